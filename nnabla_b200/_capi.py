@@ -1,4 +1,5 @@
-"""ctypes binding of libnnabla_b200.so (the C ABI declared in include/nnabla_b200.h).
+"""Bindings of libnnabla_b200.so (the C ABI declared in include/nnabla_b200.h): `native`, whose functions take torch
+tensors (csrc/native.cpp), and ctypes for the entry points that take none.
 
 There is no fallback: if the library is missing or a call fails, an exception
 is raised. Errors surface as RuntimeError carrying the library's message, the
@@ -9,6 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libnnabla_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "lib", "_native.so")
 
 c_f32p = ctypes.c_void_p
 _lib = None
@@ -34,13 +36,38 @@ def lib():
     return _lib
 
 
+class _Native:
+    """The binding module, loaded at its first use; functions become attributes as they are asked for."""
+    _module = None
+
+    def __getattr__(self, name):
+        if self._module is None:
+            lib()
+            if not os.path.exists(NATIVE_PATH):
+                raise ImportError("nnabla_b200: %s is missing. Build it with `python -m nnabla_b200.build`." % NATIVE_PATH)
+            import importlib.machinery
+            import importlib.util
+
+            import torch  # noqa: F401 - the module links against its libraries
+            loader = importlib.machinery.ExtensionFileLoader("nnabla_b200._native", NATIVE_PATH)
+            spec = importlib.util.spec_from_file_location("nnabla_b200._native", NATIVE_PATH, loader=loader)
+            module = importlib.util.module_from_spec(spec)
+            loader.exec_module(module)
+            self._module = module
+        value = getattr(self._module, name)
+        setattr(self, name, value)
+        return value
+
+
+native = _Native()
+
 _calls = 0
 _entry = {}  # entry-point name -> ctypes function with its return type set
 
 
 def calls_made():
     """Number of entry-point calls made through call() so far in this process."""
-    return _calls
+    return _calls + (native.calls() if native._module is not None else 0)
 
 
 def call(name, *args):

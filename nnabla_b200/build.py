@@ -1,5 +1,6 @@
 """Builds nnabla_b200/lib/libnnabla_b200.so from nnabla_b200/csrc/*.cu with nvcc for
-sm_100a (cross-compiles without a GPU). Usage: python -m nnabla_b200.build [--force] [-v]"""
+sm_100a (cross-compiles without a GPU), and nnabla_b200/lib/_native.so, its binding to torch
+tensors, from csrc/native.cpp. Usage: python -m nnabla_b200.build [--force] [-v]"""
 import concurrent.futures
 import os
 import shutil
@@ -12,6 +13,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(ROOT, "build", "nnabla_b200")
 LIB = os.path.join(LIBDIR, "libnnabla_b200.so")
+NATIVE = os.path.join(LIBDIR, "_native.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
@@ -65,7 +67,31 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    _build_native(force)
     return LIB
+
+
+def _build_native(force):
+    src = os.path.join(CSRC, "native.cpp")
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(ROOT, "include", "nnabla_b200.h")))
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest:
+        return
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc())))
+    include = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+               os.path.join(cuda, "include"), sysconfig.get_paths()["include"], os.path.join(ROOT, "include")]
+    libs = ["torch_python", "torch", "torch_cuda", "torch_cpu", "c10", "c10_cuda"]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-o", NATIVE, src,
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + ["-I" + d for d in include] +
+           ["-L" + os.path.join(base, "lib")] + ["-l" + n for n in libs] +
+           ["-L" + LIBDIR, "-lnnabla_b200", "-Wl,-rpath,$ORIGIN"])
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed for " + src)
 
 
 if __name__ == "__main__":

@@ -14,20 +14,12 @@ import torch
 
 from . import _capi as C
 
-
-def _check_input(x, name="x"):
-    if not isinstance(x, torch.Tensor):
-        raise TypeError("%s must be a torch.Tensor on a CUDA device" % name)
-    if not x.is_cuda:
-        raise RuntimeError("nnabla_b200 has no CPU path: %s is on %s" % (name, x.device))
-    if x.dtype != torch.float32:
-        raise TypeError("%s must be float32 (the 'float' type config), got %s" % (name, x.dtype))
-    return x if x.is_contiguous() else x.contiguous()
+L = C.native  # the entry points as functions of torch tensors
 
 
 def _output_like(x, outputs):
     if outputs is None:
-        return torch.empty_like(x)
+        return L.empty(x, x)
     y = outputs[0] if isinstance(outputs, (list, tuple)) else outputs
     _sideband.pop(id(y), None)  # about to be overwritten
     if y.shape != x.shape or y.dtype != x.dtype or y.device != x.device or not y.is_contiguous():
@@ -71,33 +63,27 @@ def fixed_point_quantize(x, sign=True, n=8, delta=2 ** -4, quantize=True, ste_fi
     """
     if not quantize:
         return x
-    x = _check_input(x)
+    x = L.f32(x)
     y = _output_like(x, outputs)
     if (codes_sideband and x.dim() == 4 and (int(x.shape[2]) * int(x.shape[3])) % 4 == 0
             and x.numel() >= SIDEBAND_MIN_VALUES
-            and int(n) - int(bool(sign)) <= 7 and int(x.shape[0]) <= 65535 and x.data_ptr() % 16 == 0
+            and int(n) - bool(sign) <= 7 and int(x.shape[0]) <= 65535 and x.data_ptr() % 16 == 0
             and y.data_ptr() % 16 == 0):
         N, Cn, inner = int(x.shape[0]), int(x.shape[1]), int(x.shape[2]) * int(x.shape[3])
-        codes = torch.empty((N, inner, codes_nhwc_slots(Cn, 1)), dtype=torch.int8, device=x.device)
-        with C.on_device(x.device):
-            C.call("nb200_fixed_point_quantize_nhwc_codes_f32", C.ptr(x), C.ptr(y), C.ptr(codes), N, Cn, inner,
-                   int(bool(sign)), int(n), C.c_float(delta), C.stream_ptr(x.device))
+        codes = L.empty_i8((N, inner, codes_nhwc_slots(Cn, 1)), x)
+        L.nb200_fixed_point_quantize_nhwc_codes_f32(x, y, codes, N, Cn, inner, bool(sign), n, delta)
         _sideband_put(y, codes, delta)
         return y
-    with C.on_device(x.device):
-        C.call("nb200_fixed_point_quantize_f32", C.ptr(x), C.ptr(y), C.size_t(x.numel()), int(bool(sign)), int(n),
-               C.c_float(delta), C.stream_ptr(x.device))
+    L.nb200_fixed_point_quantize_f32(x, y, x.numel(), bool(sign), n, delta)
     return y
 
 
 def fixed_point_quantize_with_codes(x, sign=True, n=8, delta=2 ** -4):
     """fixed_point_quantize that also returns the int8 codes k (y = k * delta)."""
-    x = _check_input(x)
-    y = torch.empty_like(x)
-    codes = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    with C.on_device(x.device):
-        C.call("nb200_fixed_point_quantize_f32_codes", C.ptr(x), C.ptr(y), C.ptr(codes), C.size_t(x.numel()),
-               int(bool(sign)), int(n), C.c_float(delta), C.stream_ptr(x.device))
+    x = L.f32(x)
+    y = L.empty(x, x)
+    codes = L.empty_i8(x, x)
+    L.nb200_fixed_point_quantize_f32_codes(x, y, codes, x.numel(), bool(sign), n, delta)
     return y, codes
 
 
@@ -108,11 +94,9 @@ def pow2_quantize(x, sign=True, with_zero=True, n=8, m=1, quantize=True, ste_fin
     """
     if not quantize:
         return x
-    x = _check_input(x)
+    x = L.f32(x)
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_pow2_quantize_f32", C.ptr(x), C.ptr(y), C.size_t(x.numel()), int(bool(sign)),
-               int(bool(with_zero)), int(n), int(m), C.stream_ptr(x.device))
+    L.nb200_pow2_quantize_f32(x, y, x.numel(), bool(sign), bool(with_zero), n, m)
     return y
 
 
@@ -126,8 +110,8 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
     """
     if not quantize:
         return x
-    x = _check_input(x)
-    qs = [_check_input(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
+    x = L.f32(x)
+    qs = [L.f32(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
                                             (ql_max, "ql_max"))]
     # Shape rules of MinMaxQuantize::setup_impl (min_max_quantize.cpp:54-83).
     if len({t.dim() for t in qs}) != 1:
@@ -141,11 +125,8 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
         if t is not orig:
             raise RuntimeError("qr_min and qr_max are updated in place and must be contiguous")
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_min_max_quantize_f32", C.ptr(x), C.i64_array(x.shape), int(x.dim()), C.ptr(qs[0]),
-               C.ptr(qs[1]), C.ptr(qs[2]), C.ptr(qs[3]), C.i64_array(qs[0].shape), C.c_float(decay),
-               int(bool(x_min_max)), int(bool(ema)), C.c_float(eps), C.ptr(y), ctypes.c_void_p(0),
-               C.stream_ptr(x.device))
+    L.nb200_min_max_quantize_f32(x, x.shape, x.dim(), qs[0], qs[1], qs[2], qs[3], qs[0].shape, decay,
+                                 bool(x_min_max), bool(ema), eps, y, None)
     return y
 
 
@@ -156,13 +137,13 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
 # ---------------------------------------------------------------------------
 
 def _grad_buffers(x, dy, dx, accum):
-    x, dy = _check_input(x), _check_input(dy, "dy")
+    x, dy = L.f32(x), L.f32(dy, "dy")
     if dy.shape != x.shape:
         raise RuntimeError("dy must have x's shape")
     if dx is None:
         if accum:
             raise RuntimeError("accum=True needs the gradient buffer dx to accumulate into")
-        dx = torch.empty_like(x)
+        dx = L.empty(x, x)
     elif dx.shape != x.shape or dx.dtype != torch.float32 or dx.device != x.device or not dx.is_contiguous():
         raise RuntimeError("dx must be a contiguous float32 tensor of x's shape and device")
     return x, dy, dx
@@ -171,20 +152,16 @@ def _grad_buffers(x, dy, dx, accum):
 def fixed_point_quantize_backward(x, dy, sign=True, n=8, delta=2 ** -4, ste_fine_grained=True, accum=False, dx=None):
     """FixedPointQuantize::backward_impl (src/nbla/function/generic/fixed_point_quantize.cpp:69-127)."""
     x, dy, dx = _grad_buffers(x, dy, dx, accum)
-    with C.on_device(x.device):
-        C.call("nb200_fixed_point_quantize_backward_f32", C.ptr(x), C.ptr(dy), C.ptr(dx), C.size_t(x.numel()),
-               int(bool(sign)), int(n), C.c_float(delta), int(bool(ste_fine_grained)), int(bool(accum)),
-               C.stream_ptr(x.device))
+    L.nb200_fixed_point_quantize_backward_f32(x, dy, dx, x.numel(), bool(sign), n, delta,
+                                              bool(ste_fine_grained), bool(accum))
     return dx
 
 
 def pow2_quantize_backward(x, dy, sign=True, with_zero=True, n=8, m=1, ste_fine_grained=True, accum=False, dx=None):
     """Pow2Quantize::backward_impl (src/nbla/function/generic/pow2_quantize.cpp:84-156)."""
     x, dy, dx = _grad_buffers(x, dy, dx, accum)
-    with C.on_device(x.device):
-        C.call("nb200_pow2_quantize_backward_f32", C.ptr(x), C.ptr(dy), C.ptr(dx), C.size_t(x.numel()),
-               int(bool(sign)), int(bool(with_zero)), int(n), int(m), int(bool(ste_fine_grained)), int(bool(accum)),
-               C.stream_ptr(x.device))
+    L.nb200_pow2_quantize_backward_f32(x, dy, dx, x.numel(), bool(sign), bool(with_zero), n, m,
+                                       bool(ste_fine_grained), bool(accum))
     return dx
 
 
@@ -197,7 +174,7 @@ def min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max=F
     left in place. Returns (dx, g_qr_min, g_qr_max); the range gradients are
     produced only when neither x_min_max nor ema is set."""
     x, dy, dx = _grad_buffers(x, dy, grads[0], accum[0])
-    qs = [_check_input(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
+    qs = [L.f32(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
                                             (ql_max, "ql_max"))]
     if len({tuple(t.shape) for t in qs}) != 1 or qs[0].dim() != x.dim():
         raise RuntimeError("All shapes among ql_min, ql_max, qr_min, and qr_max must be same.")
@@ -207,13 +184,10 @@ def min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max=F
             if acc:
                 raise RuntimeError("accum=True needs the gradient buffer to accumulate into")
             g = torch.zeros_like(qs[0])
-        gq.append(_check_input(g, "range gradient"))
-    with C.on_device(x.device):
-        C.call("nb200_min_max_quantize_backward_f32", C.ptr(x), C.i64_array(x.shape), int(x.dim()), C.ptr(qs[0]),
-               C.ptr(qs[1]), C.ptr(qs[2]), C.ptr(qs[3]), C.i64_array(qs[0].shape), C.ptr(dy), int(bool(x_min_max)),
-               int(bool(ema)), int(bool(ste_fine_grained)), C.i32_array([bool(v) for v in propagate_down]),
-               C.i32_array([bool(v) for v in accum]), C.ptr(dx), C.ptr(gq[0]), C.ptr(gq[1]),
-               C.stream_ptr(x.device))
+        gq.append(L.f32(g, "range gradient"))
+    L.nb200_min_max_quantize_backward_f32(x, x.shape, x.dim(), qs[0], qs[1], qs[2], qs[3], qs[0].shape, dy,
+                                          bool(x_min_max), bool(ema), bool(ste_fine_grained),
+                                          [bool(v) for v in propagate_down], [bool(v) for v in accum], dx, gq[0], gq[1])
     return dx, gq[0], gq[1]
 
 
@@ -232,6 +206,9 @@ def check_device_status(device=None):
 
 def _affine_dims(x, w, base_axis, bias):
     """Shape rules of Affine::setup_impl (src/nbla/function/generic/affine.cpp:29-78)."""
+    xs, ws = x.shape, w.shape
+    if base_axis == 1 and len(xs) == 2 == len(ws) and xs[1] == ws[0] and (bias is None or bias.shape == ws[1:]):
+        return xs[0], ws[0], ws[1], (xs[0], ws[1])
     if w.dim() < 2:
         raise RuntimeError("Weights(inputs[1]) must be matrix or tensor.")
     if base_axis < 0:
@@ -256,7 +233,7 @@ def _affine_dims(x, w, base_axis, bias):
 
 
 def _same_shape(a, b, what):
-    if a.dim() != b.dim() or tuple(a.shape) != tuple(b.shape):
+    if a.shape != b.shape:
         raise RuntimeError("Binary and float weights must have same size. (%s)" % what)
 
 
@@ -268,18 +245,15 @@ def binary_weight_affine(x, weight, binary_weight, alpha, bias=None, base_axis=1
     writes `binary_weight` = sign(weight) and `alpha` = mean |weight| per output,
     returns x . binary_weight * alpha + bias.
     """
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    binary_weight, alpha = _check_input(binary_weight, "binary_weight"), _check_input(alpha, "alpha")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    binary_weight, alpha = L.f32(binary_weight, "binary_weight"), L.f32(alpha, "alpha")
+    bias = L.f32(bias, "bias") if bias is not None else None
     rows, w_row, w_col, out_shape = _affine_dims(x, weight, base_axis, bias)
     _same_shape(weight, binary_weight, "float vs binary")
     if alpha.numel() != w_col:
         raise RuntimeError("Size of alpha must be equal to output size.")
-    y = torch.empty(out_shape, dtype=torch.float32, device=x.device) if outputs is None else outputs[0]
-    with C.on_device(x.device):
-        C.call("nb200_binary_weight_affine_f32", C.ptr(x), C.ptr(weight), C.ptr(binary_weight), C.ptr(alpha),
-               C.ptr(bias), C.ptr(y), ctypes.c_int64(rows), ctypes.c_int64(w_row), ctypes.c_int64(w_col),
-               C.c_float(quantize_zero_to), C.stream_ptr(x.device))
+    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    L.nb200_binary_weight_affine_f32(x, weight, binary_weight, alpha, bias, y, rows, w_row, w_col, quantize_zero_to)
     return y
 
 
@@ -289,16 +263,13 @@ def binary_connect_affine(x, weight, binary_weight, bias=None, base_axis=1, quan
 
     Forward of BinaryConnectAffine (src/nbla/function/generic/binary_connect_affine.cpp:59-71).
     """
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    binary_weight = _check_input(binary_weight, "binary_weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    binary_weight = L.f32(binary_weight, "binary_weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     rows, w_row, w_col, out_shape = _affine_dims(x, weight, base_axis, bias)
     _same_shape(weight, binary_weight, "float vs binary")
-    y = torch.empty(out_shape, dtype=torch.float32, device=x.device) if outputs is None else outputs[0]
-    with C.on_device(x.device):
-        C.call("nb200_binary_connect_affine_f32", C.ptr(x), C.ptr(weight), C.ptr(binary_weight), C.ptr(bias),
-               C.ptr(y), ctypes.c_int64(rows), ctypes.c_int64(w_row), ctypes.c_int64(w_col),
-               C.c_float(quantize_zero_to), C.stream_ptr(x.device))
+    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    L.nb200_binary_connect_affine_f32(x, weight, binary_weight, bias, y, rows, w_row, w_col, quantize_zero_to)
     return y
 
 
@@ -309,19 +280,15 @@ def affine(x, weight, bias=None, base_axis=1, n_outputs=-1, outputs=None, fixed_
     fixed_point_quantize with n <= 8 and those step sizes; the product then
     runs on the int8 tensor-core path. Otherwise the fp32-accurate split path.
     """
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     rows, w_row, w_col, out_shape = _affine_dims(x, weight, base_axis, bias)
-    y = torch.empty(out_shape, dtype=torch.float32, device=x.device) if outputs is None else outputs[0]
-    with C.on_device(x.device):
-        if fixed_point is not None:
-            dx, dw = fixed_point
-            C.call("nb200_affine_fxp8_f32", C.ptr(x), C.ptr(weight), C.c_float(dx), C.c_float(dw), C.ptr(bias),
-                   C.ptr(y), ctypes.c_int64(rows), ctypes.c_int64(w_row), ctypes.c_int64(w_col),
-                   C.stream_ptr(x.device))
-        else:
-            C.call("nb200_affine_f32", C.ptr(x), C.ptr(weight), C.ptr(bias), C.ptr(y), ctypes.c_int64(rows),
-                   ctypes.c_int64(w_row), ctypes.c_int64(w_col), C.stream_ptr(x.device))
+    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    if fixed_point is not None:
+        dx, dw = fixed_point
+        L.nb200_affine_fxp8_f32(x, weight, dx, dw, bias, y, rows, w_row, w_col)
+    else:
+        L.nb200_affine_f32(x, weight, bias, y, rows, w_row, w_col)
     return y
 
 
@@ -332,18 +299,15 @@ def affine_from_codes(x_codes, w_codes, delta_x, delta_w, bias=None):
     K2, N = w_codes.shape
     if K != K2:
         raise RuntimeError("Size of input data(inputs[0]) and weights(inputs[1]) mismatch.")
-    y = torch.empty((rows, N), dtype=torch.float32, device=x_codes.device)
-    with C.on_device(x_codes.device):
-        C.call("nb200_affine_codes_i8_f32", C.ptr(x_codes), C.ptr(w_codes), C.c_float(delta_x), C.c_float(delta_w),
-               C.ptr(bias), C.ptr(y), ctypes.c_int64(rows), ctypes.c_int64(K), ctypes.c_int64(N),
-               C.stream_ptr(x_codes.device))
+    y = L.empty((rows, N), x_codes)
+    L.nb200_affine_codes_i8_f32(x_codes, w_codes, delta_x, delta_w, bias, y, rows, K, N)
     return y
 
 
 def _affine_backward(entry, x, w, alpha, dy, base_axis, propagate_down, accum, grads):
     """Shared driver of the affine backward entry points. Returns (dx, dw, db);
     an entry whose propagate_down flag is false is returned as passed in."""
-    x, w, dy = _check_input(x), _check_input(w, "weight"), _check_input(dy, "dy")
+    x, w, dy = L.f32(x), L.f32(w, "weight"), L.f32(dy, "dy")
     rows, w_row, w_col, out_shape = _affine_dims(x, w, base_axis, None)
     if tuple(dy.shape) != tuple(out_shape):
         raise RuntimeError("dy must have the output's shape")
@@ -356,16 +320,13 @@ def _affine_backward(entry, x, w, alpha, dy, base_axis, propagate_down, accum, g
         if g is None:
             if ac:
                 raise RuntimeError("accum=True needs the gradient buffer to accumulate into")
-            g = torch.empty(tuple(shape), dtype=torch.float32, device=x.device)
+            g = L.empty(shape, x)
         elif tuple(g.shape) != tuple(shape) or g.dtype != torch.float32 or not g.is_cuda or not g.is_contiguous():
             raise RuntimeError("gradient buffers must be contiguous float32 CUDA tensors of their input's shape")
         out.append(g)
-    p = [C.ptr(g) if pd else ctypes.c_void_p(0) for g, pd in zip(out, propagate_down)]
-    args = [C.ptr(x), C.ptr(w)] + ([C.ptr(alpha)] if alpha is not None else []) + [C.ptr(dy)] + p + [
-        ctypes.c_int64(rows), ctypes.c_int64(w_row), ctypes.c_int64(w_col), int(bool(accum[0])), int(bool(accum[1])),
-        int(bool(accum[2])), C.stream_ptr(x.device)]
-    with C.on_device(x.device):
-        C.call(entry, *args)
+    p = [g if pd else None for g, pd in zip(out, propagate_down)]
+    scaled = (alpha,) if alpha is not None else ()
+    getattr(L, entry)(x, w, *scaled, dy, *p, rows, w_row, w_col, bool(accum[0]), bool(accum[1]), bool(accum[2]))
     return tuple(out)
 
 
@@ -382,7 +343,7 @@ def binary_weight_affine_backward(x, binary_weight, alpha, dy, base_axis=1, prop
     binary_weight / alpha are what the forward wrote; dw is the gradient of the
     FLOAT weights (the gradient of the scaled binary weights passes straight
     through Sign). Returns (dx, dw, db)."""
-    alpha = _check_input(alpha, "alpha")
+    alpha = L.f32(alpha, "alpha")
     return _affine_backward("nb200_binary_weight_affine_backward_f32", x, binary_weight, alpha, dy, base_axis,
                             propagate_down, accum, grads)
 
@@ -400,10 +361,8 @@ def transpose_codes(w_codes):
     a re-layout pass. Done once per weight update."""
     K, N = w_codes.shape
     Kp = (K + 15) // 16 * 16
-    out = torch.empty((N, Kp), dtype=torch.int8, device=w_codes.device)
-    with C.on_device(w_codes.device):
-        C.call("nb200_transpose_codes_i8", C.ptr(w_codes.contiguous()), C.ptr(out), ctypes.c_int64(K),
-               ctypes.c_int64(N), ctypes.c_int64(Kp), C.stream_ptr(w_codes.device))
+    out = L.empty_i8((N, Kp), w_codes)
+    L.nb200_transpose_codes_i8(w_codes.contiguous(), out, K, N, Kp)
     return out
 
 
@@ -413,11 +372,8 @@ def affine_from_kmajor_codes(x_codes, w_codes_kmajor, w_row, delta_x, delta_w, b
     N, Kp = w_codes_kmajor.shape
     if K != w_row or Kp < K:
         raise RuntimeError("Size of input data(inputs[0]) and weights(inputs[1]) mismatch.")
-    y = torch.empty((rows, N), dtype=torch.float32, device=x_codes.device)
-    with C.on_device(x_codes.device):
-        C.call("nb200_affine_codes_i8_kmajor_f32", C.ptr(x_codes), C.ptr(w_codes_kmajor), ctypes.c_int64(Kp),
-               C.c_float(delta_x), C.c_float(delta_w), C.ptr(bias), C.ptr(y), ctypes.c_int64(rows), ctypes.c_int64(K),
-               ctypes.c_int64(N), C.stream_ptr(x_codes.device))
+    y = L.empty((rows, N), x_codes)
+    L.nb200_affine_codes_i8_kmajor_f32(x_codes, w_codes_kmajor, Kp, delta_x, delta_w, bias, y, rows, K, N)
     return y
 
 
@@ -450,7 +406,7 @@ def affine_from_codes_gather(x_codes, w_codes, delta_x, delta_w, bias, y_ranks, 
 def affine_fixed_point_gather(xq, wq, delta_x, delta_w, bias, y_ranks, rank, n_total, col_begin):
     """As affine_from_codes_gather, from the fp32 outputs of fixed_point_quantize
     (xq [rows, K] multiples of delta_x, wq [K, n] multiples of delta_w)."""
-    xq, wq = _check_input(xq, "xq"), _check_input(wq, "wq")
+    xq, wq = L.f32(xq, "xq"), L.f32(wq, "wq")
     rows, K = xq.shape
     K2, n = wq.shape
     if K != K2:
@@ -467,14 +423,19 @@ def affine_fixed_point_gather(xq, wq, delta_x, delta_w, bias, y_ranks, rank, n_t
 # ---------------------------------------------------------------------------
 
 def _conv_geometry(x, w, bias, base_axis, pad, stride, dilation, group):
-    """Shape rules of Convolution::setup_impl (src/nbla/function/generic/convolution.cpp:40-158)."""
+    """Shape rules of Convolution::setup_impl (src/nbla/function/generic/convolution.cpp:40-158); x and w are
+    tensors or shapes."""
+    plain = L.conv2d(x, w, bias, base_axis, pad, stride, dilation, group)
+    if plain is not None:
+        return plain
+    xs, ws = (tuple(getattr(t, "shape", t)) for t in (x, w))
     if base_axis < 0:
-        base_axis += x.dim()
-    if not 0 <= base_axis < x.dim() - 1:
+        base_axis += len(xs)
+    if not 0 <= base_axis < len(xs) - 1:
         raise RuntimeError("base_axis must be less than ndim - 1 of inputs[0]. base_axis: %d >= ndim of inputs[0] "
-                           "- 1: %d." % (base_axis, x.dim() - 1))
-    spatial = x.dim() - base_axis - 1
-    if w.dim() != 2 + spatial:
+                           "- 1: %d." % (base_axis, len(xs) - 1))
+    spatial = len(xs) - base_axis - 1
+    if len(ws) != 2 + spatial:
         raise RuntimeError("Weights must be a tensor more than 3D.")
     if spatial != 2:
         raise C.NB200Error(4, "only 2-D convolution is implemented (got %d spatial dims)" % spatial)
@@ -485,10 +446,10 @@ def _conv_geometry(x, w, bias, base_axis, pad, stride, dilation, group):
         if len(v) != spatial:
             raise RuntimeError("%s size mismatch. %s size: %d != spatial dims: %d." % (name, name, len(v), spatial))
     batch = 1
-    for s in x.shape[:base_axis]:
+    for s in xs[:base_axis]:
         batch *= int(s)
-    Cin, H, W = (int(s) for s in x.shape[base_axis:])
-    Ko, Cg, kh, kw = (int(s) for s in w.shape)
+    Cin, H, W = (int(s) for s in xs[base_axis:])
+    Ko, Cg, kh, kw = (int(s) for s in ws)
     if Cin % group != 0:
         raise RuntimeError("Number of input channel needs to be divisible by group. Input channel: %d, group: %d."
                            % (Cin, group))
@@ -508,7 +469,7 @@ def _conv_geometry(x, w, bias, base_axis, pad, stride, dilation, group):
                                "kernel:%d, pad:%d, stride:%d, dilation:%d}." % (i, inp, k, pad[i], stride[i],
                                                                               dilation[i]))
         outs.append(o)
-    out_shape = tuple(x.shape[:base_axis]) + (Ko, outs[0], outs[1])
+    out_shape = xs[:base_axis] + (Ko, outs[0], outs[1])
     return batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape
 
 
@@ -520,21 +481,16 @@ def _binary_convolution(entry, x, weight, binary_weight, alpha, bias, base_axis,
             return binary_weight_convolution_from_codes(codes, tuple(x.shape), weight, binary_weight, alpha, bias, pad,
                                                         stride, dilation, group, quantize_zero_to, fixed_point_delta,
                                                         outputs)
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    binary_weight = _check_input(binary_weight, "binary_weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    binary_weight = L.f32(binary_weight, "binary_weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, weight, bias, base_axis, pad, stride, dilation, group)
     _same_shape(weight, binary_weight, "float vs binary")
-    y = torch.empty(out_shape, dtype=torch.float32, device=x.device) if outputs is None else outputs[0]
-    args = [C.ptr(x), C.ptr(weight), C.ptr(binary_weight)]
-    if alpha is not None:
-        args.append(C.ptr(alpha))
-    args += [C.ptr(bias), C.ptr(y), batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0], stride[1], dilation[0],
-             dilation[1], int(group), C.c_float(quantize_zero_to), C.c_float(fixed_point_delta or 0.0),
-             C.stream_ptr(x.device)]
-    with C.on_device(x.device):
-        C.call(entry, *args)
+    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    scaled = (alpha,) if alpha is not None else ()
+    getattr(L, entry)(x, weight, binary_weight, *scaled, bias, y, batch, Cin, H, W, Ko, kh, kw, *pad, *stride, *dilation,
+                      group, quantize_zero_to, fixed_point_delta or 0.0)
     return y
 
 
@@ -549,7 +505,7 @@ def binary_weight_convolution(x, weight, binary_weight, alpha, bias=None, base_a
     output of fixed_point_quantize with step d and n <= 8, which selects the
     exact int8 contraction.
     """
-    alpha = _check_input(alpha, "alpha")
+    alpha = L.f32(alpha, "alpha")
     if alpha.numel() != int(weight.shape[0]):
         raise RuntimeError("Size of alpha must be equal to the number of output maps.")
     return _binary_convolution("nb200_binary_weight_convolution_f32", x, weight, binary_weight, alpha, bias,
@@ -570,7 +526,7 @@ def binary_connect_convolution(x, weight, binary_weight, bias=None, base_axis=1,
 
 def _binary_convolution_backward(entry, x, binary_weight, alpha, dy, base_axis, pad, stride, dilation, group,
                                  propagate_down, accum, grads, fixed_point_delta):
-    x, w, dy = _check_input(x), _check_input(binary_weight, "binary_weight"), _check_input(dy, "dy")
+    x, w, dy = L.f32(x), L.f32(binary_weight, "binary_weight"), L.f32(dy, "dy")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, w, None, base_axis, pad, stride, dilation, group)
     if tuple(dy.shape) != tuple(out_shape):
@@ -584,17 +540,14 @@ def _binary_convolution_backward(entry, x, binary_weight, alpha, dy, base_axis, 
         if g is None:
             if ac:
                 raise RuntimeError("accum=True needs the gradient buffer to accumulate into")
-            g = torch.empty(tuple(shape), dtype=torch.float32, device=x.device)
+            g = L.empty(shape, x)
         elif tuple(g.shape) != tuple(shape) or g.dtype != torch.float32 or not g.is_cuda or not g.is_contiguous():
             raise RuntimeError("gradient buffers must be contiguous float32 CUDA tensors of their input's shape")
         out.append(g)
-    p = [C.ptr(g) if pd else ctypes.c_void_p(0) for g, pd in zip(out, propagate_down)]
-    args = [C.ptr(x), C.ptr(w)] + ([C.ptr(alpha)] if alpha is not None else []) + [C.ptr(dy)] + p + [
-        batch, Cin, H, W, Ko, kh, kw, int(pad[0]), int(pad[1]), int(stride[0]), int(stride[1]), int(dilation[0]),
-        int(dilation[1]), int(group), int(bool(accum[0])), int(bool(accum[1])), int(bool(accum[2])),
-        C.c_float(fixed_point_delta or 0.0), C.stream_ptr(x.device)]
-    with C.on_device(x.device):
-        C.call(entry, *args)
+    p = [g if pd else None for g, pd in zip(out, propagate_down)]
+    scaled = (alpha,) if alpha is not None else ()
+    getattr(L, entry)(x, w, *scaled, dy, *p, batch, Cin, H, W, Ko, kh, kw, *pad, *stride, *dilation, group,
+                      bool(accum[0]), bool(accum[1]), bool(accum[2]), fixed_point_delta or 0.0)
     return tuple(out)
 
 
@@ -605,7 +558,7 @@ def binary_weight_convolution_backward(x, binary_weight, alpha, dy, base_axis=1,
     (src/nbla/function/generic/binary_weight_convolution.cpp:119-146): returns
     (dx, dw, db); binary_weight / alpha are what the forward wrote, dw is the
     gradient of the float weights. fixed_point_delta as in the forward."""
-    alpha = _check_input(alpha, "alpha")
+    alpha = L.f32(alpha, "alpha")
     return _binary_convolution_backward("nb200_binary_weight_convolution_backward_f32", x, binary_weight, alpha, dy,
                                         base_axis, pad, stride, dilation, group, propagate_down, accum, grads,
                                         fixed_point_delta)
@@ -627,14 +580,13 @@ def convolution_backward(x, weight_shape, dy, base_axis=1, pad=None, stride=None
     """Gradients of the full-precision convolution
     (Convolution::backward_impl, src/nbla/function/generic/convolution.cpp:199-300).
     Returns (dx, dw, db), None where propagate_down is False; dx needs `weight`."""
-    x, dy = _check_input(x), _check_input(dy, "dy")
+    x, dy = L.f32(x), L.f32(dy, "dy")
     if weight is not None:
-        weight_shape = tuple(_check_input(weight, "weight").shape)
+        weight_shape = tuple(L.f32(weight, "weight").shape)
     elif propagate_down[0]:
         raise RuntimeError("the gradient w.r.t. x needs the weights (weight=)")
-    w_like = torch.empty(tuple(weight_shape), device="meta")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
-        x, w_like, None, base_axis, pad, stride, dilation, group)
+        x, tuple(weight_shape), None, base_axis, pad, stride, dilation, group)
     if tuple(dy.shape) != tuple(out_shape):
         raise RuntimeError("dy must have the output's shape")
     out = []
@@ -642,18 +594,17 @@ def convolution_backward(x, weight_shape, dy, base_axis=1, pad=None, stride=None
         if pd and g is None:
             if ac:
                 raise RuntimeError("accum=True needs the gradient buffer to accumulate into")
-            g = torch.empty(shape, dtype=torch.float32, device=x.device)
+            g = L.empty(shape, x)
         out.append(g if pd else None)
-    with C.on_device(x.device):
-        if propagate_down[0]:
-            C.call("nb200_convolution_input_backward_f32", C.ptr(weight), C.ptr(dy), C.ptr(out[0]), batch, Cin, H, W, Ko,
-                   kh, kw, int(pad[0]), int(pad[1]), int(stride[0]), int(stride[1]), int(dilation[0]),
-                   int(dilation[1]), int(group), int(bool(accum[0])), C.stream_ptr(x.device))
-        if propagate_down[1] or propagate_down[2]:
-            C.call("nb200_convolution_backward_f32", C.ptr(x), C.ptr(dy), C.ptr(out[1]) if propagate_down[1] else
-                   ctypes.c_void_p(0), C.ptr(out[2]) if propagate_down[2] else ctypes.c_void_p(0), batch, Cin, H, W, Ko,
-                   kh, kw, int(pad[0]), int(pad[1]), int(stride[0]), int(stride[1]), int(dilation[0]),
-                   int(dilation[1]), int(group), int(bool(accum[1])), int(bool(accum[2])), C.stream_ptr(x.device))
+    if propagate_down[0]:
+        L.nb200_convolution_input_backward_f32(weight, dy, out[0], batch, Cin, H, W, Ko, kh, kw, pad[0],
+                                               pad[1], stride[0], stride[1], dilation[0],
+                                               dilation[1], group, bool(accum[0]))
+    if propagate_down[1] or propagate_down[2]:
+        L.nb200_convolution_backward_f32(x, dy, out[1] if propagate_down[1] else None, out[2] if propagate_down[2] else
+                                         None, batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0],
+                                         stride[1], dilation[0], dilation[1], group,
+                                         bool(accum[1]), bool(accum[2]))
     return tuple(out)
 
 
@@ -671,20 +622,17 @@ def convolution(x, weight, bias=None, base_axis=1, pad=None, stride=None, dilati
     layers with few input channels (the network stem)."""
     if channel_last:
         raise C.NB200Error(4, "channel_last=True is not supported (nor by the reference's CPU Convolution)")
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, weight, bias, base_axis, pad, stride, dilation, group)
-    y = torch.empty(out_shape, dtype=torch.float32, device=x.device) if outputs is None else outputs[0]
+    y = L.empty(out_shape, x) if outputs is None else outputs[0]
     if fixed_point is not None:
-        with C.on_device(x.device):
-            C.call("nb200_convolution_fxp8_f32", C.ptr(x), C.ptr(weight), C.c_float(fixed_point[0]),
-                   C.c_float(fixed_point[1]), C.ptr(bias), C.ptr(y), batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1],
-                   stride[0], stride[1], dilation[0], dilation[1], int(group), C.stream_ptr(x.device))
+        L.nb200_convolution_fxp8_f32(x, weight, fixed_point[0], fixed_point[1], bias, y, batch, Cin, H, W, Ko, kh, kw,
+                                     pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1], group)
         return y
-    with C.on_device(x.device):
-        C.call("nb200_convolution_f32", C.ptr(x), C.ptr(weight), C.ptr(bias), C.ptr(y), batch, Cin, H, W, Ko, kh, kw,
-               pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1], int(group), C.stream_ptr(x.device))
+    L.nb200_convolution_f32(x, weight, bias, y, batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0], stride[1],
+                            dilation[0], dilation[1], group)
     return y
 
 
@@ -695,7 +643,7 @@ def batch_normalization(x, beta, gamma, mean, variance, axes=[1], decay_rate=0.9
     (src/nbla/function/generic/batch_normalization.cpp:228-260). batch_stat=True: forward_impl_batch
     (:157-226): normalises with the statistics of x and updates `mean` / `variance` (the running
     statistics) in place; output_stat=True also returns the batch mean and variance."""
-    x = _check_input(x)
+    x = L.f32(x)
     axes = list(axes)
     if len(axes) != 1:
         raise C.NB200Error(4, "one normalised axis is supported (got axes=%s)" % (axes,))
@@ -710,49 +658,41 @@ def batch_normalization(x, beta, gamma, mean, variance, axes=[1], decay_rate=0.9
         if t is None:
             params.append(None)
             continue
-        t = _check_input(t, nm)
+        t = L.f32(t, nm)
         if t.numel() != Cn:
             raise RuntimeError("%s must have %d elements (shape of the normalised axis)" % (nm, Cn))
         params.append(t)
     if params[2] is None or params[3] is None:
         raise RuntimeError("mean and variance are required")
-    y = torch.empty_like(x)
+    y = L.empty(x, x)
     if batch_stat:
-        bm = torch.empty(Cn, dtype=torch.float32, device=x.device)
-        bv = torch.empty(Cn, dtype=torch.float32, device=x.device)
-        with C.on_device(x.device):
-            C.call("nb200_batch_normalization_batch_f32", C.ptr(x), C.ptr(params[0]), C.ptr(params[1]),
-                   C.ptr(params[2]), C.ptr(params[3]), C.ptr(y), C.ptr(bm), C.ptr(bv), ctypes.c_int64(outer),
-                   ctypes.c_int64(Cn), ctypes.c_int64(inner), C.c_float(eps), C.c_float(decay_rate), 1,
-                   C.stream_ptr(x.device))
+        bm = L.empty((Cn,), x)
+        bv = L.empty((Cn,), x)
+        L.nb200_batch_normalization_batch_f32(x, params[0], params[1], params[2], params[3], y, bm, bv, outer, Cn,
+                                              inner, eps, decay_rate, 1)
         if output_stat:
             return y, bm.reshape(params[2].shape), bv.reshape(params[3].shape)
         return y
-    with C.on_device(x.device):
-        C.call("nb200_batch_normalization_inference_f32", C.ptr(x), C.ptr(params[0]), C.ptr(params[1]),
-               C.ptr(params[2]), C.ptr(params[3]), C.ptr(y), ctypes.c_int64(outer), ctypes.c_int64(Cn),
-               ctypes.c_int64(inner), C.c_float(eps), C.stream_ptr(x.device))
+    L.nb200_batch_normalization_inference_f32(x, params[0], params[1], params[2], params[3], y, outer, Cn, inner, eps)
     return y
 
 
 def relu(x, inplace=False, n_outputs=-1, outputs=None):
     """ReLU (function_bases.relu; src/nbla/function/generic/relu.cpp)."""
-    x = _check_input(x)
+    x = L.f32(x)
     y = x if inplace else _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_relu_f32", C.ptr(x), C.ptr(y), C.size_t(x.numel()), C.stream_ptr(x.device))
+    L.nb200_relu_f32(x, y, x.numel())
     return y
 
 
 def add2(x0, x1, inplace=False, n_outputs=-1, outputs=None):
     """Add2 (function_bases.add2; src/nbla/function/generic/add2.cpp), equal shapes."""
-    x0, x1 = _check_input(x0, "x0"), _check_input(x1, "x1")
+    x0, x1 = L.f32(x0, "x0"), L.f32(x1, "x1")
     if tuple(x0.shape) != tuple(x1.shape):
         raise C.NB200Error(4, "broadcasting add2 is not implemented: shapes %s and %s" % (tuple(x0.shape),
                                                                                          tuple(x1.shape)))
     y = x0 if inplace else _output_like(x0, outputs)
-    with C.on_device(x0.device):
-        C.call("nb200_add2_f32", C.ptr(x0), C.ptr(x1), C.ptr(y), C.size_t(x0.numel()), C.stream_ptr(x0.device))
+    L.nb200_add2_f32(x0, x1, y, x0.numel())
     return y
 
 
@@ -761,7 +701,7 @@ def max_pooling(x, kernel, stride=None, ignore_border=True, pad=None, channel_la
     """Max pooling (function_bases.max_pooling; src/nbla/function/generic/max_pooling.cpp:140-191), 2-D."""
     if channel_last:
         raise C.NB200Error(4, "channel_last=True is not supported (nor by the reference's CPU pooling)")
-    x = _check_input(x)
+    x = L.f32(x)
     kernel = tuple(kernel)
     if len(kernel) != 2:
         raise C.NB200Error(4, "2D Pooling only")
@@ -773,26 +713,23 @@ def max_pooling(x, kernel, stride=None, ignore_border=True, pad=None, channel_la
     maps = x.numel() // max(H * W, 1)
     Ho = (H + pad[0] - (kernel[0] - pad[0] if ignore_border else 1)) // stride[0] + 1
     Wo = (W + pad[1] - (kernel[1] - pad[1] if ignore_border else 1)) // stride[1] + 1
-    y = torch.empty(tuple(x.shape[:-2]) + (Ho, Wo), dtype=torch.float32, device=x.device)
-    with C.on_device(x.device):
-        C.call("nb200_max_pooling_f32", C.ptr(x), C.ptr(y), ctypes.c_int64(maps), H, W, kernel[0], kernel[1],
-               stride[0], stride[1], pad[0], pad[1], int(bool(ignore_border)), C.stream_ptr(x.device))
+    y = L.empty(tuple(x.shape[:-2]) + (Ho, Wo), x)
+    L.nb200_max_pooling_f32(x, y, maps, H, W, kernel[0], kernel[1], stride[0], stride[1], pad[0], pad[1],
+                            bool(ignore_border))
     return y
 
 
 def global_average_pooling(x, n_outputs=-1, outputs=None):
     """Global average pooling (function_bases.global_average_pooling;
     src/nbla/function/generic/global_average_pooling.cpp): [N, C, ...] -> [N, C, 1, 1]."""
-    x = _check_input(x)
+    x = L.f32(x)
     if x.dim() < 2:
         raise RuntimeError("GlobalAveragePooling averages across the channel, so the input's shape must have a "
                            "dimension equal to or larger than 2. actual: %d" % x.dim())
     N, Cn = int(x.shape[0]), int(x.shape[1])
     S = x.numel() // max(N * Cn, 1)
-    y = torch.empty((N, Cn, 1, 1), dtype=torch.float32, device=x.device)
-    with C.on_device(x.device):
-        C.call("nb200_global_average_pooling_f32", C.ptr(x), C.ptr(y), ctypes.c_int64(N * Cn), ctypes.c_int64(S),
-               C.stream_ptr(x.device))
+    y = L.empty((N, Cn, 1, 1), x)
+    L.nb200_global_average_pooling_f32(x, y, N * Cn, S)
     return y
 
 
@@ -817,14 +754,12 @@ def inq_update_weights(weight, indicators, state, num_bits=4, inq_iterations=(),
     if selection_algorithm not in ("largest_abs", "random"):
         raise ValueError('Provided value for selection algorithm not valid: %s. Valid values are "largest_abs" '
                          'and "random".' % selection_algorithm)
-    weight = _check_input(weight, "weight")
+    weight = L.f32(weight, "weight")
     if indicators.dtype != torch.int32 or indicators.shape != weight.shape or not indicators.is_contiguous():
         raise RuntimeError("Indicators and weights must have same size (indicators as contiguous int32).")
     n = weight.numel()
     its = [int(v) for v in inq_iterations]
-    with C.on_device(weight.device):
-        C.call("nb200_inq_restore_f32", C.ptr(weight), C.ptr(state.old_weights), C.ptr(state.old_indicators),
-               C.size_t(n), C.stream_ptr(weight.device))
+    L.nb200_inq_restore_f32(weight, state.old_weights, state.old_indicators, n)
     fix_all = 0
     if state.counter in its:
         if its[-1] == state.counter:
@@ -843,9 +778,7 @@ def inq_update_weights(weight, indicators, state, num_bits=4, inq_iterations=(),
             flat = indicators.view(-1)
             draws = torch.bernoulli(torch.full((n,), 0.5, device=weight.device), generator=state.generator).to(torch.int32)
             flat.copy_(torch.where(flat == 0, draws, flat))
-    with C.on_device(weight.device):
-        C.call("nb200_inq_quantize_f32", C.ptr(weight), C.ptr(indicators), C.ptr(state.old_weights),
-               C.ptr(state.old_indicators), C.size_t(n), int(num_bits), fix_all, C.stream_ptr(weight.device))
+    L.nb200_inq_quantize_f32(weight, indicators, state.old_weights, state.old_indicators, n, num_bits, fix_all)
     state.counter += 1
 
 
@@ -874,8 +807,8 @@ def _grad_out(like, accum, dx):
     if dx is None:
         if accum:
             raise RuntimeError("accum needs the gradient buffer to add to")
-        return torch.empty_like(like)
-    return _check_input(dx, "dx")
+        return L.empty(like, like)
+    return L.f32(dx, "dx")
 
 
 def batch_normalization_backward(x, dy, gamma, mean, variance, axes=[1], eps=1e-05, batch_stat=True, dmean=None,
@@ -884,7 +817,7 @@ def batch_normalization_backward(x, dy, gamma, mean, variance, axes=[1], eps=1e-
     """BatchNormalization::backward_impl (batch_normalization.cpp:262-486). mean / variance: the batch
     statistics the forward pass returned (batch_stat) or the running ones. Returns (dx, dbeta, dgamma),
     None where propagate_down is False."""
-    x, dy = _check_input(x), _check_input(dy, "dy")
+    x, dy = L.f32(x), L.f32(dy, "dy")
     axes = list(axes)
     if len(axes) != 1:
         raise C.NB200Error(4, "one normalised axis is supported (got axes=%s)" % (axes,))
@@ -895,63 +828,54 @@ def batch_normalization_backward(x, dy, gamma, mean, variance, axes=[1], eps=1e-
         outer *= int(s_)
     inner = x.numel() // max(outer * Cn, 1)
     dx = _grad_out(x, accum[0], grads[0]) if propagate_down[0] else None
-    like = torch.empty(Cn, dtype=torch.float32, device=x.device)
+    like = L.empty((Cn,), x)
     db = _grad_out(like, accum[1], grads[1]) if propagate_down[1] else None
     dg = _grad_out(like, accum[2], grads[2]) if propagate_down[2] else None
-    with C.on_device(x.device):
-        C.call("nb200_batch_normalization_backward_f32", C.ptr(x), C.ptr(dy), C.ptr(gamma), C.ptr(mean),
-               C.ptr(variance), C.ptr(dmean), C.ptr(dvar), C.ptr(dx), C.ptr(db), C.ptr(dg), ctypes.c_int64(outer),
-               ctypes.c_int64(Cn), ctypes.c_int64(inner), C.c_float(eps), int(bool(batch_stat)), int(bool(accum[0])),
-               int(bool(accum[1])), int(bool(accum[2])), C.stream_ptr(x.device))
+    L.nb200_batch_normalization_backward_f32(x, dy, gamma, mean, variance, dmean, dvar, dx, db, dg, outer, Cn, inner,
+                                             eps, bool(batch_stat), bool(accum[0]), bool(accum[1]),
+                                             bool(accum[2]))
     return dx, db, dg
 
 
 def relu_backward(y, dy, accum=False, dx=None):
     """ReLU::backward_impl (relu.cpp:41-66); y is the forward output."""
-    y, dy = _check_input(y), _check_input(dy, "dy")
+    y, dy = L.f32(y), L.f32(dy, "dy")
     dx = _grad_out(y, accum, dx)
-    with C.on_device(y.device):
-        C.call("nb200_relu_backward_f32", C.ptr(y), C.ptr(dy), C.ptr(dx), C.size_t(y.numel()), int(bool(accum)),
-               C.stream_ptr(y.device))
+    L.nb200_relu_backward_f32(y, dy, dx, y.numel(), bool(accum))
     return dx
 
 
 def add2_backward(dy, accum=False, dx=None):
     """Add2::backward_impl for one input of equal shape: dx (+)= dy."""
-    dy = _check_input(dy, "dy")
+    dy = L.f32(dy, "dy")
     dx = _grad_out(dy, accum, dx)
-    with C.on_device(dy.device):
-        C.call("nb200_add2_backward_f32", C.ptr(dy), C.ptr(dx), C.size_t(dy.numel()), int(bool(accum)),
-               C.stream_ptr(dy.device))
+    L.nb200_add2_backward_f32(dy, dx, dy.numel(), bool(accum))
     return dx
 
 
 def global_average_pooling_backward(x_shape, dy, accum=False, dx=None):
     """GlobalAveragePooling::backward_impl (global_average_pooling.cpp:75-117)."""
-    dy = _check_input(dy, "dy")
+    dy = L.f32(dy, "dy")
     N, Cn = int(x_shape[0]), int(x_shape[1])
     S = 1
     for s_ in x_shape[2:]:
         S *= int(s_)
-    dx = _grad_out(torch.empty(tuple(x_shape), dtype=torch.float32, device=dy.device), accum, dx)
-    with C.on_device(dy.device):
-        C.call("nb200_global_average_pooling_backward_f32", C.ptr(dy), C.ptr(dx), ctypes.c_int64(N * Cn),
-               ctypes.c_int64(S), int(bool(accum)), C.stream_ptr(dy.device))
+    dx = _grad_out(L.empty(tuple(x_shape), dy), accum, dx)
+    L.nb200_global_average_pooling_backward_f32(dy, dx, N * Cn, S, bool(accum))
     return dx
 
 
 def max_pooling_backward(x, dy, kernel, stride=None, ignore_border=True, pad=None, accum=False, dx=None):
     """MaxPooling::backward_impl (max_pooling.cpp:194-228); x is the forward input."""
-    x, dy = _check_input(x), _check_input(dy, "dy")
+    x, dy = L.f32(x), L.f32(dy, "dy")
     stride = tuple(kernel) if stride is None else tuple(stride)
     pad = (0, 0) if pad is None else tuple(pad)
     H, W = int(x.shape[-2]), int(x.shape[-1])
     maps = x.numel() // max(H * W, 1)
     dx = _grad_out(x, accum, dx)
-    with C.on_device(x.device):
-        C.call("nb200_max_pooling_backward_f32", C.ptr(x), C.ptr(dy), C.ptr(dx), ctypes.c_int64(maps), H, W,
-               int(kernel[0]), int(kernel[1]), int(stride[0]), int(stride[1]), int(pad[0]), int(pad[1]),
-               int(bool(ignore_border)), int(bool(accum)), C.stream_ptr(x.device))
+    L.nb200_max_pooling_backward_f32(x, dy, dx, maps, H, W, kernel[0], kernel[1], stride[0],
+                                     stride[1], pad[0], pad[1], bool(ignore_border),
+                                     bool(accum))
     return dx
 
 
@@ -964,7 +888,7 @@ def bn_add_relu_fixed_point(a, bn_a, b=None, bn_b=None, eps=1e-05, relu=True, qu
     adds b as it is, b=None leaves the second term out). The reference's fused
     form of the first three stages is FusedBatchNormalization
     (src/nbla/function/generic/fused_batch_normalization.cpp)."""
-    a = _check_input(a, "a")
+    a = L.f32(a, "a")
     if a.dim() < 2:
         raise RuntimeError("the normalised axis is axis 1")
     Cn = int(a.shape[1])
@@ -978,7 +902,7 @@ def bn_add_relu_fixed_point(a, bn_a, b=None, bn_b=None, eps=1e-05, relu=True, qu
                     raise RuntimeError("mean and variance are required (%s)" % what)
                 out.append(None)
                 continue
-            t = _check_input(t, nm)
+            t = L.f32(t, nm)
             if t.numel() != Cn:
                 raise RuntimeError("%s must have %d elements (shape of the normalised axis)" % (nm, Cn))
             out.append(t)
@@ -986,18 +910,15 @@ def bn_add_relu_fixed_point(a, bn_a, b=None, bn_b=None, eps=1e-05, relu=True, qu
     pa = params(bn_a, "a")
     pb = [None] * 4
     if b is not None:
-        b = _check_input(b, "b")
+        b = L.f32(b, "b")
         _same_shape(a, b, "a vs b")
         if bn_b is not None:
             pb = params(bn_b, "b")
     elif bn_b is not None:
         raise RuntimeError("bn_b without b")
     y = _output_like(a, outputs)
-    with C.on_device(a.device):
-        C.call("nb200_bn_add_relu_fxp_f32", C.ptr(a), C.ptr(pa[0]), C.ptr(pa[1]), C.ptr(pa[2]), C.ptr(pa[3]),
-               C.ptr(b), C.ptr(pb[0]), C.ptr(pb[1]), C.ptr(pb[2]), C.ptr(pb[3]), C.ptr(y), ctypes.c_int64(outer),
-               ctypes.c_int64(Cn), ctypes.c_int64(inner), C.c_float(eps), int(bool(relu)), int(bool(quantize)),
-               int(bool(sign)), int(n), C.c_float(delta), C.stream_ptr(a.device))
+    L.nb200_bn_add_relu_fxp_f32(a, pa[0], pa[1], pa[2], pa[3], b, pb[0], pb[1], pb[2], pb[3], y, outer, Cn, inner, eps,
+                                bool(relu), bool(quantize), bool(sign), n, delta)
     return y
 
 
@@ -1007,9 +928,7 @@ def bn_add_relu_fixed_point(a, bn_a, b=None, bn_b=None, eps=1e-05, relu=True, qu
 
 def codes_nhwc_slots(channels, group=1):
     """Slots per pixel of a codes tensor for `channels` channels in `group` groups."""
-    fn = C.lib().nb200_codes_nhwc_slots
-    fn.restype = ctypes.c_int64
-    n = int(fn(ctypes.c_int64(int(channels)), int(group)))
+    n = L.codes_nhwc_slots(channels, group)
     if n <= 0:
         raise RuntimeError("Number of input channel needs to be divisible by group. Input channel: %d, group: %d."
                            % (channels, group))
@@ -1026,12 +945,10 @@ def _nchw_extents(x):
 def fixed_point_codes_nhwc(xq, delta=2 ** -4, group=1):
     """xq [batch, channels, ...] (an output of fixed_point_quantize with step
     `delta` and n <= 8) -> int8 codes [batch, inner, slots], channel-last."""
-    xq = _check_input(xq, "xq")
+    xq = L.f32(xq, "xq")
     batch, ch, inner = _nchw_extents(xq)
-    codes = torch.empty((batch, inner, codes_nhwc_slots(ch, group)), dtype=torch.int8, device=xq.device)
-    with C.on_device(xq.device):
-        C.call("nb200_fixed_point_codes_nhwc", C.ptr(xq), C.ptr(codes), ctypes.c_int64(batch), ctypes.c_int64(ch),
-               ctypes.c_int64(inner), int(group), C.c_float(delta), C.stream_ptr(xq.device))
+    codes = L.empty_i8((batch, inner, codes_nhwc_slots(ch, group)), xq)
+    L.nb200_fixed_point_codes_nhwc(xq, codes, batch, ch, inner, group, delta)
     return codes
 
 
@@ -1039,7 +956,7 @@ def _check_codes(codes, batch, inner, channels, group, name="codes"):
     if not isinstance(codes, torch.Tensor) or not codes.is_cuda or codes.dtype != torch.int8:
         raise TypeError("%s must be an int8 torch.Tensor on a CUDA device" % name)
     want = (batch, inner, codes_nhwc_slots(channels, group))
-    if tuple(codes.shape) != want or not codes.is_contiguous():
+    if codes.shape != want or not codes.is_contiguous():
         raise RuntimeError("%s must be a contiguous [batch, inner, slots] = %s tensor, got %s"
                            % (name, want, tuple(codes.shape)))
     return codes
@@ -1053,10 +970,8 @@ def codes_nhwc_to_float(codes, shape, delta=2 ** -4, group=1):
     for v in shape[2:]:
         inner *= v
     codes = _check_codes(codes, batch, inner, ch, group)
-    y = torch.empty(shape, dtype=torch.float32, device=codes.device)
-    with C.on_device(codes.device):
-        C.call("nb200_codes_nhwc_to_f32", C.ptr(codes), C.ptr(y), ctypes.c_int64(batch), ctypes.c_int64(ch),
-               ctypes.c_int64(inner), int(group), C.c_float(delta), C.stream_ptr(codes.device))
+    y = L.empty(shape, codes)
+    L.nb200_codes_nhwc_to_f32(codes, y, batch, ch, inner, group, delta)
     return y
 
 
@@ -1066,7 +981,7 @@ def bn_add_relu_fixed_point_codes(a, bn_a, b=None, bn_b=None, b_codes=None, b_de
     codes (value = code * delta). The second operand is b (fp32, shaped like
     a, normalised with bn_b when given) or b_codes (codes of a tensor shaped
     like a, step b_delta, default delta)."""
-    a = _check_input(a, "a")
+    a = L.f32(a, "a")
     batch, Cn, inner = _nchw_extents(a)
 
     def params(t4, what):
@@ -1077,7 +992,7 @@ def bn_add_relu_fixed_point_codes(a, bn_a, b=None, bn_b=None, b_codes=None, b_de
                     raise RuntimeError("mean and variance are required (%s)" % what)
                 out.append(None)
                 continue
-            t = _check_input(t, nm)
+            t = L.f32(t, nm)
             if t.numel() != Cn:
                 raise RuntimeError("%s must have %d elements (shape of the normalised axis)" % (nm, Cn))
             out.append(t)
@@ -1087,7 +1002,7 @@ def bn_add_relu_fixed_point_codes(a, bn_a, b=None, bn_b=None, b_codes=None, b_de
     if b is not None and b_codes is not None:
         raise RuntimeError("the second operand is either b or b_codes")
     if b is not None:
-        b = _check_input(b, "b")
+        b = L.f32(b, "b")
         _same_shape(a, b, "a vs b")
         if bn_b is not None:
             pb = params(bn_b, "b")
@@ -1095,13 +1010,10 @@ def bn_add_relu_fixed_point_codes(a, bn_a, b=None, bn_b=None, b_codes=None, b_de
         raise RuntimeError("bn_b without b")
     if b_codes is not None:
         b_codes = _check_codes(b_codes, batch, inner, Cn, group, "b_codes")
-    y = torch.empty((batch, inner, codes_nhwc_slots(Cn, group)), dtype=torch.int8, device=a.device)
-    with C.on_device(a.device):
-        C.call("nb200_bn_add_relu_fxp_codes_nhwc", C.ptr(a), C.ptr(pa[0]), C.ptr(pa[1]), C.ptr(pa[2]), C.ptr(pa[3]),
-               C.ptr(b), C.ptr(pb[0]), C.ptr(pb[1]), C.ptr(pb[2]), C.ptr(pb[3]), C.ptr(b_codes),
-               C.c_float(delta if b_delta is None else b_delta), C.ptr(y), ctypes.c_int64(batch), ctypes.c_int64(Cn),
-               ctypes.c_int64(inner), int(group), C.c_float(eps), int(bool(relu)), int(bool(sign)), int(n),
-               C.c_float(delta), C.stream_ptr(a.device))
+    y = L.empty_i8((batch, inner, codes_nhwc_slots(Cn, group)), a)
+    L.nb200_bn_add_relu_fxp_codes_nhwc(a, pa[0], pa[1], pa[2], pa[3], b, pb[0], pb[1], pb[2], pb[3], b_codes, delta if
+                                       b_delta is None else b_delta, y, batch, Cn, inner, group, eps,
+                                       bool(relu), bool(sign), n, delta)
     return y
 
 
@@ -1122,11 +1034,9 @@ def max_pooling_codes(codes, shape, kernel, stride=None, ignore_border=True, pad
     Wo = (W + pad[1] - (kernel[1] - pad[1] if ignore_border else 1)) // stride[1] + 1
     if Ho <= 0 or Wo <= 0:
         raise RuntimeError("pooling output would be empty")
-    y = torch.empty((batch, Ho * Wo, codes.shape[2]), dtype=torch.int8, device=codes.device)
-    with C.on_device(codes.device):
-        C.call("nb200_max_pooling_codes_nhwc", C.ptr(codes), C.ptr(y), ctypes.c_int64(batch), ctypes.c_int64(Cn), H, W,
-               int(group), int(kernel[0]), int(kernel[1]), int(stride[0]), int(stride[1]), int(pad[0]), int(pad[1]),
-               int(bool(ignore_border)), C.stream_ptr(codes.device))
+    y = L.empty_i8((batch, Ho * Wo, codes.shape[2]), codes)
+    L.nb200_max_pooling_codes_nhwc(codes, y, batch, Cn, H, W, group, kernel[0], kernel[1],
+                                   stride[0], stride[1], pad[0], pad[1], bool(ignore_border))
     return y, (batch, Cn, Ho, Wo)
 
 
@@ -1136,27 +1046,24 @@ def binary_weight_convolution_from_codes(x_codes, x_shape, weight, binary_weight
     """binary_weight_convolution (binary_connect_convolution when alpha is
     None) on activations given as int8 channel-last codes of a tensor of shape
     x_shape = (batch, channels, height, width) with step activation_delta."""
-    weight = _check_input(weight, "weight")
-    binary_weight = _check_input(binary_weight, "binary_weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    weight = L.f32(weight, "weight")
+    binary_weight = L.f32(binary_weight, "binary_weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     x_shape = tuple(int(v) for v in x_shape)
     if len(x_shape) != 4:
         raise C.NB200Error(4, "only 2-D convolution with one batch axis is implemented for code tensors")
-    like = torch.empty(x_shape, dtype=torch.float32, device="meta")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
-        like, weight, bias, 1, pad, stride, dilation, group)
+        x_shape, weight, bias, 1, pad, stride, dilation, group)
     x_codes = _check_codes(x_codes, batch, H * W, Cin, group, "x_codes")
     _same_shape(weight, binary_weight, "float vs binary")
     if alpha is not None:
-        alpha = _check_input(alpha, "alpha")
+        alpha = L.f32(alpha, "alpha")
         if alpha.numel() != Ko:
             raise RuntimeError("Size of alpha must be equal to the number of output maps.")
-    y = torch.empty(out_shape, dtype=torch.float32, device=weight.device) if outputs is None else outputs[0]
-    with C.on_device(weight.device):
-        C.call("nb200_binary_convolution_codes_f32", C.ptr(x_codes), C.ptr(weight), C.ptr(binary_weight),
-               C.ptr(alpha), C.ptr(bias), C.ptr(y), batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0],
-               stride[1], dilation[0], dilation[1], int(group), C.c_float(quantize_zero_to),
-               C.c_float(activation_delta), C.stream_ptr(weight.device))
+    y = L.empty(out_shape, weight) if outputs is None else outputs[0]
+    L.nb200_binary_convolution_codes_f32(x_codes, weight, binary_weight, alpha, bias, y, batch, Cin, H, W, Ko, kh, kw,
+                                         pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1], group,
+                                         quantize_zero_to, activation_delta)
     return y
 
 
@@ -1173,44 +1080,38 @@ def prepare_binary_weights(weight, group=1, quantize_zero_to=1.0, with_alpha=Tru
     """Binarises `weight` [outmaps, channels / group, kh, kw] once: what the binary
     convolutions otherwise redo on every call (binary_weight_convolution.cpp:72-117).
     with_alpha=False gives BinaryConnect weights (no scaling)."""
-    weight = _check_input(weight, "weight")
+    weight = L.f32(weight, "weight")
     if weight.dim() != 4:
         raise C.NB200Error(4, "only 2-D convolution weights are implemented")
     Ko, Cg, kh, kw = (int(v) for v in weight.shape)
     fn = C.lib().nb200_binary_weights_side_bytes
     fn.restype = ctypes.c_int64
-    nbytes = int(fn(Ko, Cg * int(group), kh, kw, int(group)))
+    nbytes = int(fn(Ko, Cg * group, kh, kw, group))
     if nbytes <= 0 or Ko % group != 0:
         raise RuntimeError("Number of output channel needs to be divisible by group. Output channel: %d, group: %d."
                            % (Ko, group))
-    wb = torch.empty_like(weight)
-    alpha = torch.empty((Ko,), dtype=torch.float32, device=weight.device) if with_alpha else None
-    side = torch.empty((nbytes,), dtype=torch.int8, device=weight.device)
-    with C.on_device(weight.device):
-        C.call("nb200_binary_weights_prepare_i8", C.ptr(weight), C.ptr(wb), C.ptr(alpha), C.ptr(side), Ko,
-               Cg * int(group), kh, kw, int(group), C.c_float(quantize_zero_to), C.stream_ptr(weight.device))
+    wb = L.empty(weight, weight)
+    alpha = L.empty((Ko,), weight) if with_alpha else None
+    side = L.empty_i8((nbytes,), weight)
+    L.nb200_binary_weights_prepare_i8(weight, wb, alpha, side, Ko, Cg * group, kh, kw, group,
+                                      quantize_zero_to)
     return PreparedBinaryWeights(weight.shape, group, wb, alpha, side)
 
 
 def binary_convolution_from_codes_prepared(x_codes, x_shape, prepared, bias=None, pad=None, stride=None,
                                            dilation=None, activation_delta=2 ** -4, outputs=None):
     """binary_weight_convolution_from_codes with weights from prepare_binary_weights."""
-    bias = _check_input(bias, "bias") if bias is not None else None
+    bias = L.f32(bias, "bias") if bias is not None else None
     x_shape = tuple(int(v) for v in x_shape)
     if len(x_shape) != 4:
         raise C.NB200Error(4, "only 2-D convolution with one batch axis is implemented for code tensors")
-    like_x = torch.empty(x_shape, dtype=torch.float32, device="meta")
-    like_w = torch.empty(prepared.shape, dtype=torch.float32, device="meta")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
-        like_x, like_w, bias, 1, pad, stride, dilation, prepared.group)
+        x_shape, prepared.shape, bias, 1, pad, stride, dilation, prepared.group)
     x_codes = _check_codes(x_codes, batch, H * W, Cin, prepared.group, "x_codes")
-    dev = x_codes.device
-    y = torch.empty(out_shape, dtype=torch.float32, device=dev) if outputs is None else outputs[0]
-    with C.on_device(dev):
-        C.call("nb200_binary_convolution_codes_prepared_f32", C.ptr(x_codes), C.ptr(prepared.side),
-               C.ptr(prepared.alpha), C.ptr(bias), C.ptr(y), batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0],
-               stride[1], dilation[0], dilation[1], int(prepared.group), C.c_float(activation_delta),
-               C.stream_ptr(dev))
+    y = L.empty(out_shape, x_codes) if outputs is None else outputs[0]
+    L.nb200_binary_convolution_codes_prepared_f32(x_codes, prepared.side, prepared.alpha, bias, y, batch, Cin, H, W, Ko,
+                                                  kh, kw, pad[0], pad[1], stride[0], stride[1], dilation[0],
+                                                  dilation[1], prepared.group, activation_delta)
     return y
 
 
@@ -1233,19 +1134,16 @@ def convolution_codes_folded(x_codes, x_shape, prepared, scale, bias=None, pad=N
     Returns (result, (batch, outmaps, Ho, Wo))."""
     if prepared.group != 1:
         raise C.NB200Error(4, "grouped convolutions are not supported by the folded code path")
-    scale = _check_input(scale, "scale")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    scale = L.f32(scale, "scale")
+    bias = L.f32(bias, "bias") if bias is not None else None
     x_shape = tuple(int(v) for v in x_shape)
     if len(x_shape) != 4:
         raise C.NB200Error(4, "only 2-D convolution with one batch axis is implemented for code tensors")
-    like_x = torch.empty(x_shape, dtype=torch.float32, device="meta")
-    like_w = torch.empty(prepared.shape, dtype=torch.float32, device="meta")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
-        like_x, like_w, bias, 1, pad, stride, dilation, 1)
+        x_shape, prepared.shape, bias, 1, pad, stride, dilation, 1)
     x_codes = _check_codes(x_codes, batch, H * W, Cin, 1, "x_codes")
     if scale.numel() != Ko:
         raise RuntimeError("Size of scale must be equal to the number of output maps.")
-    dev = x_codes.device
     Ho, Wo = out_shape[2], out_shape[3]
     slots = codes_nhwc_slots(Ko, 1)
     if residual_codes is not None:
@@ -1254,16 +1152,15 @@ def convolution_codes_folded(x_codes, x_shape, prepared, scale, bias=None, pad=N
         raise RuntimeError("residual must be channel-last fp32 of shape %s" % ((batch, Ho * Wo, slots),))
     y_codes = y_f32 = None
     if output == "codes":
-        y_codes = torch.empty((batch, Ho * Wo, slots), dtype=torch.int8, device=dev)
+        y_codes = L.empty_i8((batch, Ho * Wo, slots), x_codes)
     elif output == "float":
-        y_f32 = torch.empty((batch, Ho * Wo, slots), dtype=torch.float32, device=dev)
+        y_f32 = L.empty((batch, Ho * Wo, slots), x_codes)
     else:
         raise ValueError("output must be 'codes' or 'float'")
-    with C.on_device(dev):
-        C.call("nb200_convolution_codes_folded_nhwc", C.ptr(x_codes), C.ptr(prepared.side), C.ptr(scale), C.ptr(bias),
-               C.ptr(residual_codes), C.c_float(residual_delta or 0.0), C.ptr(residual), C.ptr(y_codes), C.ptr(y_f32),
-               batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1],
-               int(bool(relu)), int(bool(sign)), int(n), C.c_float(delta), C.stream_ptr(dev))
+    L.nb200_convolution_codes_folded_nhwc(x_codes, prepared.side, scale, bias, residual_codes, residual_delta or 0.0,
+                                          residual, y_codes, y_f32, batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1],
+                                          stride[0], stride[1], dilation[0], dilation[1], bool(relu),
+                                          bool(sign), n, delta)
     return (y_codes if y_codes is not None else y_f32), tuple(out_shape)
 
 
@@ -1272,16 +1169,14 @@ def convolution_relu_fixed_point_codes(x, weight, bias=None, pad=None, stride=No
     """Full-precision convolution of an input with few channels (a network stem, weights and bias
     with BatchNormalization folded in), ReLU and FixedPointQuantize in one kernel; the result is
     int8 channel-last codes. Returns (codes [batch, Ho * Wo, slots], (batch, outmaps, Ho, Wo))."""
-    x, weight = _check_input(x), _check_input(weight, "weight")
-    bias = _check_input(bias, "bias") if bias is not None else None
+    x, weight = L.f32(x), L.f32(weight, "weight")
+    bias = L.f32(bias, "bias") if bias is not None else None
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, weight, bias, 1, pad, stride, None, 1)
     slots = codes_nhwc_slots(Ko, 1)
-    y = torch.empty((batch, out_shape[2] * out_shape[3], slots), dtype=torch.int8, device=x.device)
-    with C.on_device(x.device):
-        C.call("nb200_convolution_relu_fxp_codes_nhwc", C.ptr(x), C.ptr(weight), C.ptr(bias), C.ptr(y), batch, Cin, H,
-               W, Ko, kh, kw, pad[0], pad[1], stride[0], stride[1], int(bool(relu)), int(bool(sign)), int(n),
-               C.c_float(delta), C.stream_ptr(x.device))
+    y = L.empty_i8((batch, out_shape[2] * out_shape[3], slots), x)
+    L.nb200_convolution_relu_fxp_codes_nhwc(x, weight, bias, y, batch, Cin, H, W, Ko, kh, kw, pad[0], pad[1], stride[0],
+                                            stride[1], bool(relu), bool(sign), n, delta)
     return y, tuple(out_shape)
 
 
@@ -1295,10 +1190,9 @@ def global_average_pooling_codes(codes, shape, delta=2 ** -4):
 # ---------------------------------------------------------------------------
 
 def _unary(entry, x, outputs):
-    x = _check_input(x)
+    x = L.f32(x)
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call(entry, C.ptr(x), C.ptr(y), C.size_t(x.numel()), C.stream_ptr(x.device))
+    getattr(L, entry)(x, y, x.numel())
     return y
 
 
@@ -1315,8 +1209,7 @@ def binary_tanh(x, n_outputs=-1, outputs=None):
 
 def _unary_backward(entry, x, dy, accum, dx):
     x, dy, dx = _grad_buffers(x, dy, dx, accum)
-    with C.on_device(x.device):
-        C.call(entry, C.ptr(x), C.ptr(dy), C.ptr(dx), C.size_t(x.numel()), int(bool(accum)), C.stream_ptr(x.device))
+    getattr(L, entry)(x, dy, dx, x.numel(), bool(accum))
     return dx
 
 
@@ -1333,8 +1226,8 @@ _QL_DTYPES = {1: 1, 2: 2, "int8": 1, "uint8": 2, torch.int8: 1, torch.uint8: 2}
 
 
 def _linear_params(x, scale, zero_point):
-    x, scale = _check_input(x), _check_input(scale, "scale")
-    zero_point = _check_input(zero_point, "zero_point") if zero_point is not None else None
+    x, scale = L.f32(x), L.f32(scale, "scale")
+    zero_point = L.f32(zero_point, "zero_point") if zero_point is not None else None
     for t in (scale, zero_point):
         if t is not None and t.dim() != x.dim():
             raise RuntimeError("Dimensions of inputs must be same (%d, %d)." % (x.dim(), t.dim()))
@@ -1352,10 +1245,8 @@ def quantize_linear(x, scale, zero_point, round_mode="HALF_AWAY_FROM_ZERO", narr
     if dtype not in _QL_DTYPES:
         raise C.NB200Error(4, "dtype must be int8 (BYTE) or uint8 (UBYTE)")
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_quantize_linear_f32", C.ptr(x), C.i64_array(x.shape), int(x.dim()), C.ptr(scale),
-               C.i64_array(scale.shape), C.ptr(zero_point), C.i64_array(zero_point.shape), C.ptr(y),
-               _ROUND_MODES[round_mode], int(bool(narrow_range)), _QL_DTYPES[dtype], C.stream_ptr(x.device))
+    L.nb200_quantize_linear_f32(x, x.shape, x.dim(), scale, scale.shape, zero_point, zero_point.shape, y,
+                                _ROUND_MODES[round_mode], bool(narrow_range), _QL_DTYPES[dtype])
     return y
 
 
@@ -1363,19 +1254,14 @@ def dequantize_linear(x, scale, zero_point, n_outputs=-1, outputs=None):
     """(x - zero_point) * scale (src/nbla/function/generic/dequantize_linear.cpp:60-71)."""
     x, scale, zero_point = _linear_params(x, scale, zero_point)
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_dequantize_linear_f32", C.ptr(x), C.i64_array(x.shape), int(x.dim()), C.ptr(scale),
-               C.i64_array(scale.shape), C.ptr(zero_point), C.i64_array(zero_point.shape), C.ptr(y),
-               C.stream_ptr(x.device))
+    L.nb200_dequantize_linear_f32(x, x.shape, x.dim(), scale, scale.shape, zero_point, zero_point.shape, y)
     return y
 
 
 def _linear_backward(entry, dy, scale, accum, dx):
     dy, scale, _ = _linear_params(dy, scale, None)
     _, dy, dx = _grad_buffers(dy, dy, dx, accum)
-    with C.on_device(dy.device):
-        C.call(entry, C.ptr(dy), C.i64_array(dy.shape), int(dy.dim()), C.ptr(scale), C.i64_array(scale.shape),
-               C.ptr(dx), int(bool(accum)), C.stream_ptr(dy.device))
+    getattr(L, entry)(dy, dy.shape, dy.dim(), scale, scale.shape, dx, bool(accum))
     return dx
 
 
@@ -1392,17 +1278,14 @@ def dequantize_linear_backward(dy, scale, accum=False, dx=None):
 def prune(x, rate=0.9, n_outputs=-1, outputs=None):
     """Prune the input: values whose magnitude is below the rate-quantile of
     |x| become zero (python/src/nnabla/functions.py prune; src/nbla/function/generic/prune.cpp:38-72)."""
-    x = _check_input(x)
+    x = L.f32(x)
     y = _output_like(x, outputs)
-    with C.on_device(x.device):
-        C.call("nb200_prune_f32", C.ptr(x), C.ptr(y), C.size_t(x.numel()), C.c_float(rate), C.stream_ptr(x.device))
+    L.nb200_prune_f32(x, y, x.numel(), rate)
     return y
 
 
 def prune_backward(dy, accum=False, dx=None):
     """Prune::backward_impl (prune.cpp:74-88): the gradient passes unchanged."""
     _, dy, dx = _grad_buffers(dy, dy, dx, accum)
-    with C.on_device(dy.device):
-        C.call("nb200_prune_backward_f32", C.ptr(dy), C.ptr(dx), C.size_t(dy.numel()), int(bool(accum)),
-               C.stream_ptr(dy.device))
+    L.nb200_prune_backward_f32(dy, dx, dy.numel(), bool(accum))
     return dx
