@@ -293,13 +293,10 @@ static int affine_fxp8(const float *xq, const float *wq, float delta_x, float de
   NB_TRY(slab_destinations(ep, y_ranks, n_ranks, rank, N, n_total, col_begin));
   const int64_t Kp = round_up(K, 128);
   AsyncScratch scratch(st);
-  NB_TRY(scratch.alloc((size_t)(M + N) * Kp + (size_t)K * N));
+  NB_TRY(scratch.alloc((size_t)(M + N) * Kp));
   int8_t *xc = static_cast<int8_t *>(scratch.p);
   int8_t *wt = xc + (size_t)M * Kp;
-  int8_t *wc = wt + (size_t)N * Kp;
-  NB_TRY(codes_rows_i8(xq, M, (int)K, Kp, delta_x, xc, st));
-  NB_TRY(codes_rows_i8(wq, K, (int)N, N, delta_w, wc, st));
-  NB_TRY(transpose_i8(wc, (int)K, (int)N, wt, Kp, st));
+  NB_TRY(fxp8_operands(xq, M, (int)K, Kp, delta_x, xc, wq, (int)N, delta_w, wt, st));
   ep.scale = delta_x * delta_w;
   ep.col_bias = bias;
   return run_gemm(true, 1, 1, xc, Kp, wt, Kp, (int)M, (int)N, (int)K, ep, n_total, st);

@@ -47,8 +47,10 @@ int nchw_to_nhwc_half_pair(const float *x, int N, int C, int HW, int groups, int
 int transpose_i8(const int8_t *src, int R, int C, int8_t *dst, int64_t pitch, cudaStream_t st);
 // fp32 [R, C] -> [C][R].
 int transpose_f32(const float *src, int R, int C, float *dst, cudaStream_t st);
-// fp32 multiples of delta [rows, K] -> int8 [rows][pitch].
-int codes_rows_i8(const float *x, int64_t rows, int K, int64_t pitch, float delta, int8_t *out, cudaStream_t st);
+// x [M, K] multiples of delta_x -> int8 [M][Kp] and w [K, N] multiples of delta_w -> int8 [N][Kp] (transposed);
+// Kp a multiple of 128, zero padded, xc and wt 16-byte aligned.
+int fxp8_operands(const float *x, int64_t M, int K, int64_t Kp, float delta_x, int8_t *xc, const float *w, int N,
+                  float delta_w, int8_t *wt, cudaStream_t st);
 
 // ---- convolution backward (prepare_backward.cu) ------------------------------
 // dy [N][Ko][Ho][Wo] -> 3 bf16 planes [N][Hs][Ws][ctot] (pre-zeroed by the caller):

@@ -211,3 +211,15 @@ def test_fixed_point_affine_full_baseline_size(F):
     rows = slice(4000, 4016)
     ref_rows = oracle.affine(xq[rows].cpu().numpy(), wq.cpu().numpy(), b.cpu().numpy())
     assert np.array_equal(bits(y[rows].cpu().numpy()), bits(ref_rows))
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (1, 32, 10), (33, 128, 64), (5, 127, 65), (130, 129, 66), (3, 260, 61),
+                                   (7, 1028, 67), (64, 513, 132)])
+def test_fixed_point_affine_operand_tiles(F, M, K, N):
+    """Edges of the operand pass: runs of 128 values of x, tiles of 128 x 64 of w, rows of no round size."""
+    rng = np.random.RandomState(17)
+    xq = oracle.fixed_point_quantize(rng.randn(M, K).astype(np.float32), True, 8, 2.0 ** -5)
+    wq = oracle.fixed_point_quantize((0.02 * rng.randn(K, N)).astype(np.float32), True, 8, 2.0 ** -10)
+    y = F.affine(dev(xq), dev(wq), None, fixed_point=(2.0 ** -5, 2.0 ** -10)).cpu().numpy()
+    exact = (np.round(xq.astype(np.float64) * 2 ** 5) @ np.round(wq.astype(np.float64) * 2 ** 10)).astype(np.float32)
+    assert np.array_equal(y, exact * np.float32(2.0 ** -15))
