@@ -37,7 +37,7 @@ bool pixel_major_applies(const ConvGeometry &g);
 int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const float *scale, const float *bias,
                              const int8_t *res_codes, float res_delta, const float *res_f32, int8_t *y_codes,
                              float *y_f32, ConvGeometry g, int relu, int sign, int n, float delta, cudaStream_t st,
-                             float *y_nchw = nullptr, float nchw_scale = 1.0f);
+                             float *y_nchw = nullptr, float nchw_scale = 1.0f, int weight_limit = 1);
 
 // The reference's checks (src/nbla/function/generic/convolution.cpp:40-158).
 int check_geometry(ConvGeometry &g) {
@@ -237,7 +237,7 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
     // pixels on the MMA rows: same accumulators, same rounded operations in the epilogue, faster loads and stores
     return convolution_codes_folded(reinterpret_cast<const int8_t *>(act), reinterpret_cast<const int8_t *>(side),
                                     fxp_weights ? nullptr : alpha, bias, nullptr, 0.0f, nullptr, nullptr, nullptr, g, 0,
-                                    1, 8, 1.0f, st, y, ep.scale);
+                                    1, 8, 1.0f, st, y, ep.scale, fxp_weights ? 127 : 1);
   }
   if (int8) {
     // All tiles share the weights when the output maps fit one M tile: keep them in shared
@@ -520,7 +520,8 @@ void int8_side_layout(int Cg, int taps, int &c_slots, int64_t &wpitch) {
 long long *g_cc_trace = nullptr;
 #endif
 
-template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false>
+// halves = 2: two row blocks of h_box / 2 output rows each per tile (halo form).
+template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false, int kHalves = 1>
 int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot, const int8_t *side, int64_t wpitch,
                       int cblocks, int h_box, int n_box, int slots_out, const ConvCodesEpilogue &ep, cudaStream_t st) {
   CUtensorMap mx, mw;
@@ -564,11 +565,13 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
   p.slots_out = slots_out;
   p.wp = wp;
   p.hp = hp;
+  p.h_half = h_box / kHalves;
   // rows a shifted descriptor may read: the largest tap shift plus the 128 rows of the MMA, in whole
   // swizzle patterns of 8 rows (rows the box does not write hold stale data that no stored pixel uses)
-  const int rows_alloc = (((g.kh - 1) * g.dh * wp + (g.kw - 1) * g.dw + kTileM) + 7) / 8 * 8;
+  const int rows_alloc =
+      (((kHalves - 1) * p.h_half * wp + (g.kh - 1) * g.dh * wp + (g.kw - 1) * g.dw + kTileM) + 7) / 8 * 8;
   p.a_tile_bytes = (rows_alloc > hp * wp ? rows_alloc : (hp * wp + 7) / 8 * 8) * RB;
-  auto kernel = conv_codes_tcgen05_kernel<BN, STAGES, RB, kResidentB, kHalo>;
+  auto kernel = conv_codes_tcgen05_kernel<BN, STAGES, RB, kResidentB, kHalo, kHalves>;
   constexpr size_t smem_fixed = conv_codes_smem_bytes<BN, STAGES, RB, kResidentB, kHalo>();
   static_assert(smem_fixed <= 227 * 1024, "shared memory budget");
   const size_t smem = smem_fixed + (kResidentB ? (size_t)p.taps * p.cblocks * BN * RB : 0) +
@@ -598,11 +601,12 @@ bool pixel_major_applies(const ConvGeometry &g) {
 }
 
 // y_nchw != NULL: plain fp32 [batch][maps][pixels] result, acc * scale[o] (+ bias[o]) with each operation
-// rounded on its own (what the unfused functions return); no residual, ReLU or quantizer then.
+// rounded on its own (what the unfused functions return); no residual, ReLU or quantizer then. weight_limit: largest
+// magnitude of the int8 weights.
 int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const float *scale, const float *bias,
                              const int8_t *res_codes, float res_delta, const float *res_f32, int8_t *y_codes,
                              float *y_f32, ConvGeometry g, int relu, int sign, int n, float delta, cudaStream_t st,
-                             float *y_nchw, float nchw_scale) {
+                             float *y_nchw, float nchw_scale, int weight_limit) {
   NB_TRY(check_geometry(g));
   NB_CHECK(g.group == 1, NB200_ENOTIMPL, "grouped convolutions are not supported by the folded code path");
   NB_CHECK(x_codes && side && (scale || y_nchw) && (y_codes || y_f32 || y_nchw), NB200_EVALUE, "null data pointer");
@@ -626,6 +630,8 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
   ep.relu = relu;
   ep.out_scale = 1.0f;
   ep.kmax = ep.kmin = 0;
+  ep.saturate = 0;
+  ep.small_acc = weight_limit * 127ll * g.Cg * g.kh * g.kw < (1 << 22);
   if (y_codes) {
     // the quantizer's setup (fixed_point_quantize.cpp:31-42); the step must be a power of two
     NB_CHECK(n > 0 && delta > 0.f, NB200_EVALUE, "Both bit width and delta should be positive.");
@@ -638,6 +644,9 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
     ep.out_scale = 2.0f / delta;
     ep.kmax = (1 << nn) - 1;
     ep.kmin = sign ? -ep.kmax : 0;
+    ep.saturate = relu && ep.kmax == 127;
+    if (ep.saturate)
+      ep.out_scale = 0.0078125f / delta;
   }
   ep.bias_scale = ep.out_scale;
   ep.res_scale = (res_codes ? res_delta : 1.0f) * ep.out_scale;
@@ -695,8 +704,19 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
       const size_t need = 2 * cblocks * a_bytes + w_bytes * BNh + 8 * 1024;
       if (need <= 220 * 1024 && wp <= 256 && hp <= 256) {
         if (narrow_rows) {
-          if (g.Ko <= 64)
+          if (g.Ko <= 64) {
+            // two row blocks per tile, once every SM has more than one such tile to do (below that the larger tile
+            // only makes the single round of tiles longer)
+            const int h2 = 2 * hh < g.Ho ? 2 * hh : (g.Ho + 1) / 2 * 2;
+            const int64_t pairs = (int64_t)g.N * ((g.Ho + h2 - 1) / h2);
+            const int hp2 = h2 + (g.kh - 1) * g.dh;
+            const size_t a2_bytes = (size_t)(rows_alloc + (h2 / 2) * wp > hp2 * wp ? rows_alloc + (h2 / 2) * wp
+                                                                                   : (hp2 * wp + 7) / 8 * 8) * RBh;
+            if (pairs > sm_count() && h2 / 2 >= 1 && hp2 <= 256 && 2 * a2_bytes + w_bytes * BNh + 8 * 1024 <= 220 * 1024)
+              return launch_conv_codes<64, 1, 64, true, true, 2>(g, x_codes, ctot, side, wpitch, cblocks, h2, 1,
+                                                                 (int)slots_out, ep, st);
             NB_CC_HALO(64, 64);
+          }
           NB_CC_HALO(128, 64);
         }
         if (g.Ko <= 64)

@@ -43,6 +43,7 @@ struct ConvCodesProblem {
   int slots_out; // bytes per pixel of the code result / floats per pixel of the fp32 result
   // halo form (stride 1): one box of hp x wp input pixels per tile and channel block
   int wp, hp;          // wp = Wo + (kw - 1) * dw, hp = h_box + (kh - 1) * dh
+  int h_half;          // output rows of one MMA row block (h_box, or half of it with two row blocks per tile)
   int a_tile_bytes;    // bytes of one channel block's pixel tile in shared memory (readable rows included)
   __device__ __forceinline__ int num_tiles() const { return n_tiles * tiles_h * tiles_n; }
   __device__ __forceinline__ int k_blocks() const { return taps * cblocks; }
@@ -63,6 +64,9 @@ struct ConvCodesEpilogue {
                                // power of two), the activations' step for the plain fp32 result, else 1
   float bias_scale;            // factor of bias: 2 / delta when codes are written, else 1
   int kmax, kmin;              // code range
+  int saturate;                // codes with ReLU and kmax = 127: out_scale, bias_scale and res_scale hold
+                               // 1 / (128 * delta) instead of 2 / delta
+  int small_acc;               // every accumulator is below 2^22 in magnitude (see int_to_float)
 #ifdef NB200_CC_TRACE
   long long *trace; // timing experiments: block 0 writes %globaltimer at its phase boundaries
 #endif
@@ -102,6 +106,13 @@ __device__ __forceinline__ uint32_t pack_s8x4(int a, int b, int c, int d) {
 }
 
 constexpr int kCodesMaxMaps = 512;
+// a * b + c with one rounding, clamped to [0, 1] (NaN: 0).
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float d;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 constexpr int kCodesKTable = 64; // K blocks whose coordinates are tabulated once per block
 
 // kResidentB: all tiles use the same weights (one column tile) and all their K blocks fit in
@@ -119,19 +130,33 @@ constexpr int kCodesKTable = 64; // K blocks whose coordinates are tabulated onc
 // that is a whole number of rows further on reads exactly the rows further on (no base-offset
 // field is needed; setting one breaks it). This cuts the copy engine's rows per tile by the number
 // of taps.
-template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false>
+//
+// kHalves = 2 (halo form, at most 64 maps): a tile is two MMA row blocks, rows [0, 128) and the 128 rows from
+// h_half * wp on, of ONE input box of 2 * h_half output rows; their accumulators lie side by side in tensor memory.
+// With one block of 18 small MMAs per tile the hand-over between the roles (four barriers, the commits, the
+// descriptors' way into uniform registers) took as long as the MMAs themselves.
+template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false, int kHalves = 1>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     conv_codes_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                               const ConvCodesProblem prob, const ConvCodesEpilogue ep, int *status) {
   static_assert(RB == 128 || RB == 64, "operand rows are one 128-byte or 64-byte swizzle span");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N for M = 128");
   static_assert(!kHalo || kResidentB, "the halo form streams pixel tiles only");
+  static_assert(kHalves == 1 || (kHalo && kHalves == 2 && BN == 64), "two row blocks only with 64 maps");
+  constexpr int kSets = kEpilogueWarps / 4; // sets of four epilogue warps, one per TMEM lane quarter
+  constexpr int kCols = kHalves * BN;       // accumulator columns of a tile
+  // The halo forms keep the maps' scale and bias in tensor memory, the same in every lane, and read them like the
+  // accumulators. MMAs of 64 and 128 columns take 94 % of the shared-memory bandwidth (6 of 6.4 KB, 8 of 8.6 KB a
+  // call), and sixteen 128-bit broadcast reads per chunk took the rest and more: the MMAs and the epilogue of a tile
+  // ran one after the other.
+  constexpr int kScaleCol = 2 * kCols; // scale at [kScaleCol, + BN), bias behind it
   constexpr int kElems = RB;              // int8: K elements per operand row of one K block
   constexpr int kMmasPerBlock = RB / 32;  // 32 bytes of K per MMA
   constexpr uint32_t kABytes = kTileM * RB;
   constexpr uint32_t kBBytes = BN * RB;
   constexpr uint32_t kStageBytes = kABytes + (kResidentB ? 0u : kBBytes);
-  constexpr uint32_t kTmemCols = (2 * BN <= 32) ? 32 : (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
+  constexpr int kUsedCols = 2 * kCols + (kHalo ? 2 * BN : 0);
+  constexpr uint32_t kTmemCols = (kUsedCols <= 64) ? 64 : (kUsedCols <= 128) ? 128 : (kUsedCols <= 256) ? 256 : 512;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -170,7 +195,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(tmem_full + b, 1);
-      ptx::mbar_init(tmem_empty + b, kEpilogueWarps);
+      ptx::mbar_init(tmem_empty + b, 4 * kSets);
     }
     ptx::mbar_init(b_full, 1);
     for (int b = 0; b < 2; ++b) {
@@ -298,7 +323,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         ptx::tc_fence_after_sync();
         NB_CC_STAMP(3, local);
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kCols);
         uint32_t accumulate = 0;
         if constexpr (kHalo) {
           const int ab = local & 1;
@@ -311,17 +336,36 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           ptx::tc_fence_after_sync();
           const uint32_t a_base = ptx::smem_u32(smem) + (uint32_t)(ab * prob.cblocks * prob.a_tile_bytes);
           // (start addresses are 16-byte units in the low 14 bits of a descriptor; shared memory ends below 2^18)
-          const uint64_t adesc0 = ptx::smem_desc_k(a_base, RB);
-          const uint64_t bdesc0 = ptx::smem_desc_k(ptx::smem_u32(b_resident), RB);
-          for (int kb = 0; kb < k_blocks; ++kb) {
-            const uint64_t adesc = adesc0 + (uint64_t)(uint32_t)(tabulated ? kb_table[kb].x : kb_entry(kb).x);
-            const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)kb * (kBBytes >> 4));
+          const uint64_t adesc0 = ptx::smem_desc_k(a_base, RB), bdesc0 = ptx::smem_desc_k(ptx::smem_u32(b_resident), RB);
+          const uint32_t hi = (uint32_t)(adesc0 >> 32), alo = (uint32_t)adesc0, blo = (uint32_t)bdesc0;
+          const uint32_t half_step = (uint32_t)(prob.h_half * prob.wp * RB) >> 4;
+          auto issue = [&](uint32_t a_off, int kb) {
 #pragma unroll
-            for (int k = 0; k < kMmasPerBlock; ++k) {
-              ptx::mma_i8(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, accumulate);
-              accumulate = 1;
+            for (int h = 0; h < kHalves; ++h)
+#pragma unroll
+              for (int k = 0; k < kMmasPerBlock; ++k)
+                ptx::mma_i8(d_tmem + h * BN, ((uint64_t)hi << 32) | (alo + a_off + h * half_step + 2 * k),
+                            ((uint64_t)hi << 32) | (blo + (uint32_t)kb * (kBBytes >> 4) + 2 * k), idesc,
+                            k == 0 ? accumulate : 1u);
+            accumulate = 1;
+          };
+          // Offsets of kBatch K blocks first, then their MMAs back to back: descriptors reach the tensor core
+          // through uniform registers, and a loop that makes one K block's at a time spent 45 cycles an iteration
+          // on that (an MMA of 64 columns takes 51).
+          constexpr int kBatch = 4;
+          int kb = 0;
+          if (tabulated)
+            for (; kb + kBatch <= k_blocks; kb += kBatch) {
+              uint32_t off[kBatch];
+#pragma unroll
+              for (int u = 0; u < kBatch; ++u)
+                off[u] = (uint32_t)kb_table[kb + u].x;
+#pragma unroll
+              for (int u = 0; u < kBatch; ++u)
+                issue(off[u], kb + u);
             }
-          }
+          for (; kb < k_blocks; ++kb)
+            issue((uint32_t)(tabulated ? kb_table[kb].x : kb_entry(kb).x), kb);
           ptx::mma_commit(a_empty + ab); // the pixel tile is free once these MMAs have read it
           ptx::mma_commit(tmem_full + buf);
         } else {
@@ -360,42 +404,51 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;      // TMEM lanes [32 * quarter, +32) are visible to this warp
-    const int half = (warp - 2) >> 2;  // the two warps of a quarter take even / odd 32-column chunks
-    const int per_img = prob.h_box * prob.Wo;
+    const int first_col = 32 * ((warp - 2) >> 2); // this warp's first 32-column chunk of a tile's accumulators
     const float cap = (float)(2 * ep.kmax) + 0.5f;
+    // this thread's pixel of every tile: image of the box, row and column (the divisions stay out of the loop)
+    const int row = quarter * 32 + lane;
+    const int per_img = prob.h_box * prob.Wo, pitch = kHalo ? prob.wp : prob.Wo;
+    const int box_img = kHalo ? 0 : row / per_img, in_img = row - box_img * per_img;
+    const int box_y = in_img / pitch, box_x = in_img - box_y * pitch;
+    const bool box_ok = box_img < prob.n_box && box_x < prob.Wo && box_y < prob.h_half;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    if constexpr (kHalo) {
+      // one column tile: this warp's maps are the same for every tile
+      for (int c = first_col; c < BN; c += 32 * kSets) {
+        uint32_t t[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          t[j] = __float_as_uint(sb[c + j].x);
+        ptx::tmem_st_32x32(lane_base + kScaleCol + c, t);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          t[j] = __float_as_uint(sb[c + j].y);
+        ptx::tmem_st_32x32(lane_base + kScaleCol + BN + c, t);
+      }
+      ptx::tmem_st_wait();
+    }
     int local = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
       int n0, img0, oy0;
       decode(tile, n0, img0, oy0);
       const int buf = local & 1;
       const uint32_t buf_phase = (uint32_t)(local >> 1) & 1u;
-      // this thread's pixel
-      const int row = quarter * 32 + lane;
-      bool pix_ok;
-      int img, in_plane; // image and pixel inside the image's plane
-      if (kHalo) {
-        const int y = row / prob.wp, x = row - y * prob.wp;
-        img = img0;
-        pix_ok = x < prob.Wo && y < prob.h_box && oy0 + y < prob.Ho && img0 < prob.Nimg;
-        in_plane = (oy0 + y) * prob.Wo + x;
-      } else {
-        const int nn = row / per_img, q = row - nn * per_img;
-        img = img0 + nn;
-        pix_ok = nn < prob.n_box && img < prob.Nimg && q < (prob.Ho - oy0) * prob.Wo;
-        in_plane = oy0 * prob.Wo + q;
-      }
-      const int64_t pix = (int64_t)img * prob.Ho * prob.Wo + in_plane;
+      const int img = img0 + box_img;
       // the residual of this warp's first chunk is requested before the accumulator is waited for
       uint4 ra = make_uint4(0, 0, 0, 0), rb = make_uint4(0, 0, 0, 0);
-      {
-        const int col = n0 + 32 * half;
-        if (ep.res_codes && pix_ok && col < prob.slots_out) {
-          const int64_t off = pix * prob.slots_out + col;
-          ra = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off));
-          if (col + 16 < prob.slots_out)
-            rb = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off) + 1);
-        }
-      }
+      auto load_residual = [&](int64_t off, bool upper) {
+        ra = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off));
+        rb = upper ? __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off) + 1) : make_uint4(0, 0, 0, 0);
+      };
+      auto pixel_ok = [&](int half) {
+        const int y = box_y + half * prob.h_half;
+        return box_ok && img < prob.Nimg && y < prob.h_box && oy0 + y < prob.Ho;
+      };
+      auto in_plane_of = [&](int half) { return (oy0 + box_y + half * prob.h_half) * prob.Wo + box_x; };
+      const int64_t plane0 = (int64_t)img * prob.Ho * prob.Wo; // pixels before this image
+      if (ep.res_codes && pixel_ok(0) && n0 + first_col < prob.slots_out)
+        load_residual((plane0 + in_plane_of(0)) * prob.slots_out + n0 + first_col, n0 + first_col + 16 < prob.slots_out);
       if (threadIdx.x == 64)
         NB_CC_STAMP(5, local);
       const bool got = ptx::mbar_wait(tmem_full + buf, buf_phase, abort_flag);
@@ -411,18 +464,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (threadIdx.x == 64)
         NB_CC_STAMP(6, local);
 #pragma unroll 1
-      for (int c0 = 32 * half; c0 < BN; c0 += 64) {
-        const int col = n0 + c0; // first output map of the chunk
-        const bool live = pix_ok && col < (ep.y_nchw ? prob.Ko : prob.slots_out);
-        const int64_t off = pix * prob.slots_out + col;
+      for (int c0 = first_col; c0 < kCols; c0 += 32 * kSets) {
+        const int col = n0 + c0 % BN; // first output map of the chunk
+        const int half = c0 / BN; // row block
+        const bool live = pixel_ok(half) && col < (ep.y_nchw ? prob.Ko : prob.slots_out);
+        const int in_plane = in_plane_of(half); // inside the image's plane
+        const int64_t off = (plane0 + in_plane) * prob.slots_out + col;
         const bool upper = col + 16 < prob.slots_out; // the pixel's row ends in the middle of this chunk otherwise
-        if (c0 != 32 * half && ep.res_codes && live) { // later chunks: fetched here
-          ra = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off));
-          rb = upper ? __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off) + 1) : make_uint4(0, 0, 0, 0);
-        }
+        if (c0 != first_col && ep.res_codes && live) // later chunks: fetched here
+          load_residual(off, upper);
         uint32_t r[32];
-        ptx::tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), r);
-        ptx::tmem_ld_wait();
+        ptx::tmem_ld_32x32(lane_base + (uint32_t)(buf * kCols + c0), r);
+        float scale[32], bias[32]; // (maps past Ko have scale = bias = 0)
+        if constexpr (kHalo) {
+          uint32_t (&us)[32] = reinterpret_cast<uint32_t (&)[32]>(scale), (&ub)[32] = reinterpret_cast<uint32_t (&)[32]>(bias);
+          ptx::tmem_ld_32x32(lane_base + kScaleCol + (uint32_t)(c0 % BN), us);
+          ptx::tmem_ld_32x32(lane_base + kScaleCol + BN + (uint32_t)(c0 % BN), ub);
+          ptx::tmem_ld_wait();
+        } else {
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int j2 = 0; j2 < 16; ++j2) {
+            const float4 k = sb2[(col >> 1) + j2]; // (scale, bias) of two neighbouring maps
+            scale[2 * j2] = k.x;
+            bias[2 * j2] = k.y;
+            scale[2 * j2 + 1] = k.z;
+            bias[2 * j2 + 1] = k.w;
+          }
+        }
         if (threadIdx.x == 64)
           NB_CC_STAMP(7, local);
         if (!live)
@@ -434,15 +503,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           // all 32 values first, without branches (maps past Ko have scale = bias = 0), then the stores:
           // with a test per map in between, the maps went through the pipes one after the other
           float val[32];
+          if (ep.small_acc) {
 #pragma unroll
-          for (int j2 = 0; j2 < 16; ++j2) {
-            const float4 k = sb2[(col >> 1) + j2]; // (scale, bias) of two neighbouring maps
-            val[2 * j2] = __fmul_rn((float)(int)r[2 * j2], k.x);
-            val[2 * j2 + 1] = __fmul_rn((float)(int)r[2 * j2 + 1], k.z);
-            if (ep.has_bias) {
-              val[2 * j2] = __fadd_rn(val[2 * j2], k.y);
-              val[2 * j2 + 1] = __fadd_rn(val[2 * j2 + 1], k.w);
-            }
+            for (int j = 0; j < 32; ++j)
+              val[j] = int_to_float((int)r[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              val[j] = (float)(int)r[j];
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            val[j] = __fmul_rn(val[j], scale[j]);
+          if (ep.has_bias) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              val[j] = __fadd_rn(val[j], bias[j]);
           }
           if (col + 32 <= prob.Ko) {
 #pragma unroll
@@ -456,62 +532,83 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           continue;
         }
-        // u = acc * scale + bias, one fused multiply-add (scale and bias already carry the factor
-        // 2 / delta when codes are written, so u is twice the quantizer's argument)
         // Integers become floats on the add / multiply pipes instead of the (much narrower) conversion
         // pipe: for |a| < 2^22, the bit pattern of 1.5 * 2^23 plus a IS the float 1.5 * 2^23 + a.
-        float v[32];
-#pragma unroll
-        for (int j2 = 0; j2 < 16; ++j2) {
-          const float4 k = sb2[(col >> 1) + j2]; // (scale, bias) of two neighbouring maps
-          v[2 * j2] = __fmaf_rn(int_to_float((int)r[2 * j2]), k.x, k.y);
-          v[2 * j2 + 1] = __fmaf_rn(int_to_float((int)r[2 * j2 + 1]), k.z, k.w);
-        }
-        if (ep.res_codes) {
-          // code + 128 (one XOR per word) lands in the low mantissa byte of 1.5 * 2^23
-          const uint32_t w[8] = {ra.x ^ 0x80808080u, ra.y ^ 0x80808080u, ra.z ^ 0x80808080u, ra.w ^ 0x80808080u,
-                                 rb.x ^ 0x80808080u, rb.y ^ 0x80808080u, rb.z ^ 0x80808080u, rb.w ^ 0x80808080u};
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float rc = __fsub_rn(__uint_as_float(__byte_perm(w[j >> 2], 0x4B400000u, 0x7650 + (j & 3))),
-                                       12582912.0f + 128.0f);
-            v[j] = __fmaf_rn(rc, ep.res_scale, v[j]);
-          }
-        } else if (ep.res_f32) {
-          const float4 *rp = reinterpret_cast<const float4 *>(ep.res_f32 + off);
-#pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 t = (j4 < 4 || upper) ? __ldg(rp + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
-            v[4 * j4 + 0] = __fmaf_rn(t.x, ep.res_scale, v[4 * j4 + 0]);
-            v[4 * j4 + 1] = __fmaf_rn(t.y, ep.res_scale, v[4 * j4 + 1]);
-            v[4 * j4 + 2] = __fmaf_rn(t.z, ep.res_scale, v[4 * j4 + 2]);
-            v[4 * j4 + 3] = __fmaf_rn(t.w, ep.res_scale, v[4 * j4 + 3]);
-          }
-        }
-        if (ep.y_f32) {
-          float4 *yp = reinterpret_cast<float4 *>(ep.y_f32 + off);
-#pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4)
-            if (j4 < 4 || upper)
-              yp[j4] = make_float4(v[4 * j4], v[4 * j4 + 1], v[4 * j4 + 2], v[4 * j4 + 3]);
-          continue;
-        }
+        // code + 128 of a residual (one XOR per word) lands in the low mantissa byte of 1.5 * 2^23
+        const uint32_t rw[8] = {ra.x ^ 0x80808080u, ra.y ^ 0x80808080u, ra.z ^ 0x80808080u, ra.w ^ 0x80808080u,
+                                rb.x ^ 0x80808080u, rb.y ^ 0x80808080u, rb.z ^ 0x80808080u, rb.w ^ 0x80808080u};
+        auto residual = [&](int j) {
+          return __fsub_rn(__uint_as_float(__byte_perm(rw[j >> 2], 0x4B400000u, 0x7650 + (j & 3))), 12582912.0f + 128.0f);
+        };
         uint32_t w[8];
-        if (ep.relu && ep.kmax == 127) {
-          // ReLU, then the quantizer of a non-negative value: code = (floor(u) + 1) >> 1, capped at 127
-          // by the saturating pack (maps past Ko have scale = bias = 0 and give code 0 on their own)
+        if (ep.saturate) {
+          // ReLU and a quantizer with codes up to 127: scale, bias and residual carry 1 / (128 * delta), so that the
+          // last fused multiply-add saturated to [0, 1] is the ReLU, the upper limit and a NaN's 0 at once. Adding
+          // 256.00390625 = 2^8 + 2^-8 rounded DOWN leaves floor(128 v + 0.5), 0 to 128, in mantissa bits 8 to 15,
+          // and of four codes in a word a 128 becomes 127 by subtracting its top bit: 8.5 instructions a value with a
+          // residual, where limits, conversion and packing one by one took 14.
+          // (one test of the residual's kind per chunk: a test per value keeps the values from overlapping)
+          float v[32];
+          if (ep.res_codes) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              v[j] = fma_sat(residual(j), ep.res_scale, __fmaf_rn(int_to_float((int)r[j]), scale[j], bias[j]));
+          } else if (ep.res_f32) {
+            const float4 *rp = reinterpret_cast<const float4 *>(ep.res_f32 + off);
+#pragma unroll
+            for (int j4 = 0; j4 < 8; ++j4) {
+              const float4 t = (j4 < 4 || upper) ? __ldg(rp + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
+              const float f[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int j = 4 * j4 + i;
+                v[j] = fma_sat(f[i], ep.res_scale, __fmaf_rn(int_to_float((int)r[j]), scale[j], bias[j]));
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              v[j] = fma_sat(int_to_float((int)r[j]), scale[j], bias[j]);
+          }
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
-            int c[4];
+            uint32_t c[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              // floor of 0 <= u < 2^23 without the conversion pipe: u + 2^23 rounded DOWN has it in its mantissa
-              const float t = __fadd_rd(fminf(fmaxf(v[4 * j4 + k], 0.0f), cap), 8388608.0f); // a NaN becomes 0
-              c[k] = (__float_as_int(t) - 0x4B000000 + 1) >> 1;
-            }
-            w[j4] = (uint32_t)c[0] | ((uint32_t)c[1] << 8) | ((uint32_t)c[2] << 16) | ((uint32_t)c[3] << 24); // each <= 127
+            for (int i = 0; i < 4; ++i)
+              c[i] = __float_as_uint(__fadd_rd(v[4 * j4 + i], 256.00390625f));
+            const uint32_t packed = __byte_perm(__byte_perm(c[0], c[1], 0x0051), __byte_perm(c[2], c[3], 0x0051), 0x5410);
+            w[j4] = packed - ((packed >> 7) & 0x01010101u);
           }
         } else {
+          // u = acc * scale + bias, one fused multiply-add (scale and bias already carry the factor
+          // 2 / delta when codes are written, so u is twice the quantizer's argument)
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            v[j] = __fmaf_rn(int_to_float((int)r[j]), scale[j], bias[j]);
+          if (ep.res_codes) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              v[j] = __fmaf_rn(residual(j), ep.res_scale, v[j]);
+          } else if (ep.res_f32) {
+            const float4 *rp = reinterpret_cast<const float4 *>(ep.res_f32 + off);
+#pragma unroll
+            for (int j4 = 0; j4 < 8; ++j4) {
+              const float4 t = (j4 < 4 || upper) ? __ldg(rp + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
+              v[4 * j4 + 0] = __fmaf_rn(t.x, ep.res_scale, v[4 * j4 + 0]);
+              v[4 * j4 + 1] = __fmaf_rn(t.y, ep.res_scale, v[4 * j4 + 1]);
+              v[4 * j4 + 2] = __fmaf_rn(t.z, ep.res_scale, v[4 * j4 + 2]);
+              v[4 * j4 + 3] = __fmaf_rn(t.w, ep.res_scale, v[4 * j4 + 3]);
+            }
+          }
+          if (ep.y_f32) {
+            float4 *yp = reinterpret_cast<float4 *>(ep.y_f32 + off);
+#pragma unroll
+            for (int j4 = 0; j4 < 8; ++j4)
+              if (j4 < 4 || upper)
+                yp[j4] = make_float4(v[4 * j4], v[4 * j4 + 1], v[4 * j4 + 2], v[4 * j4 + 3]);
+            continue;
+          }
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
             uint32_t packed = 0;

@@ -295,3 +295,29 @@ def test_fusion_converter_gives_the_as_written_logits(F):
     as_written = resnet18.Runner(F, gp, gz)(dev(x))
     by_hand = resnet18.Runner(F, gp, gz, fused=True)(dev(x))
     assert torch.equal(got, as_written) and torch.equal(got, by_hand)
+
+
+@pytest.mark.parametrize("batch,channels,maps,height,width", [(40, 64, 64, 17, 56), (150, 16, 40, 7, 7), (80, 33, 64, 30, 41)])
+def test_two_row_blocks_per_tile(F, batch, channels, maps, height, width):
+    """More tiles than SMs and at most 64 maps: two MMA row blocks per tile, ragged images."""
+    rng = np.random.RandomState(batch)
+    w = torch.from_numpy(rng.randn(maps, channels, 3, 3).astype(np.float32)).cuda()
+    prep = F.prepare_binary_weights(w)
+    scale = torch.from_numpy((0.002 + 0.002 * rng.rand(maps)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.randn(maps).astype(np.float32)).cuda()
+    codes = torch.zeros(batch, height * width, F.codes_nhwc_slots(channels), dtype=torch.int8, device="cuda")
+    codes[:, :, :channels] = torch.from_numpy(rng.randint(0, 128, (batch, height * width, channels)).astype(np.int8)).cuda()
+    res = torch.zeros(batch, height * width, F.codes_nhwc_slots(maps), dtype=torch.int8, device="cuda")
+    res[:, :, :maps] = torch.from_numpy(rng.randint(-127, 128, (batch, height * width, maps)).astype(np.int8)).cuda()
+    y, shape = F.convolution_codes_folded(codes, (batch, channels, height, width), prep, scale, bias, (1, 1),
+                                          residual_codes=res, residual_delta=2.0 ** -5, delta=2.0 ** -4)
+    F.check_device_status()
+    x = codes[:, :, :channels].double().transpose(1, 2).reshape(batch, channels, height, width)
+    acc = torch.nn.functional.conv2d(x, prep.binary_weight.double(), padding=1)
+    v = (acc * scale.double().view(1, -1, 1, 1) + bias.double().view(1, -1, 1, 1)).float()
+    r = res[:, :, :maps].double().transpose(1, 2).reshape(batch, maps, height, width)
+    v = (r * 2.0 ** -5 + v.double()).float()
+    want = torch.floor(v.clamp(min=0).double() * 16 + 0.5).clamp(max=127).to(torch.int8)
+    got = y[:, :, :maps].transpose(1, 2).reshape(batch, maps, height, width)
+    assert shape == (batch, maps, height, width) and torch.equal(got, want)
+    assert not y[:, :, maps:].any()
