@@ -13,6 +13,8 @@
 #include <cstring>
 
 #include "conv_codes.cuh"
+#include "conv_planes.cuh"
+#include "conv_wgrad.cuh"
 #include "gemm.cuh"
 #include "prepare.cuh"
 
@@ -292,6 +294,329 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
 //       output is the kh x kw filter window. One launch per group.
 //  db = sums of dy over batch and pixels.
 // ---------------------------------------------------------------------------
+// The pixel-major convolution of planes (conv_planes.cuh). A: [planes][N][Hin][Win][ctot], B: [total_maps][taps][k_slots],
+// both 16-bit; output pixel (iy, ix) of p.H x p.W reads input pixel (iy + pad - k * dil) / s of tap k along either axis
+// (flip: the gradient's direction) or iy - pad + k * dil (s = 1).
+struct PlanesAxis {
+  int k, dil, pad, s;
+  bool flip;
+  int residue(int t) const { return flip ? ((t * dil - pad) % s + s) % s : 0; }
+  int offset(int t) const { return flip ? (residue(t) + pad - t * dil) / s : t * dil - pad; }
+  int min_offset() const {
+    int m = offset(0);
+    for (int t = 1; t < k; ++t)
+      m = offset(t) < m ? offset(t) : m;
+    return m;
+  }
+  int max_offset() const {
+    int m = offset(0);
+    for (int t = 1; t < k; ++t)
+      m = offset(t) > m ? offset(t) : m;
+    return m;
+  }
+};
+
+struct PlanesPlan {
+  ConvPlanesProblem p;
+  int bn;
+  bool resident;
+  size_t smem;
+};
+
+constexpr size_t kPlanesSmem = 226 * 1024; // of 227 KB; the barriers are static
+
+// Fills p's tiling for an output of p.H x p.W with p.maps maps per group; false: the kernel does not apply.
+bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, int channels_g) {
+  ConvPlanesProblem &p = plan.p;
+  const int taps = ay.k * ax.k;
+  if (taps > kPlanesMaxTaps || ay.s * ax.s > 16)
+    return false;
+  p.sy = ay.s;
+  p.sx = ax.s;
+  p.Wu = (p.W + ax.s - 1) / ax.s;
+  const int Hu = (p.H + ay.s - 1) / ay.s;
+  p.y0 = ay.min_offset();
+  p.x0 = ax.min_offset();
+  p.wp = p.Wu + ax.max_offset() - p.x0;
+  const int span_y = ay.max_offset() - p.y0;
+  p.cblocks = (channels_g + 63) / 64;
+  p.k_slots = p.cblocks * 64;
+  if (p.Wu > 128 || p.wp > 256)
+    return false;
+  p.h_box = (128 - p.Wu) / p.wp + 1; // (h_box - 1) * wp + Wu <= 128
+  p.h_box = p.h_box < Hu ? p.h_box : Hu;
+  for (int h = p.h_box; h >= 1; --h) // prefer a divisor of the rows unless it wastes over a third of the tile
+    if (Hu % h == 0) {
+      if (3 * h >= 2 * p.h_box)
+        p.h_box = h;
+      break;
+    }
+  p.hp = p.h_box + span_y;
+  if (p.hp > 256)
+    return false;
+  p.tiles_h = (Hu + p.h_box - 1) / p.h_box;
+  p.plane_bytes = (p.hp * p.wp + 7) / 8 * 8 * kRowBytes;
+  int n = 0, max_row = 0;
+  for (int ry = 0; ry < ay.s; ++ry)
+    for (int rx = 0; rx < ax.s; ++rx) {
+      p.class_tap[ry * ax.s + rx] = n;
+      for (int ky = 0; ky < ay.k; ++ky)
+        for (int kx = 0; kx < ax.k; ++kx)
+          if (ay.residue(ky) == ry && ax.residue(kx) == rx) {
+            p.tap_row[n] = (ay.offset(ky) - p.y0) * p.wp + ax.offset(kx) - p.x0;
+            max_row = p.tap_row[n] > max_row ? p.tap_row[n] : max_row;
+            p.tap_k[n++] = ky * ax.k + kx;
+          }
+    }
+  p.class_tap[ay.s * ax.s] = n;
+  // the 128 rows read from the last tap's row on may reach past the last box
+  int over = (max_row + kTileM) * kRowBytes - p.plane_bytes;
+  over = over > 0 ? over : 0;
+  plan.bn = p.maps <= 64 ? 64 : 128;
+  p.n_tiles = (p.maps + plan.bn - 1) / plan.bn;
+  const size_t b_tile = (size_t)plan.bn * kRowBytes, fixed = 1024 + over;
+  // all weights beside three single-plane boxes at least, and the accumulation short enough without chunks
+  const size_t b_all = (size_t)taps * p.cblocks * b_tile;
+  plan.resident = p.groups == 1 && p.n_tiles == 1 && taps * p.cblocks * 4 <= 96 &&
+                  fixed + b_all + 3 * (size_t)p.plane_bytes <= kPlanesSmem;
+  if (plan.resident) {
+    int st = (int)((kPlanesSmem - fixed - b_all) / p.plane_bytes);
+    p.a_stages = st > 4 ? 4 : st;
+    p.b_stages = 1;
+    p.chunk = 0;
+    plan.smem = fixed + b_all + (size_t)p.a_stages * p.plane_bytes;
+    return true;
+  }
+  const size_t stage = (size_t)p.planes * p.plane_bytes;
+  p.a_stages = 2;
+  if (fixed + 2 * stage + 2 * b_tile > kPlanesSmem)
+    return false;
+  int st = (int)((kPlanesSmem - fixed - 2 * stage) / b_tile);
+  p.b_stages = st > 6 ? 6 : st;
+  p.chunk = k_chunk_blocks(p.planes * 4);
+  plan.smem = fixed + 2 * stage + (size_t)p.b_stages * b_tile;
+  return true;
+}
+
+template <int BN, int PG, bool kResident, bool kF16>
+int launch_planes_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const PlanesPlan &plan, cudaStream_t st) {
+  auto kernel = conv_planes_tcgen05_kernel<BN, PG, kResident, kF16>;
+  static bool configured[64];
+  int dev = 0;
+  NB_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63]) {
+    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanesSmem));
+    configured[dev & 63] = true;
+  }
+  int *status = nullptr;
+  NB_TRY(device_status_word(&status));
+  const int tiles = plan.p.num_tiles();
+  kernel<<<tiles < sm_count() ? tiles : sm_count(), kGemmThreads, plan.smem, st>>>(ma, mb, plan.p, status);
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+// act: [planes][N][Hin][Win][ctot], side: [total_maps][taps * k_slots].
+int launch_planes(const PlanesPlan &plan, const void *act, int Hin, int Win, int64_t ctot, const void *side, int taps,
+                  bool f16, cudaStream_t st) {
+  const ConvPlanesProblem &p = plan.p;
+  CUtensorMap ma, mb;
+  const uint64_t dims[5] = {(uint64_t)ctot, (uint64_t)Win, (uint64_t)Hin, (uint64_t)p.Nimg, (uint64_t)p.planes};
+  const uint64_t strides[4] = {(uint64_t)ctot * 2, (uint64_t)ctot * 2 * Win, (uint64_t)ctot * 2 * Win * Hin,
+                               (uint64_t)ctot * 2 * Win * Hin * p.Nimg};
+  const uint32_t box[5] = {64, (uint32_t)p.wp, (uint32_t)p.hp, 1, 1};
+  NB_TRY(encode_tiled(&ma, 0, 5, act, dims, strides, box, nullptr, kRowBytes));
+  const int64_t pitch = (int64_t)taps * p.k_slots;
+  NB_TRY(make_operand_map(&mb, side, false, pitch, pitch, p.total_maps, 1, plan.bn));
+  if (f16) {
+    NB_CHECK(p.planes == 2, NB200_EVALUE, "fp16 planes come in pairs");
+    if (plan.resident)
+      return plan.bn == 64 ? launch_planes_kernel<64, 1, true, true>(ma, mb, plan, st)
+                           : launch_planes_kernel<128, 1, true, true>(ma, mb, plan, st);
+    return plan.bn == 64 ? launch_planes_kernel<64, 2, false, true>(ma, mb, plan, st)
+                         : launch_planes_kernel<128, 2, false, true>(ma, mb, plan, st);
+  }
+  NB_CHECK(p.planes == 3, NB200_EVALUE, "bf16 planes come in threes");
+  if (plan.resident)
+    return plan.bn == 64 ? launch_planes_kernel<64, 1, true, false>(ma, mb, plan, st)
+                         : launch_planes_kernel<128, 1, true, false>(ma, mb, plan, st);
+  return plan.bn == 64 ? launch_planes_kernel<64, 3, false, false>(ma, mb, plan, st)
+                       : launch_planes_kernel<128, 3, false, false>(ma, mb, plan, st);
+}
+
+// Tasks and boxes of the weight gradient of one geometry; false: the kernel does not apply.
+bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t &smem) {
+  const int taps = g.kh * g.kw;
+  if (taps > kWgradMaxTaps || g.Wo > 256)
+    return false;
+  auto residue = [](int t, int d, int pad, int s) { return ((t * d - pad) % s + s) % s; };
+  auto offset = [&](int t, int d, int pad, int s) { return (t * d - pad - residue(t, d, pad, s)) / s; };
+  // offsets grow with the tap
+  p.y0 = offset(0, g.dh, g.ph, g.sh);
+  p.x0 = offset(0, g.dw, g.pw, g.sw);
+  const int span_y = offset(g.kh - 1, g.dh, g.ph, g.sh) - p.y0;
+  p.wp = g.Wo + offset(g.kw - 1, g.dw, g.pw, g.sw) - p.x0;
+  if (p.wp * g.sw > 256)
+    return false;
+  p.sy = g.sh;
+  p.sx = g.sw;
+  p.groups = g.group;
+  p.o_blocks = (g.Kog + 63) / 64;
+  p.c_blocks = (g.Cg + 63) / 64;
+  p.x_planes = x_planes;
+  int n = 0, groups = 0;
+  p.tg_tap[0] = p.tg_pair[0] = 0;
+  for (int ry = 0; ry < g.sh; ++ry)
+    for (int rx = 0; rx < g.sw; ++rx) {
+      int in_group = 0;
+      for (int ky = 0; ky < g.kh; ++ky)
+        for (int kx = 0; kx < g.kw; ++kx) {
+          if (residue(ky, g.dh, g.ph, g.sh) != ry || residue(kx, g.dw, g.pw, g.sw) != rx)
+            continue;
+          if (in_group == 0 || in_group == kWgradTaps) {
+            p.tg_ry[groups] = ry;
+            p.tg_rx[groups] = rx;
+            ++groups;
+            in_group = 0;
+          }
+          p.tap_row[n] = (offset(ky, g.dh, g.ph, g.sh) - p.y0) * p.wp + offset(kx, g.dw, g.pw, g.sw) - p.x0;
+          p.tap_id[n++] = ky * g.kw + kx;
+          ++in_group;
+          p.tg_tap[groups] = n;
+          p.tg_pair[groups] = p.tg_pair[groups - 1] + (in_group + 1) / 2;
+        }
+    }
+  p.tap_groups = groups;
+  // Box height: as few accumulation steps per image as possible, where a box costs about one step beside its own, and
+  // two boxes must fit in shared memory.
+  const int max_shift = span_y * p.wp + p.wp - g.Wo;
+  double best = 0.0;
+  p.h_box = 0;
+  for (int h = 1; h <= g.Ho && h + span_y <= 256 / g.sh; ++h) {
+    const int k16 = (h * p.wp + 15) / 16, x_rows = (max_shift + 16 * k16 + 7) / 8 * 8;
+    const size_t stage = (size_t)(3 * 16 * k16 + x_planes * x_rows) * kRowBytes;
+    if (2 * stage + 1024 > kPlanesSmem || k16 > 96)
+      break;
+    const double cost = (double)((g.Ho + h - 1) / h) * (k16 + 1);
+    if (p.h_box == 0 || cost < best) {
+      best = cost;
+      p.h_box = h;
+    }
+  }
+  if (p.h_box == 0)
+    return false;
+  p.hp = p.h_box + span_y;
+  p.k16 = (p.h_box * p.wp + 15) / 16;
+  p.dy_bytes = 16 * p.k16 * kRowBytes;
+  p.x_bytes = (max_shift + 16 * p.k16 + 7) / 8 * 8 * kRowBytes;
+  const size_t stage = 3 * (size_t)p.dy_bytes + (size_t)x_planes * p.x_bytes;
+  const int fit = (int)((kPlanesSmem - 1024) / stage);
+  p.stages = fit < kWgradMaxStages ? fit : kWgradMaxStages;
+  smem = 1024 + p.stages * stage;
+  p.flush = 96 / p.k16;
+  p.tiles_h = (g.Ho + p.h_box - 1) / p.h_box;
+  const int64_t boxes = (int64_t)g.N * p.tiles_h, group_work = boxes * p.tg_pair[groups];
+  const int64_t work = group_work * p.groups * p.o_blocks * p.c_blocks;
+  if (work >= (1ll << 30))
+    return false;
+  p.boxes = (int)boxes;
+  p.group_work = (int)group_work;
+  p.work = (int)work;
+  p.per_block = (int)((work + sm_count() - 1) / sm_count());
+  p.per_block = p.per_block < 4 ? 4 : p.per_block;
+  return true;
+}
+
+// Input gradient (dx) and weight gradient (dw) from the channel-last pieces of dy and x, for weights exact in one bf16
+// piece. *did_dx / *did_dw: which of the two it computed (the geometries its kernels do not take are left to the caller).
+int planes_backward(const float *x, const float *wb, const float *alpha, const float *dy, float *dx, float *dw,
+                    const ConvGeometry &g, int accum_dx, int accum_dw, float act_delta, cudaStream_t st, bool *did_dx,
+                    bool *did_dw) {
+  const int taps = g.kh * g.kw, k_pad_g = (int)round_up(g.Kog, 16), c_pad_g = (int)round_up(g.Cg, 16);
+  // activations that are multiples of act_delta with |code| <= 127 are exact in one bf16 piece
+  const int x_planes = act_delta > 0.0f ? 1 : 3;
+  PlanesPlan plan{};
+  ConvPlanesProblem &p = plan.p;
+  if (dx) {
+    p.Nimg = g.N;
+    p.maps = g.Cg;
+    p.total_maps = g.C;
+    p.groups = g.group;
+    p.H = g.H;
+    p.W = g.W;
+    p.planes = 3;
+    const PlanesAxis ay{g.kh, g.dh, g.ph, g.sh, true}, ax{g.kw, g.dw, g.pw, g.sw, true};
+    *did_dx = plan_planes(plan, ay, ax, g.Kog);
+  }
+  ConvWgradProblem q{};
+  size_t smem_w = 0;
+  if (dw)
+    *did_dw = plan_wgrad(q, g, x_planes, smem_w);
+  if (!*did_dx && !*did_dw)
+    return NB200_OK;
+  const int64_t k_tot = (int64_t)g.group * k_pad_g < 64 ? 64 : (int64_t)g.group * k_pad_g;
+  const int64_t c_tot = (int64_t)g.group * c_pad_g < 64 ? 64 : (int64_t)g.group * c_pad_g;
+  const bool two = *did_dx && *did_dw && alpha; // dy * alpha for dx, dy for dw
+  const size_t dy_bytes = round_up((size_t)3 * g.N * g.Ho * g.Wo * k_tot * 2, 1024);
+  const size_t x_bytes = *did_dw ? round_up((size_t)x_planes * g.N * g.H * g.W * c_tot * 2, 1024) : 0;
+  const size_t side_bytes = *did_dx ? round_up((size_t)g.C * taps * p.k_slots * 2, 1024) : 0;
+  const int grid_w = *did_dw ? (q.work + q.per_block - 1) / q.per_block : 0;
+  const size_t slot_bytes = *did_dw ? (size_t)(grid_w + q.tasks()) * kWgradSlotFloats * 4 : 0;
+  AsyncScratch scratch(st);
+  NB_TRY(scratch.alloc((two ? 2 : 1) * dy_bytes + x_bytes + side_bytes + slot_bytes));
+  uint8_t *at = static_cast<uint8_t *>(scratch.p);
+  uint8_t *dys = at, *dyp = two ? at + dy_bytes : at; // pieces of dy * alpha (or dy) and of dy
+  at += (two ? 2 : 1) * dy_bytes;
+  uint8_t *xp = at, *side = xp + x_bytes;
+  q.slots = reinterpret_cast<float *>(side + side_bytes);
+  const bool scaled = *did_dx && alpha;
+  NB_TRY(nhwc_pieces(dy, g.N, g.Ko, g.Ho * g.Wo, g.group, g.Kog, k_pad_g, (int)k_tot, 3, scaled ? alpha : nullptr,
+                     scaled ? dys : nullptr, scaled ? (two ? dyp : nullptr) : dyp, st));
+  if (*did_dx) {
+    p.c_group_stride = k_pad_g;
+    p.y = dx;
+    p.accumulate = accum_dx;
+    NB_TRY(transpose_binary_weights(wb, g.Ko, g.Cg, taps, g.group, p.k_slots, side, st));
+    NB_TRY(launch_planes(plan, dys, g.Ho, g.Wo, k_tot, side, taps, false, st));
+  }
+  if (!*did_dw)
+    return NB200_OK;
+  NB_TRY(nhwc_pieces(x, g.N, g.C, g.H * g.W, g.group, g.Cg, c_pad_g, (int)c_tot, x_planes, nullptr, nullptr, xp, st));
+  q.k_stride = k_pad_g;
+  q.c_stride = c_pad_g;
+  CUtensorMap mx, md;
+  {
+    const uint64_t dims[5] = {(uint64_t)c_tot, (uint64_t)g.W, (uint64_t)g.H, (uint64_t)g.N, (uint64_t)x_planes};
+    const uint64_t strides[4] = {(uint64_t)c_tot * 2, (uint64_t)c_tot * 2 * g.W, (uint64_t)c_tot * 2 * g.W * g.H,
+                                 (uint64_t)c_tot * 2 * g.W * g.H * g.N};
+    const uint32_t box[5] = {64, (uint32_t)(q.wp * g.sw), (uint32_t)(q.hp * g.sh), 1, 1};
+    const uint32_t estr[5] = {1, (uint32_t)g.sw, (uint32_t)g.sh, 1, 1};
+    NB_TRY(encode_tiled(&mx, 0, 5, xp, dims, strides, box, estr, kRowBytes));
+  }
+  {
+    const uint64_t dims[5] = {(uint64_t)k_tot, (uint64_t)g.Wo, (uint64_t)g.Ho, (uint64_t)g.N, 3};
+    const uint64_t strides[4] = {(uint64_t)k_tot * 2, (uint64_t)k_tot * 2 * g.Wo, (uint64_t)k_tot * 2 * g.Wo * g.Ho,
+                                 (uint64_t)k_tot * 2 * g.Wo * g.Ho * g.N};
+    const uint32_t box[5] = {64, (uint32_t)q.wp, (uint32_t)q.h_box, 1, 1};
+    NB_TRY(encode_tiled(&md, 0, 5, dyp, dims, strides, box, nullptr, kRowBytes));
+  }
+  auto kernel = x_planes == 1 ? conv_wgrad_tcgen05_kernel<1> : conv_wgrad_tcgen05_kernel<3>;
+  static bool configured[64][2];
+  int dev = 0;
+  NB_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63][x_planes == 3]) {
+    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanesSmem));
+    configured[dev & 63][x_planes == 3] = true;
+  }
+  int *status = nullptr;
+  NB_TRY(device_status_word(&status));
+  kernel<<<grid_w, kGemmThreads, smem_w, st>>>(mx, md, q, status);
+  NB_LAUNCH_CHECK();
+  conv_wgrad_finish_kernel<<<dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), 256, 0, st>>>(q, g.Kog, g.Cg, taps, dw, accum_dw);
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
 // full_precision: the weights are arbitrary fp32 values (three bf16 pieces, the products that matter at fp32
 // resolution) instead of values exact in one bf16 piece
 int conv_input_grad(const float *wb, const float *alpha, const float *dy, float *dx, const ConvGeometry &g,
@@ -424,12 +749,16 @@ int convolution_backward(const float *x, const float *w_exact, const float *alph
                          float act_delta, cudaStream_t st, bool full_precision_weights = false) {
   NB_TRY(check_geometry(g));
   NB_CHECK(dy != nullptr, NB200_EVALUE, "dy is NULL");
-  if (dx) {
-    NB_CHECK(w_exact != nullptr, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
+  NB_CHECK(!dx || w_exact != nullptr, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
+  NB_CHECK(!dw || x != nullptr, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
+  bool did_dx = false, did_dw = false;
+  if ((dx && !full_precision_weights) || dw)
+    NB_TRY(planes_backward(x, w_exact, alpha, dy, full_precision_weights ? nullptr : dx, dw, g, accum_dx, accum_dw,
+                           act_delta, st, &did_dx, &did_dw));
+  if (dx && !did_dx) {
     NB_TRY(conv_input_grad(w_exact, alpha, dy, dx, g, accum_dx, st, full_precision_weights));
   }
-  if (dw) {
-    NB_CHECK(x != nullptr, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
+  if (dw && !did_dw) {
     NB_TRY(conv_weight_grad(x, dy, dw, g, accum_dw, act_delta, st));
   }
   if (db) {

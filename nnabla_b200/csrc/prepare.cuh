@@ -53,6 +53,13 @@ int fxp8_operands(const float *x, int64_t M, int K, int64_t Kp, float delta_x, i
                   float delta_w, int8_t *wt, cudaStream_t st);
 
 // ---- convolution backward (prepare_backward.cu) ------------------------------
+// src [N][C][HW] fp32 -> channel-last bf16 pieces [planes][N][HW][ctot] (planes = 3 or 1), of src * chan_scale[c] in
+// `scaled` and of src in `plain` (either may be NULL).
+int nhwc_pieces(const float *src, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, int planes,
+                const float *chan_scale, void *scaled, void *plain, cudaStream_t st);
+// wb [Ko][Cg][taps] of values exact in bf16 -> [groups * Cg][taps][k_slots] bf16, zero padded.
+int transpose_binary_weights(const float *wb, int Ko, int Cg, int taps, int groups, int k_slots, void *side,
+                             cudaStream_t st);
 // dy [N][Ko][Ho][Wo] -> 3 bf16 planes [N][Hs][Ws][ctot] (pre-zeroed by the caller):
 // pixel (oy, ox) at (oy * sh, ox * sw), map o of group g at slot g * k_pad_g + o - g * Kog,
 // multiplied by chan_scale[o] first when given.

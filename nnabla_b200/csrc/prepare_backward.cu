@@ -11,6 +11,7 @@
 //   bias gradient:   sums of dy over batch and pixels  -> channel_sums
 #include <cuda_bf16.h>
 
+#include "pdl.cuh"
 #include "prepare.cuh"
 
 namespace nb200 {
@@ -63,6 +64,93 @@ __global__ void __launch_bounds__(256) dy_to_nhwc_stuffed_kernel(const float *__
       out[plane_stride + dst] = m;
       out[2 * plane_stride + dst] = l;
     }
+  }
+}
+
+// src [N][C][HW] fp32 -> channel-last bf16 planes [planes][N][HW][ctot]: the pieces (hi, mid, lo) of every value, channel
+// c of group g at slot g * c_pad_g + c - g * Cg, all other slots zero. `scaled` receives the pieces of
+// src * chan_scale[c] (one rounding: dy * alpha), `plain` those of src itself; either may be NULL, so that dy is read
+// once for both gradients. HBM-bound: 4 B read and 2 B per piece written per value. Blocks of 64 pixels x 64 slots, a
+// thread converts four slots of four pixels; a pixel's row of 64 slots is transposed through shared memory in 16-byte
+// chunks (XORed with the pixel quad, at most two lanes to a bank) and leaves as 128 bytes.
+template <bool kVec, int PLANES>
+__global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restrict__ src, int C, int HW, int groups, int Cg,
+                                                          int c_pad_g, int ctot, const float *__restrict__ chan_scale,
+                                                          __nv_bfloat16 *__restrict__ scaled,
+                                                          __nv_bfloat16 *__restrict__ plain, int64_t plane_stride) {
+  __shared__ uint4 tile[PLANES][64][8];
+  pdl_wait();
+  pdl_trigger();
+  const int n = blockIdx.z, p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
+  const int px4 = threadIdx.x & 15, chq = threadIdx.x >> 4;
+  const int p = p0 + 4 * px4, dq = d0 + 4 * chq;
+  const int g = dq / c_pad_g, cc0 = dq - g * c_pad_g; // c_pad_g is a multiple of 16: one group for the four slots
+  const bool ok = dq < ctot && g < groups;
+  const float *base = src + ((int64_t)n * C + (g * Cg + cc0)) * HW + p;
+  float v[4][4], f[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const bool live = ok && cc0 + r < Cg;
+    f[r] = live && scaled && chan_scale ? __ldg(chan_scale + g * Cg + cc0 + r) : 1.0f;
+    if (kVec) {
+      const float4 q = live && p < HW ? __ldcs(reinterpret_cast<const float4 *>(base + (int64_t)r * HW))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[r][0] = q.x, v[r][1] = q.y, v[r][2] = q.z, v[r][3] = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        v[r][k] = live && p + k < HW ? __ldcs(base + (int64_t)r * HW + k) : 0.0f;
+    }
+  }
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+    __nv_bfloat16 *out = pass == 0 ? scaled : plain;
+    if (!out)
+      continue;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      __nv_bfloat16 h[4], m[4], l[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        split3(pass == 0 && chan_scale ? __fmul_rn(v[r][k], f[r]) : v[r][k], h[r], m[r], l[r]);
+      const int chunk = (chq >> 1) ^ (px4 & 7);
+#pragma unroll
+      for (int pl = 0; pl < PLANES; ++pl) {
+        const __nv_bfloat16 *s = pl == 0 ? h : (pl == 1 ? m : l);
+        const __nv_bfloat162 a = __halves2bfloat162(s[0], s[1]), b = __halves2bfloat162(s[2], s[3]);
+        reinterpret_cast<uint2 *>(&tile[pl][4 * px4 + k][chunk])[chq & 1] =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < 2; ++it) {
+      const int i = threadIdx.x + 256 * it, pp = i >> 3, c = i & 7;
+      const int pix = p0 + pp, d = d0 + 8 * c;
+      if (pix < HW && d < ctot) {
+        const int64_t dst = ((int64_t)n * HW + pix) * ctot + d;
+#pragma unroll
+        for (int pl = 0; pl < PLANES; ++pl)
+          *reinterpret_cast<uint4 *>(out + pl * plane_stride + dst) = tile[pl][pp][c ^ ((pp >> 2) & 7)];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// wb [Ko][Cg][kh][kw] of +-1 (exact in bf16) -> side [C][kh * kw][k_slots] bf16, row g * Cg + c, maps of the group
+// innermost, zero past them: the weights of the input gradient, one block per row.
+__global__ void __launch_bounds__(256) transpose_binary_weights_kernel(const float *__restrict__ wb, int Cg, int taps,
+                                                                       int Kog, int k_slots,
+                                                                       __nv_bfloat16 *__restrict__ side) {
+  pdl_wait();
+  pdl_trigger();
+  const int row = blockIdx.x, g = row / Cg, c = row - g * Cg;
+  const float *src = wb + ((int64_t)g * Kog * Cg + c) * taps;
+  __nv_bfloat16 *dst = side + (int64_t)row * taps * k_slots;
+  for (int i = threadIdx.x; i < taps * k_slots; i += 256) {
+    const int t = i / k_slots, o = i - t * k_slots;
+    dst[i] = o < Kog ? __float2bfloat16_rn(__ldg(src + (int64_t)o * Cg * taps + t)) : __float2bfloat16_rn(0.0f);
   }
 }
 
@@ -195,6 +283,28 @@ int dy_to_nhwc_stuffed(const float *dy, int N, int Ko, int Ho, int Wo, int group
   dy_to_nhwc_stuffed_kernel<<<grid, 256, 0, st>>>(dy, Ko, Ho, Wo, groups, Kog, k_pad_g, ctot, Hs, Ws, sh, sw,
                                                   chan_scale, reinterpret_cast<__nv_bfloat16 *>(out),
                                                   (int64_t)N * Hs * Ws * ctot);
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+int nhwc_pieces(const float *src, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, int planes,
+                const float *chan_scale, void *scaled, void *plain, cudaStream_t st) {
+  NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
+  const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
+  const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  auto kernel = planes == 3 ? (vec ? nhwc_pieces_kernel<true, 3> : nhwc_pieces_kernel<false, 3>)
+                            : (vec ? nhwc_pieces_kernel<true, 1> : nhwc_pieces_kernel<false, 1>);
+  NB_CUDA(launch_dependent(kernel, grid, dim3(256), 0, st, src, C, HW, groups, Cg, c_pad_g, ctot, chan_scale,
+                           static_cast<__nv_bfloat16 *>(scaled), static_cast<__nv_bfloat16 *>(plain),
+                           (int64_t)N * HW * ctot));
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+int transpose_binary_weights(const float *wb, int Ko, int Cg, int taps, int groups, int k_slots, void *side,
+                             cudaStream_t st) {
+  NB_CUDA(launch_dependent(transpose_binary_weights_kernel, dim3(groups * Cg), dim3(256), 0, st, wb, Cg, taps, Ko / groups,
+                           k_slots, static_cast<__nv_bfloat16 *>(side)));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -1,0 +1,43 @@
+"""Convolution gradients at the edges of the pixel-major kernels (boxes, tap groups, classes of a stride, channel and
+map blocks) against float64 convolutions: dx and dW within 1e-5 of their RMS."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# batch, channels, height, width, maps, kernel, pad, stride, dilation, group
+CASES = [
+    (1, 64, 64, 64, 64, 3, 1, 1, 1, 1),     # the widest rows of a box
+    (2, 130, 13, 61, 70, 3, 1, 1, 1, 1),    # several channel and map blocks, ragged rows
+    (3, 48, 11, 9, 40, 5, 2, 1, 1, 1),      # 25 taps: seven tap groups
+    (5, 16, 29, 31, 200, 3, 1, 2, 1, 1),    # four classes of a stride, two column tiles
+    (2, 20, 23, 17, 33, 3, 2, 3, 2, 1),     # classes without taps
+    (4, 96, 10, 10, 64, 1, 0, 2, 1, 1),     # one tap, three empty classes
+    (2, 72, 14, 15, 136, 3, 0, 1, 1, 2),    # groups whose slots are padded
+    (300, 8, 3, 3, 8, 3, 1, 1, 1, 1),       # many tiny images
+    (1, 24, 7, 120, 16, 3, 1, 1, 1, 1),     # rows near the width limit
+]
+
+
+@pytest.mark.parametrize("n,c,h,w,o,k,pad,stride,dil,group", CASES)
+@pytest.mark.parametrize("delta", [None, 2.0 ** -4])
+def test_gradients(n, c, h, w, o, k, pad, stride, dil, group, delta):
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(n + c)
+    x = torch.randn(n, c, h, w, device="cuda", generator=g)
+    if delta:
+        x = (x / delta).round().clamp(-127, 127) * delta
+    wb = torch.randn(o, c // group, k, k, device="cuda", generator=g).sign()
+    alpha = torch.rand(o, device="cuda", generator=g) + 0.5
+    geometry = dict(pad=(pad, pad), stride=(stride, stride), dilation=(dil, dil), group=group)
+    xd, wd = x.double().requires_grad_(), (wb.double() * alpha.double().view(-1, 1, 1, 1)).requires_grad_()
+    y = torch.nn.functional.conv2d(xd, wd, None, stride, pad, dil, group)
+    dy = torch.randn(*y.shape, device="cuda", generator=g)
+    y.backward(dy.double())
+    dx, dw, db = F.binary_weight_convolution_backward(x, wb, alpha, dy, fixed_point_delta=delta, **geometry)
+    dx0, dw0 = torch.ones_like(x), torch.ones_like(wb)
+    F.binary_weight_convolution_backward(x, wb, alpha, dy, propagate_down=(True, True, False), accum=(True, True, False),
+                                         grads=(dx0, dw0, None), fixed_point_delta=delta, **geometry)
+    F.check_device_status()
+    for got, want in ((dx, xd.grad), (dw, wd.grad), (dx0 - 1, xd.grad), (dw0 - 1, wd.grad), (db, dy.double().sum((0, 2, 3)))):
+        assert (got.double() - want).norm() <= 1e-5 * want.norm() + 1e-6 * want.numel() ** 0.5
