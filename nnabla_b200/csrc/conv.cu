@@ -392,8 +392,9 @@ bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, i
   if (fixed + 2 * stage + 2 * b_tile > kPlanesSmem)
     return false;
   int st = (int)((kPlanesSmem - fixed - 2 * stage) / b_tile);
-  p.b_stages = st > 6 ? 6 : st;
-  p.chunk = k_chunk_blocks(p.planes * 4);
+  p.b_stages = st >= 6 ? 6 : (st >= 4 ? 4 : 2); // even: they alternate between the issuing warps
+  // two accumulators share a chunk; half the usual length each: no step of a strided gradient multiplies zeros here
+  p.chunk = 2 * k_chunk_blocks(p.planes * 8);
   plan.smem = fixed + 2 * stage + (size_t)p.b_stages * b_tile;
   return true;
 }
@@ -411,7 +412,7 @@ int launch_planes_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const Pla
   int *status = nullptr;
   NB_TRY(device_status_word(&status));
   const int tiles = plan.p.num_tiles();
-  kernel<<<tiles < sm_count() ? tiles : sm_count(), kGemmThreads, plan.smem, st>>>(ma, mb, plan.p, status);
+  kernel<<<tiles < sm_count() ? tiles : sm_count(), kPlanesThreads, plan.smem, st>>>(ma, mb, plan.p, status);
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -487,15 +488,16 @@ bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t
         }
     }
   p.tap_groups = groups;
-  // Box height: as few accumulation steps per image as possible, where a box costs about one step beside its own, and
-  // two boxes must fit in shared memory.
+  // Box height: as few accumulation steps per image as possible, where a box costs about one step beside its own. Three
+  // boxes must fit in shared memory when a box has one plane of x (its MMAs take about as long as its copies: with two
+  // boxes the MMAs waited), two when it has three.
   const int max_shift = span_y * p.wp + p.wp - g.Wo;
   double best = 0.0;
   p.h_box = 0;
   for (int h = 1; h <= g.Ho && h + span_y <= 256 / g.sh; ++h) {
     const int k16 = (h * p.wp + 15) / 16, x_rows = (max_shift + 16 * k16 + 7) / 8 * 8;
     const size_t stage = (size_t)(3 * 16 * k16 + x_planes * x_rows) * kRowBytes;
-    if (2 * stage + 1024 > kPlanesSmem || k16 > 96)
+    if ((x_planes == 1 ? 3 : 2) * stage + 1024 > kPlanesSmem || k16 > 96)
       break;
     const double cost = (double)((g.Ho + h - 1) / h) * (k16 + 1);
     if (p.h_box == 0 || cost < best) {

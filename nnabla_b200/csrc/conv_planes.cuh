@@ -15,7 +15,9 @@
 // fetched a box of pixels per filter tap: 540 us for the input gradient of a 64 -> 64 3 x 3 layer on [128, 64, 56, 56],
 // 71 us of MMAs at the rates above.
 //
-// Warp 0 loads (TMA), warp 1 issues the MMAs, eight epilogue warps store. A stage of the pixel ring is the input box
+// Warp 0 loads (TMA), two warps issue the MMAs, eight epilogue warps store. The issuing warps take alternate tiles
+// (kResident) or alternate weight tiles into accumulators of their own: a thread that decodes a tile, waits for
+// barriers and comes back to the head of its unrolled loop leaves the tensor core idle, 27 % of the time with one. A stage of the pixel ring is the input box
 // of PG planes of one 64-channel block; the weights of one tap and channel block come through a second ring
 // (kResident: all of them are loaded once). With kResident the planes come one after the other, smallest pieces
 // first, which also keeps the number of accumulation steps at full magnitude down; otherwise the planes of a box are
@@ -27,6 +29,7 @@ namespace nb200 {
 
 constexpr int kPlanesMaxTaps = 64;
 constexpr int kPlanesMaxStages = 8;
+constexpr int kPlanesThreads = kGemmThreads + 32; // the second issuing warp stands behind the epilogue warps
 
 struct ConvPlanesProblem {
   int Nimg, maps, total_maps, groups; // output maps per group and in all
@@ -41,7 +44,7 @@ struct ConvPlanesProblem {
   int k_slots;                        // weight slots per tap
   int plane_bytes;                    // of one plane's box in shared memory
   int planes;                         // planes of A
-  int chunk;                          // weight tiles (tap, channel block) per accumulation in tensor memory, 0 = all
+  int chunk;                          // weight tiles (tap, channel block) per accumulation in tensor memory, even; 0 = all
   int a_stages, b_stages;
   int class_tap[17];                  // taps of class k: [class_tap[k], class_tap[k + 1])
   int tap_row[kPlanesMaxTaps];        // first row of the box that tap reads
@@ -53,12 +56,13 @@ struct ConvPlanesProblem {
 };
 
 template <int BN, int PG, bool kResident, bool kF16>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kPlanesThreads, 1)
     conv_planes_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ ConvPlanesProblem prob, int *status) {
   static_assert(BN == 64 || BN == 128, "column tiles of 64 or 128 maps");
   constexpr uint32_t kBBytes = BN * kRowBytes;
-  constexpr uint32_t kTmemCols = 2 * BN;
+  constexpr int kAccs = kResident ? 1 : 2; // accumulators of a chunk: one per issuing warp, which share its tiles
+  constexpr uint32_t kTmemCols = 2 * kAccs * BN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t stage_bytes = (uint32_t)PG * prob.plane_bytes;
@@ -79,12 +83,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   if (threadIdx.x == 0) {
     for (int i = 0; i < kPlanesMaxStages; ++i) {
       ptx::mbar_init(a_full + i, 1);
-      ptx::mbar_init(a_empty + i, 1);
+      ptx::mbar_init(a_empty + i, 2); // both issuers: a barrier's phase must not run past one that has not seen it
       ptx::mbar_init(b_full + i, 1);
       ptx::mbar_init(b_empty + i, 1);
     }
     for (int b = 0; b < 2; ++b) {
-      ptx::mbar_init(tmem_full + b, 1);
+      ptx::mbar_init(tmem_full + b, kAccs);
       ptx::mbar_init(tmem_empty + b, kEpilogueWarps);
     }
     abort_word = 0;
@@ -176,65 +180,79 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
       }
     }
-  } else if (warp == 1) {
-    // -------------------------------------------------------------- MMA issuer
+  } else if (warp == 1 || warp == 2 + kEpilogueWarps) {
+    // ------------------------------------------------------------- MMA issuers
+    const int who = warp == 1 ? 0 : 1;
     if (ptx::elect_one()) {
-      int as = 0, bs = 0, local = 0;
+      int as = 0, bs = 0, local = 0; // stages and chunk (or tile) counted over both issuers' work
       uint32_t aphase = 0, bphase = 0;
       bool ok = true;
       const uint32_t idesc = ptx::make_idesc(1u, kF16 ? 0u : 1u, kTileM, BN);
-      const uint64_t desc0 = ptx::smem_desc_k(0, kRowBytes);
-      const uint32_t hi = (uint32_t)(desc0 >> 32);
+      const uint32_t hi = (uint32_t)(ptx::smem_desc_k(0, kRowBytes) >> 32);
       const uint32_t a_lo = ptx::smem_u32(a_base) >> 4, b_lo = ptx::smem_u32(b_base) >> 4; // below 2^14
-      if (kResident && (int)blockIdx.x < num_tiles) {
-        if (!ptx::mbar_wait(b_full, 0u, abort_flag)) {
+      auto next_a = [&]() {
+        if (++as == prob.a_stages) {
+          as = 0;
+          aphase ^= 1u;
+        }
+      };
+      uint32_t accumulate = 0, d_tmem = 0;
+      auto open_chunk = [&]() { // waits for the accumulator of the next chunk
+        const int buf = local & 1;
+        if (!ptx::mbar_wait(tmem_empty + buf, ((uint32_t)(local >> 1) & 1u) ^ 1u, abort_flag)) {
           gave_up(kStatusMmaTimeout);
-          ok = false;
+          return false;
         }
         ptx::tc_fence_after_sync();
-      }
+        d_tmem = tmem_base + (uint32_t)((buf * kAccs + (kResident ? 0 : who)) * BN);
+        accumulate = 0;
+        return true;
+      };
+      auto wait = [&](uint64_t *bar, uint32_t phase) {
+        if (!ptx::mbar_wait(bar, phase, abort_flag)) {
+          gave_up(kStatusMmaTimeout);
+          return false;
+        }
+        ptx::tc_fence_after_sync();
+        return true;
+      };
+      auto issue = [&](uint32_t a_row16, uint32_t b16) {
+#pragma unroll
+        for (int p = 0; p < PG; ++p)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            ptx::mma_bf16(d_tmem, ((uint64_t)hi << 32) | (a_row16 + p * ((uint32_t)prob.plane_bytes >> 4) + 2 * k),
+                          ((uint64_t)hi << 32) | (b16 + 2 * k), idesc, accumulate);
+            accumulate = 1;
+          }
+      };
+      if (kResident && (int)blockIdx.x < num_tiles)
+        ok = wait(b_full, 0u);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileAt t = decode(tile);
         const int tap0 = prob.class_tap[t.cls], tap1 = prob.class_tap[t.cls + 1];
         if (tap0 == tap1)
           continue;
-        int in_chunk = 0;
-        uint32_t accumulate = 0, d_tmem = 0;
-        auto open_chunk = [&]() { // waits for the accumulator of the next chunk
-          const int buf = local & 1;
-          if (!ptx::mbar_wait(tmem_empty + buf, ((uint32_t)(local >> 1) & 1u) ^ 1u, abort_flag)) {
-            gave_up(kStatusMmaTimeout);
-            return false;
-          }
-          ptx::tc_fence_after_sync();
-          d_tmem = tmem_base + (uint32_t)(buf * BN);
-          accumulate = 0;
-          in_chunk = 0;
-          return true;
-        };
-        ok = open_chunk();
-        for (int cb = 0; cb < prob.cblocks && ok; ++cb)
-          for (int pg = 0; pg < plane_groups && ok; ++pg) {
-            if (!ptx::mbar_wait(a_full + as, aphase, abort_flag)) {
-              gave_up(kStatusMmaTimeout);
-              ok = false;
-              break;
+        if constexpr (kResident) {
+          if ((local & 1) != who) { // the other issuer's tile: its boxes are released as soon as they have come
+            for (int i = 0; i < prob.cblocks * plane_groups; ++i) {
+              if (!(ok = wait(a_full + as, aphase)))
+                break;
+              ptx::mbar_arrive(a_empty + as);
+              next_a();
             }
-            ptx::tc_fence_after_sync();
-            const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
-            auto issue = [&](uint32_t a_row16, uint32_t b16) {
-#pragma unroll
-              for (int p = 0; p < PG; ++p)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  ptx::mma_bf16(d_tmem, ((uint64_t)hi << 32) | (a_row16 + p * ((uint32_t)prob.plane_bytes >> 4) + 2 * k),
-                                ((uint64_t)hi << 32) | (b16 + 2 * k), idesc, accumulate);
-                  accumulate = 1;
-                }
-            };
-            if (kResident) {
+            ++local;
+            continue;
+          }
+          ok = open_chunk();
+          for (int cb = 0; cb < prob.cblocks && ok; ++cb)
+            for (int pg = 0; pg < plane_groups; ++pg) {
+              if (!(ok = wait(a_full + as, aphase)))
+                break;
+              const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
+              // in batches: the descriptors of three taps before their MMAs
               int tap = tap0;
-              for (; tap + 3 <= tap1; tap += 3) { // in batches: the descriptors of several taps before their MMAs
+              for (; tap + 3 <= tap1; tap += 3) {
                 uint32_t off[3];
 #pragma unroll
                 for (int u = 0; u < 3; ++u)
@@ -246,35 +264,42 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
               for (; tap < tap1; ++tap)
                 issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4),
                       b_lo + (uint32_t)(tap * prob.cblocks + cb) * (kBBytes >> 4));
-            } else {
+              ptx::mma_commit(a_empty + as); // the boxes are free once these MMAs have read them
+              next_a();
+            }
+        } else {
+          // Weight stages alternate between the issuers (their number is even), so that each sees every phase of its own.
+          int in_chunk = 0;
+          ok = open_chunk();
+          for (int cb = 0; cb < prob.cblocks && ok; ++cb)
+            for (int pg = 0; pg < plane_groups && ok; ++pg) {
+              if (!(ok = wait(a_full + as, aphase)))
+                break;
+              const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
               for (int tap = tap0; tap < tap1; ++tap) {
                 if (prob.chunk > 0 && in_chunk == prob.chunk) {
                   ptx::mma_commit(tmem_full + (local & 1));
                   ++local;
+                  in_chunk = 0;
                   if (!(ok = open_chunk()))
                     break;
                 }
-                ++in_chunk;
-                if (!ptx::mbar_wait(b_full + bs, bphase, abort_flag)) {
-                  gave_up(kStatusMmaTimeout);
-                  ok = false;
-                  break;
+                if ((bs & 1) == who) {
+                  if (!(ok = wait(b_full + bs, bphase)))
+                    break;
+                  issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4), b_lo + (uint32_t)bs * (kBBytes >> 4));
+                  ptx::mma_commit(b_empty + bs);
                 }
-                ptx::tc_fence_after_sync();
-                issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4), b_lo + (uint32_t)bs * (kBBytes >> 4));
-                ptx::mma_commit(b_empty + bs);
+                ++in_chunk;
                 if (++bs == prob.b_stages) {
                   bs = 0;
                   bphase ^= 1u;
                 }
               }
+              ptx::mma_commit(a_empty + as);
+              next_a();
             }
-            ptx::mma_commit(a_empty + as); // the boxes are free once these MMAs have read them
-            if (++as == prob.a_stages) {
-              as = 0;
-              aphase ^= 1u;
-            }
-          }
+        }
         if (ok) {
           ptx::mma_commit(tmem_full + (local & 1));
           ++local;
@@ -288,7 +313,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int64_t plane = (int64_t)prob.H * prob.W;
     constexpr int kMine = BN / 64; // chunks of 32 columns per warp
-    int local = 0;
+    int local = 0, b_at = 0;       // chunks, weight tiles so far
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const TileAt t = decode(tile);
@@ -314,14 +339,26 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           break;
         }
         ptx::tc_fence_after_sync();
+        // a chunk of one weight tile lies in the accumulator of the issuer that had it
+        const int in_chunk = prob.chunk == 0 || tiles_k - kc * prob.chunk < prob.chunk ? tiles_k - kc * prob.chunk : prob.chunk;
+        const bool both = kAccs == 2 && in_chunk > 1;
+        const int only = kAccs == 2 && in_chunk == 1 ? b_at & 1 : 0;
+        b_at += in_chunk;
 #pragma unroll
         for (int ci = 0; ci < kMine; ++ci) {
-          uint32_t r[32];
-          ptx::tmem_ld_32x32(lane_base + (uint32_t)(buf * BN + 32 * set + 64 * ci), r);
+          const uint32_t at = lane_base + (uint32_t)((buf * kAccs + only) * BN + 32 * set + 64 * ci);
+          uint32_t r[32], r2[32];
+          ptx::tmem_ld_32x32(at, r);
+          if (both)
+            ptx::tmem_ld_32x32(at + BN, r2);
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) // chunk sums in fp32, round to nearest (the first addend is 0)
             acc[ci][j] = __fadd_rn(acc[ci][j], __uint_as_float(r[j]));
+          if (both)
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              acc[ci][j] = __fadd_rn(acc[ci][j], __uint_as_float(r2[j]));
         }
         ptx::tc_fence_before_sync();
         __syncwarp();

@@ -15,6 +15,7 @@ CASES = [
     (4, 96, 10, 10, 64, 1, 0, 2, 1, 1),     # one tap, three empty classes
     (2, 72, 14, 15, 136, 3, 0, 1, 1, 2),    # groups whose slots are padded
     (300, 8, 3, 3, 8, 3, 1, 1, 1, 1),       # many tiny images
+    (80, 128, 27, 27, 256, 1, 0, 2, 1, 1),  # a tile with more boxes than the ring, several tiles per block
     (1, 24, 7, 120, 16, 3, 1, 1, 1, 1),     # rows near the width limit
 ]
 
