@@ -11,6 +11,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace nb200 {
 namespace {
@@ -31,6 +32,8 @@ inline unsigned grid_for(size_t items, int per_thread = 1) {
 template <int kOp, bool kAccum>
 __global__ void __launch_bounds__(kThreads) grad_pass_kernel(const float *__restrict__ y, const float *__restrict__ dy,
                                                              float *__restrict__ dx, size_t total, bool vec) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   const size_t first = (size_t)blockIdx.x * kThreads + threadIdx.x;
   auto one = [](float yv, float g, float old) {
@@ -56,6 +59,8 @@ __global__ void __launch_bounds__(kThreads) grad_pass_kernel(const float *__rest
 template <bool kAccum>
 __global__ void __launch_bounds__(kThreads) gap_backward_kernel(const float *__restrict__ dy, float *__restrict__ dx,
                                                                 size_t total, unsigned S) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += stride) {
     const float g = __fdiv_rn(__ldg(dy + i / S), (float)S);
@@ -71,6 +76,8 @@ __global__ void __launch_bounds__(kThreads) gap_backward_kernel(const float *__r
 __global__ void __launch_bounds__(kThreads)
     max_pooling_index_kernel(const float *__restrict__ x, int *__restrict__ index, size_t outputs, int H, int W,
                              int Ho, int Wo, int kh, int kw, int sh, int sw, int ph, int pw) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   for (size_t o = (size_t)blockIdx.x * kThreads + threadIdx.x; o < outputs; o += stride) {
     const int ox = (int)(o % Wo);
@@ -100,6 +107,8 @@ __global__ void __launch_bounds__(kThreads)
     max_pooling_backward_kernel(const int *__restrict__ index, const float *__restrict__ dy, float *__restrict__ dx,
                                 size_t total, int H, int W, int Ho, int Wo, int kh, int kw, int sh, int sw, int ph,
                                 int pw) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += stride) {
     const int ix = (int)(i % W);
@@ -171,33 +180,58 @@ template <int K> __device__ __forceinline__ void block_sums(float (&v)[K], float
   }
 }
 
+// Calls f(flat element, live) for this block's items of channel c, four at a time with their loads before their use:
+// the sums are HBM-bound and one load in flight per thread reached half of the copy bandwidth.
+template <int kW, typename Load, typename Use>
+__device__ __forceinline__ void channel_sum_loop(unsigned N, unsigned C, unsigned S, Load load, Use use) {
+  const unsigned c = blockIdx.y, P = gridDim.x, Su = S / kW;
+  ChannelItems it((size_t)blockIdx.x * kThreads + threadIdx.x, (size_t)P * kThreads, Su, N);
+  while (it.valid()) {
+    decltype(load((size_t)0)) v[4];
+    bool live[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      live[u] = it.valid();
+      if (live[u])
+        v[u] = load(((size_t)it.n * C + c) * S + (size_t)kW * it.s);
+      it.next();
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (live[u])
+        use(v[u]);
+  }
+}
+
 // partial sums of x and x^2 of channel blockIdx.y over the items of block blockIdx.x: partial[c][p][2]
 template <bool kVec>
 __global__ void __launch_bounds__(kThreads) bn_stats_kernel(const float *__restrict__ x, unsigned N, unsigned C,
                                                             unsigned S, float *__restrict__ partial) {
-  const unsigned c = blockIdx.y, P = gridDim.x;
-  const unsigned Su = kVec ? S / 4 : S;
+  pdl_wait();
+  pdl_trigger();
   float v[2] = {0.0f, 0.0f};
-  ChannelItems it((size_t)blockIdx.x * kThreads + threadIdx.x, (size_t)P * kThreads, Su, N);
-  for (; it.valid(); it.next()) {
-    const size_t base = ((size_t)it.n * C + c) * S;
-    if (kVec) {
-      const float4 a = __ldg(reinterpret_cast<const float4 *>(x + base) + it.s);
-      v[0] += (a.x + a.y) + (a.z + a.w);
-      v[1] += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
-    } else {
-      const float a = __ldg(x + base + it.s);
-      v[0] += a;
-      v[1] += a * a;
-    }
+  if constexpr (kVec) {
+    channel_sum_loop<4>(N, C, S, [&](size_t i) { return __ldg(reinterpret_cast<const float4 *>(x + i)); },
+                        [&](float4 a) {
+                          v[0] += (a.x + a.y) + (a.z + a.w);
+                          v[1] += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
+                        });
+  } else {
+    channel_sum_loop<1>(N, C, S, [&](size_t i) { return __ldg(x + i); },
+                        [&](float a) {
+                          v[0] += a;
+                          v[1] += a * a;
+                        });
   }
-  block_sums<2>(v, partial + ((size_t)c * P + blockIdx.x) * 2);
+  block_sums<2>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 2);
 }
 
 // batch_normalization.cpp:191-205 given the channel's sums: mean, variance, running statistics.
 __global__ void bn_stats_finish_kernel(const float *__restrict__ partial, unsigned P, unsigned C, float count,
                                        float decay, int update, float *__restrict__ m, float *__restrict__ v,
                                        float *__restrict__ rm, float *__restrict__ rv) {
+  pdl_wait();
+  pdl_trigger();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C)
     return;
@@ -218,47 +252,43 @@ __global__ void bn_stats_finish_kernel(const float *__restrict__ partial, unsign
   }
 }
 
-// partial[c][p][5]: sum dy*scale*(x-m), sum dy*scale, sum (x-m), sum dy, sum dy*(x-m)/sqrt(v+eps)   (batch)
-//                   -, -, -, sum dy, sum dy*((x-m)*rstd_inv)                                          (global)
+// partial[c][p][3]: sum dy, sum dy * (x - m), sum (x - m) (the last for batch statistics only). The reference's sums
+// over dy * scale * (x - m), dy * scale and dy * (x - m) / sqrt(v + eps) are these times a constant of the channel.
 template <bool kVec, bool kBatch>
 __global__ void __launch_bounds__(kThreads)
-    bn_backward_sums_kernel(const float *__restrict__ x, const float *__restrict__ dy, const float *__restrict__ gamma,
-                            const float *__restrict__ mean, const float *__restrict__ var, float eps, unsigned N,
-                            unsigned C, unsigned S, float *__restrict__ partial) {
-  const unsigned c = blockIdx.y, P = gridDim.x;
-  const unsigned Su = kVec ? S / 4 : S;
-  const float m = mean[c], scale = gamma ? gamma[c] : 1.0f;
-  const float sd = __fsqrt_rn(__fadd_rn(var[c], eps));
-  const float rstd_inv = kBatch ? 0.0f : inv_sqrt_rn(__fadd_rn(var[c], eps));
-  float v[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    bn_backward_sums_kernel(const float *__restrict__ x, const float *__restrict__ dy, const float *__restrict__ mean,
+                            unsigned N, unsigned C, unsigned S, float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
+  const float m = mean[blockIdx.y];
+  float v[3] = {0.0f, 0.0f, 0.0f};
   auto one = [&](float xv, float g) {
     const float cx = __fsub_rn(xv, m);
-    if (kBatch) {
-      const float dxh = __fmul_rn(g, scale);
-      v[0] += __fmul_rn(dxh, cx);
-      v[1] += dxh;
+    v[0] += g;
+    v[1] += __fmul_rn(g, cx);
+    if (kBatch)
       v[2] += cx;
-      v[4] += __fdiv_rn(__fmul_rn(g, cx), sd);
-    } else {
-      v[4] += __fmul_rn(g, __fmul_rn(cx, rstd_inv));
-    }
-    v[3] += g;
   };
-  ChannelItems it((size_t)blockIdx.x * kThreads + threadIdx.x, (size_t)P * kThreads, Su, N);
-  for (; it.valid(); it.next()) {
-    const size_t base = ((size_t)it.n * C + c) * S;
-    if (kVec) {
-      const float4 a = __ldg(reinterpret_cast<const float4 *>(x + base) + it.s);
-      const float4 g = __ldg(reinterpret_cast<const float4 *>(dy + base) + it.s);
-      one(a.x, g.x);
-      one(a.y, g.y);
-      one(a.z, g.z);
-      one(a.w, g.w);
-    } else {
-      one(__ldg(x + base + it.s), __ldg(dy + base + it.s));
-    }
+  if constexpr (kVec) {
+    struct Pair {
+      float4 a, g;
+    };
+    channel_sum_loop<4>(N, C, S,
+                        [&](size_t i) {
+                          return Pair{__ldg(reinterpret_cast<const float4 *>(x + i)),
+                                      __ldg(reinterpret_cast<const float4 *>(dy + i))};
+                        },
+                        [&](const Pair &p) {
+                          one(p.a.x, p.g.x);
+                          one(p.a.y, p.g.y);
+                          one(p.a.z, p.g.z);
+                          one(p.a.w, p.g.w);
+                        });
+  } else {
+    channel_sum_loop<1>(N, C, S, [&](size_t i) { return make_float2(__ldg(x + i), __ldg(dy + i)); },
+                        [&](float2 p) { one(p.x, p.y); });
   }
-  block_sums<5>(v, partial + ((size_t)c * P + blockIdx.x) * 5);
+  block_sums<3>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 3);
 }
 
 // coef[c][4] for the dx pass: {dvar * 2, dmean / n, gamma * (v + eps)^-0.5, -}. Batch mode
@@ -269,15 +299,20 @@ __global__ void bn_backward_finish_kernel(const float *__restrict__ partial, uns
                                           const float *__restrict__ dm, const float *__restrict__ dv, int batch,
                                           float *__restrict__ coef, float *__restrict__ dbeta, int accum_dbeta,
                                           float *__restrict__ dgamma, int accum_dgamma) {
+  pdl_wait();
+  pdl_trigger();
   const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C)
     return;
-  double s[5] = {0, 0, 0, 0, 0};
+  double t[3] = {0, 0, 0};
   if (partial)
     for (unsigned p = 0; p < P; ++p)
-      for (int k = 0; k < 5; ++k)
-        s[k] += (double)partial[((size_t)c * P + p) * 5 + k];
+      for (int k = 0; k < 3; ++k)
+        t[k] += (double)partial[((size_t)c * P + p) * 3 + k];
   const float ve = __fadd_rn(var[c], eps);
+  const double scale = gamma ? (double)gamma[c] : 1.0;
+  // sum dy*scale*(x-m), sum dy*scale, sum (x-m), sum dy, sum dy*(x-m)/sqrt(v+eps)
+  const double s[5] = {scale * t[1], scale * t[0], t[2], t[0], t[1] / sqrt((double)ve)};
   {
     const float r = inv_sqrt_rn(ve);
     coef[c * 4 + 2] = gamma ? __fmul_rn(gamma[c], r) : r;
@@ -304,6 +339,8 @@ __global__ void __launch_bounds__(kThreads)
                           const float *__restrict__ mean, const float *__restrict__ var, float eps,
                           const float *__restrict__ coef, float count, size_t total, unsigned C, unsigned S,
                           float *__restrict__ dx) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   const size_t first = (size_t)blockIdx.x * kThreads + threadIdx.x;
   ChannelWalk walk(first, stride, S, C);
@@ -323,41 +360,88 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// The same for planes of whole float4: one block per (plane, chunk), the channel's constants taken once.
-template <bool kBatch, bool kAccum>
+// a / d for many a and one d > 0: a times 1 / d held in two floats, hi rounded toward zero and lo > 0 (an infinite a stays
+// infinite). Within 2^-23 ulp of the quotient before its one rounding, in two instructions instead of a division's dozen.
+struct Quotient {
+  float hi, lo;
+  __device__ __forceinline__ explicit Quotient(float d) {
+    hi = __frcp_rz(d);
+    if (__fmaf_rn(-hi, d, 1.0f) == 0.0f)
+      hi = __int_as_float(__float_as_int(hi) - 1);
+    lo = isinf(hi) ? hi : __fmul_rn(__fmaf_rn(-hi, d, 1.0f), hi);
+  }
+  __device__ __forceinline__ float operator()(float a) const { return __fmaf_rn(a, hi, __fmul_rn(a, lo)); }
+};
+
+// The same for planes of whole float4: a warp takes a run of up to 32 * kRun float4 of one plane, `runs` of them per
+// plane, with all its loads in flight before the channel's constants are made. The run length is chosen so that the last
+// run of a plane is nearly full (a block per 512 float4 left 784-float4 planes a quarter idle: 66 us for
+// [128, 64, 56, 56] against 47 us of traffic).
+template <int kRun, bool kBatch, bool kAccum>
 __global__ void __launch_bounds__(kThreads)
     bn_backward_dx_plane_kernel(const float *__restrict__ x, const float *__restrict__ dy,
                                 const float *__restrict__ gamma, const float *__restrict__ mean,
                                 const float *__restrict__ var, float eps, const float *__restrict__ coef, float count,
-                                int C, int S4, float *__restrict__ dx) {
-  const unsigned plane = blockIdx.x;
-  const int c = (int)(plane % (unsigned)C);
+                                unsigned C, int S4, unsigned runs, size_t total_runs, float *__restrict__ dx) {
+  pdl_wait();
+  pdl_trigger();
+  const size_t run = (size_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (run >= total_runs)
+    return;
+  const size_t plane = run / runs;
+  const int c = (int)(plane % C), i0 = (int)(run - plane * runs) * (32 * kRun) + (int)(threadIdx.x & 31);
+  const float4 *xp = reinterpret_cast<const float4 *>(x) + plane * S4;
+  const float4 *gp = reinterpret_cast<const float4 *>(dy) + plane * S4;
+  float4 *op = reinterpret_cast<float4 *>(dx) + plane * S4;
+  float4 g[kRun], xv[kRun], o[kRun];
+#pragma unroll
+  for (int u = 0; u < kRun; ++u) {
+    const int i = i0 + 32 * u;
+    if (i < S4) {
+      g[u] = __ldcs(gp + i);
+      if (kBatch)
+        xv[u] = __ldcs(xp + i);
+      if (kAccum)
+        o[u] = op[i];
+    }
+  }
   const float scale = gamma ? __ldg(gamma + c) : 1.0f;
-  const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
+  const Quotient by_sd(__fsqrt_rn(__fadd_rn(__ldg(var + c), eps))), by_count(count);
   const float m = __ldg(mean + c), k0 = __ldg(coef + c * 4), k1 = __ldg(coef + c * 4 + 1), k2 = __ldg(coef + c * 4 + 2);
-  const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)plane * S4;
-  const float4 *gp = reinterpret_cast<const float4 *>(dy) + (size_t)plane * S4;
-  float4 *op = reinterpret_cast<float4 *>(dx) + (size_t)plane * S4;
-  auto one = [&](float xv, float g, float old) {
+  auto one = [&](float xe, float ge, float old) {
     float r;
     if (kBatch) {
-      const float a = __fdiv_rn(__fmul_rn(g, scale), sd);
-      const float b = __fdiv_rn(__fmul_rn(k0, __fsub_rn(xv, m)), count);
+      const float a = by_sd(__fmul_rn(ge, scale));
+      const float b = by_count(__fmul_rn(k0, __fsub_rn(xe, m)));
       r = __fadd_rn(__fadd_rn(a, b), k1);
     } else {
-      r = __fmul_rn(g, k2);
+      r = __fmul_rn(ge, k2);
     }
     return kAccum ? __fadd_rn(old, r) : r;
   };
-  for (int i = blockIdx.y * kThreads + threadIdx.x; i < S4; i += gridDim.y * kThreads) {
-    const float4 g = __ldcs(gp + i);
-    float4 xv = make_float4(0, 0, 0, 0), o = make_float4(0, 0, 0, 0);
-    if (kBatch)
-      xv = __ldcs(xp + i);
-    if (kAccum)
-      o = op[i];
-    op[i] = make_float4(one(xv.x, g.x, o.x), one(xv.y, g.y, o.y), one(xv.z, g.z, o.z), one(xv.w, g.w, o.w));
+#pragma unroll
+  for (int u = 0; u < kRun; ++u) {
+    const int i = i0 + 32 * u;
+    if (i < S4) {
+      const float4 a = kBatch ? xv[u] : make_float4(0, 0, 0, 0), b = kAccum ? o[u] : make_float4(0, 0, 0, 0);
+      op[i] = make_float4(one(a.x, g[u].x, b.x), one(a.y, g[u].y, b.y), one(a.z, g[u].z, b.z), one(a.w, g[u].w, b.w));
+    }
   }
+}
+
+template <int kRun>
+int bn_backward_dx_planes(const float *x, const float *dy, const float *gamma, const float *mean, const float *var,
+                          float eps, const float *coef, float count, size_t planes, unsigned C, int S4, float *dx,
+                          bool batch, bool accum, cudaStream_t st) {
+  const unsigned runs = (unsigned)((S4 + 32 * kRun - 1) / (32 * kRun));
+  const size_t total = planes * runs, blocks = (total + kThreads / 32 - 1) / (kThreads / 32);
+  NB_CHECK(blocks < (1ull << 31), NB200_ENOTIMPL, "tensor too large");
+  auto kernel = batch ? (accum ? bn_backward_dx_plane_kernel<kRun, true, true> : bn_backward_dx_plane_kernel<kRun, true, false>)
+                      : (accum ? bn_backward_dx_plane_kernel<kRun, false, true> : bn_backward_dx_plane_kernel<kRun, false, false>);
+  NB_CUDA(launch_dependent(kernel, dim3((unsigned)blocks), dim3(kThreads), 0, st, x, dy, gamma, mean, var, eps, coef,
+                           count,
+                           C, S4, runs, total, dx));
+  return NB200_OK;
 }
 
 int channel_blocks(int64_t outer, int64_t channels, int64_t inner, bool vec) {
@@ -394,15 +478,11 @@ int nb200_batch_normalization_batch_f32(const float *x, const float *beta, const
   NB_TRY(scratch.alloc((size_t)channels * P * 2 * sizeof(float)));
   float *partial = static_cast<float *>(scratch.p);
   const dim3 grid((unsigned)P, (unsigned)channels);
-  if (vec)
-    bn_stats_kernel<true><<<grid, kThreads, 0, st>>>(x, (unsigned)outer, (unsigned)channels, (unsigned)inner, partial);
-  else
-    bn_stats_kernel<false><<<grid, kThreads, 0, st>>>(x, (unsigned)outer, (unsigned)channels, (unsigned)inner, partial);
-  NB_LAUNCH_CHECK();
-  bn_stats_finish_kernel<<<(unsigned)((channels + 127) / 128), 128, 0, st>>>(
-      partial, (unsigned)P, (unsigned)channels, (float)(outer * inner), decay_rate, update_running, batch_mean,
-      batch_var, running_mean, running_var);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(vec ? bn_stats_kernel<true> : bn_stats_kernel<false>, grid, dim3(kThreads), 0, st, x,
+                           (unsigned)outer, (unsigned)channels, (unsigned)inner, partial));
+  NB_CUDA(launch_dependent(bn_stats_finish_kernel, dim3((unsigned)((channels + 127) / 128)), dim3(128), 0, st, partial,
+                           (unsigned)P, (unsigned)channels, (float)(outer * inner), decay_rate, update_running,
+                           batch_mean, batch_var, running_mean, running_var));
   return nb200_batch_normalization_inference_f32(x, beta, gamma, batch_mean, batch_var, y, outer, channels, inner,
                                                  eps, stream);
 }
@@ -421,68 +501,42 @@ int nb200_batch_normalization_backward_f32(const float *x, const float *dy, cons
   const bool vec = (inner % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
   const int P = channel_blocks(outer, channels, inner, vec);
   AsyncScratch scratch(st);
-  NB_TRY(scratch.alloc((size_t)channels * (P * 5 + 4) * sizeof(float)));
+  NB_TRY(scratch.alloc((size_t)channels * (P * 3 + 4) * sizeof(float)));
   float *partial = static_cast<float *>(scratch.p);
-  float *coef = partial + (size_t)channels * P * 5;
+  float *coef = partial + (size_t)channels * P * 3;
   const bool sums = (batch_stat && dx) || dbeta || dgamma;
   if (sums) {
     const dim3 grid((unsigned)P, (unsigned)channels);
-#define NB_BN_SUMS(V, B)                                                                                               \
-  bn_backward_sums_kernel<V, B><<<grid, kThreads, 0, st>>>(x, dy, gamma, mean, var, eps, (unsigned)outer,              \
-                                                            (unsigned)channels, (unsigned)inner, partial)
-    if (vec && batch_stat)
-      NB_BN_SUMS(true, true);
-    else if (vec)
-      NB_BN_SUMS(true, false);
-    else if (batch_stat)
-      NB_BN_SUMS(false, true);
-    else
-      NB_BN_SUMS(false, false);
-#undef NB_BN_SUMS
-    NB_LAUNCH_CHECK();
+    auto kernel = vec ? (batch_stat ? bn_backward_sums_kernel<true, true> : bn_backward_sums_kernel<true, false>)
+                      : (batch_stat ? bn_backward_sums_kernel<false, true> : bn_backward_sums_kernel<false, false>);
+    NB_CUDA(launch_dependent(kernel, grid, dim3(kThreads), 0, st, x, dy, mean, (unsigned)outer, (unsigned)channels,
+                             (unsigned)inner, partial));
   }
-  bn_backward_finish_kernel<<<(unsigned)((channels + 127) / 128), 128, 0, st>>>(
-      sums ? partial : nullptr, (unsigned)P, (unsigned)channels, (float)(outer * inner), gamma, var, eps, dmean, dvar,
-      batch_stat, coef, sums ? dbeta : nullptr, accum_dbeta, sums ? dgamma : nullptr, accum_dgamma);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(bn_backward_finish_kernel, dim3((unsigned)((channels + 127) / 128)), dim3(128), 0, st,
+                           sums ? partial : nullptr, (unsigned)P, (unsigned)channels, (float)(outer * inner), gamma, var,
+                           eps, dmean, dvar, batch_stat, coef, sums ? dbeta : nullptr, accum_dbeta,
+                           sums ? dgamma : nullptr, accum_dgamma));
   if (dx) {
     const size_t total = (size_t)outer * channels * inner;
     const unsigned grid = grid_for(total, 4);
-    const bool planes = vec && inner >= 4 * kThreads && outer * channels < (1ll << 31) &&
-                        (reinterpret_cast<uintptr_t>(dx) & 15) == 0;
-    if (planes) {
+    // runs of float4 from planes of 32 values on (below that a warp would be mostly idle)
+    if (vec && inner >= 32 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0) {
       const int S4 = (int)(inner / 4);
-      int chunks = (S4 + 2 * kThreads - 1) / (2 * kThreads);
-      chunks = chunks > 64 ? 64 : chunks;
-      const dim3 pgrid((unsigned)(outer * channels), (unsigned)chunks);
-#define NB_BN_DXP(B, A)                                                                                                \
-  bn_backward_dx_plane_kernel<B, A><<<pgrid, kThreads, 0, st>>>(x, dy, gamma, mean, var, eps, coef,                    \
-                                                                (float)(outer * inner), (int)channels, S4, dx)
-      if (batch_stat && accum_dx)
-        NB_BN_DXP(true, true);
-      else if (batch_stat)
-        NB_BN_DXP(true, false);
-      else if (accum_dx)
-        NB_BN_DXP(false, true);
-      else
-        NB_BN_DXP(false, false);
-#undef NB_BN_DXP
-      NB_LAUNCH_CHECK();
-      return NB200_OK;
+      const size_t planes = (size_t)outer * channels;
+      auto idle = [&](int run) { return (double)((S4 + 32 * run - 1) / (32 * run) * (32 * run)) / S4; };
+      int best = 2;
+      for (int run : {4, 5, 7})
+        if (idle(run) <= idle(best) + 1e-9)
+          best = run;
+      auto launch = best == 2 ? bn_backward_dx_planes<2>
+                              : (best == 4 ? bn_backward_dx_planes<4> : (best == 5 ? bn_backward_dx_planes<5> : bn_backward_dx_planes<7>));
+      return launch(x, dy, gamma, mean, var, eps, coef, (float)(outer * inner), planes, (unsigned)channels, S4, dx,
+                    batch_stat != 0, accum_dx != 0, st);
     }
-#define NB_BN_DX(B, A)                                                                                                 \
-  bn_backward_dx_kernel<B, A><<<grid, kThreads, 0, st>>>(x, dy, gamma, mean, var, eps, coef, (float)(outer * inner),   \
-                                                          total, (unsigned)channels, (unsigned)inner, dx)
-    if (batch_stat && accum_dx)
-      NB_BN_DX(true, true);
-    else if (batch_stat)
-      NB_BN_DX(true, false);
-    else if (accum_dx)
-      NB_BN_DX(false, true);
-    else
-      NB_BN_DX(false, false);
-#undef NB_BN_DX
-    NB_LAUNCH_CHECK();
+    auto kernel = batch_stat ? (accum_dx ? bn_backward_dx_kernel<true, true> : bn_backward_dx_kernel<true, false>)
+                             : (accum_dx ? bn_backward_dx_kernel<false, true> : bn_backward_dx_kernel<false, false>);
+    NB_CUDA(launch_dependent(kernel, dim3(grid), dim3(kThreads), 0, st, x, dy, gamma, mean, var, eps, coef,
+                             (float)(outer * inner), total, (unsigned)channels, (unsigned)inner, dx));
   }
   return NB200_OK;
 }
@@ -494,11 +548,9 @@ int nb200_relu_backward_f32(const float *y, const float *dy, float *dx, size_t s
   const bool vec =
       ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
   const unsigned grid = grid_for(size / 4 + 1, 2);
-  if (accum)
-    grad_pass_kernel<0, true><<<grid, kThreads, 0, as_stream(stream)>>>(y, dy, dx, size, vec);
-  else
-    grad_pass_kernel<0, false><<<grid, kThreads, 0, as_stream(stream)>>>(y, dy, dx, size, vec);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(accum ? grad_pass_kernel<0, true> : grad_pass_kernel<0, false>, dim3(grid), dim3(kThreads),
+                           0,
+                           as_stream(stream), y, dy, dx, size, vec));
   return NB200_OK;
 }
 
@@ -508,11 +560,9 @@ int nb200_add2_backward_f32(const float *dy, float *dx, size_t size, int accum, 
   NB_CHECK(dy && dx, NB200_EVALUE, "null data pointer");
   const bool vec = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
   const unsigned grid = grid_for(size / 4 + 1, 2);
-  if (accum)
-    grad_pass_kernel<1, true><<<grid, kThreads, 0, as_stream(stream)>>>(nullptr, dy, dx, size, vec);
-  else
-    grad_pass_kernel<1, false><<<grid, kThreads, 0, as_stream(stream)>>>(nullptr, dy, dx, size, vec);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(accum ? grad_pass_kernel<1, true> : grad_pass_kernel<1, false>, dim3(grid), dim3(kThreads),
+                           0,
+                           as_stream(stream), (const float *)nullptr, dy, dx, size, vec));
   return NB200_OK;
 }
 
@@ -523,11 +573,8 @@ int nb200_global_average_pooling_backward_f32(const float *dy, float *dx, int64_
   if (total == 0)
     return NB200_OK;
   NB_CHECK(dy && dx, NB200_EVALUE, "null data pointer");
-  if (accum)
-    gap_backward_kernel<true><<<grid_for(total, 4), kThreads, 0, as_stream(stream)>>>(dy, dx, total, (unsigned)spatial);
-  else
-    gap_backward_kernel<false><<<grid_for(total, 4), kThreads, 0, as_stream(stream)>>>(dy, dx, total, (unsigned)spatial);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(accum ? gap_backward_kernel<true> : gap_backward_kernel<false>, dim3(grid_for(total, 4)),
+                           dim3(kThreads), 0, as_stream(stream), dy, dx, total, (unsigned)spatial));
   return NB200_OK;
 }
 
@@ -551,17 +598,12 @@ int nb200_max_pooling_backward_f32(const float *x, const float *dy, float *dx, i
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc(outputs * sizeof(int)));
   int *index = static_cast<int *>(scratch.p);
-  max_pooling_index_kernel<<<grid_for(outputs, 1), kThreads, 0, st>>>(x, index, outputs, height, width, Ho, Wo,
-                                                                       kernel_h, kernel_w, stride_h, stride_w, pad_h,
-                                                                       pad_w);
-  NB_LAUNCH_CHECK();
-  if (accum)
-    max_pooling_backward_kernel<true><<<grid_for(total, 1), kThreads, 0, st>>>(
-        index, dy, dx, total, height, width, Ho, Wo, kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w);
-  else
-    max_pooling_backward_kernel<false><<<grid_for(total, 1), kThreads, 0, st>>>(
-        index, dy, dx, total, height, width, Ho, Wo, kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w);
-  NB_LAUNCH_CHECK();
+  NB_CUDA(launch_dependent(max_pooling_index_kernel, dim3(grid_for(outputs, 1)), dim3(kThreads), 0, st, x, index,
+                           outputs,
+                           height, width, Ho, Wo, kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w));
+  NB_CUDA(launch_dependent(accum ? max_pooling_backward_kernel<true> : max_pooling_backward_kernel<false>,
+                           dim3(grid_for(total, 1)), dim3(kThreads), 0, st, index, dy, dx, total, height, width, Ho, Wo,
+                           kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w));
   return NB200_OK;
 }
 

@@ -186,3 +186,22 @@ def test_against_the_golden_fixtures(F):
                 assert np.abs(host(got[0]) - want).max() <= 2e-5 * (np.abs(want).max() + 1e-6)
                 assert np.allclose(host(got[1]).reshape(-1), g[k + "_dbeta"].reshape(-1), rtol=2e-5, atol=2e-5 * np.sqrt(n))
                 assert np.allclose(host(got[2]).reshape(-1), g[k + "_dgamma"].reshape(-1), rtol=2e-5, atol=2e-5 * np.sqrt(n))
+
+
+@pytest.mark.parametrize("side", [(4, 8), (6, 6), (7, 28), (28, 28), (30, 34), (56, 56), (64, 70)])
+@pytest.mark.parametrize("accum", [False, True])
+@pytest.mark.parametrize("batch_stat", [True, False])
+def test_batch_normalization_backward_plane_runs(F, side, accum, batch_stat):
+    """Planes of whole float4 around the lengths of a warp's run, against float64."""
+    g = torch.Generator(device="cuda").manual_seed(side[1])
+    x, dy, old = (torch.randn(3, 5, *side, device="cuda", generator=g) for _ in range(3))
+    gamma = torch.rand(5, device="cuda", generator=g) + 0.5
+    m, v = (x.mean((0, 2, 3)), x.var((0, 2, 3), unbiased=False)) if batch_stat else (gamma - 1, gamma * 2)
+    xd = x.double().requires_grad_()
+    want, = torch.autograd.grad(torch.nn.functional.batch_norm(xd, m.double(), v.double(), gamma.double(), None, batch_stat,
+                                                               0.0, 1e-5), xd, dy.double())
+    dx = old.clone()
+    F.batch_normalization_backward(x, dy, gamma, m, v, [1], 1e-5, batch_stat, propagate_down=(True, False, False),
+                                   accum=(accum, False, False), grads=(dx, None, None))
+    want = want + old.double() if accum else want
+    assert (dx.double() - want).abs().max() <= 2e-6 * want.abs().max()
