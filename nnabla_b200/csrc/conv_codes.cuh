@@ -216,6 +216,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const bool tabulated = k_blocks <= kCodesKTable;
   for (int kb = threadIdx.x; kb < k_blocks && kb < kCodesKTable; kb += kGemmThreads)
     kb_table[kb] = kb_entry(kb);
+  pdl_wait();
+  pdl_trigger();
   for (int c = threadIdx.x; c < prob.n_tiles * BN; c += kGemmThreads)
     sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
                                       ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)

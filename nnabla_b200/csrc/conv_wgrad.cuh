@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
+  pdl_wait();
+  pdl_trigger();
   auto gave_up = [&](int code) {
     if (*abort_flag == 0)
       atomicCAS(status, 0, code);
@@ -343,6 +345,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 __global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const __grid_constant__ ConvWgradProblem prob, int Kog,
                                                                 int Cg, int taps, float *__restrict__ dw,
                                                                 int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const int task = blockIdx.x;
   const int tg = task % prob.tap_groups;
   int r = task / prob.tap_groups;

@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "pdl.cuh"
 #include "prepare.cuh"
 
 namespace nb200 {
@@ -68,6 +69,8 @@ template <bool kVec, int kSecond, bool kFast = false>
 __global__ void __launch_bounds__(kThreads) bn_add_relu_fxp_kernel(BnTerm A, BnTerm B, size_t total, int C, int S,
                                                                    float eps, int relu, int quantize, FxpParams P,
                                                                    int cached, float *__restrict__ y) {
+  pdl_wait();
+  pdl_trigger();
   // the channels' constants (a square root and a reciprocal each) are worked out once per
   // block into shared memory when they fit (cached != 0), else per item
   extern __shared__ __align__(16) uint8_t consts_raw[];
@@ -172,14 +175,14 @@ int launch(const BnTerm &A, const BnTerm &B, size_t total, int C, int S, float e
   // the largest code must be exact in fp32 arithmetic for the short form (codes below 2^22: twice the code plus one half is exact)
   const bool fast = vec && relu && quantize && P.pow2 && P.maxv * P.inv_delta < 4194304.0f;
   if (fast)
-    bn_add_relu_fxp_kernel<true, kSecond, true><<<grid, kThreads, cached ? smem : 0, st>>>(A, B, total, C, S, eps, relu,
-                                                                                            quantize, P, cached, y);
+    NB_CUDA(launch_dependent(bn_add_relu_fxp_kernel<true, kSecond, true>, grid, dim3(kThreads), cached ? smem : 0, st,
+                             A, B, total, C, S, eps, relu, quantize, P, cached, y));
   else if (vec)
-    bn_add_relu_fxp_kernel<true, kSecond><<<grid, kThreads, cached ? smem : 0, st>>>(A, B, total, C, S, eps, relu,
-                                                                                      quantize, P, cached, y);
+    NB_CUDA(launch_dependent(bn_add_relu_fxp_kernel<true, kSecond>, grid, dim3(kThreads), cached ? smem : 0, st, A, B,
+                             total, C, S, eps, relu, quantize, P, cached, y));
   else
-    bn_add_relu_fxp_kernel<false, kSecond><<<grid, kThreads, cached ? smem : 0, st>>>(A, B, total, C, S, eps, relu,
-                                                                                       quantize, P, cached, y);
+    NB_CUDA(launch_dependent(bn_add_relu_fxp_kernel<false, kSecond>, grid, dim3(kThreads), cached ? smem : 0, st, A, B,
+                             total, C, S, eps, relu, quantize, P, cached, y));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -222,6 +225,8 @@ __global__ void __launch_bounds__(256) bn_add_relu_fxp_codes_kernel(BnTerm A, Bn
                                                                     const int8_t *__restrict__ b_codes, float b_delta,
                                                                     CodesLayout L, float eps, int relu, FxpParams P,
                                                                     int kmax, int kmin, int8_t *__restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[kTilePx * kTilePitch];
   __shared__ ChannelConsts consts_a[kTileSlots], consts_b[kSecond == 2 ? kTileSlots : 1];
   __shared__ int channel_of[kTileSlots]; // channel held by each slot of the tile, -1 = padding
@@ -339,6 +344,8 @@ __global__ void __launch_bounds__(256) bn_add_relu_fxp_codes_kernel(BnTerm A, Bn
 // codes [batch][HW][slots] -> y [batch][C][HW] = code * delta (64 x 64 tiles through shared memory)
 __global__ void __launch_bounds__(256) codes_nhwc_to_f32_kernel(const int8_t *__restrict__ codes, CodesLayout L,
                                                                 float delta, float *__restrict__ y) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int8_t tile[kTilePx][kTileSlots + 4];
   const int n = blockIdx.z;
   const int p0 = blockIdx.x * kTilePx, d0 = blockIdx.y * kTileSlots;
@@ -374,6 +381,8 @@ struct PoolGeom {
 
 __global__ void __launch_bounds__(256) max_pooling_codes_kernel(const int8_t *__restrict__ in, int slots, PoolGeom G,
                                                                 int8_t *__restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   // grid = (chunks of an output row, output rows, samples): no wide divisions per item
   const int vecs = slots / 16; // 16-slot groups per pixel
   const int item = blockIdx.x * 256 + threadIdx.x;
@@ -496,10 +505,11 @@ extern "C" int nb200_bn_add_relu_fxp_codes_nhwc(const float *a, const float *bet
   cudaStream_t st = as_stream(stream);
   const int second = b_codes ? 3 : (b == nullptr ? 0 : (mean_b == nullptr ? 1 : 2));
 #define NB_LAUNCH_CODES(V, S)                                                                                          \
-  bn_add_relu_fxp_codes_kernel<V, S><<<grid, 256, 0, st>>>(A, B, b_codes, b_delta, L, eps, relu, P, kmax, kmin, y_codes)
+  NB_CUDA(launch_dependent(bn_add_relu_fxp_codes_kernel<V, S>, grid, dim3(256), 0, st, A, B, b_codes, b_delta, L, eps, \
+                           relu, P, kmax, kmin, y_codes))
 #define NB_LAUNCH_CODES_FAST(S)                                                                                        \
-  bn_add_relu_fxp_codes_kernel<true, S, true><<<grid, 256, 0, st>>>(A, B, b_codes, b_delta, L, eps, relu, P, kmax,     \
-                                                                    kmin, y_codes)
+  NB_CUDA(launch_dependent(bn_add_relu_fxp_codes_kernel<true, S, true>, grid, dim3(256), 0, st, A, B, b_codes, b_delta,\
+                           L, eps, relu, P, kmax, kmin, y_codes))
   const bool fast = vec && relu && P.pow2 && group == 1 && L.slots == L.C && kmin <= 0;
   if (fast) {
     switch (second) {
@@ -535,7 +545,7 @@ extern "C" int nb200_codes_nhwc_to_f32(const int8_t *codes, float *y, int64_t ba
   NB_CHECK(codes && y, NB200_EVALUE, "null data pointer");
   NB_CHECK((reinterpret_cast<uintptr_t>(codes) & 3) == 0, NB200_EVALUE, "code tensors must be 4-byte aligned");
   const dim3 grid((L.HW + kTilePx - 1) / kTilePx, (L.slots + kTileSlots - 1) / kTileSlots, (unsigned)batch);
-  codes_nhwc_to_f32_kernel<<<grid, 256, 0, as_stream(stream)>>>(codes, L, delta, y);
+  NB_CUDA(launch_dependent(codes_nhwc_to_f32_kernel, grid, dim3(256), 0, as_stream(stream), codes, L, delta, y));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -564,7 +574,7 @@ extern "C" int nb200_max_pooling_codes_nhwc(const int8_t *codes, int8_t *y_codes
   const int slots = (int)codes_slots(channels, group);
   NB_CHECK(batch <= 65535 && G.Ho <= 65535, NB200_ENOTIMPL, "more than 65535 samples or output rows");
   const dim3 grid((unsigned)((G.Wo * (slots / 16) + 255) / 256), (unsigned)G.Ho, (unsigned)batch);
-  max_pooling_codes_kernel<<<grid, 256, 0, as_stream(stream)>>>(codes, slots, G, y_codes);
+  NB_CUDA(launch_dependent(max_pooling_codes_kernel, grid, dim3(256), 0, as_stream(stream), codes, slots, G, y_codes));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

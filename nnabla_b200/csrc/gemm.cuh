@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "pdl.cuh"
 #include "ptx.cuh"
 
 namespace nb200 {
@@ -260,6 +261,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -663,7 +666,7 @@ inline int launch_contraction(const CUtensorMap &ma, const CUtensorMap &mb, cons
     epd.debug = dbg;
   }
 #endif
-  kernel<<<grid, kGemmThreads, smem, st>>>(ma, mb, prob, epd, status);
+  NB_CUDA(launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), smem, st, ma, mb, prob, epd, status));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -168,6 +168,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   ptx::cluster_sync(); // the peer's barriers are initialised before anything is signalled remotely
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -411,7 +413,7 @@ inline int launch_pair_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M,
   int pairs = sm_count() / 2;
   if (pairs > tiles)
     pairs = tiles;
-  kernel<<<2 * pairs, kPairThreads, smem, st>>>(ma, mb, my, prob, ep, status);
+  NB_CUDA(launch_dependent(kernel, dim3(2 * pairs), dim3(kPairThreads), smem, st, ma, mb, my, prob, ep, status));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

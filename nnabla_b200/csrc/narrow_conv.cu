@@ -41,6 +41,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "pdl.cuh"
 #include "narrow_conv.cuh"
 #include "ptx.cuh"
 
@@ -114,6 +115,8 @@ __device__ __forceinline__ void split2(float v, __half &p0, __half &p1) {
 // max |x| of every sample as fp32 bits (non-negative floats order like their bits; a NaN ends above infinity)
 __global__ void __launch_bounds__(256) narrow_conv_absmax_kernel(const float *__restrict__ x, int64_t per_sample,
                                                                  uint32_t *__restrict__ maxbits) {
+  pdl_wait();
+  pdl_trigger();
   const int n = blockIdx.y;
   const float *xs = x + (int64_t)n * per_sample;
   uint32_t m = 0;
@@ -145,6 +148,8 @@ template <int SW>
 __global__ void __launch_bounds__(256) narrow_conv_split_kernel(const float *__restrict__ x, NarrowConv g,
                                                                 const uint32_t *__restrict__ maxbits,
                                                                 uint8_t *__restrict__ xs, float *__restrict__ xscale) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int cpp = 8 / SW; // channel slots per pixel
   const int n = blockIdx.y;
   const int e = scale_exponent(maxbits[n], 14);
@@ -181,6 +186,8 @@ __global__ void __launch_bounds__(256) narrow_conv_split_kernel(const float *__r
 // for itself: the filter is a few thousand values); wscale[0] = 2^-S.
 __global__ void __launch_bounds__(256) narrow_conv_weights_kernel(const float *__restrict__ w, NarrowConv g,
                                                                   __half *__restrict__ out, float *__restrict__ wscale) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ uint32_t part[8];
   const int count = g.Ko * g.C * g.kh * g.kw;
   uint32_t m = 0;
@@ -260,12 +267,6 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
            *tmem_empty = bars + 2 * kInFlight + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kInFlight + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  // bias of every map (0 past Ko or without bias), times 2 / delta when codes are written
-  __shared__ float bias_s[kN];
-  if (threadIdx.x < kN)
-    bias_s[threadIdx.x] = (bias && (int)threadIdx.x < g.Ko)
-                              ? (co.codes ? __fmul_rn(bias[threadIdx.x], co.two_inv) : bias[threadIdx.x])
-                              : 0.0f;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // consecutive output rows per block, so that a tile finds most of its input rows in the ring
   const int num_tiles = g.N * g.Ho;
@@ -289,6 +290,14 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
     ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();
   }
+  pdl_wait();
+  pdl_trigger();
+  // bias of every map (0 past Ko or without bias), times 2 / delta when codes are written
+  __shared__ float bias_s[kN];
+  if (threadIdx.x < kN)
+    bias_s[threadIdx.x] = (bias && (int)threadIdx.x < g.Ko)
+                              ? (co.codes ? __fmul_rn(bias[threadIdx.x], co.two_inv) : bias[threadIdx.x])
+                              : 0.0f;
   {
     // resident weights (already in the tensor core's layout) and zeros behind the ring
     const uint4 *src = reinterpret_cast<const uint4 *>(wprep);
@@ -561,15 +570,17 @@ int narrow_conv_tc(const float *x, const float *w, const float *bias, float *y, 
   int blocks = (int)((per_sample / 4 + 255) / 256);
   const int cap = (8 * sm_count() + batch - 1) / batch;
   blocks = blocks < 1 ? 1 : (blocks > cap ? (cap < 1 ? 1 : cap) : blocks);
-  narrow_conv_absmax_kernel<<<dim3((unsigned)blocks, (unsigned)batch), 256, 0, st>>>(x, per_sample, maxbits);
+  NB_CUDA(launch_dependent(narrow_conv_absmax_kernel, dim3((unsigned)blocks, (unsigned)batch), dim3(256), 0, st, x,
+                           per_sample, maxbits));
   NB_LAUNCH_CHECK();
-  narrow_conv_weights_kernel<<<p.steps, 256, 0, st>>>(w, g, reinterpret_cast<__half *>(wprep), wscale);
+  NB_CUDA(launch_dependent(narrow_conv_weights_kernel, dim3(p.steps), dim3(256), 0, st, w, g, reinterpret_cast<__half
+                           *>(wprep), wscale));
   NB_LAUNCH_CHECK();
   const dim3 split_grid((unsigned)((g.Hp + kSplitRows - 1) / kSplitRows), (unsigned)batch);
   if (stride_w == 2)
-    narrow_conv_split_kernel<2><<<split_grid, 256, 0, st>>>(x, g, maxbits, xs, xscale);
+    NB_CUDA(launch_dependent(narrow_conv_split_kernel<2>, split_grid, dim3(256), 0, st, x, g, maxbits, xs, xscale));
   else
-    narrow_conv_split_kernel<1><<<split_grid, 256, 0, st>>>(x, g, maxbits, xs, xscale);
+    NB_CUDA(launch_dependent(narrow_conv_split_kernel<1>, split_grid, dim3(256), 0, st, x, g, maxbits, xs, xscale));
   NB_LAUNCH_CHECK();
   static bool configured[64];
   int dev = 0;
@@ -595,7 +606,8 @@ int narrow_conv_tc(const float *x, const float *w, const float *bias, float *y, 
   NB_TRY(device_status_word(&status));
   const int tiles = batch * Ho;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  narrow_conv_tcgen05_kernel<<<grid, kThreadsNC, p.smem, st>>>(map_y, box_store ? 1 : 0, xs, wprep, xscale, wscale, bias, y, g, status, co);
+  NB_CUDA(launch_dependent(narrow_conv_tcgen05_kernel, dim3(grid), dim3(kThreadsNC), p.smem, st, map_y,
+                           box_store ? 1 : 0, xs, wprep, xscale, wscale, bias, y, g, status, co));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -4,9 +4,10 @@
 // dozen images per GPU a network is a chain of kernels of a few microseconds each, and the gap between two
 // kernels (launch processing, grid start) is a large part of the step; this hides most of it.
 //
-// Rules that keep it correct: (1) every kernel launched this way executes pdl_wait() as its first
-// statement, in every thread, before any global-memory access (so its completion implies the
-// predecessor's, and ordering stays transitive along the stream); (2) pdl_trigger() only says "my
+// Rules that keep it correct: (1) every kernel launched this way executes pdl_wait() in every thread, before any
+// global-memory access: as its first statement, or in the tensor-core kernels after the barriers and the tensor
+// memory are set up, which touches nothing outside the SM (so its completion implies the predecessor's, and
+// ordering stays transitive along the stream); (2) pdl_trigger() only says "my
 // successor may be scheduled", it orders nothing. Kernels launched the ordinary way in between serialize
 // fully, as before. NNABLA_B200_PDL=0 turns the attribute off (ordinary launches; the waits are no-ops).
 #pragma once

@@ -285,11 +285,13 @@ int fxp_nhwc_codes(const float *x, float *y, int8_t *codes, int64_t batch, int64
   const dim3 grid((unsigned)((inner + 63) / 64), (unsigned)((slots + 63) / 64), (unsigned)batch);
   if (L.pow2) {
     FxpOp<true, false> op{L.maxv, L.minv, delta, L.inv, L.code_max, L.code_min, nullptr};
-    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<true>, grid, dim3(256), 0, st, x, y, codes, (int)channels, (int)inner,
+    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<true>, grid, dim3(256), 0, st, x, y, codes, (int)channels,
+                             (int)inner,
                              slots, op));
   } else {
     FxpOp<false, false> op{L.maxv, L.minv, delta, L.inv, L.code_max, L.code_min, nullptr};
-    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<false>, grid, dim3(256), 0, st, x, y, codes, (int)channels, (int)inner,
+    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<false>, grid, dim3(256), 0, st, x, y, codes, (int)channels,
+                             (int)inner,
                              slots, op));
   }
   NB_LAUNCH_CHECK();
@@ -677,6 +679,8 @@ __device__ __forceinline__ float extremum_value(unsigned long long key, bool is_
 }
 
 __global__ void minmax_init_kernel(unsigned long long *mn, unsigned long long *mx, size_t Q) {
+  pdl_wait();
+  pdl_trigger();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < Q) {
     mn[i] = extremum_start(true);
@@ -689,6 +693,8 @@ __global__ void minmax_init_kernel(unsigned long long *mn, unsigned long long *m
 // is the element's position in the reference's scan over the reduced axes.
 __global__ void __launch_bounds__(kThreads) minmax_reduce_kernel(const float *__restrict__ x, MinMaxView V,
                                                                  unsigned long long *mn, unsigned long long *mx) {
+  pdl_wait();
+  pdl_trigger();
   const size_t q = blockIdx.y;
   const size_t per_q = V.outer * V.inner;
   float lo = 1e8f, hi = -1e8f;
@@ -736,6 +742,8 @@ __global__ void minmax_params_kernel(size_t Q, float *qr_min, float *qr_max, con
                                      int x_min_max, int ema, float decay_f,
                                      float one_minus_decay_f, float eps, float *m_out, float *M_out, float *s_out,
                                      float *scale_user) {
+  pdl_wait();
+  pdl_trigger();
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q >= Q)
     return;
@@ -860,7 +868,7 @@ int minmax_run(const float *x, const MinMaxView &V, float *qr_min, float *qr_max
   const unsigned qblocks = (unsigned)((V.Q + 255) / 256);
   if (x_min_max) {
     NB_CHECK(V.size > 0, NB200_EVALUE, "min/max of an empty tensor");
-    minmax_init_kernel<<<qblocks, 256, 0, st>>>(mn, mx, V.Q);
+    NB_CUDA(launch_dependent(minmax_init_kernel, dim3(qblocks), dim3(256), 0, st, mn, mx, V.Q));
     NB_LAUNCH_CHECK();
     NB_CHECK(V.Q <= 65535, NB200_ENOTIMPL, "more than 65535 quantization ranges");
     const size_t per_q = V.outer * V.inner;
@@ -872,13 +880,14 @@ int minmax_run(const float *x, const MinMaxView &V, float *qr_min, float *qr_max
       splits = cap;
     if (splits == 0)
       splits = 1;
-    minmax_reduce_kernel<<<dim3((unsigned)splits, (unsigned)V.Q), kThreads, 0, st>>>(x, V, mn, mx);
+    NB_CUDA(launch_dependent(minmax_reduce_kernel, dim3((unsigned)splits, (unsigned)V.Q), dim3(kThreads), 0, st, x, V,
+                             mn, mx));
     NB_LAUNCH_CHECK();
   }
   // (T)decay_ and (T)(1.0 - decay_) as in min_max_quantize.cpp:105-106.
   const float d1 = decay, d2 = (float)(1.0 - (double)decay);
-  minmax_params_kernel<<<qblocks, 256, 0, st>>>(V.Q, qr_min, qr_max, ql_min, ql_max, mn, mx, x_min_max, ema, d1, d2,
-                                                 eps, m, M, s, scale);
+  NB_CUDA(launch_dependent(minmax_params_kernel, dim3(qblocks), dim3(256), 0, st, V.Q, qr_min, qr_max, ql_min, ql_max,
+                           mn, mx, x_min_max, ema, d1, d2, eps, m, M, s, scale));
   NB_LAUNCH_CHECK();
   MinMaxOp op{m, M, s, V.Q, V.inner};
   return launch_elementwise(x, y, V.size, op, st);

@@ -31,6 +31,8 @@ __device__ __forceinline__ float grad_combine(const Op &op, const typename Op::S
 template <typename Op, bool kAccum>
 __global__ void __launch_bounds__(kThreads) grad_vec_kernel(const float *__restrict__ x, const float *__restrict__ dy,
                                                             float *__restrict__ dx, size_t size, size_t n4, Op op) {
+  pdl_wait();
+  pdl_trigger();
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   const float4 *dy4 = reinterpret_cast<const float4 *>(dy);
   float4 *dx4 = reinterpret_cast<float4 *>(dx);
@@ -80,6 +82,8 @@ template <typename Op, bool kAccum>
 __global__ void __launch_bounds__(kThreads) grad_scalar_kernel(const float *__restrict__ x,
                                                                const float *__restrict__ dy, float *__restrict__ dx,
                                                                size_t size, Op op) {
+  pdl_wait();
+  pdl_trigger();
   const size_t stride = (size_t)gridDim.x * kThreads;
   const typename Op::State st = op.init();
   for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < size; i += stride)
@@ -91,11 +95,12 @@ int launch_gradient_t(const float *x, const float *dy, float *dx, size_t size, c
   const uintptr_t all = (Op::kNeedsX ? reinterpret_cast<uintptr_t>(x) : 0) | reinterpret_cast<uintptr_t>(dy) |
                         reinterpret_cast<uintptr_t>(dx);
   if (all & 15) {
-    grad_scalar_kernel<Op, kAccum><<<grid_for(size), kThreads, 0, st>>>(x, dy, dx, size, op);
+    NB_CUDA(launch_dependent(grad_scalar_kernel<Op, kAccum>, dim3(grid_for(size)), dim3(kThreads), 0, st, x, dy, dx,
+                             size, op));
   } else {
     const size_t n4 = size / 4;
-    grad_vec_kernel<Op, kAccum>
-        <<<grid_for((n4 + kUnroll - 1) / kUnroll), kThreads, 0, st>>>(x, dy, dx, size, n4, op);
+    NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum>, dim3(grid_for((n4 + kUnroll - 1) / kUnroll)), dim3(kThreads),
+                             0, st, x, dy, dx, size, n4, op));
   }
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -197,6 +202,8 @@ int pow2_gradient_threshold(const Pow2Params &P, uint32_t *threshold_bits) {
 // (nudge_qr_min_max, :362-390, with the scale of :184-186).
 __global__ void minmax_nudged_kernel(size_t Q, const float *qr_min, const float *qr_max, const float *ql_min,
                                      const float *ql_max, float *m_out, float *M_out) {
+  pdl_wait();
+  pdl_trigger();
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q >= Q)
     return;
@@ -258,6 +265,8 @@ __global__ void __launch_bounds__(kThreads) minmax_range_grad_kernel(const float
                                                                      const float *__restrict__ m,
                                                                      const float *__restrict__ M, float *partial,
                                                                      float *__restrict__ dx) {
+  pdl_wait();
+  pdl_trigger();
   const size_t q = blockIdx.y;
   const size_t per_q = V.outer * V.inner;
   const float lo = __ldg(m + q), hi = __ldg(M + q);
@@ -332,6 +341,8 @@ __global__ void __launch_bounds__(kThreads) minmax_range_grad_kernel(const float
 __global__ void __launch_bounds__(kThreads) minmax_range_finish_kernel(const float *partial, unsigned splits,
                                                                        float *g_min, float *g_max, int do_min,
                                                                        int do_max, int accum_min, int accum_max) {
+  pdl_wait();
+  pdl_trigger();
   const size_t q = blockIdx.x;
   float s_lo = 0.0f, s_hi = 0.0f;
   for (unsigned s = threadIdx.x; s < splits; s += kThreads) {
@@ -375,7 +386,8 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
   float *m = static_cast<float *>(scratch.p), *M = m + V.Q, *partial = M + V.Q;
   if (need_nudged) {
     NB_CHECK(qr_min && qr_max && ql_min && ql_max, NB200_EVALUE, "null range pointer");
-    minmax_nudged_kernel<<<(unsigned)((V.Q + 255) / 256), 256, 0, st>>>(V.Q, qr_min, qr_max, ql_min, ql_max, m, M);
+    NB_CUDA(launch_dependent(minmax_nudged_kernel, dim3((unsigned)((V.Q + 255) / 256)), dim3(256), 0, st, V.Q, qr_min,
+                             qr_max, ql_min, ql_max, m, M));
     NB_LAUNCH_CHECK();
   }
   // Per-tensor ranges with aligned buffers: one pass produces dx and the range sums.
@@ -395,21 +407,26 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
     NB_CHECK(V.size == 0 || (x && dy), NB200_EVALUE, "null data pointer");
     const dim3 grid((unsigned)splits, (unsigned)V.Q);
     if (!fused) {
-      minmax_range_grad_kernel<0, false><<<grid, kThreads, 0, st>>>(x, dy, V, m, M, partial, nullptr);
+      NB_CUDA(launch_dependent(minmax_range_grad_kernel<0, false>, grid, dim3(kThreads), 0, st, x, dy, V, m, M, partial,
+                               nullptr));
     } else {
       NB_CHECK(dx != nullptr, NB200_EVALUE, "null data pointer");
       if (fine && accum[0])
-        minmax_range_grad_kernel<2, true><<<grid, kThreads, 0, st>>>(x, dy, V, m, M, partial, dx);
+        NB_CUDA(launch_dependent(minmax_range_grad_kernel<2, true>, grid, dim3(kThreads), 0, st, x, dy, V, m, M,
+                                 partial, dx));
       else if (fine)
-        minmax_range_grad_kernel<1, true><<<grid, kThreads, 0, st>>>(x, dy, V, m, M, partial, dx);
+        NB_CUDA(launch_dependent(minmax_range_grad_kernel<1, true>, grid, dim3(kThreads), 0, st, x, dy, V, m, M,
+                                 partial, dx));
       else if (accum[0])
-        minmax_range_grad_kernel<2, false><<<grid, kThreads, 0, st>>>(x, dy, V, m, M, partial, dx);
+        NB_CUDA(launch_dependent(minmax_range_grad_kernel<2, false>, grid, dim3(kThreads), 0, st, x, dy, V, m, M,
+                                 partial, dx));
       else
-        minmax_range_grad_kernel<1, false><<<grid, kThreads, 0, st>>>(x, dy, V, m, M, partial, dx);
+        NB_CUDA(launch_dependent(minmax_range_grad_kernel<1, false>, grid, dim3(kThreads), 0, st, x, dy, V, m, M,
+                                 partial, dx));
     }
     NB_LAUNCH_CHECK();
-    minmax_range_finish_kernel<<<(unsigned)V.Q, kThreads, 0, st>>>(partial, (unsigned)splits, g_min, g_max, prop[1],
-                                                                   prop[2], accum[1], accum[2]);
+    NB_CUDA(launch_dependent(minmax_range_finish_kernel, dim3((unsigned)V.Q), dim3(kThreads), 0, st, partial,
+                             (unsigned)splits, g_min, g_max, prop[1], prop[2], accum[1], accum[2]));
     NB_LAUNCH_CHECK();
   }
   return NB200_OK;
