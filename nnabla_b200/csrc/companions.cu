@@ -670,7 +670,8 @@ int nb200_batch_normalization_inference_f32(const float *x, const float *beta, c
     const dim3 grid((planes + kThreads / 32 - 1) / (kThreads / 32));
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
     if (vec)
-      NB_CUDA(launch_dependent(bn_inference_warp_kernel<true>, grid, dim3(kThreads), 0, as_stream(stream), x, beta, gamma,
+      NB_CUDA(launch_dependent(bn_inference_warp_kernel<true>, grid, dim3(kThreads), 0, as_stream(stream), x, beta,
+                               gamma,
                                mean, var, planes, (int)channels, (int)inner, eps, y));
     else if (aligned && planes % 4 == 0)
       NB_CUDA(launch_dependent(bn_inference_warp4_kernel, dim3((planes / 4 + kThreads / 32 - 1) / (kThreads / 32)),

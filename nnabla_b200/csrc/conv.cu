@@ -138,6 +138,167 @@ int launch_conv(const ConvGeometry &g, const void *act, int planes_b, int64_t ct
                                                                                             p.taps * p.cblocks);
 }
 
+// The pixel-major convolution of planes (conv_planes.cuh). A: [planes][N][Hin][Win][ctot], B: [total_maps][taps][k_slots],
+// both 16-bit; along either axis output pixel i of p.H x p.W reads input pixel i * s - pad + k * dil of tap k, or
+// (i + pad - k * dil) / s in the gradient's direction.
+struct PlanesAxis {
+  int k, dil, pad, s;
+  bool flip; // the gradient's direction: the classes are the output's
+  int residue(int t) const { return ((t * dil - pad) % s + s) % s; }
+  int offset(int t) const { return (flip ? residue(t) + pad - t * dil : t * dil - pad - residue(t)) / s; }
+  int min_offset() const {
+    int m = offset(0);
+    for (int t = 1; t < k; ++t)
+      m = offset(t) < m ? offset(t) : m;
+    return m;
+  }
+  int max_offset() const {
+    int m = offset(0);
+    for (int t = 1; t < k; ++t)
+      m = offset(t) > m ? offset(t) : m;
+    return m;
+  }
+};
+
+struct PlanesPlan {
+  ConvPlanesProblem p;
+  int bn;
+  bool resident;
+  size_t smem;
+};
+
+// Channel slots per pixel of a planes tensor.
+inline int64_t planes_slots(int group, int c_pad_g) {
+  const int64_t n = (int64_t)group * c_pad_g;
+  return n < 64 ? 64 : n;
+}
+
+constexpr size_t kPlanesSmem = 226 * 1024; // of 227 KB; the barriers are static
+
+// Fills p's tiling for an output of p.H x p.W with p.maps maps per group; false: the kernel does not apply.
+bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, int channels_g) {
+  ConvPlanesProblem &p = plan.p;
+  const int taps = ay.k * ax.k;
+  if (taps > kPlanesMaxTaps || ay.s * ax.s > 16)
+    return false;
+  p.sy = ay.flip ? ay.s : 1;
+  p.sx = ax.flip ? ax.s : 1;
+  p.in_sy = ay.flip ? 1 : ay.s;
+  p.in_sx = ax.flip ? 1 : ax.s;
+  p.Wu = (p.W + p.sx - 1) / p.sx;
+  const int Hu = (p.H + p.sy - 1) / p.sy;
+  p.y0 = ay.min_offset();
+  p.x0 = ax.min_offset();
+  p.wp = p.Wu + ax.max_offset() - p.x0;
+  const int span_y = ay.max_offset() - p.y0;
+  p.cblocks = (channels_g + 63) / 64;
+  p.k_slots = p.cblocks * 64;
+  if (p.Wu > 128 || p.wp * p.in_sx > 256)
+    return false;
+  p.h_box = (128 - p.Wu) / p.wp + 1; // (h_box - 1) * wp + Wu <= 128
+  p.h_box = p.h_box < Hu ? p.h_box : Hu;
+  for (int h = p.h_box; h >= 1; --h) // prefer a divisor of the rows unless it wastes over a third of the tile
+    if (Hu % h == 0) {
+      if (3 * h >= 2 * p.h_box)
+        p.h_box = h;
+      break;
+    }
+  p.hp = p.h_box + span_y;
+  if (p.hp * p.in_sy > 256)
+    return false;
+  p.tiles_h = (Hu + p.h_box - 1) / p.h_box;
+  p.plane_bytes = (p.hp * p.wp + 7) / 8 * 8 * kRowBytes;
+  int n = 0, max_row = 0;
+  for (int ry = 0; ry < ay.s; ++ry)
+    for (int rx = 0; rx < ax.s; ++rx) {
+      p.class_tap[ry * ax.s + rx] = n;
+      for (int ky = 0; ky < ay.k; ++ky)
+        for (int kx = 0; kx < ax.k; ++kx)
+          if (ay.residue(ky) == ry && ax.residue(kx) == rx) {
+            p.tap_row[n] = (ay.offset(ky) - p.y0) * p.wp + ax.offset(kx) - p.x0;
+            max_row = p.tap_row[n] > max_row ? p.tap_row[n] : max_row;
+            p.tap_k[n++] = ky * ax.k + kx;
+          }
+    }
+  p.class_tap[ay.s * ax.s] = n;
+  // the 128 rows read from the last tap's row on may reach past the last box
+  int over = (max_row + kTileM) * kRowBytes - p.plane_bytes;
+  over = over > 0 ? over : 0;
+  plan.bn = p.maps <= 64 ? 64 : 128;
+  p.n_tiles = (p.maps + plan.bn - 1) / plan.bn;
+  const size_t b_tile = (size_t)plan.bn * kRowBytes, fixed = 1024 + over;
+  // all weights beside three single-plane boxes at least, and the accumulation short enough without chunks
+  const size_t b_all = (size_t)taps * p.cblocks * b_tile;
+  plan.resident = p.groups == 1 && p.n_tiles == 1 && taps * p.cblocks * 4 <= 96 &&
+                  fixed + b_all + 3 * (size_t)p.plane_bytes <= kPlanesSmem;
+  if (plan.resident) {
+    int st = (int)((kPlanesSmem - fixed - b_all) / p.plane_bytes);
+    p.a_stages = st > 4 ? 4 : st;
+    p.b_stages = 1;
+    p.chunk = 0;
+    plan.smem = fixed + b_all + (size_t)p.a_stages * p.plane_bytes;
+    return true;
+  }
+  const size_t stage = (size_t)p.planes * p.plane_bytes;
+  p.a_stages = 2;
+  if (fixed + 2 * stage + 2 * b_tile > kPlanesSmem)
+    return false;
+  int st = (int)((kPlanesSmem - fixed - 2 * stage) / b_tile);
+  p.b_stages = st >= 6 ? 6 : (st >= 4 ? 4 : 2); // even: they alternate between the issuing warps
+  // two accumulators share a chunk; half the usual length each: no step of a strided gradient multiplies zeros here
+  p.chunk = 2 * k_chunk_blocks(p.planes * 8);
+  plan.smem = fixed + 2 * stage + (size_t)p.b_stages * b_tile;
+  return true;
+}
+
+template <int BN, int PG, bool kResident, bool kF16>
+int launch_planes_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const PlanesPlan &plan, cudaStream_t st) {
+  auto kernel = conv_planes_tcgen05_kernel<BN, PG, kResident, kF16>;
+  static bool configured[64];
+  int dev = 0;
+  NB_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63]) {
+    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanesSmem));
+    configured[dev & 63] = true;
+  }
+  int *status = nullptr;
+  NB_TRY(device_status_word(&status));
+  const int tiles = plan.p.num_tiles();
+  NB_CUDA(launch_dependent(kernel, dim3(tiles < sm_count() ? tiles : sm_count()), dim3(kPlanesThreads), plan.smem, st,
+                           ma, mb, plan.p, status));
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+// act: [planes][N][Hin][Win][ctot], side: [total_maps][taps * k_slots].
+int launch_planes(const PlanesPlan &plan, const void *act, int Hin, int Win, int64_t ctot, const void *side, int taps,
+                  bool f16, cudaStream_t st) {
+  const ConvPlanesProblem &p = plan.p;
+  CUtensorMap ma, mb;
+  const uint64_t dims[5] = {(uint64_t)ctot, (uint64_t)Win, (uint64_t)Hin, (uint64_t)p.Nimg, (uint64_t)p.planes};
+  const uint64_t strides[4] = {(uint64_t)ctot * 2, (uint64_t)ctot * 2 * Win, (uint64_t)ctot * 2 * Win * Hin,
+                               (uint64_t)ctot * 2 * Win * Hin * p.Nimg};
+  const uint32_t box[5] = {64, (uint32_t)(p.wp * p.in_sx), (uint32_t)(p.hp * p.in_sy), 1, 1};
+  const uint32_t estr[5] = {1, (uint32_t)p.in_sx, (uint32_t)p.in_sy, 1, 1};
+  NB_TRY(encode_tiled(&ma, 0, 5, act, dims, strides, box, estr, kRowBytes));
+  const int64_t pitch = (int64_t)taps * p.k_slots;
+  NB_TRY(make_operand_map(&mb, side, false, pitch, pitch, p.total_maps, 1, plan.bn));
+  if (f16) {
+    NB_CHECK(p.planes == 2, NB200_EVALUE, "fp16 planes come in pairs");
+    if (plan.resident)
+      return plan.bn == 64 ? launch_planes_kernel<64, 1, true, true>(ma, mb, plan, st)
+                           : launch_planes_kernel<128, 1, true, true>(ma, mb, plan, st);
+    return plan.bn == 64 ? launch_planes_kernel<64, 2, false, true>(ma, mb, plan, st)
+                         : launch_planes_kernel<128, 2, false, true>(ma, mb, plan, st);
+  }
+  NB_CHECK(p.planes == 3, NB200_EVALUE, "bf16 planes come in threes");
+  if (plan.resident)
+    return plan.bn == 64 ? launch_planes_kernel<64, 1, true, false>(ma, mb, plan, st)
+                         : launch_planes_kernel<128, 1, true, false>(ma, mb, plan, st);
+  return plan.bn == 64 ? launch_planes_kernel<64, 3, false, false>(ma, mb, plan, st)
+                       : launch_planes_kernel<128, 3, false, false>(ma, mb, plan, st);
+}
+
 // Shared body of BinaryWeightConvolution / BinaryConnectConvolution forward.
 // weight_delta > 0: w itself holds multiples of weight_delta (a fixed-point convolution of two
 // 8-bit operands: no binarisation, wb / alpha unused, int8 path only).
@@ -170,9 +331,26 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
            "output rows wider than 256 pixels (Wo=%d, stride %d) are not supported", g.Wo, g.sw);
   const int es = int8 ? 1 : 2;
   const int c_pad_g = (int)round_up(g.Cg, 16);
+  // fp32 activations against +-1 weights: two fp16 pieces of the activations scaled by a power of two
+  // (x * 2^-e = p0 + p1), two thirds of the operand rows and MMAs of the exact three-piece bf16 split;
+  // the bf16 form stays for a quantize_zero_to other than -1, 0, 1
+  const bool half_pair = !int8 && (zero_to == 1.0f || zero_to == -1.0f || zero_to == 0.0f);
+  // Those run with the pixels on the MMA rows, and a scale per image, where a tile's boxes fit in a block's shared memory.
+  PlanesPlan plan{};
+  bool planes_form = false;
+  if (half_pair) {
+    plan.p.Nimg = g.N;
+    plan.p.maps = g.Kog;
+    plan.p.total_maps = g.Ko;
+    plan.p.groups = g.group;
+    plan.p.H = g.Ho;
+    plan.p.W = g.Wo;
+    plan.p.planes = 2;
+    planes_form = plan_planes(plan, PlanesAxis{g.kh, g.dh, g.ph, g.sh, false}, PlanesAxis{g.kw, g.dw, g.pw, g.sw, false}, g.Cg);
+  }
   // One K block is one filter tap over E channel slots. With few channels per
   // group a 128-byte row would be half zero padding: use 64-byte rows then.
-  const bool narrow_rows = c_pad_g * es <= 64;
+  const bool narrow_rows = !planes_form && c_pad_g * es <= 64;
   const int E = (narrow_rows ? 64 : kRowBytes) / es;
   const int cblocks = (c_pad_g + E - 1) / E;
   const int c_slots = cblocks * E;
@@ -182,14 +360,10 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
   NB_CHECK(!int8 || ctot == codes_slots(g.C, g.group), NB200_EVALUE, "activation code layout mismatch");
   const int taps = g.kh * g.kw;
   const int64_t wpitch = (int64_t)taps * c_slots;
-  // fp32 activations against +-1 weights: two fp16 pieces of the activations scaled by a power of two
-  // (x * 2^-e = p0 + p1), two thirds of the operand rows and MMAs of the exact three-piece bf16 split;
-  // the bf16 form stays for a quantize_zero_to other than -1, 0, 1
-  const bool half_pair = !int8 && (zero_to == 1.0f || zero_to == -1.0f || zero_to == 0.0f);
   const int planes = int8 ? 1 : (half_pair ? 2 : 3);
   const size_t act_bytes = x_codes ? 0 : (size_t)planes * g.N * g.H * g.W * ctot * es;
   const size_t side_bytes = prepared_side ? 0 : (size_t)g.Ko * wpitch * es;
-  const size_t extra_bytes = half_pair ? round_up((size_t)g.Ko * 4 + 16, 1024) : 0;
+  const size_t extra_bytes = half_pair ? round_up((planes_form ? (size_t)g.N * (1 + kHalfPairParts) : (size_t)g.Ko) * 4 + 16, 1024) : 0;
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc(round_up(act_bytes, 1024) + round_up(side_bytes, 1024) + extra_bytes));
   const uint8_t *act = x_codes ? reinterpret_cast<const uint8_t *>(x_codes) : static_cast<uint8_t *>(scratch.p);
@@ -212,8 +386,19 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
       NB_TRY(binarize_rows(w, g.Ko, g.Cg, g.kh, g.kw, zero_to, wb, alpha, side, wpitch, c_slots, int8, st, half_pair));
   }
   float *row_scale_half = nullptr;
+  uint8_t *extra = static_cast<uint8_t *>(scratch.p) + round_up(act_bytes, 1024) + round_up(side_bytes, 1024);
+  if (planes_form) {
+    ConvPlanesProblem &p = plan.p;
+    p.image_max = reinterpret_cast<uint32_t *>(extra);
+    NB_TRY(nchw_to_nhwc_half_pair_images(x, g.N, g.C, g.H * g.W, g.group, g.Cg, c_pad_g, (int)ctot, scratch.p,
+                                         reinterpret_cast<uint32_t *>(extra), st));
+    p.c_group_stride = c_pad_g;
+    p.y = y;
+    p.scale = alpha;
+    p.bias = bias;
+    return launch_planes(plan, act, g.H, g.W, ctot, side, taps, true, st);
+  }
   if (half_pair) {
-    uint8_t *extra = static_cast<uint8_t *>(scratch.p) + round_up(act_bytes, 1024) + round_up(side_bytes, 1024);
     row_scale_half = reinterpret_cast<float *>(extra + 16);
     NB_TRY(nchw_to_nhwc_half_pair(x, g.N, g.C, g.H * g.W, g.group, g.Cg, c_pad_g, (int)ctot, scratch.p,
                                   reinterpret_cast<uint32_t *>(extra), alpha, g.Ko, row_scale_half, st));
@@ -294,157 +479,6 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
 //       output is the kh x kw filter window. One launch per group.
 //  db = sums of dy over batch and pixels.
 // ---------------------------------------------------------------------------
-// The pixel-major convolution of planes (conv_planes.cuh). A: [planes][N][Hin][Win][ctot], B: [total_maps][taps][k_slots],
-// both 16-bit; output pixel (iy, ix) of p.H x p.W reads input pixel (iy + pad - k * dil) / s of tap k along either axis
-// (flip: the gradient's direction) or iy - pad + k * dil (s = 1).
-struct PlanesAxis {
-  int k, dil, pad, s;
-  bool flip;
-  int residue(int t) const { return flip ? ((t * dil - pad) % s + s) % s : 0; }
-  int offset(int t) const { return flip ? (residue(t) + pad - t * dil) / s : t * dil - pad; }
-  int min_offset() const {
-    int m = offset(0);
-    for (int t = 1; t < k; ++t)
-      m = offset(t) < m ? offset(t) : m;
-    return m;
-  }
-  int max_offset() const {
-    int m = offset(0);
-    for (int t = 1; t < k; ++t)
-      m = offset(t) > m ? offset(t) : m;
-    return m;
-  }
-};
-
-struct PlanesPlan {
-  ConvPlanesProblem p;
-  int bn;
-  bool resident;
-  size_t smem;
-};
-
-constexpr size_t kPlanesSmem = 226 * 1024; // of 227 KB; the barriers are static
-
-// Fills p's tiling for an output of p.H x p.W with p.maps maps per group; false: the kernel does not apply.
-bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, int channels_g) {
-  ConvPlanesProblem &p = plan.p;
-  const int taps = ay.k * ax.k;
-  if (taps > kPlanesMaxTaps || ay.s * ax.s > 16)
-    return false;
-  p.sy = ay.s;
-  p.sx = ax.s;
-  p.Wu = (p.W + ax.s - 1) / ax.s;
-  const int Hu = (p.H + ay.s - 1) / ay.s;
-  p.y0 = ay.min_offset();
-  p.x0 = ax.min_offset();
-  p.wp = p.Wu + ax.max_offset() - p.x0;
-  const int span_y = ay.max_offset() - p.y0;
-  p.cblocks = (channels_g + 63) / 64;
-  p.k_slots = p.cblocks * 64;
-  if (p.Wu > 128 || p.wp > 256)
-    return false;
-  p.h_box = (128 - p.Wu) / p.wp + 1; // (h_box - 1) * wp + Wu <= 128
-  p.h_box = p.h_box < Hu ? p.h_box : Hu;
-  for (int h = p.h_box; h >= 1; --h) // prefer a divisor of the rows unless it wastes over a third of the tile
-    if (Hu % h == 0) {
-      if (3 * h >= 2 * p.h_box)
-        p.h_box = h;
-      break;
-    }
-  p.hp = p.h_box + span_y;
-  if (p.hp > 256)
-    return false;
-  p.tiles_h = (Hu + p.h_box - 1) / p.h_box;
-  p.plane_bytes = (p.hp * p.wp + 7) / 8 * 8 * kRowBytes;
-  int n = 0, max_row = 0;
-  for (int ry = 0; ry < ay.s; ++ry)
-    for (int rx = 0; rx < ax.s; ++rx) {
-      p.class_tap[ry * ax.s + rx] = n;
-      for (int ky = 0; ky < ay.k; ++ky)
-        for (int kx = 0; kx < ax.k; ++kx)
-          if (ay.residue(ky) == ry && ax.residue(kx) == rx) {
-            p.tap_row[n] = (ay.offset(ky) - p.y0) * p.wp + ax.offset(kx) - p.x0;
-            max_row = p.tap_row[n] > max_row ? p.tap_row[n] : max_row;
-            p.tap_k[n++] = ky * ax.k + kx;
-          }
-    }
-  p.class_tap[ay.s * ax.s] = n;
-  // the 128 rows read from the last tap's row on may reach past the last box
-  int over = (max_row + kTileM) * kRowBytes - p.plane_bytes;
-  over = over > 0 ? over : 0;
-  plan.bn = p.maps <= 64 ? 64 : 128;
-  p.n_tiles = (p.maps + plan.bn - 1) / plan.bn;
-  const size_t b_tile = (size_t)plan.bn * kRowBytes, fixed = 1024 + over;
-  // all weights beside three single-plane boxes at least, and the accumulation short enough without chunks
-  const size_t b_all = (size_t)taps * p.cblocks * b_tile;
-  plan.resident = p.groups == 1 && p.n_tiles == 1 && taps * p.cblocks * 4 <= 96 &&
-                  fixed + b_all + 3 * (size_t)p.plane_bytes <= kPlanesSmem;
-  if (plan.resident) {
-    int st = (int)((kPlanesSmem - fixed - b_all) / p.plane_bytes);
-    p.a_stages = st > 4 ? 4 : st;
-    p.b_stages = 1;
-    p.chunk = 0;
-    plan.smem = fixed + b_all + (size_t)p.a_stages * p.plane_bytes;
-    return true;
-  }
-  const size_t stage = (size_t)p.planes * p.plane_bytes;
-  p.a_stages = 2;
-  if (fixed + 2 * stage + 2 * b_tile > kPlanesSmem)
-    return false;
-  int st = (int)((kPlanesSmem - fixed - 2 * stage) / b_tile);
-  p.b_stages = st >= 6 ? 6 : (st >= 4 ? 4 : 2); // even: they alternate between the issuing warps
-  // two accumulators share a chunk; half the usual length each: no step of a strided gradient multiplies zeros here
-  p.chunk = 2 * k_chunk_blocks(p.planes * 8);
-  plan.smem = fixed + 2 * stage + (size_t)p.b_stages * b_tile;
-  return true;
-}
-
-template <int BN, int PG, bool kResident, bool kF16>
-int launch_planes_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const PlanesPlan &plan, cudaStream_t st) {
-  auto kernel = conv_planes_tcgen05_kernel<BN, PG, kResident, kF16>;
-  static bool configured[64];
-  int dev = 0;
-  NB_CUDA(cudaGetDevice(&dev));
-  if (!configured[dev & 63]) {
-    NB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanesSmem));
-    configured[dev & 63] = true;
-  }
-  int *status = nullptr;
-  NB_TRY(device_status_word(&status));
-  const int tiles = plan.p.num_tiles();
-  kernel<<<tiles < sm_count() ? tiles : sm_count(), kPlanesThreads, plan.smem, st>>>(ma, mb, plan.p, status);
-  NB_LAUNCH_CHECK();
-  return NB200_OK;
-}
-
-// act: [planes][N][Hin][Win][ctot], side: [total_maps][taps * k_slots].
-int launch_planes(const PlanesPlan &plan, const void *act, int Hin, int Win, int64_t ctot, const void *side, int taps,
-                  bool f16, cudaStream_t st) {
-  const ConvPlanesProblem &p = plan.p;
-  CUtensorMap ma, mb;
-  const uint64_t dims[5] = {(uint64_t)ctot, (uint64_t)Win, (uint64_t)Hin, (uint64_t)p.Nimg, (uint64_t)p.planes};
-  const uint64_t strides[4] = {(uint64_t)ctot * 2, (uint64_t)ctot * 2 * Win, (uint64_t)ctot * 2 * Win * Hin,
-                               (uint64_t)ctot * 2 * Win * Hin * p.Nimg};
-  const uint32_t box[5] = {64, (uint32_t)p.wp, (uint32_t)p.hp, 1, 1};
-  NB_TRY(encode_tiled(&ma, 0, 5, act, dims, strides, box, nullptr, kRowBytes));
-  const int64_t pitch = (int64_t)taps * p.k_slots;
-  NB_TRY(make_operand_map(&mb, side, false, pitch, pitch, p.total_maps, 1, plan.bn));
-  if (f16) {
-    NB_CHECK(p.planes == 2, NB200_EVALUE, "fp16 planes come in pairs");
-    if (plan.resident)
-      return plan.bn == 64 ? launch_planes_kernel<64, 1, true, true>(ma, mb, plan, st)
-                           : launch_planes_kernel<128, 1, true, true>(ma, mb, plan, st);
-    return plan.bn == 64 ? launch_planes_kernel<64, 2, false, true>(ma, mb, plan, st)
-                         : launch_planes_kernel<128, 2, false, true>(ma, mb, plan, st);
-  }
-  NB_CHECK(p.planes == 3, NB200_EVALUE, "bf16 planes come in threes");
-  if (plan.resident)
-    return plan.bn == 64 ? launch_planes_kernel<64, 1, true, false>(ma, mb, plan, st)
-                         : launch_planes_kernel<128, 1, true, false>(ma, mb, plan, st);
-  return plan.bn == 64 ? launch_planes_kernel<64, 3, false, false>(ma, mb, plan, st)
-                       : launch_planes_kernel<128, 3, false, false>(ma, mb, plan, st);
-}
-
 // Tasks and boxes of the weight gradient of one geometry; false: the kernel does not apply.
 bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t &smem) {
   const int taps = g.kh * g.kw;
@@ -556,8 +590,8 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
     *did_dw = plan_wgrad(q, g, x_planes, smem_w);
   if (!*did_dx && !*did_dw)
     return NB200_OK;
-  const int64_t k_tot = (int64_t)g.group * k_pad_g < 64 ? 64 : (int64_t)g.group * k_pad_g;
-  const int64_t c_tot = (int64_t)g.group * c_pad_g < 64 ? 64 : (int64_t)g.group * c_pad_g;
+  const int64_t k_tot = planes_slots(g.group, k_pad_g);
+  const int64_t c_tot = planes_slots(g.group, c_pad_g);
   const bool two = *did_dx && *did_dw && alpha; // dy * alpha for dx, dy for dw
   const size_t dy_bytes = round_up((size_t)3 * g.N * g.Ho * g.Wo * k_tot * 2, 1024);
   const size_t x_bytes = *did_dw ? round_up((size_t)x_planes * g.N * g.H * g.W * c_tot * 2, 1024) : 0;
@@ -612,9 +646,10 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   }
   int *status = nullptr;
   NB_TRY(device_status_word(&status));
-  kernel<<<grid_w, kGemmThreads, smem_w, st>>>(mx, md, q, status);
+  NB_CUDA(launch_dependent(kernel, dim3(grid_w), dim3(kGemmThreads), smem_w, st, mx, md, q, status));
   NB_LAUNCH_CHECK();
-  conv_wgrad_finish_kernel<<<dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), 256, 0, st>>>(q, g.Kog, g.Cg, taps, dw, accum_dw);
+  NB_CUDA(launch_dependent(conv_wgrad_finish_kernel, dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), dim3(256), 0, st, q,
+                           g.Kog, g.Cg, taps, dw, accum_dw));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -920,7 +955,7 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
   NB_TRY(device_status_word(&status));
   const int tiles = p.n_tiles * p.tiles_h * p.tiles_n;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kernel<<<grid, kGemmThreads, smem, st>>>(mx, mw, p, ep, status);
+  NB_CUDA(launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), smem, st, mx, mw, p, ep, status));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -8,7 +8,8 @@
 //    s * s classes of input pixels (row and column residues mod s): each class is a stride-1 convolution of dy with
 //    the taps that reach it, so that no zeros are multiplied (spreading dy over the input grid multiplied s * s times
 //    as much and stored it first);
-//  * the forward convolution of fp32 activations: A = two fp16 pieces of the scaled activations, B = +-1 weights.
+//  * the forward convolution of fp32 activations: A = two fp16 pieces of the scaled activations, B = +-1 weights. A
+//    stride s makes s * s classes of taps, each reading one of the s * s interleaved images of x.
 //
 // What bounds it: the tensor core (an MMA of 128 rows takes 51 / 67 cycles for 64 / 128 columns, limited by the
 // shared-memory reads of A). The previous form put the maps on the 128 MMA rows, half of them empty for 64 maps, and
@@ -24,6 +25,7 @@
 // multiplied with a weight tile together, so that each weight tile is fetched once per box.
 #pragma once
 #include "gemm.cuh"
+#include "prepare.cuh"
 
 namespace nb200 {
 
@@ -35,10 +37,11 @@ struct ConvPlanesProblem {
   int Nimg, maps, total_maps, groups; // output maps per group and in all
   int H, W;                           // output image
   int sy, sx;                         // output pixel (sy * u + ry, sx * v + rx) belongs to class ry * sx + rx
+  int in_sy, in_sx;                   // a tile sums in_sy * in_sx classes of input pixels (1 with output classes)
   int Wu;                             // columns of a class's grid: ceil(W / sx)
   int h_box, tiles_h, n_tiles;        // class rows per tile, tiles per class and image, column tiles
   int wp, hp;                         // input box: hp rows of wp pixels
-  int y0, x0;                         // its origin relative to the tile's first class row / column
+  int y0, x0;                         // its origin relative to the tile's first class row / column (class pixels)
   int cblocks;                        // 64-channel blocks of one group
   int c_group_stride;                 // channel slots between groups in A
   int k_slots;                        // weight slots per tap
@@ -50,6 +53,7 @@ struct ConvPlanesProblem {
   int tap_row[kPlanesMaxTaps];        // first row of the box that tap reads
   int tap_k[kPlanesMaxTaps];          // its index in the weights
   const float *scale, *bias;          // per output map, may be NULL
+  const uint32_t *image_max;          // per image: bits of the magnitude that its scaling was chosen from, may be NULL
   float *y;
   int accumulate;
   __host__ __device__ __forceinline__ int num_tiles() const { return n_tiles * sy * sx * groups * tiles_h * Nimg; }
@@ -67,7 +71,9 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t stage_bytes = (uint32_t)PG * prob.plane_bytes;
   uint8_t *b_base = smem; // weights first: MMAs may read up to 128 rows past a box (rows of no stored pixel)
-  const uint32_t b_tiles = kResident ? (uint32_t)(prob.class_tap[prob.sy * prob.sx] * prob.cblocks) : (uint32_t)prob.b_stages;
+  const int in_classes = prob.in_sy * prob.in_sx;
+  const uint32_t b_tiles =
+      kResident ? (uint32_t)(prob.class_tap[prob.sy * prob.sx * in_classes] * prob.cblocks) : (uint32_t)prob.b_stages;
   uint8_t *a_base = smem + b_tiles * kBBytes;
 
   __shared__ __align__(8) uint64_t a_full[kPlanesMaxStages], a_empty[kPlanesMaxStages], b_full[kPlanesMaxStages],
@@ -104,6 +110,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   struct TileAt {
     int n0, cls, group, row0, img;
@@ -120,6 +128,26 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
     t.row0 = (tile % prob.tiles_h) * prob.h_box;
     t.img = tile / prob.tiles_h;
     return t;
+  };
+  // boxes of a tile, in the order of the ring: (channel block, input class, plane group)
+  struct BoxAt {
+    int cb, cls, pg, ry, rx;
+  };
+  const int boxes_per_tile = prob.cblocks * in_classes * plane_groups;
+  auto box_at = [&](const TileAt &t, int i) {
+    BoxAt b;
+    b.pg = i % plane_groups;
+    i /= plane_groups;
+    const int ic = i % in_classes;
+    b.cb = i / in_classes;
+    b.cls = t.cls * in_classes + ic; // one of the two counts is 1
+    b.ry = ic / prob.in_sx;
+    b.rx = ic - b.ry * prob.in_sx;
+    return b;
+  };
+  // whether a tile has any tap (an output class may have none)
+  auto empty_tile = [&](const TileAt &t) {
+    return prob.class_tap[t.cls * in_classes] == prob.class_tap[(t.cls + 1) * in_classes];
   };
   auto gave_up = [&](int code) {
     if (*abort_flag == 0)
@@ -142,42 +170,43 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
       }
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileAt t = decode(tile);
-        const int tap0 = prob.class_tap[t.cls], tap1 = prob.class_tap[t.cls + 1];
-        if (tap0 == tap1)
-          continue;
-        for (int cb = 0; cb < prob.cblocks && ok; ++cb)
-          for (int pg = 0; pg < plane_groups && ok; ++pg) {
-            if (!ptx::mbar_wait(a_empty + as, aphase ^ 1u, abort_flag)) {
-              gave_up(kStatusProducerTimeout);
-              ok = false;
-              break;
-            }
-            ptx::mbar_expect_tx(a_full + as, (uint32_t)(PG * prob.hp * prob.wp * kRowBytes));
-#pragma unroll
-            for (int p = 0; p < PG; ++p)
-              ptx::tma_load_5d(a_base + as * stage_bytes + p * prob.plane_bytes, &map_a, a_full + as,
-                               t.group * prob.c_group_stride + cb * 64, prob.x0, t.row0 + prob.y0, t.img,
-                               prob.planes - 1 - (pg * PG + p)); // smallest pieces first
-            if (++as == prob.a_stages) {
-              as = 0;
-              aphase ^= 1u;
-            }
-            if (!kResident)
-              for (int tap = tap0; tap < tap1; ++tap) {
-                if (!ptx::mbar_wait(b_empty + bs, bphase ^ 1u, abort_flag)) {
-                  gave_up(kStatusProducerTimeout);
-                  ok = false;
-                  break;
-                }
-                ptx::mbar_expect_tx(b_full + bs, kBBytes);
-                ptx::tma_load_3d(b_base + bs * kBBytes, &map_b, b_full + bs, prob.tap_k[tap] * prob.k_slots + cb * 64,
-                                 t.group * prob.maps + t.n0, 0);
-                if (++bs == prob.b_stages) {
-                  bs = 0;
-                  bphase ^= 1u;
-                }
-              }
+        for (int i = 0; i < boxes_per_tile && ok; ++i) {
+          const BoxAt at = box_at(t, i);
+          const int cb = at.cb, pg = at.pg, tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+          if (tap0 == tap1)
+            continue;
+          if (!ptx::mbar_wait(a_empty + as, aphase ^ 1u, abort_flag)) {
+            gave_up(kStatusProducerTimeout);
+            ok = false;
+            break;
           }
+          ptx::mbar_expect_tx(a_full + as, (uint32_t)(PG * prob.hp * prob.wp * kRowBytes));
+#pragma unroll
+          for (int p = 0; p < PG; ++p)
+            ptx::tma_load_5d(a_base + as * stage_bytes + p * prob.plane_bytes, &map_a, a_full + as,
+                             t.group * prob.c_group_stride + cb * 64, prob.x0 * prob.in_sx + at.rx,
+                             (t.row0 + prob.y0) * prob.in_sy + at.ry, t.img,
+                             prob.planes - 1 - (pg * PG + p)); // smallest pieces first
+          if (++as == prob.a_stages) {
+            as = 0;
+            aphase ^= 1u;
+          }
+          if (!kResident)
+            for (int tap = tap0; tap < tap1; ++tap) {
+              if (!ptx::mbar_wait(b_empty + bs, bphase ^ 1u, abort_flag)) {
+                gave_up(kStatusProducerTimeout);
+                ok = false;
+                break;
+              }
+              ptx::mbar_expect_tx(b_full + bs, kBBytes);
+              ptx::tma_load_3d(b_base + bs * kBBytes, &map_b, b_full + bs, prob.tap_k[tap] * prob.k_slots + cb * 64,
+                               t.group * prob.maps + t.n0, 0);
+              if (++bs == prob.b_stages) {
+                bs = 0;
+                bphase ^= 1u;
+              }
+            }
+        }
       }
     }
   } else if (warp == 1 || warp == 2 + kEpilogueWarps) {
@@ -230,12 +259,14 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
         ok = wait(b_full, 0u);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileAt t = decode(tile);
-        const int tap0 = prob.class_tap[t.cls], tap1 = prob.class_tap[t.cls + 1];
-        if (tap0 == tap1)
+        if (empty_tile(t))
           continue;
         if constexpr (kResident) {
           if ((local & 1) != who) { // the other issuer's tile: its boxes are released as soon as they have come
-            for (int i = 0; i < prob.cblocks * plane_groups; ++i) {
+            for (int i = 0; i < boxes_per_tile; ++i) {
+              const int cls = box_at(t, i).cls;
+              if (prob.class_tap[cls] == prob.class_tap[cls + 1])
+                continue;
               if (!(ok = wait(a_full + as, aphase)))
                 break;
               ptx::mbar_arrive(a_empty + as);
@@ -245,60 +276,66 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
             continue;
           }
           ok = open_chunk();
-          for (int cb = 0; cb < prob.cblocks && ok; ++cb)
-            for (int pg = 0; pg < plane_groups; ++pg) {
-              if (!(ok = wait(a_full + as, aphase)))
-                break;
-              const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
-              // in batches: the descriptors of three taps before their MMAs
-              int tap = tap0;
-              for (; tap + 3 <= tap1; tap += 3) {
-                uint32_t off[3];
+          for (int i = 0; i < boxes_per_tile && ok; ++i) {
+            const BoxAt at = box_at(t, i);
+            const int cb = at.cb, tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+            if (tap0 == tap1)
+              continue;
+            if (!(ok = wait(a_full + as, aphase)))
+              break;
+            const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
+            // in batches: the descriptors of three taps before their MMAs
+            int tap = tap0;
+            for (; tap + 3 <= tap1; tap += 3) {
+              uint32_t off[3];
 #pragma unroll
-                for (int u = 0; u < 3; ++u)
-                  off[u] = a_stage + (uint32_t)prob.tap_row[tap + u] * (kRowBytes >> 4);
+              for (int u = 0; u < 3; ++u)
+                off[u] = a_stage + (uint32_t)prob.tap_row[tap + u] * (kRowBytes >> 4);
 #pragma unroll
-                for (int u = 0; u < 3; ++u)
-                  issue(off[u], b_lo + (uint32_t)((tap + u) * prob.cblocks + cb) * (kBBytes >> 4));
-              }
-              for (; tap < tap1; ++tap)
-                issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4),
-                      b_lo + (uint32_t)(tap * prob.cblocks + cb) * (kBBytes >> 4));
-              ptx::mma_commit(a_empty + as); // the boxes are free once these MMAs have read them
-              next_a();
+              for (int u = 0; u < 3; ++u)
+                issue(off[u], b_lo + (uint32_t)((tap + u) * prob.cblocks + cb) * (kBBytes >> 4));
             }
+            for (; tap < tap1; ++tap)
+              issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4),
+                    b_lo + (uint32_t)(tap * prob.cblocks + cb) * (kBBytes >> 4));
+            ptx::mma_commit(a_empty + as); // the boxes are free once these MMAs have read them
+            next_a();
+          }
         } else {
           // Weight stages alternate between the issuers (their number is even), so that each sees every phase of its own.
           int in_chunk = 0;
           ok = open_chunk();
-          for (int cb = 0; cb < prob.cblocks && ok; ++cb)
-            for (int pg = 0; pg < plane_groups && ok; ++pg) {
-              if (!(ok = wait(a_full + as, aphase)))
-                break;
-              const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
-              for (int tap = tap0; tap < tap1; ++tap) {
-                if (prob.chunk > 0 && in_chunk == prob.chunk) {
-                  ptx::mma_commit(tmem_full + (local & 1));
-                  ++local;
-                  in_chunk = 0;
-                  if (!(ok = open_chunk()))
-                    break;
-                }
-                if ((bs & 1) == who) {
-                  if (!(ok = wait(b_full + bs, bphase)))
-                    break;
-                  issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4), b_lo + (uint32_t)bs * (kBBytes >> 4));
-                  ptx::mma_commit(b_empty + bs);
-                }
-                ++in_chunk;
-                if (++bs == prob.b_stages) {
-                  bs = 0;
-                  bphase ^= 1u;
-                }
+          for (int i = 0; i < boxes_per_tile && ok; ++i) {
+            const BoxAt at = box_at(t, i);
+            const int tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+            if (tap0 == tap1)
+              continue;
+            if (!(ok = wait(a_full + as, aphase)))
+              break;
+            const uint32_t a_stage = a_lo + ((uint32_t)as * stage_bytes >> 4);
+            for (int tap = tap0; tap < tap1; ++tap) {
+              if (prob.chunk > 0 && in_chunk == prob.chunk) {
+                ptx::mma_commit(tmem_full + (local & 1));
+                ++local;
+                in_chunk = 0;
+                if (!(ok = open_chunk()))
+                  break;
               }
-              ptx::mma_commit(a_empty + as);
-              next_a();
+              if ((bs & 1) == who) {
+                if (!(ok = wait(b_full + bs, bphase)))
+                  break;
+                issue(a_stage + (uint32_t)prob.tap_row[tap] * (kRowBytes >> 4), b_lo + (uint32_t)bs * (kBBytes >> 4));
+                ptx::mma_commit(b_empty + bs);
+              }
+              ++in_chunk;
+              if (++bs == prob.b_stages) {
+                bs = 0;
+                bphase ^= 1u;
+              }
             }
+            ptx::mma_commit(a_empty + as);
+            next_a();
+          }
         }
         if (ok) {
           ptx::mma_commit(tmem_full + (local & 1));
@@ -317,7 +354,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const TileAt t = decode(tile);
-      const int taps = prob.class_tap[t.cls + 1] - prob.class_tap[t.cls];
+      const int taps = prob.class_tap[(t.cls + 1) * in_classes] - prob.class_tap[t.cls * in_classes];
       const int ry = t.cls / prob.sx, rx = t.cls - ry * prob.sx;
       const int iy = (t.row0 + box_y) * prob.sy + ry, ix = box_x * prob.sx + rx;
       const bool pix_ok = box_y < prob.h_box && box_x < prob.Wu && iy < prob.H && ix < prob.W;
@@ -374,8 +411,12 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
           continue;
         const int map0 = t.group * prob.maps + col;
         float *yp = prob.y + ((int64_t)t.img * prob.total_maps + map0) * plane + (int64_t)iy * prob.W + ix;
-        if (prob.scale || prob.bias) { // one rounding per operation, like the reference's product and bias addition
-          const float ls = prob.scale && lane < left ? __ldg(prob.scale + map0 + lane) : 1.0f;
+        if (prob.scale || prob.bias || prob.image_max) {
+          // one rounding per operation, like the reference's product and bias addition (the image's factor is a power
+          // of two)
+          const float up = prob.image_max ? __int_as_float((127 + half_pair_exponent(__ldg(prob.image_max + t.img))) << 23)
+                                          : 1.0f;
+          const float ls = __fmul_rn(prob.scale && lane < left ? __ldg(prob.scale + map0 + lane) : 1.0f, up);
           const float lb = prob.bias && lane < left ? __ldg(prob.bias + map0 + lane) : 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {

@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(256) binarize_columns_kernel(const float *__re
                                                                float zero_to, float *__restrict__ wb,
                                                                void *__restrict__ side, int64_t side_pitch,
                                                                float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float s_sign[kBT][kBT + 1];
   __shared__ float s_sum[4][kBT];
   const int c0 = blockIdx.x * kBT, r0 = blockIdx.y * kBT;
@@ -75,6 +77,8 @@ __global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *
                                                                    float zero_to, float *__restrict__ wb,
                                                                    void *__restrict__ side, int64_t side_pitch,
                                                                    float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float s_sign[kBT][kBT + 1];
   __shared__ float s_sum[16][kBT];
   const int c0 = blockIdx.x * kBT, r0 = blockIdx.y * kBT;
@@ -134,6 +138,8 @@ __global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *
 
 __global__ void finalize_alpha_kernel(const float *__restrict__ partial, int blocks, int C, float inv,
                                       float *__restrict__ alpha) {
+  pdl_wait();
+  pdl_trigger();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C)
     return;
@@ -207,6 +213,8 @@ __global__ void __launch_bounds__(256) binarize_rows_kernel(const float *__restr
 __global__ void __launch_bounds__(256) codes_conv_weights_kernel(const float *__restrict__ wq, int Cg, int kh, int kw,
                                                                  float inv_delta, int8_t *__restrict__ side,
                                                                  int64_t side_pitch, int c_pad) {
+  pdl_wait();
+  pdl_trigger();
   const int o = blockIdx.x;
   const int taps = kh * kw, Kd = Cg * taps;
   const float *wr = wq + (int64_t)o * Kd;
@@ -233,6 +241,8 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 
 __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict__ x, int64_t rows, int K, int64_t Kp,
                                                          int planes, const float *__restrict__ col_scale,
                                                          __nv_bfloat16 *__restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   const int k = blockIdx.x * 64 + threadIdx.x;
   const int64_t plane_stride = rows * Kp;
   const float cs = (col_scale != nullptr && k < K) ? col_scale[k] : 1.0f;
@@ -256,6 +266,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
 // columns), a second kernel adds the `splits` partials of each column in order.
 __global__ void __launch_bounds__(256) column_partial_sums_kernel(const float *__restrict__ a, int64_t rows, int C,
                                                                   float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= C)
     return;
@@ -276,6 +288,8 @@ __global__ void __launch_bounds__(256) column_partial_sums_kernel(const float *_
 
 __global__ void __launch_bounds__(256) column_finish_kernel(const float *__restrict__ partial, int C, int splits,
                                                             float *__restrict__ out, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= C)
     return;
@@ -294,6 +308,8 @@ template <typename OutT, int PLANES>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const float *__restrict__ x, int C, int HW, int groups,
                                                            int Cg, int c_pad_g, int ctot, OutT *__restrict__ out,
                                                            int64_t plane_stride, float inv_delta) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[32][33];
   const int n = blockIdx.z;
   const int p0 = blockIdx.x * 32, d0 = blockIdx.y * 32; // d = destination channel slot
@@ -358,6 +374,8 @@ __device__ __forceinline__ void nchw_to_nhwc_i8_tile(int bx, int by, int n, cons
 __global__ void __launch_bounds__(256) nchw_to_nhwc_i8_kernel(const float *__restrict__ x, int C, int HW, int groups,
                                                               int Cg, int c_pad_g, int ctot,
                                                               int8_t *__restrict__ out, float inv_delta) {
+  pdl_wait();
+  pdl_trigger();
   nchw_to_nhwc_i8_tile(blockIdx.x, blockIdx.y, blockIdx.z, x, C, HW, groups, Cg, c_pad_g, ctot, out, inv_delta);
 }
 
@@ -439,6 +457,8 @@ __global__ void __launch_bounds__(256)
 // int8 [R, C] -> [C][pitch] (transpose), tile 64 x 64 through shared memory.
 __global__ void __launch_bounds__(256) transpose_i8_kernel(const int8_t *__restrict__ src, int R, int C,
                                                            int8_t *__restrict__ dst, int64_t pitch) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int8_t tile[64][65];
   const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
@@ -457,6 +477,8 @@ __global__ void __launch_bounds__(256) transpose_i8_kernel(const int8_t *__restr
 // fp32 [R, C] -> [C][R] (transpose), tile 32 x 32 through shared memory.
 __global__ void __launch_bounds__(256) transpose_f32_kernel(const float *__restrict__ src, int R, int C,
                                                             float *__restrict__ dst) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -564,17 +586,22 @@ int binarize_columns(const float *w, int R, int C, float zero_to, float *wb, flo
                    ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(wb)) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(side) & 7) == 0;
   if (vec && int8)
-    binarize_columns_vec_kernel<true><<<grid, 256, 0, st>>>(w, R, C, zero_to, wb, side, side_pitch, partial);
+    NB_CUDA(launch_dependent(binarize_columns_vec_kernel<true>, grid, dim3(256), 0, st, w, R, C, zero_to, wb, side,
+                             side_pitch, partial));
   else if (vec)
-    binarize_columns_vec_kernel<false><<<grid, 256, 0, st>>>(w, R, C, zero_to, wb, side, side_pitch, partial);
+    NB_CUDA(launch_dependent(binarize_columns_vec_kernel<false>, grid, dim3(256), 0, st, w, R, C, zero_to, wb, side,
+                             side_pitch, partial));
   else if (int8)
-    binarize_columns_kernel<true><<<grid, 256, 0, st>>>(w, R, C, zero_to, wb, side, side_pitch, partial);
+    NB_CUDA(launch_dependent(binarize_columns_kernel<true>, grid, dim3(256), 0, st, w, R, C, zero_to, wb, side,
+                             side_pitch, partial));
   else
-    binarize_columns_kernel<false><<<grid, 256, 0, st>>>(w, R, C, zero_to, wb, side, side_pitch, partial);
+    NB_CUDA(launch_dependent(binarize_columns_kernel<false>, grid, dim3(256), 0, st, w, R, C, zero_to, wb, side,
+                             side_pitch, partial));
   NB_LAUNCH_CHECK();
   if (alpha) {
     const float inv = (float)1 / R; // binary_weight_affine.cpp:68
-    finalize_alpha_kernel<<<(C + 255) / 256, 256, 0, st>>>(partial, (int)grid.y, C, inv, alpha);
+    NB_CUDA(launch_dependent(finalize_alpha_kernel, dim3((C + 255) / 256), dim3(256), 0, st, partial, (int)grid.y, C,
+                             inv, alpha));
     NB_LAUNCH_CHECK();
   }
   return NB200_OK;
@@ -584,12 +611,15 @@ int binarize_rows(const float *w, int Ko, int Cg, int kh, int kw, float zero_to,
                   int64_t side_pitch, int c_pad, bool int8, cudaStream_t st, bool half) {
   const float inv = (float)1 / (Cg * kh * kw); // binary_weight_convolution.cpp:66
   if (int8)
-    NB_CUDA(launch_dependent(binarize_rows_kernel<1>, dim3(Ko), dim3(256), 0, st, w, Cg, kh, kw, zero_to, inv, wb, alpha,
+    NB_CUDA(launch_dependent(binarize_rows_kernel<1>, dim3(Ko), dim3(256), 0, st, w, Cg, kh, kw, zero_to, inv, wb,
+                             alpha,
                              side, side_pitch, c_pad));
   else if (half)
-    binarize_rows_kernel<2><<<Ko, 256, 0, st>>>(w, Cg, kh, kw, zero_to, inv, wb, alpha, side, side_pitch, c_pad);
+    NB_CUDA(launch_dependent(binarize_rows_kernel<2>, dim3(Ko), dim3(256), 0, st, w, Cg, kh, kw, zero_to, inv, wb,
+                             alpha, side, side_pitch, c_pad));
   else
-    binarize_rows_kernel<0><<<Ko, 256, 0, st>>>(w, Cg, kh, kw, zero_to, inv, wb, alpha, side, side_pitch, c_pad);
+    NB_CUDA(launch_dependent(binarize_rows_kernel<0>, dim3(Ko), dim3(256), 0, st, w, Cg, kh, kw, zero_to, inv, wb,
+                             alpha, side, side_pitch, c_pad));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -621,8 +651,8 @@ int binary_conv_operands_i8(const float *w, int Ko, int Cg, int kh, int kw, floa
 
 int codes_conv_weights(const float *wq, int Ko, int Cg, int kh, int kw, float delta, void *side, int64_t side_pitch,
                        int c_pad, cudaStream_t st) {
-  codes_conv_weights_kernel<<<Ko, 256, 0, st>>>(wq, Cg, kh, kw, 1.0f / delta, reinterpret_cast<int8_t *>(side),
-                                                side_pitch, c_pad);
+  NB_CUDA(launch_dependent(codes_conv_weights_kernel, dim3(Ko), dim3(256), 0, st, wq, Cg, kh, kw, 1.0f / delta,
+                           reinterpret_cast<int8_t *>(side), side_pitch, c_pad));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -634,8 +664,8 @@ int split_rows_bf16(const float *x, int64_t rows, int K, int64_t Kp, int planes,
   const int64_t cap = (int64_t)sm_count() * 64;
   gy = gy > cap ? cap : (gy < 1 ? 1 : gy);
   gy = gy > 65535 ? 65535 : gy;
-  split_rows_kernel<<<dim3((unsigned)(Kp / 64), (unsigned)gy), dim3(64, 4), 0, st>>>(
-      x, rows, K, Kp, planes, col_scale, reinterpret_cast<__nv_bfloat16 *>(out));
+  NB_CUDA(launch_dependent(split_rows_kernel, dim3((unsigned)(Kp / 64), (unsigned)gy), dim3(64, 4), 0, st, x, rows, K,
+                           Kp, planes, col_scale, reinterpret_cast<__nv_bfloat16 *>(out)));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -646,16 +676,10 @@ int split_rows_bf16(const float *x, int64_t rows, int K, int64_t Kp, int planes,
 // significant bits for every element within 2^-18 of the maximum, an absolute error of at most 2^-40
 // of the maximum below that (p1 is then subnormal), which no fp32 sum over a filter window resolves.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int half_pair_exponent(uint32_t maxbits) {
-  const int E = (int)(maxbits >> 23);
-  if (E == 0 || E >= 255)
-    return 0; // zero, denormal or non-finite maximum: no scaling
-  const int e = E - 127 - 14;
-  return e < -100 ? -100 : e;
-}
-
 __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restrict__ x, size_t n,
                                                           uint32_t *__restrict__ maxbits) {
+  pdl_wait();
+  pdl_trigger();
   uint32_t m = 0;
   const size_t stride = (size_t)gridDim.x * 256;
   const size_t n4 = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) ? n / 4 : 0;
@@ -674,6 +698,8 @@ __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restric
 // out[i] = (in ? in[i] : 1) * 2^e: the per-row factor that undoes the activation scaling
 __global__ void half_pair_row_scale_kernel(const float *__restrict__ in, int n, const uint32_t *__restrict__ maxbits,
                                            float *__restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     const float up = __int_as_float((127 + half_pair_exponent(*maxbits)) << 23);
@@ -688,6 +714,8 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_half_pair_kernel(const float
                                                                      int groups, int Cg, int c_pad_g, int ctot,
                                                                      const uint32_t *__restrict__ maxbits,
                                                                      __half *__restrict__ out, int64_t plane_stride) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[64][33];
   const float down = __int_as_float((127 - half_pair_exponent(*maxbits)) << 23);
   const int n = blockIdx.z;
@@ -725,14 +753,15 @@ int nchw_to_nhwc_half_pair(const float *x, int N, int C, int HW, int groups, int
   size_t blocks = (n / 4 + 255) / 256;
   const size_t cap = (size_t)sm_count() * 16;
   blocks = blocks < 1 ? 1 : (blocks > cap ? cap : blocks);
-  absmax_bits_kernel<<<(unsigned)blocks, 256, 0, st>>>(x, n, maxbits);
+  NB_CUDA(launch_dependent(absmax_bits_kernel, dim3((unsigned)blocks), dim3(256), 0, st, x, n, maxbits));
   NB_LAUNCH_CHECK();
-  half_pair_row_scale_kernel<<<(rows + 255) / 256, 256, 0, st>>>(row_scale_in, rows, maxbits, row_scale_out);
+  NB_CUDA(launch_dependent(half_pair_row_scale_kernel, dim3((rows + 255) / 256), dim3(256), 0, st, row_scale_in, rows,
+                           maxbits, row_scale_out));
   NB_LAUNCH_CHECK();
   NB_CHECK(ctot % 2 == 0, NB200_EVALUE, "channel slots must come in pairs");
   const dim3 grid((HW + 31) / 32, (ctot + 63) / 64, N);
-  nchw_to_nhwc_half_pair_kernel<<<grid, 256, 0, st>>>(x, C, HW, groups, Cg, c_pad_g, ctot, maxbits,
-                                                      reinterpret_cast<__half *>(out), (int64_t)N * HW * ctot);
+  NB_CUDA(launch_dependent(nchw_to_nhwc_half_pair_kernel, grid, dim3(256), 0, st, x, C, HW, groups, Cg, c_pad_g, ctot,
+                           maxbits, reinterpret_cast<__half *>(out), (int64_t)N * HW * ctot));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -749,14 +778,14 @@ int nchw_to_nhwc_planes(const float *x, int N, int C, int HW, int groups, int Cg
       NB_CUDA(launch_dependent(nchw_to_nhwc_i8_vec_kernel, grid8, dim3(256), 0, st, x, C, HW, groups, Cg, c_pad_g, ctot,
                                reinterpret_cast<int8_t *>(out), 1.0f / delta));
     else
-      nchw_to_nhwc_i8_kernel<<<grid8, 256, 0, st>>>(x, C, HW, groups, Cg, c_pad_g, ctot,
-                                                    reinterpret_cast<int8_t *>(out), 1.0f / delta);
+      NB_CUDA(launch_dependent(nchw_to_nhwc_i8_kernel, grid8, dim3(256), 0, st, x, C, HW, groups, Cg, c_pad_g, ctot,
+                               reinterpret_cast<int8_t *>(out), 1.0f / delta));
   } else if (planes == 3) {
-    nchw_to_nhwc_kernel<__nv_bfloat16, 3><<<grid, 256, 0, st>>>(x, C, HW, groups, Cg, c_pad_g, ctot,
-                                                                reinterpret_cast<__nv_bfloat16 *>(out), ps, 0.f);
+    NB_CUDA(launch_dependent(nchw_to_nhwc_kernel<__nv_bfloat16, 3>, grid, dim3(256), 0, st, x, C, HW, groups, Cg,
+                             c_pad_g, ctot, reinterpret_cast<__nv_bfloat16 *>(out), ps, 0.f));
   } else {
-    nchw_to_nhwc_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(x, C, HW, groups, Cg, c_pad_g, ctot,
-                                                                reinterpret_cast<__nv_bfloat16 *>(out), ps, 0.f);
+    NB_CUDA(launch_dependent(nchw_to_nhwc_kernel<__nv_bfloat16, 1>, grid, dim3(256), 0, st, x, C, HW, groups, Cg,
+                             c_pad_g, ctot, reinterpret_cast<__nv_bfloat16 *>(out), ps, 0.f));
   }
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -765,23 +794,24 @@ int nchw_to_nhwc_planes(const float *x, int N, int C, int HW, int groups, int Cg
 int column_sums(const float *a, int64_t rows, int C, float *out, int accumulate, float *partial, int splits,
                 cudaStream_t st) {
   const dim3 grid((C + 255) / 256, splits);
-  column_partial_sums_kernel<<<grid, 256, 0, st>>>(a, rows, C, partial);
+  NB_CUDA(launch_dependent(column_partial_sums_kernel, grid, dim3(256), 0, st, a, rows, C, partial));
   NB_LAUNCH_CHECK();
-  column_finish_kernel<<<(C + 255) / 256, 256, 0, st>>>(partial, C, splits, out, accumulate);
+  NB_CUDA(launch_dependent(column_finish_kernel, dim3((C + 255) / 256), dim3(256), 0, st, partial, C, splits, out,
+                           accumulate));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
 
 int transpose_i8(const int8_t *src, int R, int C, int8_t *dst, int64_t pitch, cudaStream_t st) {
   const dim3 grid((C + 63) / 64, (R + 63) / 64);
-  transpose_i8_kernel<<<grid, 256, 0, st>>>(src, R, C, dst, pitch);
+  NB_CUDA(launch_dependent(transpose_i8_kernel, grid, dim3(256), 0, st, src, R, C, dst, pitch));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
 
 int transpose_f32(const float *src, int R, int C, float *dst, cudaStream_t st) {
   const dim3 grid((C + 31) / 32, (R + 31) / 32);
-  transpose_f32_kernel<<<grid, 256, 0, st>>>(src, R, C, dst);
+  NB_CUDA(launch_dependent(transpose_f32_kernel, grid, dim3(256), 0, st, src, R, C, dst));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -43,6 +43,19 @@ int nchw_to_nhwc_planes(const float *x, int N, int C, int HW, int groups, int Cg
 int nchw_to_nhwc_half_pair(const float *x, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, void *out,
                            uint32_t *maxbits, const float *row_scale_in, int rows, float *row_scale_out,
                            cudaStream_t st);
+// The same with a scale per image: image_max [N][1 + kHalfPairParts] is scratch; its first N words receive the bits of
+// every image's largest magnitude.
+constexpr int kHalfPairParts = 64;
+int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, void *out,
+                                  uint32_t *image_max, cudaStream_t st);
+// Exponent e of the scaling x * 2^-e of the two fp16 pieces, from the bits of the largest magnitude.
+__host__ __device__ __forceinline__ int half_pair_exponent(uint32_t maxbits) {
+  const int E = (int)(maxbits >> 23);
+  if (E == 0 || E >= 255)
+    return 0; // zero, denormal or non-finite maximum: no scaling
+  const int e = E - 127 - 14;
+  return e < -100 ? -100 : e;
+}
 // int8 [R, C] -> [C][pitch].
 int transpose_i8(const int8_t *src, int R, int C, int8_t *dst, int64_t pitch, cudaStream_t st);
 // fp32 [R, C] -> [C][R].

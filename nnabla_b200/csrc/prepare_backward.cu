@@ -10,6 +10,7 @@
 //                    stride and dilation exchanged     -> batch_to_inner
 //   bias gradient:   sums of dy over batch and pixels  -> channel_sums
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "pdl.cuh"
 #include "prepare.cuh"
@@ -35,6 +36,8 @@ __global__ void __launch_bounds__(256) dy_to_nhwc_stuffed_kernel(const float *__
                                                                  const float *__restrict__ chan_scale,
                                                                  __nv_bfloat16 *__restrict__ out,
                                                                  int64_t plane_stride) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[32][33];
   const int n = blockIdx.z;
   const int HW = Ho * Wo;
@@ -67,31 +70,80 @@ __global__ void __launch_bounds__(256) dy_to_nhwc_stuffed_kernel(const float *__
   }
 }
 
+// parts[n][gridDim.x]: the bits of the largest magnitude of image n's shares (non-negative floats order like their bits; a
+// NaN ends above infinity). HBM-bound, four loads in flight per thread.
+__global__ void __launch_bounds__(256) image_absmax_kernel(const float *__restrict__ x, int64_t per_image,
+                                                           uint32_t *__restrict__ parts) {
+  pdl_wait();
+  pdl_trigger();
+  const float *xs = x + (int64_t)blockIdx.y * per_image;
+  const int64_t begin = per_image / 4 * blockIdx.x / gridDim.x * 4;
+  const int64_t end = blockIdx.x + 1 == gridDim.x ? per_image : per_image / 4 * (blockIdx.x + 1) / gridDim.x * 4;
+  uint32_t m = 0;
+  if (((reinterpret_cast<uintptr_t>(x) & 15) | (per_image & 3)) == 0) {
+#pragma unroll 4
+    for (int64_t i = begin + 4 * threadIdx.x; i < end; i += 1024) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(xs + i));
+      m = max(max(m, __float_as_uint(fabsf(v.x))), max(__float_as_uint(fabsf(v.y)), __float_as_uint(fabsf(v.z))));
+      m = max(m, __float_as_uint(fabsf(v.w)));
+    }
+  } else {
+#pragma unroll 8
+    for (int64_t i = begin + threadIdx.x; i < end; i += 256)
+      m = max(m, __float_as_uint(fabsf(__ldg(xs + i))));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  __shared__ uint32_t warps[8];
+  if ((threadIdx.x & 31) == 0)
+    warps[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = __reduce_max_sync(0xffffffffu, threadIdx.x < 8 ? warps[threadIdx.x] : 0u);
+    if (threadIdx.x == 0)
+      parts[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = m;
+  }
+}
+
 // src [N][C][HW] fp32 -> channel-last bf16 planes [planes][N][HW][ctot]: the pieces (hi, mid, lo) of every value, channel
 // c of group g at slot g * c_pad_g + c - g * Cg, all other slots zero. `scaled` receives the pieces of
 // src * chan_scale[c] (one rounding: dy * alpha), `plain` those of src itself; either may be NULL, so that dy is read
 // once for both gradients. HBM-bound: 4 B read and 2 B per piece written per value. Blocks of 64 pixels x 64 slots, a
 // thread converts four slots of four pixels; a pixel's row of 64 slots is transposed through shared memory in 16-byte
 // chunks (XORed with the pixel quad, at most two lanes to a bank) and leaves as 128 bytes.
-template <bool kVec, int PLANES>
+// kHalf: two fp16 pieces of src * 2^-e with e from the image's largest magnitude, the maximum of image_parts[n][parts],
+// left in image_max[n]. The images go last to first, against the order that the maxima were taken in, so that most of
+// them still come from L2: [128, 256, 28, 28] 50 us for the two passes (82 us with the maximum of the whole tensor and
+// 4-byte stores).
+template <bool kVec, int PLANES, bool kHalf>
 __global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restrict__ src, int C, int HW, int groups, int Cg,
                                                           int c_pad_g, int ctot, const float *__restrict__ chan_scale,
-                                                          __nv_bfloat16 *__restrict__ scaled,
-                                                          __nv_bfloat16 *__restrict__ plain, int64_t plane_stride) {
+                                                          uint16_t *__restrict__ scaled, uint16_t *__restrict__ plain,
+                                                          int64_t plane_stride, const uint32_t *__restrict__ image_parts,
+                                                          int parts, uint32_t *__restrict__ image_max) {
   __shared__ uint4 tile[PLANES][64][8];
   pdl_wait();
   pdl_trigger();
-  const int n = blockIdx.z, p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
+  const int n = kHalf ? gridDim.z - 1 - blockIdx.z : blockIdx.z, p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
   const int px4 = threadIdx.x & 15, chq = threadIdx.x >> 4;
   const int p = p0 + 4 * px4, dq = d0 + 4 * chq;
   const int g = dq / c_pad_g, cc0 = dq - g * c_pad_g; // c_pad_g is a multiple of 16: one group for the four slots
   const bool ok = dq < ctot && g < groups;
   const float *base = src + ((int64_t)n * C + (g * Cg + cc0)) * HW + p;
+  float down = 1.0f;
+  if (kHalf) {
+    uint32_t m = 0;
+    for (int i = threadIdx.x & 31; i < parts; i += 32)
+      m = max(m, __ldg(image_parts + (int64_t)n * parts + i));
+    m = __reduce_max_sync(0xffffffffu, m);
+    down = __int_as_float((127 - half_pair_exponent(m)) << 23);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+      image_max[n] = m;
+  }
   float v[4][4], f[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const bool live = ok && cc0 + r < Cg;
-    f[r] = live && scaled && chan_scale ? __ldg(chan_scale + g * Cg + cc0 + r) : 1.0f;
+    f[r] = kHalf ? down : live && scaled && chan_scale ? __ldg(chan_scale + g * Cg + cc0 + r) : 1.0f;
     if (kVec) {
       const float4 q = live && p < HW ? __ldcs(reinterpret_cast<const float4 *>(base + (int64_t)r * HW))
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -103,24 +155,33 @@ __global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restric
     }
   }
 #pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-    __nv_bfloat16 *out = pass == 0 ? scaled : plain;
+  for (int pass = 0; pass < (kHalf ? 1 : 2); ++pass) {
+    uint16_t *out = pass == 0 ? scaled : plain;
     if (!out)
       continue;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      __nv_bfloat16 h[4], m[4], l[4];
+      uint16_t piece[3][4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        split3(pass == 0 && chan_scale ? __fmul_rn(v[r][k], f[r]) : v[r][k], h[r], m[r], l[r]);
+      for (int r = 0; r < 4; ++r) {
+        const float a = kHalf || (pass == 0 && chan_scale) ? __fmul_rn(v[r][k], f[r]) : v[r][k];
+        if (kHalf) {
+          const __half h = __float2half_rn(a);
+          piece[0][r] = __half_as_ushort(h);
+          piece[1][r] = __half_as_ushort(__float2half_rn(__fsub_rn(a, __half2float(h))));
+        } else {
+          __nv_bfloat16 h, m, l;
+          split3(a, h, m, l);
+          piece[0][r] = __bfloat16_as_ushort(h);
+          piece[1][r] = __bfloat16_as_ushort(m);
+          piece[2][r] = __bfloat16_as_ushort(l);
+        }
+      }
       const int chunk = (chq >> 1) ^ (px4 & 7);
 #pragma unroll
-      for (int pl = 0; pl < PLANES; ++pl) {
-        const __nv_bfloat16 *s = pl == 0 ? h : (pl == 1 ? m : l);
-        const __nv_bfloat162 a = __halves2bfloat162(s[0], s[1]), b = __halves2bfloat162(s[2], s[3]);
+      for (int pl = 0; pl < PLANES; ++pl)
         reinterpret_cast<uint2 *>(&tile[pl][4 * px4 + k][chunk])[chq & 1] =
-            make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
-      }
+            make_uint2(piece[pl][0] | (uint32_t)piece[pl][1] << 16, piece[pl][2] | (uint32_t)piece[pl][3] << 16);
     }
     __syncthreads();
 #pragma unroll
@@ -160,6 +221,8 @@ __global__ void __launch_bounds__(256) transpose_binary_weights_kernel(const flo
 template <int PLANES>
 __global__ void flip_transpose_weights_kernel(const float *__restrict__ wb, int Ko, int Cg, int kh, int kw, int Kog,
                                               int k_slots, __nv_bfloat16 *__restrict__ side, int64_t plane_stride) {
+  pdl_wait();
+  pdl_trigger();
   const int taps = kh * kw;
   const int64_t total = (int64_t)Ko * Cg * taps;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -189,6 +252,8 @@ template <int PLANES>
 __global__ void __launch_bounds__(256) batch_to_inner_kernel(const float *__restrict__ src, int N, int64_t R,
                                                              int64_t src_row_stride, int Np,
                                                              __nv_bfloat16 *__restrict__ out, int64_t plane_stride) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.x * 32;
   const int n0 = blockIdx.y * 32;
@@ -220,6 +285,8 @@ __global__ void __launch_bounds__(256) batch_to_inner_kernel(const float *__rest
 // a second kernel adds the partials of each map in order.
 __global__ void __launch_bounds__(256) channel_partial_sums_kernel(const float *__restrict__ dy, int N, int Ko, int HW,
                                                                    float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
   const int o = blockIdx.x, s = blockIdx.y, splits = gridDim.y;
   float acc = 0.0f;
   for (int n = s; n < N; n += splits) {
@@ -241,6 +308,8 @@ __global__ void __launch_bounds__(256) channel_partial_sums_kernel(const float *
 
 __global__ void channel_finish_kernel(const float *__restrict__ partial, int Ko, int splits, float *__restrict__ out,
                                       int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= Ko)
     return;
@@ -255,6 +324,8 @@ __global__ void channel_finish_kernel(const float *__restrict__ partial, int Ko,
 // dW[o][c][taps]: the splits are added in order, then dW is overwritten or added to.
 __global__ void permute_weight_grad_kernel(const float *__restrict__ staged, int splits, int Cg, int Kog, int taps,
                                            float *__restrict__ dw, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t total = (int64_t)Cg * Kog * taps;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int t = (int)(i % taps);
@@ -280,9 +351,9 @@ int dy_to_nhwc_stuffed(const float *dy, int N, int Ko, int Ho, int Wo, int group
                        int Hs, int Ws, int sh, int sw, const float *chan_scale, void *out, cudaStream_t st) {
   NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
   const dim3 grid((Ho * Wo + 31) / 32, (ctot + 31) / 32, N);
-  dy_to_nhwc_stuffed_kernel<<<grid, 256, 0, st>>>(dy, Ko, Ho, Wo, groups, Kog, k_pad_g, ctot, Hs, Ws, sh, sw,
-                                                  chan_scale, reinterpret_cast<__nv_bfloat16 *>(out),
-                                                  (int64_t)N * Hs * Ws * ctot);
+  NB_CUDA(launch_dependent(dy_to_nhwc_stuffed_kernel, grid, dim3(256), 0, st, dy, Ko, Ho, Wo, groups, Kog, k_pad_g,
+                           ctot, Hs, Ws, sh, sw, chan_scale, reinterpret_cast<__nv_bfloat16 *>(out), (int64_t)N * Hs *
+                           Ws * ctot));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -292,18 +363,34 @@ int nhwc_pieces(const float *src, int N, int C, int HW, int groups, int Cg, int 
   NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
   const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
   const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  auto kernel = planes == 3 ? (vec ? nhwc_pieces_kernel<true, 3> : nhwc_pieces_kernel<false, 3>)
-                            : (vec ? nhwc_pieces_kernel<true, 1> : nhwc_pieces_kernel<false, 1>);
+  auto kernel = planes == 3 ? (vec ? nhwc_pieces_kernel<true, 3, false> : nhwc_pieces_kernel<false, 3, false>)
+                            : (vec ? nhwc_pieces_kernel<true, 1, false> : nhwc_pieces_kernel<false, 1, false>);
   NB_CUDA(launch_dependent(kernel, grid, dim3(256), 0, st, src, C, HW, groups, Cg, c_pad_g, ctot, chan_scale,
-                           static_cast<__nv_bfloat16 *>(scaled), static_cast<__nv_bfloat16 *>(plain),
-                           (int64_t)N * HW * ctot));
-  NB_LAUNCH_CHECK();
+                           static_cast<uint16_t *>(scaled), static_cast<uint16_t *>(plain), (int64_t)N * HW * ctot,
+                           (const uint32_t *)nullptr, 0, (uint32_t *)nullptr));
+  return NB200_OK;
+}
+
+int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot,
+                                  void *out, uint32_t *image_max, cudaStream_t st) {
+  NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
+  const int64_t per_image = (int64_t)C * HW;
+  // 4096 values per block, a few loads per thread, up to what a warp reads back in two
+  const int parts = (int)(per_image < 4096 ? 1 : per_image / 4096 < kHalfPairParts ? per_image / 4096 : kHalfPairParts);
+  NB_CUDA(launch_dependent(image_absmax_kernel, dim3(parts, N), dim3(256), 0, st, x, per_image, image_max + N));
+  const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
+  const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  NB_CUDA(launch_dependent(vec ? nhwc_pieces_kernel<true, 2, true> : nhwc_pieces_kernel<false, 2, true>, grid,
+                           dim3(256),
+                           0, st, x, C, HW, groups, Cg, c_pad_g, ctot, (const float *)nullptr, static_cast<uint16_t *>(out),
+                           (uint16_t *)nullptr, (int64_t)N * HW * ctot, image_max + N, parts, image_max));
   return NB200_OK;
 }
 
 int transpose_binary_weights(const float *wb, int Ko, int Cg, int taps, int groups, int k_slots, void *side,
                              cudaStream_t st) {
-  NB_CUDA(launch_dependent(transpose_binary_weights_kernel, dim3(groups * Cg), dim3(256), 0, st, wb, Cg, taps, Ko / groups,
+  NB_CUDA(launch_dependent(transpose_binary_weights_kernel, dim3(groups * Cg), dim3(256), 0, st, wb, Cg, taps, Ko /
+                           groups,
                            k_slots, static_cast<__nv_bfloat16 *>(side)));
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -313,11 +400,13 @@ int flip_transpose_weights(const float *wb, int Ko, int Cg, int kh, int kw, int 
                            cudaStream_t st, int planes) {
   const int64_t plane_stride = (int64_t)groups * Cg * kh * kw * k_slots;
   if (planes == 3)
-    flip_transpose_weights_kernel<3><<<capped((int64_t)Ko * Cg * kh * kw, 256), 256, 0, st>>>(
-        wb, Ko, Cg, kh, kw, Ko / groups, k_slots, reinterpret_cast<__nv_bfloat16 *>(side), plane_stride);
+    NB_CUDA(launch_dependent(flip_transpose_weights_kernel<3>, dim3(capped((int64_t)Ko * Cg * kh * kw, 256)), dim3(256),
+                             0, st, wb, Ko, Cg, kh, kw, Ko / groups, k_slots, reinterpret_cast<__nv_bfloat16 *>(side),
+                             plane_stride));
   else
-    flip_transpose_weights_kernel<1><<<capped((int64_t)Ko * Cg * kh * kw, 256), 256, 0, st>>>(
-        wb, Ko, Cg, kh, kw, Ko / groups, k_slots, reinterpret_cast<__nv_bfloat16 *>(side), plane_stride);
+    NB_CUDA(launch_dependent(flip_transpose_weights_kernel<1>, dim3(capped((int64_t)Ko * Cg * kh * kw, 256)), dim3(256),
+                             0, st, wb, Ko, Cg, kh, kw, Ko / groups, k_slots, reinterpret_cast<__nv_bfloat16 *>(side),
+                             plane_stride));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -328,9 +417,11 @@ int batch_to_inner(const float *src, int N, int64_t R, int64_t src_row_stride, i
   const dim3 grid((unsigned)((R + 31) / 32), (unsigned)((N + 31) / 32));
   __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out);
   if (planes == 3)
-    batch_to_inner_kernel<3><<<grid, 256, 0, st>>>(src, N, R, src_row_stride, Np, o, R * Np);
+    NB_CUDA(launch_dependent(batch_to_inner_kernel<3>, grid, dim3(256), 0, st, src, N, R, src_row_stride, Np, o, R *
+                             Np));
   else
-    batch_to_inner_kernel<1><<<grid, 256, 0, st>>>(src, N, R, src_row_stride, Np, o, R * Np);
+    NB_CUDA(launch_dependent(batch_to_inner_kernel<1>, grid, dim3(256), 0, st, src, N, R, src_row_stride, Np, o, R *
+                             Np));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
@@ -338,17 +429,18 @@ int batch_to_inner(const float *src, int N, int64_t R, int64_t src_row_stride, i
 int channel_sums(const float *dy, int N, int Ko, int HW, float *out, int accumulate, float *partial, int splits,
                  cudaStream_t st) {
   NB_CHECK(splits >= 1 && splits <= 65535, NB200_EVALUE, "bad split count");
-  channel_partial_sums_kernel<<<dim3(Ko, splits), 256, 0, st>>>(dy, N, Ko, HW, partial);
+  NB_CUDA(launch_dependent(channel_partial_sums_kernel, dim3(Ko, splits), dim3(256), 0, st, dy, N, Ko, HW, partial));
   NB_LAUNCH_CHECK();
-  channel_finish_kernel<<<(Ko + 255) / 256, 256, 0, st>>>(partial, Ko, splits, out, accumulate);
+  NB_CUDA(launch_dependent(channel_finish_kernel, dim3((Ko + 255) / 256), dim3(256), 0, st, partial, Ko, splits, out,
+                           accumulate));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
 
 int permute_weight_grad(const float *staged, int splits, int Cg, int Kog, int taps, float *dw, int accumulate,
                         cudaStream_t st) {
-  permute_weight_grad_kernel<<<capped((int64_t)Cg * Kog * taps, 256), 256, 0, st>>>(staged, splits, Cg, Kog, taps, dw,
-                                                                                      accumulate);
+  NB_CUDA(launch_dependent(permute_weight_grad_kernel, dim3(capped((int64_t)Cg * Kog * taps, 256)), dim3(256), 0, st,
+                           staged, splits, Cg, Kog, taps, dw, accumulate));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -42,3 +42,19 @@ def test_gradients(n, c, h, w, o, k, pad, stride, dil, group, delta):
     F.check_device_status()
     for got, want in ((dx, xd.grad), (dw, wd.grad), (dx0 - 1, xd.grad), (dw0 - 1, wd.grad), (db, dy.double().sum((0, 2, 3)))):
         assert (got.double() - want).norm() <= 1e-5 * want.norm() + 1e-6 * want.numel() ** 0.5
+
+
+@pytest.mark.parametrize("n,c,h,w,o,k,pad,stride,dil,group", CASES)
+def test_forward(n, c, h, w, o, k, pad, stride, dil, group):
+    """Images of very different magnitudes: each has a scale of its own."""
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(n + c)
+    x = torch.randn(n, c, h, w, device="cuda", generator=g)
+    x *= torch.exp2(torch.randint(-30, 30, (n, 1, 1, 1), device="cuda", generator=g).float())
+    wt = torch.randn(o, c // group, k, k, device="cuda", generator=g)
+    wb, alpha = torch.empty_like(wt), torch.empty(o, device="cuda")
+    y = F.binary_weight_convolution(x, wt, wb, alpha, None, 1, (pad, pad), (stride, stride), (dil, dil), group)
+    F.check_device_status()
+    want = torch.nn.functional.conv2d(x.double(), wb.double() * alpha.double().view(-1, 1, 1, 1), None, stride, pad, dil, group)
+    error = (y.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+    assert error.max() <= 2e-6
