@@ -259,6 +259,10 @@ int nb200_fixed_point_codes_nhwc(const float *xq, int8_t *codes, int64_t batch, 
 /* codes_nhwc -> y [batch, channels, inner] fp32 = code * delta. */
 int nb200_codes_nhwc_to_f32(const int8_t *codes, float *y, int64_t batch, int64_t channels, int64_t inner, int group,
                             float delta, void *stream);
+/* GlobalAveragePooling of codes_nhwc (group 1): y [batch, channels] fp32, the same bits as
+ * nb200_global_average_pooling_f32 of nb200_codes_nhwc_to_f32. */
+int nb200_global_average_pooling_codes_f32(const int8_t *codes, float *y, int64_t batch, int64_t channels,
+                                           int64_t inner, float delta, void *stream);
 /* nb200_bn_add_relu_fxp_f32 whose result is written as codes_nhwc (the
  * quantizer is always applied; n - sign <= 7). The second operand is either
  * b (fp32 [batch, channels, inner], with or without its own normalisation) or

@@ -410,6 +410,34 @@ __global__ void __launch_bounds__(256) max_pooling_codes_kernel(const int8_t *__
   reinterpret_cast<uint4 *>(out)[((n * G.Ho + oy) * (size_t)G.Wo + ox) * vecs + v] = best;
 }
 
+// GlobalAveragePooling (src/nbla/function/generic/global_average_pooling.cpp) of codes: the values code * delta of a map
+// added in ascending pixel order, then one division. A thread has four slots of a sample; neighbours read whole lines.
+__global__ void __launch_bounds__(128) global_average_pooling_codes_kernel(const int8_t *__restrict__ codes, CodesLayout L,
+                                                                           float delta, float *__restrict__ y) {
+  pdl_wait();
+  pdl_trigger();
+  const int d = 4 * (blockIdx.x * 128 + threadIdx.x), n = blockIdx.y;
+  if (d >= L.slots)
+    return;
+  const int8_t *src = codes + (int64_t)n * L.HW * L.slots + d;
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+  for (int p = 0; p < L.HW; ++p) {
+    const char4 q = __ldg(reinterpret_cast<const char4 *>(src + (int64_t)p * L.slots));
+    s[0] = __fadd_rn(s[0], __fmul_rn((float)q.x, delta));
+    s[1] = __fadd_rn(s[1], __fmul_rn((float)q.y, delta));
+    s[2] = __fadd_rn(s[2], __fmul_rn((float)q.z, delta));
+    s[3] = __fadd_rn(s[3], __fmul_rn((float)q.w, delta));
+  }
+  const int g = d / L.c_pad_g; // c_pad_g is a multiple of 16: one group for the four slots
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int cc = d + j - g * L.c_pad_g;
+    if (g < L.groups && cc < L.Cg)
+      y[(int64_t)n * L.C + g * L.Cg + cc] = __fdiv_rn(s[j], (float)L.HW);
+  }
+}
+
 int fill_fxp(FxpParams &P, int sign, int n, float delta) {
   // the reference's setup (fixed_point_quantize.cpp:31-42)
   NB_CHECK(n > 0 && delta > 0.f, NB200_EVALUE, "Both bit width and delta should be positive.");
@@ -547,6 +575,20 @@ extern "C" int nb200_codes_nhwc_to_f32(const int8_t *codes, float *y, int64_t ba
   const dim3 grid((L.HW + kTilePx - 1) / kTilePx, (L.slots + kTileSlots - 1) / kTileSlots, (unsigned)batch);
   NB_CUDA(launch_dependent(codes_nhwc_to_f32_kernel, grid, dim3(256), 0, as_stream(stream), codes, L, delta, y));
   NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+extern "C" int nb200_global_average_pooling_codes_f32(const int8_t *codes, float *y, int64_t batch, int64_t channels,
+                                                      int64_t inner, float delta, void *stream) {
+  CodesLayout L;
+  NB_TRY(codes_layout(L, batch, channels, inner, 1));
+  NB_CHECK(delta > 0.f, NB200_EVALUE, "delta should be positive");
+  if (batch == 0)
+    return NB200_OK;
+  NB_CHECK(codes && y, NB200_EVALUE, "null data pointer");
+  NB_CHECK((reinterpret_cast<uintptr_t>(codes) & 3) == 0, NB200_EVALUE, "code tensors must be 4-byte aligned");
+  NB_CUDA(launch_dependent(global_average_pooling_codes_kernel, dim3((unsigned)((L.slots + 511) / 512), (unsigned)batch),
+                           dim3(128), 0, as_stream(stream), codes, L, delta, y));
   return NB200_OK;
 }
 

@@ -7,6 +7,7 @@
 
 #include "gemm.cuh"
 #include "gemm2.cuh"
+#include "small_gemm.cuh"
 #include "prepare.cuh"
 
 namespace nb200 {
@@ -195,6 +196,15 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
   NB_CHECK(x && w && wb && y, NB200_EVALUE, "null data pointer");
   NB_CHECK(bf16_exact(zero_to), NB200_ENOTIMPL,
            "quantize_zero_to = %g is not representable in bf16; the exact tensor-core path needs it to be", zero_to);
+  if (small_gemm_binarized(M, N, K)) {
+    SmallGemm P{};
+    P.a = x, P.b = w, P.y = y;
+    P.M = (int)M, P.N = (int)N, P.K = (int)K;
+    P.col_bias = bias;
+    P.zero_to = zero_to, P.inv = (float)1 / K; // binary_weight_affine.cpp:68
+    P.wb = wb, P.alpha = alpha;
+    return launch_small_gemm<false, false, SmallB::kBinarize>(P, st);
+  }
   const int64_t Kp = round_up(K, 64);
   const size_t planes_bytes = (size_t)3 * M * Kp * 2;
   const size_t side_bytes = (size_t)N * Kp * 2;
@@ -321,6 +331,17 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
   NB_CHECK(dy != nullptr, NB200_EVALUE, "dy is NULL");
   if (dx) {
     NB_CHECK(w != nullptr, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
+    if (w_exact_bf16 ? small_gemm_scaled(M, K, N) : small_gemm_plain(M, K, N)) {
+      SmallGemm P{};
+      P.a = dy, P.b = w, P.y = dx;
+      P.M = (int)M, P.N = (int)K, P.K = (int)N;
+      P.a_scale = w_col_scale;
+      P.accumulate = accum_dx;
+      NB_TRY((launch_small_gemm<false, true, SmallB::kPlain>(P, st)));
+      dx = nullptr;
+    }
+  }
+  if (dx) {
     const int64_t Np = round_up(N, 64);
     const int planes_w = w_exact_bf16 ? 1 : 3;
     const size_t a_bytes = round_up((size_t)3 * M * Np * 2, 256), b_bytes = (size_t)planes_w * K * Np * 2;
@@ -337,6 +358,21 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
   }
   if (dw) {
     NB_CHECK(x != nullptr, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
+    if (small_gemm_transposed(K, N, M)) {
+      SmallGemm P{};
+      P.a = x, P.b = dy, P.y = dw;
+      P.M = (int)K, P.N = (int)N, P.K = (int)M;
+      P.accumulate = accum_dw;
+      P.sums = db;
+      P.accumulate_sums = accum_db;
+      if (db)
+        NB_TRY((launch_small_gemm<true, false, SmallB::kColumnSums>(P, st)));
+      else
+        NB_TRY((launch_small_gemm<true, false, SmallB::kPlain>(P, st)));
+      dw = db = nullptr;
+    }
+  }
+  if (dw) {
     const int64_t Mp = round_up(M, 64);
     const size_t xt_bytes = round_up((size_t)K * M * 4, 256), dyt_bytes = round_up((size_t)N * M * 4, 256);
     const size_t a_bytes = round_up((size_t)3 * K * Mp * 2, 256), b_bytes = round_up((size_t)3 * N * Mp * 2, 256);
@@ -433,6 +469,13 @@ int nb200_affine_f32(const float *x, const float *w, const float *bias, float *y
   NB_CHECK(M < (1ll << 31) && K < (1ll << 31) && N < (1ll << 31), NB200_EVALUE, "extent exceeds 2^31");
   NB_CHECK(x && w && y, NB200_EVALUE, "null data pointer");
   cudaStream_t st = as_stream(stream);
+  if (small_gemm_plain(M, N, K)) {
+    SmallGemm P{};
+    P.a = x, P.b = w, P.y = y;
+    P.M = (int)M, P.N = (int)N, P.K = (int)K;
+    P.col_bias = bias;
+    return launch_small_gemm<false, false, SmallB::kPlain>(P, st);
+  }
   const int64_t Kp = round_up(K, 64);
   // w [K, N] is transposed through a fp32 staging pass into [N][K] planes.
   AsyncScratch scratch(st);

@@ -346,6 +346,7 @@ PyMethodDef methods[] = {
     ENTRY(nb200_binary_weights_prepare_i8),
     ENTRY(nb200_fixed_point_codes_nhwc),
     ENTRY(nb200_codes_nhwc_to_f32),
+    ENTRY(nb200_global_average_pooling_codes_f32),
     ENTRY(nb200_max_pooling_f32),
     ENTRY(nb200_max_pooling_backward_f32),
     ENTRY(nb200_max_pooling_codes_nhwc),

@@ -1182,7 +1182,15 @@ def convolution_relu_fixed_point_codes(x, weight, bias=None, pad=None, stride=No
 
 def global_average_pooling_codes(codes, shape, delta=2 ** -4):
     """GlobalAveragePooling of a tensor held as channel-last codes: [batch, channels, 1, 1] fp32."""
-    return global_average_pooling(codes_nhwc_to_float(codes, shape, delta))
+    shape = tuple(int(v) for v in shape)
+    batch, ch = shape[0], shape[1]
+    inner = 1
+    for v in shape[2:]:
+        inner *= v
+    codes = _check_codes(codes, batch, inner, ch, 1)
+    y = L.empty((batch, ch, 1, 1), codes)
+    L.nb200_global_average_pooling_codes_f32(codes, y, batch, ch, inner, delta)
+    return y
 
 
 # ---------------------------------------------------------------------------

@@ -223,3 +223,29 @@ def test_fixed_point_affine_operand_tiles(F, M, K, N):
     y = F.affine(dev(xq), dev(wq), None, fixed_point=(2.0 ** -5, 2.0 ** -10)).cpu().numpy()
     exact = (np.round(xq.astype(np.float64) * 2 ** 5) @ np.round(wq.astype(np.float64) * 2 ** 10)).astype(np.float32)
     assert np.array_equal(y, exact * np.float32(2.0 ** -15))
+
+
+# around the tile (16 or 32 x 32), the 128-value chunk, the ring of stages and the rows that are not whole float4
+@pytest.mark.parametrize("rows,inmaps,outmaps", [(1, 1, 1), (15, 127, 31), (17, 129, 33), (32, 128, 32), (33, 512, 130),
+                                                 (5, 700, 1000), (300, 64, 500), (130, 900, 260), (3, 2048, 40)])
+@pytest.mark.parametrize("accum", [False, True])
+def test_small_products(rows, inmaps, outmaps, accum):
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, w, b, dy = (torch.randn(*s, device="cuda", generator=g) for s in ((rows, inmaps), (inmaps, outmaps), (outmaps,),
+                                                                       (rows, outmaps)))
+    close = lambda got, want: (got.double() - want).norm() <= 3e-6 * want.norm() + 1e-9
+    assert close(F.affine(x, w, b), x.double() @ w.double() + b.double())
+    wb, alpha = torch.full_like(w, 7.0), torch.full((outmaps,), 7.0, device="cuda")
+    y = F.binary_weight_affine(x, w, wb, alpha, b)
+    signs = torch.where(w > 0, 1.0, torch.where(w < 0, -1.0, 1.0))
+    assert torch.equal(wb, signs) and close(alpha, w.double().abs().mean(0))
+    scaled = signs.double() * alpha.double()
+    assert close(y, x.double() @ scaled + b.double())
+    for weight, grads in ((scaled, lambda *a, **k: F.binary_weight_affine_backward(x, wb, alpha, dy, **k)),
+                          (w.double(), lambda *a, **k: F.affine_backward(x, w, dy, **k))):
+        wants = (dy.double() @ weight.t(), x.double().t() @ dy.double(), dy.double().sum(0))
+        old = [torch.ones_like(x), torch.ones_like(w), torch.ones_like(b)] if accum else [None] * 3
+        got = grads(accum=(accum,) * 3, grads=tuple(old))
+        assert all(close(a, t + accum) for a, t in zip(got, wants))
+    F.check_device_status()

@@ -321,3 +321,13 @@ def test_two_row_blocks_per_tile(F, batch, channels, maps, height, width):
     got = y[:, :, :maps].transpose(1, 2).reshape(batch, maps, height, width)
     assert shape == (batch, maps, height, width) and torch.equal(got, want)
     assert not y[:, :, maps:].any()
+
+
+@pytest.mark.parametrize("batch,channels,height,width", [(1, 512, 7, 7), (3, 20, 1, 1), (2, 1030, 5, 9)])
+def test_global_average_pooling_of_codes(batch, channels, height, width):
+    """The same bits as the pooling of the fp32 tensor."""
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(channels)
+    x = torch.randint(-127, 128, (batch, channels, height, width), device="cuda", generator=g) * 0.0625
+    codes = F.fixed_point_codes_nhwc(x, 0.0625)
+    assert torch.equal(F.global_average_pooling_codes(codes, x.shape, 0.0625), F.global_average_pooling(x))
