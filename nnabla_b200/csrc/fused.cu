@@ -373,12 +373,14 @@ __global__ void __launch_bounds__(256) codes_nhwc_to_f32_kernel(const int8_t *__
 // ---------------------------------------------------------------------------
 // Max-pooling on codes (channel-last): the value code * delta grows with the
 // code, so the window maximum of the codes is the code of the window maximum.
-// One thread per output pixel and 16 slots: kh * kw 128-bit loads, bytewise maxima.
+// One thread per output pixel and 16 slots: kh * kw 128-bit loads, bytewise maxima. KH x KW windows (0 x 0: any) have all
+// their loads in flight; past the border they read a position of the window again, which changes no maximum.
 // ---------------------------------------------------------------------------
 struct PoolGeom {
   int H, W, Ho, Wo, kh, kw, sh, sw, ph, pw;
 };
 
+template <int KH, int KW>
 __global__ void __launch_bounds__(256) max_pooling_codes_kernel(const int8_t *__restrict__ in, int slots, PoolGeom G,
                                                                 int8_t *__restrict__ out) {
   pdl_wait();
@@ -397,7 +399,25 @@ __global__ void __launch_bounds__(256) max_pooling_codes_kernel(const int8_t *__
   y0 = max(y0, 0);
   x0 = max(x0, 0);
   uint4 best = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
-  for (int iy = y0; iy < y1; ++iy) {
+  if (KH > 0 && y0 < y1 && x0 < x1) {
+    uint4 q[KH > 0 ? KH : 1][KH > 0 ? KW : 1];
+#pragma unroll
+    for (int a = 0; a < KH; ++a)
+#pragma unroll
+      for (int b = 0; b < KW; ++b)
+        q[a][b] = __ldg(reinterpret_cast<const uint4 *>(
+                            in + ((n * G.H + min(y0 + a, y1 - 1)) * (size_t)G.W + min(x0 + b, x1 - 1)) * slots) + v);
+#pragma unroll
+    for (int a = 0; a < KH; ++a)
+#pragma unroll
+      for (int b = 0; b < KW; ++b) {
+        best.x = __vmaxs4(best.x, q[a][b].x);
+        best.y = __vmaxs4(best.y, q[a][b].y);
+        best.z = __vmaxs4(best.z, q[a][b].z);
+        best.w = __vmaxs4(best.w, q[a][b].w);
+      }
+  }
+  for (int iy = y0; KH == 0 && iy < y1; ++iy) {
     const uint4 *row = reinterpret_cast<const uint4 *>(in + ((n * G.H + iy) * (size_t)G.W) * slots) + v;
     for (int ix = x0; ix < x1; ++ix) {
       const uint4 q = __ldg(row + (size_t)ix * vecs);
@@ -616,7 +636,10 @@ extern "C" int nb200_max_pooling_codes_nhwc(const int8_t *codes, int8_t *y_codes
   const int slots = (int)codes_slots(channels, group);
   NB_CHECK(batch <= 65535 && G.Ho <= 65535, NB200_ENOTIMPL, "more than 65535 samples or output rows");
   const dim3 grid((unsigned)((G.Wo * (slots / 16) + 255) / 256), (unsigned)G.Ho, (unsigned)batch);
-  NB_CUDA(launch_dependent(max_pooling_codes_kernel, grid, dim3(256), 0, as_stream(stream), codes, slots, G, y_codes));
+  auto kernel = kernel_h == 3 && kernel_w == 3   ? max_pooling_codes_kernel<3, 3>
+                : kernel_h == 2 && kernel_w == 2 ? max_pooling_codes_kernel<2, 2>
+                                                 : max_pooling_codes_kernel<0, 0>;
+  NB_CUDA(launch_dependent(kernel, grid, dim3(256), 0, as_stream(stream), codes, slots, G, y_codes));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

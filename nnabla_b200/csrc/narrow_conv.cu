@@ -38,6 +38,7 @@
 // falls through to the common teardown.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -112,53 +113,26 @@ __device__ __forceinline__ void split2(float v, __half &p0, __half &p1) {
   p1 = __float2half_rn(__fmul_rn(__fsub_rn(v, __half2float(p0)), 2048.0f));
 }
 
-// max |x| of every sample as fp32 bits (non-negative floats order like their bits; a NaN ends above infinity)
-__global__ void __launch_bounds__(256) narrow_conv_absmax_kernel(const float *__restrict__ x, int64_t per_sample,
-                                                                 uint32_t *__restrict__ maxbits) {
-  pdl_wait();
-  pdl_trigger();
-  const int n = blockIdx.y;
-  const float *xs = x + (int64_t)n * per_sample;
-  uint32_t m = 0;
-  const int64_t vecs = ((reinterpret_cast<uintptr_t>(xs) & 15) == 0) ? per_sample / 4 : 0;
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < vecs; i += (int64_t)gridDim.x * 256) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(xs) + i);
-    m = max(max(m, __float_as_uint(fabsf(v.x))), max(__float_as_uint(fabsf(v.y)), __float_as_uint(fabsf(v.z))));
-    m = max(m, __float_as_uint(fabsf(v.w)));
-  }
-  for (int64_t i = vecs * 4 + (int64_t)blockIdx.x * 256 + threadIdx.x; i < per_sample; i += (int64_t)gridDim.x * 256)
-    m = max(m, __float_as_uint(fabsf(__ldg(xs + i))));
-  m = __reduce_max_sync(0xffffffffu, m);
-  __shared__ uint32_t part[8];
-  if ((threadIdx.x & 31) == 0)
-    part[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; ++i)
-      m = max(m, part[i]);
-    atomicMax(maxbits + n, m);
-  }
-}
-
 // x [N][C][H][W] fp32 -> xs [N][Hp][piece][row_bytes] fp16: unit u of a row holds the stride_w pixels
 // u * stride_w .. (padded column), 8 / stride_w channel slots each; zero outside the image and past C.
-// One block per (kSplitRows staged rows, sample); xscale[n] = 2^e of the sample.
-constexpr int kSplitRows = 8;
+// One block per (split_rows staged rows, sample); xscale[n] = 2^e of the sample.
+constexpr int kAbsmaxParts = 32; // shares of a sample, what a warp reads back at once
 template <int SW>
-__global__ void __launch_bounds__(256) narrow_conv_split_kernel(const float *__restrict__ x, NarrowConv g,
-                                                                const uint32_t *__restrict__ maxbits,
+__global__ void __launch_bounds__(256) narrow_conv_split_kernel(const float *__restrict__ x, NarrowConv g, int split_rows,
+                                                                const uint32_t *__restrict__ maxbits, int parts,
                                                                 uint8_t *__restrict__ xs, float *__restrict__ xscale) {
   pdl_wait();
   pdl_trigger();
   constexpr int cpp = 8 / SW; // channel slots per pixel
   const int n = blockIdx.y;
-  const int e = scale_exponent(maxbits[n], 14);
+  const int lane = threadIdx.x & 31;
+  const int e = scale_exponent(__reduce_max_sync(0xffffffffu, lane < parts ? __ldg(maxbits + n * parts + lane) : 0u), 14);
   const float down = pow2i(-e);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     xscale[n] = pow2i(e);
   const int units = g.row_bytes >> 4;
-  const int py0 = blockIdx.x * kSplitRows;
-  const int rows = min(kSplitRows, g.Hp - py0);
+  const int py0 = blockIdx.x * split_rows;
+  const int rows = min(split_rows, g.Hp - py0);
   for (int i = threadIdx.x; i < rows * units; i += 256) {
     const int r = i / units, u = i - r * units;
     const int py = py0 + r, iy = py - g.ph;
@@ -184,15 +158,48 @@ __global__ void __launch_bounds__(256) narrow_conv_split_kernel(const float *__r
 // chunk stride 128, group stride 256 bytes). Step = (ky, j); value k of chunk c2 is tap
 // kx = (2 j + c2) * stride_w + k / cpp, channel k % cpp. One block per step (every block finds max |w|
 // for itself: the filter is a few thousand values); wscale[0] = 2^-S.
-__global__ void __launch_bounds__(256) narrow_conv_weights_kernel(const float *__restrict__ w, NarrowConv g,
-                                                                  __half *__restrict__ out, float *__restrict__ wscale) {
+// The blocks behind those of the weights take shares of the samples: maxbits[sample][parts] receives the fp32 bits of
+// each share's largest |x| (non-negative floats order like their bits; a NaN ends above infinity).
+__global__ void __launch_bounds__(256) narrow_conv_prepare_kernel(const float *__restrict__ w, NarrowConv g, int steps,
+                                                                  __half *__restrict__ out, float *__restrict__ wscale,
+                                                                  const float *__restrict__ x, int64_t per_sample,
+                                                                  int parts, uint32_t *__restrict__ maxbits) {
   pdl_wait();
   pdl_trigger();
   __shared__ uint32_t part[8];
-  const int count = g.Ko * g.C * g.kh * g.kw;
   uint32_t m = 0;
+  if ((int)blockIdx.x >= steps) {
+    const int share = blockIdx.x - steps, n = share / parts, q = share - n * parts;
+    const float *xs = x + (int64_t)n * per_sample;
+    const int64_t begin = per_sample / 4 * q / parts * 4;
+    const int64_t end = q + 1 == parts ? per_sample : per_sample / 4 * (q + 1) / parts * 4;
+    if (((reinterpret_cast<uintptr_t>(x) & 15) | (per_sample & 3)) == 0) {
+#pragma unroll 4
+      for (int64_t i = begin + 4 * threadIdx.x; i < end; i += 1024) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(xs + i));
+        m = max(max(m, __float_as_uint(fabsf(v.x))), max(__float_as_uint(fabsf(v.y)), __float_as_uint(fabsf(v.z))));
+        m = max(m, __float_as_uint(fabsf(v.w)));
+      }
+    } else {
+#pragma unroll 8
+      for (int64_t i = begin + threadIdx.x; i < end; i += 256)
+        m = max(m, __float_as_uint(fabsf(__ldg(xs + i))));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0)
+      part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      m = __reduce_max_sync(0xffffffffu, threadIdx.x < 8 ? part[threadIdx.x] : 0u);
+      if (threadIdx.x == 0)
+        maxbits[share] = m;
+    }
+    return;
+  }
+  const int count = g.Ko * g.C * g.kh * g.kw;
+#pragma unroll 8
   for (int i = threadIdx.x; i < count; i += 256)
-    m = max(m, __float_as_uint(fabsf(w[i])));
+    m = max(m, __float_as_uint(fabsf(__ldg(w + i))));
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0)
     part[threadIdx.x >> 5] = m;
@@ -355,13 +362,28 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
       int seq = 0;
       bool ok = true;
       const uint32_t idesc128 = ptx::make_idesc(1u, 0u, kM, 128), idesc64 = ptx::make_idesc(1u, 0u, kM, 64);
-      const uint32_t b_base = ptx::smem_u32(b_res), ring_base = ptx::smem_u32(ring);
+      // The MMAs of a tile are issued from one straight piece of code with every address at hand: a loop that worked
+      // them out per step issued 28 MMAs in 2700 cycles that take the tensor core 1650.
+      const uint64_t a_base = ptx::smem_desc_k_plain(ptx::smem_u32(ring), 16u, 128u);
+      const uint64_t b_base = ptx::smem_desc_k_plain(ptx::smem_u32(b_res), 128u, 256u);
+      const uint32_t slot_units = slot_bytes >> 4, piece_units = (uint32_t)g.row_bytes >> 4;
+      int step_ky[kMaxSteps];
+      uint32_t step_unit[kMaxSteps];
+#pragma unroll
+      for (int s = 0; s < kMaxSteps; ++s) {
+        step_ky[s] = s / g.jsteps;
+        step_unit[s] = 2u * (uint32_t)(s - step_ky[s] * g.jsteps);
+      }
+      int n = tile_first / g.Ho, oy = tile_first - n * g.Ho;
       for (int tile = tile_first; tile < tile_last && ok; ++tile, ++seq) {
         const int buf = seq & 1;
         const uint32_t buf_phase = (uint32_t)(seq >> 1) & 1u;
-        const int n = tile / g.Ho, oy = tile - n * g.Ho;
         int first, s0;
         walk.next(n, oy * g.sh, g.kh, first, s0);
+        uint32_t a_unit[kMaxSteps]; // rows 16 bytes apart, the second K chunk 16 bytes behind the first: sliding windows
+#pragma unroll
+        for (int s = 0; s < kMaxSteps; ++s)
+          a_unit[s] = (uint32_t)((s0 + step_ky[s]) & (kRing - 1)) * slot_units + step_unit[s];
         if (!ptx::mbar_wait(tmem_empty + buf, buf_phase ^ 1u, abort_flag) ||
             !ptx::mbar_wait(full_bar + (seq & (kInFlight - 1)), (uint32_t)(seq / kInFlight) & 1u, abort_flag)) {
           if (*abort_flag == 0)
@@ -371,20 +393,16 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
         }
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kAccCols);
-        uint32_t accumulate = 0;
-        int step = 0;
-        for (int ky = 0; ky < g.kh; ++ky) {
-          const uint32_t row = ring_base + (uint32_t)((s0 + ky) % kRing) * slot_bytes;
-          for (int j = 0; j < g.jsteps; ++j, ++step) {
-            // rows 16 bytes apart, the second K chunk 16 bytes behind the first: sliding windows
-            const uint64_t a0 = ptx::smem_desc_k_plain(row + (uint32_t)j * 32u, 16u, 128u);
-            const uint64_t a1 = ptx::smem_desc_k_plain(row + (uint32_t)g.row_bytes + (uint32_t)j * 32u, 16u, 128u);
-            const uint64_t b = ptx::smem_desc_k_plain(b_base + (uint32_t)step * kStepBytes, 128u, 256u);
-            ptx::mma_bf16(d_tmem, a0, b, idesc128, accumulate);  // x0 x [w0; w1] -> columns 0..127
-            ptx::mma_bf16(d_tmem + kN, a1, b, idesc64, 1u);      // x1 x [w0]     -> columns 64..127
-            accumulate = 1;
+#pragma unroll
+        for (int s = 0; s < kMaxSteps; ++s) {
+          if (s < steps) {
+            const uint64_t a0 = a_base + a_unit[s], b = b_base + (uint64_t)(s * (kStepBytes / 16));
+            ptx::mma_bf16(d_tmem, a0, b, idesc128, s > 0);                  // x0 x [w0; w1] -> columns 0..127
+            ptx::mma_bf16(d_tmem + kN, a0 + piece_units, b, idesc64, 1u);   // x1 x [w0]     -> columns 64..127
           }
         }
+        if (++oy == g.Ho)
+          oy = 0, ++n;
         ptx::mma_commit(done_bar + (seq & (kInFlight - 1)));
         ptx::mma_commit(tmem_full + buf);
       }
@@ -557,30 +575,29 @@ int narrow_conv_tc(const float *x, const float *w, const float *bias, float *y, 
   // scratch: weights | staged input | per-sample maxima (bits) | per-sample 2^e | 2^-S
   const size_t w_bytes = (size_t)p.steps * kStepBytes;
   const size_t xs_bytes = (size_t)batch * g.Hp * 2 * p.row_bytes;
-  const size_t tail_bytes = ((size_t)batch * 8 + 16 + 255) & ~size_t(255);
+  const size_t tail_bytes = ((size_t)batch * 4 * (kAbsmaxParts + 1) + 16 + 255) & ~size_t(255);
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc(w_bytes + xs_bytes + tail_bytes));
   uint8_t *wprep = static_cast<uint8_t *>(scratch.p);
   uint8_t *xs = wprep + w_bytes;
   uint32_t *maxbits = reinterpret_cast<uint32_t *>(xs + xs_bytes);
-  float *xscale = reinterpret_cast<float *>(maxbits + batch);
+  float *xscale = reinterpret_cast<float *>(maxbits + (size_t)batch * kAbsmaxParts);
   float *wscale = xscale + batch;
-  NB_CUDA(cudaMemsetAsync(maxbits, 0, (size_t)batch * 4, st));
   const int64_t per_sample = (int64_t)channels * height * width;
-  int blocks = (int)((per_sample / 4 + 255) / 256);
-  const int cap = (8 * sm_count() + batch - 1) / batch;
-  blocks = blocks < 1 ? 1 : (blocks > cap ? (cap < 1 ? 1 : cap) : blocks);
-  NB_CUDA(launch_dependent(narrow_conv_absmax_kernel, dim3((unsigned)blocks, (unsigned)batch), dim3(256), 0, st, x,
-                           per_sample, maxbits));
-  NB_LAUNCH_CHECK();
-  NB_CUDA(launch_dependent(narrow_conv_weights_kernel, dim3(p.steps), dim3(256), 0, st, w, g, reinterpret_cast<__half
-                           *>(wprep), wscale));
-  NB_LAUNCH_CHECK();
-  const dim3 split_grid((unsigned)((g.Hp + kSplitRows - 1) / kSplitRows), (unsigned)batch);
+  // shares of at least 4096 values, not many more than fill the chip twice (a block's start and end cost two microseconds)
+  const int64_t most = std::min<int64_t>(kAbsmaxParts, 16ll * sm_count() / batch);
+  const int parts = (int)std::max<int64_t>(1, std::min(per_sample / 4096, most));
+  NB_CUDA(launch_dependent(narrow_conv_prepare_kernel, dim3((unsigned)(p.steps + batch * parts)), dim3(256), 0, st, w, g,
+                           p.steps, reinterpret_cast<__half *>(wprep), wscale, x, per_sample, parts, maxbits));
+  // eight rows per block (a few units per thread) where that gives every SM several blocks
+  const int split_rows = (int64_t)batch * g.Hp >= 64ll * sm_count() ? 8 : 2;
+  const dim3 split_grid((unsigned)((g.Hp + split_rows - 1) / split_rows), (unsigned)batch);
   if (stride_w == 2)
-    NB_CUDA(launch_dependent(narrow_conv_split_kernel<2>, split_grid, dim3(256), 0, st, x, g, maxbits, xs, xscale));
+    NB_CUDA(launch_dependent(narrow_conv_split_kernel<2>, split_grid, dim3(256), 0, st, x, g, split_rows, maxbits, parts,
+                             xs, xscale));
   else
-    NB_CUDA(launch_dependent(narrow_conv_split_kernel<1>, split_grid, dim3(256), 0, st, x, g, maxbits, xs, xscale));
+    NB_CUDA(launch_dependent(narrow_conv_split_kernel<1>, split_grid, dim3(256), 0, st, x, g, split_rows, maxbits, parts,
+                             xs, xscale));
   NB_LAUNCH_CHECK();
   static bool configured[64];
   int dev = 0;

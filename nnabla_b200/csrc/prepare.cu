@@ -166,19 +166,28 @@ __device__ __forceinline__ void binarize_row(int o, const float *__restrict__ w,
   const int taps = kh * kw, Kd = Cg * taps;
   const float *wr = w + (int64_t)o * Kd;
   float acc = 0.0f;
-  for (int k = threadIdx.x; k < Kd; k += 256) {
-    const float v = wr[k];
-    const float s = sign_of(v, zero_to);
-    wb[(int64_t)o * Kd + k] = s;
-    acc += fabsf(v);
-    const int c = k / taps, t = k - c * taps;
-    const int64_t dst = (int64_t)o * side_pitch + (int64_t)t * c_pad + c;
-    if (kMode == 1) {
-      reinterpret_cast<int8_t *>(side)[dst] = (int8_t)(int)s;
-    } else if (kMode == 2) {
-      reinterpret_cast<__half *>(side)[dst] = __float2half_rn(s);
-    } else {
-      reinterpret_cast<__nv_bfloat16 *>(side)[dst] = __float2bfloat16_rn(s);
+  for (int k0 = threadIdx.x; k0 < Kd; k0 += 8 * 256) { // eight loads in flight
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      v[u] = k0 + 256 * u < Kd ? __ldg(wr + k0 + 256 * u) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + 256 * u;
+      if (k >= Kd)
+        break;
+      const float s = sign_of(v[u], zero_to);
+      wb[(int64_t)o * Kd + k] = s;
+      acc += fabsf(v[u]);
+      const int c = k / taps, t = k - c * taps;
+      const int64_t dst = (int64_t)o * side_pitch + (int64_t)t * c_pad + c;
+      if (kMode == 1) {
+        reinterpret_cast<int8_t *>(side)[dst] = (int8_t)(int)s;
+      } else if (kMode == 2) {
+        reinterpret_cast<__half *>(side)[dst] = __float2half_rn(s);
+      } else {
+        reinterpret_cast<__nv_bfloat16 *>(side)[dst] = __float2bfloat16_rn(s);
+      }
     }
   }
   if (alpha == nullptr)
@@ -341,29 +350,44 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const float *__restri
   }
 }
 
-// fp32 NCHW (multiples of delta) -> int8 NHWC codes, 64 pixels x 64 channel
-// slots per block. Reads are coalesced along the pixels of one channel plane;
-// the codes are transposed through shared memory (row pitch 17 words, so both
-// the byte writes and the word reads are bank-conflict free) and written as
-// 64-byte runs per pixel.
+// Codes of four multiples of delta as one word: round(v / delta) on the add pipe, where for |t| < 2^22 the low
+// byte of 1.5 * 2^23 + t is the two's complement code.
+__device__ __forceinline__ uint32_t pack_codes(float a, float b, float c, float d, float inv_delta) {
+  const uint32_t i = __float_as_uint(__fadd_rn(__fmul_rn(a, inv_delta), 12582912.0f));
+  const uint32_t j = __float_as_uint(__fadd_rn(__fmul_rn(b, inv_delta), 12582912.0f));
+  const uint32_t k = __float_as_uint(__fadd_rn(__fmul_rn(c, inv_delta), 12582912.0f));
+  const uint32_t l = __float_as_uint(__fadd_rn(__fmul_rn(d, inv_delta), 12582912.0f));
+  return __byte_perm(__byte_perm(i, j, 0x0040), __byte_perm(k, l, 0x0040), 0x5410);
+}
+
+// fp32 NCHW (multiples of delta) -> int8 NHWC codes, 64 pixels x 64 channel slots per block. A thread converts four
+// neighbouring slots of four pixels 16 apart, sixteen loads in flight; the four codes of a pixel go to shared memory as
+// one word and leave in 64-byte runs per pixel. For planes that 128-bit loads cannot read (the loop over single values
+// with one load in flight took 27 us for [256, 512, 7, 7]).
 __device__ __forceinline__ void nchw_to_nhwc_i8_tile(int bx, int by, int n, const float *__restrict__ x, int C, int HW,
                                                      int groups, int Cg, int c_pad_g, int ctot,
                                                      int8_t *__restrict__ out, float inv_delta) {
   __shared__ uint32_t tile[64][17]; // [pixel][16 words of 4 codes + 1 pad]
-  int8_t *tile8 = reinterpret_cast<int8_t *>(&tile[0][0]);
   const int p0 = bx * 64, d0 = by * 64;
-  const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-  const int p = p0 + tx;
-  for (int dd = ty; dd < 64; dd += 4) {
-    const int d = d0 + dd;
-    const int g = d / c_pad_g, cc = d - g * c_pad_g;
-    float v = 0.0f;
-    if (d < ctot && g < groups && cc < Cg && p < HW)
-      v = __ldcs(x + ((int64_t)n * C + (g * Cg + cc)) * HW + p);
-    tile8[tx * 68 + dd] = (int8_t)__float2int_rn(__fmul_rn(v, inv_delta));
-  }
+  const int px = threadIdx.x & 15, chq = threadIdx.x >> 4;
+  const int dq = d0 + 4 * chq;
+  const int g = dq / c_pad_g, cc0 = dq - g * c_pad_g; // c_pad_g is a multiple of 16: one group for the four slots
+  const bool ok = dq < ctot && g < groups;
+  const float *base = x + ((int64_t)n * C + (g * Cg + cc0)) * HW;
+  float v[4][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int p = p0 + px + 16 * k;
+      v[k][r] = ok && cc0 + r < Cg && p < HW ? __ldcs(base + (int64_t)r * HW + p) : 0.0f;
+    }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    tile[px + 16 * k][chq] = pack_codes(v[k][0], v[k][1], v[k][2], v[k][3], inv_delta);
   __syncthreads();
   const int word = threadIdx.x & 15, prow = threadIdx.x >> 4; // 16 pixels per pass
+#pragma unroll
   for (int pp = prow; pp < 64; pp += 16) {
     const int pix = p0 + pp, d = d0 + 4 * word;
     if (pix < HW && d < ctot)
@@ -492,16 +516,6 @@ __global__ void __launch_bounds__(256) transpose_f32_kernel(const float *__restr
     if (c < C && r < R)
       dst[(int64_t)c * R + r] = tile[tx][cc];
   }
-}
-
-// Codes of four multiples of delta as one word: round(v / delta) on the add pipe, where for |t| < 2^22 the low
-// byte of 1.5 * 2^23 + t is the two's complement code.
-__device__ __forceinline__ uint32_t pack_codes(float a, float b, float c, float d, float inv_delta) {
-  const uint32_t i = __float_as_uint(__fadd_rn(__fmul_rn(a, inv_delta), 12582912.0f));
-  const uint32_t j = __float_as_uint(__fadd_rn(__fmul_rn(b, inv_delta), 12582912.0f));
-  const uint32_t k = __float_as_uint(__fadd_rn(__fmul_rn(c, inv_delta), 12582912.0f));
-  const uint32_t l = __float_as_uint(__fadd_rn(__fmul_rn(d, inv_delta), 12582912.0f));
-  return __byte_perm(__byte_perm(i, j, 0x0040), __byte_perm(k, l, 0x0040), 0x5410);
 }
 
 // Four neighbouring values of a row of `extent` floats from column k on, zero past its end; kVec: one 128-bit load

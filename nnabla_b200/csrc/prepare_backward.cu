@@ -12,6 +12,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "pdl.cuh"
 #include "prepare.cuh"
 
@@ -375,8 +377,9 @@ int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int grou
                                   void *out, uint32_t *image_max, cudaStream_t st) {
   NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
   const int64_t per_image = (int64_t)C * HW;
-  // 4096 values per block, a few loads per thread, up to what a warp reads back in two
-  const int parts = (int)(per_image < 4096 ? 1 : per_image / 4096 < kHalfPairParts ? per_image / 4096 : kHalfPairParts);
+  // shares of at least 4096 values, not many more than fill the chip twice (a block's start and end cost two microseconds)
+  const int64_t most = std::min<int64_t>(kHalfPairParts, 16ll * sm_count() / N);
+  const int parts = (int)std::max<int64_t>(1, std::min(per_image / 4096, most));
   NB_CUDA(launch_dependent(image_absmax_kernel, dim3(parts, N), dim3(256), 0, st, x, per_image, image_max + N));
   const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
   const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
