@@ -32,8 +32,11 @@
 //      (main + 2^-11 cross) * 2^(e - S). The product left out, x1 w1, is 2^-22 of
 //      the main one, the size of the representation error.
 //
-// Warps: 0-7 epilogue (TMEM lanes = pixels, columns = maps; warp w takes lanes 32 (w % 4) and
-// maps 32 (w / 4)), 8 MMA issue + TMEM allocation, 9 loader. Every mbarrier wait is time-bounded; a wait that gives
+// Warps: two sets of eight for the epilogue (TMEM lanes = pixels, columns = maps; warp w of a set takes lanes 32 (w % 4)
+// and maps 32 (w / 4)), two MMA issuers, each with every other tile and an accumulator of its own, and a loader. With one
+// issuer and one set the tensor core waited for the issue of 28 MMAs with their addresses (each MMA is as short as its
+// issue) and for the epilogue of the tile before the last: 2680 cycles per tile of 1660 cycles of MMAs, 73 us for the
+// codes of 64 x 3 x 224 x 224, now 64. Every mbarrier wait is time-bounded; a wait that gives
 // up stores a code in *status and raises the block's abort flag, every role then
 // falls through to the common teardown.
 #include <cuda_fp16.h>
@@ -54,8 +57,8 @@ int encode_tiled(CUtensorMap *map, int dtype_code, int rank, const void *base, c
 
 namespace {
 
-constexpr int kThreadsNC = 320;
-constexpr int kEpilogueWarps = 8, kMmaWarp = 8, kLoadWarp = 9;
+constexpr int kSetWarps = 8, kEpilogueWarps = 2 * kSetWarps, kMmaWarp = kEpilogueWarps, kLoadWarp = kMmaWarp + 2;
+constexpr int kThreadsNC = 32 * (kLoadWarp + 1);
 constexpr int kM = 128, kN = 64;
 constexpr int kMaxSteps = 16;             // K steps of 16 values: kernel_h * ceil(kernel_w / (2 * stride_w))
 constexpr int kStepBytes = 2 * kN * 32;   // resident weights of one K step: [w0; w1] x 16 values
@@ -267,9 +270,9 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
   const uint32_t tail = (uint32_t)(kM + 2 * g.jsteps) * 16u;
   uint8_t *b_res = smem;                           // [step][16 groups][2 chunks][8 rows][16 B]
   uint8_t *ring = b_res + (size_t)steps * kStepBytes; // [slot][piece][row_bytes]
-  // fp32 result: every epilogue warp stages [32 maps][32 pixels] boxes (two, used in turn) for bulk stores
+  // fp32 result: every epilogue warp stages a [32 maps][32 pixels] box for bulk stores
   float *stage = reinterpret_cast<float *>(ring + ((kRing * slot_bytes + tail + 127u) & ~127u));
-  uint64_t *bars = reinterpret_cast<uint64_t *>(stage + kEpilogueWarps * 2 * 1024);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(stage + kEpilogueWarps * 1024);
   uint64_t *full_bar = bars, *done_bar = bars + kInFlight, *tmem_full = bars + 2 * kInFlight,
            *tmem_empty = bars + 2 * kInFlight + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kInFlight + 4);
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
     }
     for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(tmem_full + s, 1);
-      ptx::mbar_init(tmem_empty + s, kEpilogueWarps);
+      ptx::mbar_init(tmem_empty + s, kSetWarps);
     }
     *abort_flag = 0;
     ptx::mbar_fence_init();
@@ -299,11 +302,12 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
   }
   pdl_wait();
   pdl_trigger();
-  // bias of every map (0 past Ko or without bias), times 2 / delta when codes are written
-  __shared__ float bias_s[kN];
+  // bias of every map (0 past Ko or without bias), times 2 / delta (ReLU: over 256) when codes are written
+  __shared__ __align__(16) float bias_s[kN];
   if (threadIdx.x < kN)
     bias_s[threadIdx.x] = (bias && (int)threadIdx.x < g.Ko)
-                              ? (co.codes ? __fmul_rn(bias[threadIdx.x], co.two_inv) : bias[threadIdx.x])
+                              ? (co.codes ? __fmul_rn(bias[threadIdx.x], co.relu ? co.two_inv * 0.00390625f : co.two_inv)
+                                          : bias[threadIdx.x])
                               : 0.0f;
   {
     // resident weights (already in the tensor core's layout) and zeros behind the ring
@@ -323,18 +327,19 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------ loader: the new rows of every tile
     if (ptx::elect_one()) {
-      RowWalk walk;
-      int s0_of[2 * kInFlight];
-      int seq = 0, oldest = 0;
+      RowWalk walk, behind; // of the tile to load, of the oldest tile that may still be read
+      int seq = 0, oldest = 0, ignored, oldest_s0;
+      int n = tile_first / g.Ho, oy = tile_first - n * g.Ho, old_n = n, old_oy = oy;
+      behind.next(old_n, old_oy * g.sh, g.kh, ignored, oldest_s0);
       bool ok = true;
       for (int tile = tile_first; tile < tile_last && ok; ++tile, ++seq) {
-        const int n = tile / g.Ho, oy = tile - n * g.Ho;
         int first, s0;
         const int count_before = walk.count;
         const int nload = walk.next(n, oy * g.sh, g.kh, first, s0);
-        // ring slots about to be overwritten, and the barrier of this tile, must have been released
-        // by the tiles that used them
-        while (oldest < seq && (s0_of[oldest & (2 * kInFlight - 1)] + kRing < walk.count || seq - oldest >= kInFlight)) {
+        // ring slots about to be overwritten must have been released by the tiles that used them, and the barrier of
+        // this tile by the tile seven before: an issuer also waits for the barrier of the tile before its own, which
+        // must not have gone round by then
+        while (oldest < seq && (oldest_s0 + kRing < walk.count || seq - oldest >= kInFlight - 1)) {
           if (!ptx::mbar_wait(done_bar + (oldest & (kInFlight - 1)), (uint32_t)(oldest / kInFlight) & 1u, abort_flag)) {
             if (*abort_flag == 0)
               atomicCAS(status, 0, kStatusNcLoadTimeout);
@@ -343,27 +348,31 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
             break;
           }
           ++oldest;
+          if (++old_oy == g.Ho)
+            old_oy = 0, ++old_n;
+          behind.next(old_n, old_oy * g.sh, g.kh, ignored, oldest_s0);
         }
         if (!ok)
           break;
-        s0_of[seq & (2 * kInFlight - 1)] = s0;
         uint64_t *bar = full_bar + (seq & (kInFlight - 1));
         ptx::mbar_expect_tx(bar, (uint32_t)nload * slot_bytes);
         const uint8_t *src = xs + ((int64_t)n * g.Hp + first) * slot_bytes;
         for (int i = 0; i < nload; ++i)
           ptx::bulk_load(ring + (uint32_t)((count_before + i) % kRing) * slot_bytes, src + (int64_t)i * slot_bytes,
                          slot_bytes, bar);
+        if (++oy == g.Ho)
+          oy = 0, ++n;
       }
     }
-  } else if (warp == kMmaWarp) {
-    // -------------------------------------------------------------- MMA issuer
+  } else if (warp >= kMmaWarp) {
+    // ------------------------------------------------------------- MMA issuers
     if (ptx::elect_one()) {
+      const int who = warp - kMmaWarp; // takes the tiles with seq % 2 == who
       RowWalk walk;
       int seq = 0;
       bool ok = true;
       const uint32_t idesc128 = ptx::make_idesc(1u, 0u, kM, 128), idesc64 = ptx::make_idesc(1u, 0u, kM, 64);
-      // The MMAs of a tile are issued from one straight piece of code with every address at hand: a loop that worked
-      // them out per step issued 28 MMAs in 2700 cycles that take the tensor core 1650.
+      // the MMAs of a tile are issued from one straight piece of code with every address at hand
       const uint64_t a_base = ptx::smem_desc_k_plain(ptx::smem_u32(ring), 16u, 128u);
       const uint64_t b_base = ptx::smem_desc_k_plain(ptx::smem_u32(b_res), 128u, 256u);
       const uint32_t slot_units = slot_bytes >> 4, piece_units = (uint32_t)g.row_bytes >> 4;
@@ -376,15 +385,20 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
       }
       int n = tile_first / g.Ho, oy = tile_first - n * g.Ho;
       for (int tile = tile_first; tile < tile_last && ok; ++tile, ++seq) {
-        const int buf = seq & 1;
-        const uint32_t buf_phase = (uint32_t)(seq >> 1) & 1u;
         int first, s0;
         walk.next(n, oy * g.sh, g.kh, first, s0);
+        if (++oy == g.Ho)
+          oy = 0, ++n;
+        if ((seq & 1) != who)
+          continue;
         uint32_t a_unit[kMaxSteps]; // rows 16 bytes apart, the second K chunk 16 bytes behind the first: sliding windows
 #pragma unroll
         for (int s = 0; s < kMaxSteps; ++s)
           a_unit[s] = (uint32_t)((s0 + step_ky[s]) & (kRing - 1)) * slot_units + step_unit[s];
-        if (!ptx::mbar_wait(tmem_empty + buf, buf_phase ^ 1u, abort_flag) ||
+        // rows of this tile that an earlier one asked for too came with that one's barrier
+        const int before = seq == 0 ? 0 : seq - 1;
+        if (!ptx::mbar_wait(tmem_empty + who, ((uint32_t)(seq >> 1) & 1u) ^ 1u, abort_flag) ||
+            !ptx::mbar_wait(full_bar + (before & (kInFlight - 1)), (uint32_t)(before / kInFlight) & 1u, abort_flag) ||
             !ptx::mbar_wait(full_bar + (seq & (kInFlight - 1)), (uint32_t)(seq / kInFlight) & 1u, abort_flag)) {
           if (*abort_flag == 0)
             atomicCAS(status, 0, kStatusNcMmaTimeout);
@@ -392,7 +406,7 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
           break;
         }
         ptx::tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kAccCols);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(who * kAccCols);
 #pragma unroll
         for (int s = 0; s < kMaxSteps; ++s) {
           if (s < steps) {
@@ -401,26 +415,23 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
             ptx::mma_bf16(d_tmem + kN, a0 + piece_units, b, idesc64, 1u);   // x1 x [w0]     -> columns 64..127
           }
         }
-        if (++oy == g.Ho)
-          oy = 0, ++n;
         ptx::mma_commit(done_bar + (seq & (kInFlight - 1)));
-        ptx::mma_commit(tmem_full + buf);
+        ptx::mma_commit(tmem_full + who);
       }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3; // TMEM lanes [32 * quarter, 32 * quarter + 32)
-    const int half = warp >> 2;   // maps [32 * half, 32 * half + 32)
-    int local = 0;
+    const int half = warp >> 2 & 1; // maps [32 * half, 32 * half + 32)
+    const int set = warp / kSetWarps; // tiles with seq % 2 == set, in its issuer's accumulator
+    uint32_t phase = 0;
     const int px = quarter * 32 + lane;
     const int64_t plane = (int64_t)g.Ho * g.Wo;
     const float ws = __ldg(wscale);
-    for (int tile = tile_first; tile < tile_last; ++tile, ++local) {
-      const int buf = local & 1;
-      const uint32_t buf_phase = (uint32_t)(local >> 1) & 1u;
-      const int n = tile / g.Ho, oy = tile - n * g.Ho;
+    int n = (tile_first + set) / g.Ho, oy = tile_first + set - n * g.Ho;
+    for (int tile = tile_first + set; tile < tile_last; tile += 2, phase ^= 1u) {
       const float scale = __fmul_rn(__ldg(xscale + n), ws); // 2^(e - S)
-      const bool got = ptx::mbar_wait_backoff(tmem_full + buf, buf_phase, abort_flag, 100u);
+      const bool got = ptx::mbar_wait_backoff(tmem_full + set, phase, abort_flag, 20u);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) {
           if (*abort_flag == 0)
@@ -431,36 +442,62 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
       }
       ptx::tc_fence_after_sync();
       float *yrow = y + (int64_t)n * g.Ko * plane + (int64_t)oy * g.Wo + px;
-      const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kAccCols);
+      const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * kAccCols);
       {
         uint32_t r0[32], r1[32];
         ptx::tmem_ld_32x32(t0 + (uint32_t)(half * 32), r0);      // x0 w0
         ptx::tmem_ld_32x32(t0 + (uint32_t)(kN + half * 32), r1); // x0 w1 + x1 w0, times 2^11
         ptx::tmem_ld_wait();
+        // the accumulator is in registers: the MMAs of the tile after the next may start
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0)
+          ptx::mbar_arrive(tmem_empty + set);
         if (co.codes != nullptr) {
           if (px < g.Wo && half * 32 < co.slots) {
             // u = conv * (2 / delta) + bias * (2 / delta), one fused multiply-add; then ReLU and the
             // quantizer of a non-negative value, (floor(u) + 1) >> 1 capped at kmax
-            const float cap = (float)(2 * co.kmax) + 0.5f;
-            const float k2 = __fmul_rn(scale, co.two_inv);
             uint32_t wds[8];
+            if (co.relu) {
+              // floor(u) + 1 on the FMA pipe: u / 256 saturated to [0, 1] (a NaN becomes 0), capped, and scaled back
+              // by an addition to 2^23 + 1 that rounds down; at most 255, so four of them shift as one word. Decided
+              // per value, the branch and the conversions took 30 instructions where these are five.
+              const float cap = (float)(2 * co.kmax) + 0.5f;
+              const float k256 = __fmul_rn(__fmul_rn(scale, co.two_inv), 0.00390625f), cap256 = __fmul_rn(cap, 0.00390625f);
 #pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
-              int c[4];
+              for (int j4 = 0; j4 < 8; ++j4) {
+                uint32_t c[4];
+                const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + half * 32 + 4 * j4);
+                const float b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const int j = 4 * j4 + k;
-                const float raw = __fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j]));
-                const float u = __fmaf_rn(raw, k2, bias_s[half * 32 + j]);
-                if (co.relu) {
-                  c[k] = (__float2int_rd(fminf(fmaxf(u, 0.0f), cap)) + 1) >> 1; // a NaN becomes 0
-                } else {
+                for (int k = 0; k < 4; ++k) {
+                  const int j = 4 * j4 + k;
+                  const float raw = __fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j]));
+                  const float u = fminf(__saturatef(__fmaf_rn(raw, k256, b[k])), cap256);
+                  c[k] = __float_as_uint(__fmaf_rd(u, 256.0f, 8388609.0f));
+                }
+                wds[j4] = __byte_perm(__byte_perm(c[0], c[1], 0x0040), __byte_perm(c[2], c[3], 0x0040), 0x5410) >> 1 &
+                          0x7f7f7f7fu;
+              }
+            } else {
+              const float cap = (float)(2 * co.kmax) + 0.5f;
+              const float k2 = __fmul_rn(scale, co.two_inv);
+#pragma unroll
+              for (int j4 = 0; j4 < 8; ++j4) {
+                int c[4];
+                const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + half * 32 + 4 * j4);
+                const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const int j = 4 * j4 + k;
+                  const float raw = __fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j]));
+                  const float u = __fmaf_rn(raw, k2, b[k]);
                   const int m = (__float2int_rd(fminf(fabsf(u), cap)) + 1) >> 1;
                   c[k] = u < 0.0f ? max(-m, co.kmin) : m;
                 }
+                // maps past Ko have zero weights and zero bias: their code is 0 on its own
+                wds[j4] = pack_codes4(c[0], c[1], c[2], c[3]);
               }
-              // maps past Ko have zero weights and zero bias: their code is 0 on its own
-              wds[j4] = pack_codes4(c[0], c[1], c[2], c[3]);
             }
             uint4 *cp = reinterpret_cast<uint4 *>(co.codes + ((int64_t)n * plane + (int64_t)oy * g.Wo + px) * co.slots +
                                                   half * 32);
@@ -470,16 +507,25 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
           }
         } else if (box_store) {
           // the copy engine writes the box: whole lines, clipped at Wo and Ko, while the warp goes on
-          float *box = stage + (warp * 2 + (local & 1)) * 1024;
+          float *box = stage + warp * 1024;
           if (lane == 0)
-            ptx::tma_store_wait_read<1>(); // the store before the previous one read this box
+            ptx::tma_store_wait_read<0>(); // the previous store has read the box
           __syncwarp();
+          if (bias) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float v = __fmul_rn(__fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j])), scale);
-            if (bias)
-              v = __fadd_rn(v, bias_s[half * 32 + j]);
-            box[j * 32 + lane] = v;
+            for (int j4 = 0; j4 < 8; ++j4) {
+              const float4 b4 = *reinterpret_cast<const float4 *>(bias_s + half * 32 + 4 * j4);
+              const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+              for (int j = 4 * j4; j < 4 * j4 + 4; ++j)
+                box[j * 32 + lane] = __fadd_rn(
+                    __fmul_rn(__fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j])), scale), b[j - 4 * j4]);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              box[j * 32 + lane] =
+                  __fmul_rn(__fmaf_rn(__uint_as_float(r1[j]), 0.00048828125f, __uint_as_float(r0[j])), scale);
           }
           ptx::fence_async_shared();
           __syncwarp();
@@ -501,10 +547,8 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
           }
         }
       }
-      ptx::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0)
-        ptx::mbar_arrive(tmem_empty + buf);
+      for (oy += 2; oy >= g.Ho; oy -= g.Ho)
+        ++n;
     }
   }
 
@@ -540,7 +584,7 @@ NarrowPlan narrow_plan(int width, int kernel_h, int kernel_w, int pad_w, int str
   const int units_read = Wo - 1 + 2 * p.jsteps; // by rows that hold an output pixel
   p.row_bytes = 16 * (units_image > units_read ? units_image : units_read);
   const size_t ring = ((size_t)kRing * 2 * p.row_bytes + (size_t)(kM + 2 * p.jsteps) * 16 + 127) & ~size_t(127);
-  p.smem = (size_t)p.steps * kStepBytes + ring + kEpilogueWarps * 2 * 4096 + (2 * kInFlight + 4) * 8 + 16 + 128;
+  p.smem = (size_t)p.steps * kStepBytes + ring + kEpilogueWarps * 4096 + (2 * kInFlight + 4) * 8 + 16 + 128;
   return p;
 }
 
