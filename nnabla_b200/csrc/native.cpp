@@ -12,6 +12,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <cstdint>
@@ -253,6 +254,28 @@ bool read_pair(PyObject *o, int64_t fallback, int64_t out[2]) {
   return !PyErr_Occurred();
 }
 
+// Geometry of a 2-D convolution with one batch axis; false where the operands do not fit together.
+struct Geometry {
+  int64_t x[4], w[4], pad[2], stride[2], dil[2], out[2];
+  bool read(const c10::SmallVector<int64_t, 8> &xs, const c10::SmallVector<int64_t, 8> &ws, PyObject *p, PyObject *st,
+            PyObject *d, long group) {
+    if (xs.size() != 4 || ws.size() != 4 || group <= 0)
+      return false;
+    std::copy(xs.begin(), xs.end(), x);
+    std::copy(ws.begin(), ws.end(), w);
+    bool ok = read_pair(p, 0, pad) && read_pair(st, 1, stride) && read_pair(d, 1, dil) && x[1] % group == 0 &&
+              w[0] % group == 0 && x[1] / group == w[1];
+    for (int i = 0; ok && i < 2; ++i) {
+      const int64_t span = x[2 + i] + 2 * pad[i] - (dil[i] * (w[2 + i] - 1) + 1);
+      ok = span >= 0 && stride[i] > 0;
+      out[i] = ok ? span / stride[i] + 1 : 0;
+    }
+    if (!ok)
+      PyErr_Clear();
+    return ok;
+  }
+};
+
 // conv2d(x, w, bias, base_axis, pad, stride, dilation, group): the geometry of a 2-D convolution with one batch axis,
 // (batch, channels, height, width, outmaps, kh, kw, pad, stride, dilation, output shape); x and w are tensors or
 // shapes. None where the operands are of another form or do not fit together: the caller's full checks say why.
@@ -260,29 +283,21 @@ PyObject *conv2d(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   if (nargs != 8)
     return PyErr_Format(PyExc_TypeError, "expected 8 arguments, got %zd", nargs);
-  c10::SmallVector<int64_t, 8> x, w;
-  int64_t pad[2], stride[2], dil[2], out[2];
+  c10::SmallVector<int64_t, 8> x, w, b;
+  Geometry g;
   const long base_axis = PyLong_AsLong(args[3]), group = PyLong_AsLong(args[7]);
-  bool ok = !PyErr_Occurred() && read_shape(args[0], x) && read_shape(args[1], w) && x.size() == 4 && w.size() == 4 &&
-            base_axis == 1 && read_pair(args[4], 0, pad) && read_pair(args[5], 1, stride) &&
-            read_pair(args[6], 1, dil) && group > 0 && x[1] % group == 0 && w[0] % group == 0 && x[1] / group == w[1];
-  if (ok && args[2] != Py_None) {
-    c10::SmallVector<int64_t, 8> b;
+  bool ok = !PyErr_Occurred() && base_axis == 1 && read_shape(args[0], x) && read_shape(args[1], w) &&
+            g.read(x, w, args[4], args[5], args[6], group);
+  if (ok && args[2] != Py_None)
     ok = read_shape(args[2], b) && b.size() == 1 && b[0] == w[0];
-  }
-  for (int i = 0; ok && i < 2; ++i) {
-    const int64_t span = x[2 + i] + 2 * pad[i] - (dil[i] * (w[2 + i] - 1) + 1);
-    ok = span >= 0 && stride[i] > 0;
-    out[i] = ok ? span / stride[i] + 1 : 0;
-  }
   if (!ok) {
     PyErr_Clear();
     Py_RETURN_NONE;
   }
   return Py_BuildValue("LLLLLLL(LL)(LL)(LL)(LLLL)", (long long)x[0], (long long)x[1], (long long)x[2], (long long)x[3],
-                       (long long)w[0], (long long)w[2], (long long)w[3], (long long)pad[0], (long long)pad[1],
-                       (long long)stride[0], (long long)stride[1], (long long)dil[0], (long long)dil[1],
-                       (long long)x[0], (long long)w[0], (long long)out[0], (long long)out[1]);
+                       (long long)w[0], (long long)w[2], (long long)w[3], (long long)g.pad[0], (long long)g.pad[1],
+                       (long long)g.stride[0], (long long)g.stride[1], (long long)g.dil[0], (long long)g.dil[1],
+                       (long long)x[0], (long long)w[0], (long long)g.out[0], (long long)g.out[1]);
   END_HANDLE_TH_ERRORS
 }
 
@@ -294,6 +309,358 @@ PyObject *codes_nhwc_slots(PyObject *, PyObject *const *args, Py_ssize_t nargs) 
   if (nargs != 2 || !channels.read(args[0], unused) || !group.read(args[1], unused))
     return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_TypeError, "expected channels and group");
   return PyLong_FromLongLong(nb200_codes_nhwc_slots(channels.v, group.v));
+  END_HANDLE_TH_ERRORS
+}
+
+// ---- whole calls of the mirror -------------------------------------------------------------------------------------
+// The functions that networks and training blocks call per layer, from their Python arguments to the launch: checks,
+// geometry and allocations in Python cost a folded convolution 3.9 us on top of 3.3. Each returns None, before anything
+// is written or launched, where an argument is not of the plain form; the caller's full path then does the work or says
+// what is wrong.
+
+// Tensors, shapes and options of one call; ok turns false at the first that is not of the plain form.
+struct Plain {
+  bool ok = true;
+  const at::Tensor *first = nullptr;
+  // a contiguous float32 CUDA tensor on the device of the first one
+  const at::Tensor *f32(PyObject *o) { return tensor(o, at::kFloat); }
+  const at::Tensor *i8(PyObject *o) { return tensor(o, at::kChar); }
+  const at::Tensor *tensor(PyObject *o, at::ScalarType type) {
+    if (!ok || !THPVariable_Check(o))
+      return fail();
+    const at::Tensor &t = THPVariable_Unpack(o);
+    if (!t.is_cuda() || t.scalar_type() != type || !t.is_contiguous() || (first && t.get_device() != first->get_device()))
+      return fail();
+    if (!first)
+      first = &t;
+    return &t;
+  }
+  // the same, or NULL for None
+  const at::Tensor *f32_or_none(PyObject *o) { return o == Py_None ? nullptr : f32(o); }
+  const at::Tensor *fail() {
+    ok = false;
+    return nullptr;
+  }
+  void require(bool condition) { ok = ok && condition; }
+  // the truth of a bool; anything else is not plain
+  bool truth(PyObject *o) {
+    require(o == Py_True || o == Py_False);
+    return o == Py_True;
+  }
+  long integer(PyObject *o) {
+    const long v = ok && PyLong_Check(o) ? PyLong_AsLong(o) : (ok = false, 0);
+    if (v == -1 && PyErr_Occurred()) {
+      PyErr_Clear();
+      ok = false;
+    }
+    return v;
+  }
+  float number(PyObject *o) {
+    if (ok && (PyFloat_Check(o) || PyLong_Check(o))) {
+      const double d = PyFloat_AsDouble(o);
+      if (!(d == -1.0 && PyErr_Occurred()))
+        return (float)d;
+      PyErr_Clear();
+    }
+    ok = false;
+    return 0.0f;
+  }
+};
+
+template <typename P> P *data(const at::Tensor *t) { return t ? static_cast<P *>(t->data_ptr()) : nullptr; }
+
+at::Tensor empty_like_of(const at::Tensor &like, at::IntArrayRef shape, at::ScalarType type) {
+  return at::detail::empty_cuda(shape, type, like.device(), std::nullopt);
+}
+
+// Runs an entry point on the tensors' device and torch's current stream of it; NULL after raising its error.
+template <typename F> bool run_on(const at::Tensor &t, F &&f) {
+  const int device = t.get_device(), current = c10::cuda::current_device();
+  if (device != current)
+    c10::cuda::set_device((c10::DeviceIndex)device);
+  void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+  g_calls.fetch_add(1, std::memory_order_relaxed);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS;
+  rc = f(stream);
+  Py_END_ALLOW_THREADS;
+  if (device != current)
+    c10::cuda::set_device((c10::DeviceIndex)current);
+  if (rc != 0)
+    raise_status(rc);
+  return rc == 0;
+}
+
+PyObject *not_plain() {
+  PyErr_Clear();
+  Py_RETURN_NONE;
+}
+
+// folded_convolution(x_codes, x_shape, side, group, w_shape, scale, bias, pad, stride, dilation, residual_codes,
+//                    residual_delta, residual, relu, sign, n, delta, output): functions.convolution_codes_folded
+PyObject *folded_convolution(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 18)
+    return PyErr_Format(PyExc_TypeError, "expected 18 arguments, got %zd", nargs);
+  Plain p;
+  c10::SmallVector<int64_t, 8> xs, ws;
+  Geometry g;
+  const at::Tensor *x = p.i8(a[0]), *side = p.i8(a[2]), *scale = p.f32(a[5]), *bias = p.f32_or_none(a[6]);
+  const at::Tensor *res_codes = a[10] == Py_None ? nullptr : p.i8(a[10]), *res = p.f32_or_none(a[12]);
+  const float res_delta = a[11] == Py_None ? 0.0f : p.number(a[11]);
+  const bool relu = p.truth(a[13]), sign = p.truth(a[14]);
+  const long n = p.integer(a[15]);
+  const float delta = p.number(a[16]);
+  const char *output = PyUnicode_Check(a[17]) ? PyUnicode_AsUTF8(a[17]) : nullptr;
+  const bool codes = output && strcmp(output, "codes") == 0;
+  p.require(output && (codes || strcmp(output, "float") == 0) && p.integer(a[3]) == 1);
+  if (!p.ok || !read_shape(a[1], xs) || !read_shape(a[4], ws) || !g.read(xs, ws, a[7], a[8], a[9], 1))
+    return not_plain();
+  const int64_t pixels = g.out[0] * g.out[1], slots = nb200_codes_nhwc_slots(g.w[0], 1);
+  const int64_t want_x[3] = {g.x[0], g.x[2] * g.x[3], nb200_codes_nhwc_slots(g.x[1], 1)}, want_y[3] = {g.x[0], pixels, slots};
+  const at::IntArrayRef y_shape(want_y, 3);
+  p.require(x->sizes() == at::IntArrayRef(want_x, 3) && scale->numel() == g.w[0] &&
+            (!bias || (bias->dim() == 1 && bias->numel() == g.w[0])) && (!res_codes || res_codes->sizes() == y_shape) &&
+            (!res || res->sizes() == y_shape));
+  if (!p.ok)
+    return not_plain();
+  const at::Tensor y = empty_like_of(*x, y_shape, codes ? at::kChar : at::kFloat);
+  if (!run_on(*x, [&](void *stream) {
+        return nb200_convolution_codes_folded_nhwc(
+            data<int8_t>(x), data<int8_t>(side), data<float>(scale), data<float>(bias), data<int8_t>(res_codes), res_delta,
+            data<float>(res), codes ? data<int8_t>(&y) : nullptr, codes ? nullptr : data<float>(&y), (int)g.x[0], (int)g.x[1],
+            (int)g.x[2], (int)g.x[3], (int)g.w[0], (int)g.w[2], (int)g.w[3], (int)g.pad[0], (int)g.pad[1],
+            (int)g.stride[0], (int)g.stride[1], (int)g.dil[0], (int)g.dil[1], relu, sign, (int)n, delta, stream);
+      }))
+    return nullptr;
+  return Py_BuildValue("N(LLLL)", THPVariable_Wrap(y), (long long)g.x[0], (long long)g.w[0], (long long)g.out[0],
+                       (long long)g.out[1]);
+  END_HANDLE_TH_ERRORS
+}
+
+// binary_convolution(x, weight, binary_weight, alpha, bias, pad, stride, dilation, group, quantize_zero_to, delta):
+// y of binary_weight_convolution (alpha a tensor) or binary_connect_convolution (alpha None); delta None or a number
+PyObject *binary_convolution(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 11)
+    return PyErr_Format(PyExc_TypeError, "expected 11 arguments, got %zd", nargs);
+  Plain p;
+  c10::SmallVector<int64_t, 8> xs, ws;
+  Geometry g;
+  const at::Tensor *x = p.f32(a[0]), *w = p.f32(a[1]), *wb = p.f32(a[2]), *alpha = p.f32_or_none(a[3]),
+                   *bias = p.f32_or_none(a[4]);
+  const long group = p.integer(a[8]);
+  const float zero_to = p.number(a[9]), delta = a[10] == Py_None ? 0.0f : p.number(a[10]);
+  if (!p.ok || !read_shape(a[0], xs) || !read_shape(a[1], ws) || !g.read(xs, ws, a[5], a[6], a[7], group))
+    return not_plain();
+  p.require(w->sizes() == wb->sizes() && (!alpha || alpha->numel() == g.w[0]) &&
+            (!bias || (bias->dim() == 1 && bias->numel() == g.w[0])));
+  if (!p.ok)
+    return not_plain();
+  const int64_t out[4] = {g.x[0], g.w[0], g.out[0], g.out[1]};
+  const at::Tensor y = empty_like_of(*x, at::IntArrayRef(out, 4), at::kFloat);
+  const int c[13] = {(int)g.x[0],   (int)g.x[1],   (int)g.x[2],      (int)g.x[3],      (int)g.w[0],   (int)g.w[2],  (int)g.w[3],
+                     (int)g.pad[0], (int)g.pad[1], (int)g.stride[0], (int)g.stride[1], (int)g.dil[0], (int)g.dil[1]};
+  if (!run_on(*x, [&](void *stream) {
+        return alpha ? nb200_binary_weight_convolution_f32(data<float>(x), data<float>(w), data<float>(wb),
+                                                           data<float>(alpha), data<float>(bias), data<float>(&y), c[0], c[1],
+                                                           c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10], c[11],
+                                                           c[12], (int)group, zero_to, delta, stream)
+                     : nb200_binary_connect_convolution_f32(data<float>(x), data<float>(w), data<float>(wb),
+                                                            data<float>(bias), data<float>(&y), c[0], c[1], c[2], c[3], c[4],
+                                                            c[5], c[6], c[7], c[8], c[9], c[10], c[11], c[12], (int)group,
+                                                            zero_to, delta, stream);
+      }))
+    return nullptr;
+  return THPVariable_Wrap(y);
+  END_HANDLE_TH_ERRORS
+}
+
+bool read_flags(Plain &p, PyObject *o, bool out[3]) {
+  if (!PyTuple_Check(o) || PyTuple_GET_SIZE(o) != 3)
+    return p.ok = false;
+  for (int i = 0; i < 3; ++i)
+    out[i] = p.truth(PyTuple_GET_ITEM(o, i));
+  return p.ok;
+}
+
+// binary_convolution_backward(x, binary_weight, alpha, dy, pad, stride, dilation, group, propagate_down, accum, grads,
+// delta): (dx, dw, db) with what grads holds where propagate_down is False
+PyObject *binary_convolution_backward(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 12)
+    return PyErr_Format(PyExc_TypeError, "expected 12 arguments, got %zd", nargs);
+  Plain p;
+  c10::SmallVector<int64_t, 8> xs, ws;
+  Geometry g;
+  const at::Tensor *x = p.f32(a[0]), *wb = p.f32(a[1]), *alpha = p.f32_or_none(a[2]), *dy = p.f32(a[3]);
+  const long group = p.integer(a[7]);
+  bool down[3], accum[3];
+  read_flags(p, a[8], down);
+  read_flags(p, a[9], accum);
+  const float delta = a[11] == Py_None ? 0.0f : p.number(a[11]);
+  p.require(PyTuple_Check(a[10]) && PyTuple_GET_SIZE(a[10]) == 3);
+  if (!p.ok || !read_shape(a[0], xs) || !read_shape(a[1], ws) || !g.read(xs, ws, a[4], a[5], a[6], group))
+    return not_plain();
+  const int64_t out[4] = {g.x[0], g.w[0], g.out[0], g.out[1]};
+  p.require(dy->sizes() == at::IntArrayRef(out, 4));
+  const at::IntArrayRef shapes[3] = {x->sizes(), wb->sizes(), at::IntArrayRef(g.w, 1)};
+  at::Tensor grad[3];
+  for (int i = 0; p.ok && i < 3; ++i) {
+    PyObject *given = PyTuple_GET_ITEM(a[10], i);
+    if (!down[i])
+      continue;
+    if (given == Py_None) {
+      p.require(!accum[i]);
+    } else {
+      const at::Tensor *t = p.f32(given);
+      p.require(t && t->sizes() == shapes[i]);
+      if (p.ok)
+        grad[i] = *t;
+    }
+  }
+  if (!p.ok)
+    return not_plain();
+  for (int i = 0; i < 3; ++i)
+    if (down[i] && !grad[i].defined())
+      grad[i] = empty_like_of(*x, shapes[i], at::kFloat);
+  float *d[3];
+  for (int i = 0; i < 3; ++i)
+    d[i] = down[i] ? data<float>(&grad[i]) : nullptr;
+  const int c[13] = {(int)g.x[0],   (int)g.x[1],   (int)g.x[2],      (int)g.x[3],      (int)g.w[0],   (int)g.w[2],  (int)g.w[3],
+                     (int)g.pad[0], (int)g.pad[1], (int)g.stride[0], (int)g.stride[1], (int)g.dil[0], (int)g.dil[1]};
+  if (!run_on(*x, [&](void *stream) {
+        return alpha ? nb200_binary_weight_convolution_backward_f32(
+                           data<float>(x), data<float>(wb), data<float>(alpha), data<float>(dy), d[0], d[1], d[2], c[0], c[1],
+                           c[2], c[3], c[4], c[5], c[6], c[7], c[8], c[9], c[10], c[11], c[12], (int)group, accum[0],
+                           accum[1], accum[2], delta, stream)
+                     : nb200_binary_connect_convolution_backward_f32(
+                           data<float>(x), data<float>(wb), data<float>(dy), d[0], d[1], d[2], c[0], c[1], c[2], c[3], c[4],
+                           c[5], c[6], c[7], c[8], c[9], c[10], c[11], c[12], (int)group, accum[0], accum[1], accum[2],
+                           delta, stream);
+      }))
+    return nullptr;
+  PyObject *r = PyTuple_New(3);
+  for (int i = 0; r && i < 3; ++i) {
+    PyObject *given = PyTuple_GET_ITEM(a[10], i);
+    if (!down[i] || given != Py_None) {
+      Py_INCREF(given);
+      PyTuple_SET_ITEM(r, i, given);
+    } else {
+      PyTuple_SET_ITEM(r, i, THPVariable_Wrap(grad[i]));
+    }
+  }
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// channel axis 1, given as [1] or (1,)
+bool axis_one(PyObject *o) {
+  if (!(PyList_Check(o) || PyTuple_Check(o)) || PySequence_Fast_GET_SIZE(o) != 1)
+    return false;
+  PyObject *e = PySequence_Fast_GET_ITEM(o, 0);
+  return PyLong_Check(e) && PyLong_AsLong(e) == 1;
+}
+
+// batch_normalization(x, beta, gamma, mean, variance, axes, decay_rate, eps, batch_stat, output_stat)
+PyObject *batch_normalization(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 10)
+    return PyErr_Format(PyExc_TypeError, "expected 10 arguments, got %zd", nargs);
+  Plain p;
+  const at::Tensor *x = p.f32(a[0]), *beta = p.f32_or_none(a[1]), *gamma = p.f32_or_none(a[2]), *mean = p.f32(a[3]),
+                   *var = p.f32(a[4]);
+  const float decay = p.number(a[6]), eps = p.number(a[7]);
+  const bool batch = p.truth(a[8]), stats = p.truth(a[9]);
+  p.require(axis_one(a[5]) && p.ok && x->dim() >= 2);
+  if (!p.ok)
+    return not_plain();
+  const int64_t outer = x->size(0), C = x->size(1), inner = x->numel() / std::max<int64_t>(outer * C, 1);
+  for (const at::Tensor *t : {beta, gamma, mean, var})
+    p.require(!t || t->numel() == C);
+  if (!p.ok)
+    return not_plain();
+  const at::Tensor y = empty_like_of(*x, x->sizes(), at::kFloat);
+  at::Tensor bm, bv;
+  if (batch) {
+    bm = empty_like_of(*x, mean->sizes(), at::kFloat);
+    bv = empty_like_of(*x, var->sizes(), at::kFloat);
+  }
+  if (!run_on(*x, [&](void *stream) {
+        return batch ? nb200_batch_normalization_batch_f32(data<float>(x), data<float>(beta), data<float>(gamma),
+                                                           data<float>(mean), data<float>(var), data<float>(&y),
+                                                           data<float>(&bm), data<float>(&bv), outer, C, inner, eps, decay, 1,
+                                                           stream)
+                     : nb200_batch_normalization_inference_f32(data<float>(x), data<float>(beta), data<float>(gamma),
+                                                               data<float>(mean), data<float>(var), data<float>(&y), outer,
+                                                               C, inner, eps, stream);
+      }))
+    return nullptr;
+  if (batch && stats)
+    return Py_BuildValue("NNN", THPVariable_Wrap(y), THPVariable_Wrap(bm), THPVariable_Wrap(bv));
+  return THPVariable_Wrap(y);
+  END_HANDLE_TH_ERRORS
+}
+
+// batch_normalization_backward(x, dy, gamma, mean, variance, axes, eps, batch_stat, dmean, dvar, propagate_down, accum,
+// grads): (dx, dbeta, dgamma), None where propagate_down is False
+PyObject *batch_normalization_backward(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 13)
+    return PyErr_Format(PyExc_TypeError, "expected 13 arguments, got %zd", nargs);
+  Plain p;
+  const at::Tensor *x = p.f32(a[0]), *dy = p.f32(a[1]), *gamma = p.f32_or_none(a[2]), *mean = p.f32(a[3]),
+                   *var = p.f32(a[4]), *dmean = p.f32_or_none(a[8]), *dvar = p.f32_or_none(a[9]);
+  const float eps = p.number(a[6]);
+  const bool batch = p.truth(a[7]);
+  bool down[3], accum[3];
+  read_flags(p, a[10], down);
+  read_flags(p, a[11], accum);
+  p.require(axis_one(a[5]) && PyTuple_Check(a[12]) && PyTuple_GET_SIZE(a[12]) == 3 && p.ok && x->dim() >= 2 &&
+            dy->sizes() == x->sizes());
+  if (!p.ok)
+    return not_plain();
+  const int64_t outer = x->size(0), C = x->size(1), inner = x->numel() / std::max<int64_t>(outer * C, 1);
+  for (const at::Tensor *t : {gamma, mean, var, dmean, dvar})
+    p.require(!t || t->numel() == C);
+  const at::IntArrayRef shapes[3] = {x->sizes(), at::IntArrayRef(C), at::IntArrayRef(C)};
+  at::Tensor grad[3];
+  for (int i = 0; p.ok && i < 3; ++i) {
+    PyObject *given = PyTuple_GET_ITEM(a[12], i);
+    if (!down[i])
+      continue;
+    if (given == Py_None) {
+      p.require(!accum[i]);
+    } else {
+      const at::Tensor *t = p.f32(given);
+      p.require(t && t->numel() == (i == 0 ? x->numel() : C));
+      if (p.ok)
+        grad[i] = *t;
+    }
+  }
+  if (!p.ok)
+    return not_plain();
+  float *d[3] = {nullptr, nullptr, nullptr};
+  for (int i = 0; i < 3; ++i)
+    if (down[i]) {
+      if (!grad[i].defined())
+        grad[i] = empty_like_of(*x, shapes[i], at::kFloat);
+      d[i] = data<float>(&grad[i]);
+    }
+  if (!run_on(*x, [&](void *stream) {
+        return nb200_batch_normalization_backward_f32(data<float>(x), data<float>(dy), data<float>(gamma), data<float>(mean),
+                                                      data<float>(var), data<float>(dmean), data<float>(dvar), d[0], d[1],
+                                                      d[2], outer, C, inner, eps, batch, accum[0], accum[1], accum[2],
+                                                      stream);
+      }))
+    return nullptr;
+  PyObject *r = PyTuple_New(3);
+  for (int i = 0; r && i < 3; ++i) {
+    PyObject *given = PyTuple_GET_ITEM(a[12], i);
+    PyObject *o = !down[i] ? Py_NewRef(Py_None) : given != Py_None ? Py_NewRef(given) : THPVariable_Wrap(grad[i]);
+    PyTuple_SET_ITEM(r, i, o);
+  }
+  return r;
   END_HANDLE_TH_ERRORS
 }
 
@@ -366,6 +733,11 @@ PyMethodDef methods[] = {
     HELPER("empty", empty<at::kFloat>),
     HELPER("empty_i8", empty<at::kChar>),
     HELPER("conv2d", conv2d),
+    HELPER("folded_convolution", folded_convolution),
+    HELPER("binary_convolution", binary_convolution),
+    HELPER("binary_convolution_backward", binary_convolution_backward),
+    HELPER("batch_normalization", batch_normalization),
+    HELPER("batch_normalization_backward", batch_normalization_backward),
     HELPER("codes_nhwc_slots", codes_nhwc_slots),
     {nullptr, nullptr, 0, nullptr},
 };

@@ -481,6 +481,11 @@ def _binary_convolution(entry, x, weight, binary_weight, alpha, bias, base_axis,
             return binary_weight_convolution_from_codes(codes, tuple(x.shape), weight, binary_weight, alpha, bias, pad,
                                                         stride, dilation, group, quantize_zero_to, fixed_point_delta,
                                                         outputs)
+    if outputs is None and base_axis == 1:
+        y = L.binary_convolution(x, weight, binary_weight, alpha, bias, pad, stride, dilation, group, quantize_zero_to,
+                                 fixed_point_delta)
+        if y is not None:
+            return y
     x, weight = L.f32(x), L.f32(weight, "weight")
     binary_weight = L.f32(binary_weight, "binary_weight")
     bias = L.f32(bias, "bias") if bias is not None else None
@@ -526,6 +531,11 @@ def binary_connect_convolution(x, weight, binary_weight, bias=None, base_axis=1,
 
 def _binary_convolution_backward(entry, x, binary_weight, alpha, dy, base_axis, pad, stride, dilation, group,
                                  propagate_down, accum, grads, fixed_point_delta):
+    if base_axis == 1:
+        out = L.binary_convolution_backward(x, binary_weight, alpha, dy, pad, stride, dilation, group, propagate_down,
+                                            accum, grads, fixed_point_delta)
+        if out is not None:
+            return out
     x, w, dy = L.f32(x), L.f32(binary_weight, "binary_weight"), L.f32(dy, "dy")
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, w, None, base_axis, pad, stride, dilation, group)
@@ -643,6 +653,9 @@ def batch_normalization(x, beta, gamma, mean, variance, axes=[1], decay_rate=0.9
     (src/nbla/function/generic/batch_normalization.cpp:228-260). batch_stat=True: forward_impl_batch
     (:157-226): normalises with the statistics of x and updates `mean` / `variance` (the running
     statistics) in place; output_stat=True also returns the batch mean and variance."""
+    fast = L.batch_normalization(x, beta, gamma, mean, variance, axes, decay_rate, eps, batch_stat, output_stat)
+    if fast is not None:
+        return fast
     x = L.f32(x)
     axes = list(axes)
     if len(axes) != 1:
@@ -817,6 +830,10 @@ def batch_normalization_backward(x, dy, gamma, mean, variance, axes=[1], eps=1e-
     """BatchNormalization::backward_impl (batch_normalization.cpp:262-486). mean / variance: the batch
     statistics the forward pass returned (batch_stat) or the running ones. Returns (dx, dbeta, dgamma),
     None where propagate_down is False."""
+    fast = L.batch_normalization_backward(x, dy, gamma, mean, variance, axes, eps, batch_stat, dmean, dvar, propagate_down,
+                                          accum, grads)
+    if fast is not None:
+        return fast
     x, dy = L.f32(x), L.f32(dy, "dy")
     axes = list(axes)
     if len(axes) != 1:
@@ -1132,6 +1149,10 @@ def convolution_codes_folded(x_codes, x_shape, prepared, scale, bias=None, pad=N
     output="codes": int8 codes [batch, Ho * Wo, slots]; output="float": the fp32 value before ReLU
     and quantizer, channel-last (what a shortcut branch hands to the main branch's epilogue).
     Returns (result, (batch, outmaps, Ho, Wo))."""
+    fast = L.folded_convolution(x_codes, x_shape, prepared.side, prepared.group, prepared.shape, scale, bias, pad, stride,
+                                dilation, residual_codes, residual_delta, residual, relu, sign, n, delta, output)
+    if fast is not None:
+        return fast
     if prepared.group != 1:
         raise C.NB200Error(4, "grouped convolutions are not supported by the folded code path")
     scale = L.f32(scale, "scale")
