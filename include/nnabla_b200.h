@@ -407,7 +407,8 @@ int nb200_pow2_quantize_backward_f32(const float *x, const float *dy, float *dx,
  * as in nb200_min_max_quantize_f32. propagate_down[3] / accum[3] are the
  * flags of x, qr_min, qr_max. g_qr_min / g_qr_max (q-shaped) are written only
  * when neither x_min_max nor ema is set (the reference returns before them,
- * :300-301). */
+ * :300-301); a flag of theirs with bit 1 set (2 or 3) has the buffer zeroed where
+ * it is not written. */
 int nb200_min_max_quantize_backward_f32(const float *x, const int64_t *x_shape, int ndim, const float *qr_min,
                                         const float *qr_max, const float *ql_min, const float *ql_max,
                                         const int64_t *q_shape, const float *dy, int x_min_max, int ema,

@@ -109,6 +109,12 @@ inline unsigned grid_for(size_t work_items) {
   return (unsigned)blocks;
 }
 
+// For the kernels that take kUnroll float4 per thread and round: one per thread as long as that leaves every SM room for
+// all its blocks at once, so that small tensors spread over the chip.
+inline unsigned grid_for_quads(size_t n4) {
+  return n4 <= (size_t)sm_count() * 4 * kThreads ? grid_for(n4) : grid_for((n4 + kUnroll - 1) / kUnroll);
+}
+
 template <typename Op> int launch_elementwise(const float *x, float *y, size_t size, Op op, cudaStream_t st) {
   if (size == 0)
     return NB200_OK;
@@ -125,8 +131,7 @@ template <typename Op> int launch_elementwise(const float *x, float *y, size_t s
     return NB200_OK;
   }
   const size_t n4 = (size - head) / 4;
-  NB_CUDA(launch_dependent(ew_vec_kernel<Op>, dim3(grid_for((n4 + kUnroll - 1) / kUnroll)), dim3(kThreads), 0, st, x, y,
-                           size, head, n4, op));
+  NB_CUDA(launch_dependent(ew_vec_kernel<Op>, dim3(grid_for_quads(n4)), dim3(kThreads), 0, st, x, y, size, head, n4, op));
   return NB200_OK;
 }
 
@@ -734,6 +739,39 @@ __global__ void __launch_bounds__(kThreads) minmax_reduce_kernel(const float *__
   }
 }
 
+struct MinMaxNudged {
+  float m, M, s;
+};
+// The scale (:184-186) and nudge_qr_min_max (:362-390), with every fp32 operation rounded on its own.
+__device__ __forceinline__ MinMaxNudged minmax_nudge(float rmin, float rmax, float lmin, float lmax) {
+  const float s = __fdiv_rn(__fsub_rn(rmax, rmin), __fsub_rn(lmax, lmin));
+  const float z = __fsub_rn(lmin, __fdiv_rn(rmin, s));
+  float zp;
+  if (z <= lmin)
+    zp = lmin;
+  else if (z >= lmax)
+    zp = lmax;
+  else
+    zp = roundf(z);
+  return {__fmul_rn(__fsub_rn(lmin, zp), s), __fmul_rn(__fsub_rn(lmax, zp), s), s};
+}
+
+// The moving average (:159-178) and nudge_range (:352-361) of one range, in place.
+__device__ __forceinline__ void minmax_update(float &rmin, float &rmax, float mn, float mx, int x_min_max, int ema,
+                                              float decay_f, float one_minus_decay_f, float eps) {
+  if (x_min_max) {
+    if (ema) {
+      rmin = __fadd_rn(__fmul_rn(rmin, decay_f), __fmul_rn(mn, one_minus_decay_f));
+      rmax = __fadd_rn(__fmul_rn(rmax, decay_f), __fmul_rn(mx, one_minus_decay_f));
+    } else {
+      rmin = mn;
+      rmax = mx;
+    }
+  }
+  if (__fsub_rn(rmax, rmin) < eps)
+    rmax = __fadd_rn(rmin, eps);
+}
+
 // Parameter step, one thread per q: the moving average (:159-178), nudge_range
 // (:352-361), the scale (:184-186) and nudge_qr_min_max (:362-390), with every
 // fp32 operation rounded on its own.
@@ -748,35 +786,17 @@ __global__ void minmax_params_kernel(size_t Q, float *qr_min, float *qr_max, con
   if (q >= Q)
     return;
   float rmin = qr_min[q], rmax = qr_max[q];
-  if (x_min_max) {
-    const float mn = extremum_value(mn_key[q], true), mx = extremum_value(mx_key[q], false);
-    if (ema) {
-      rmin = __fadd_rn(__fmul_rn(rmin, decay_f), __fmul_rn(mn, one_minus_decay_f));
-      rmax = __fadd_rn(__fmul_rn(rmax, decay_f), __fmul_rn(mx, one_minus_decay_f));
-    } else {
-      rmin = mn;
-      rmax = mx;
-    }
+  minmax_update(rmin, rmax, x_min_max ? extremum_value(mn_key[q], true) : 0.0f,
+                x_min_max ? extremum_value(mx_key[q], false) : 0.0f, x_min_max, ema, decay_f, one_minus_decay_f, eps);
+  if (x_min_max)
     qr_min[q] = rmin;
-  }
-  if (__fsub_rn(rmax, rmin) < eps)
-    rmax = __fadd_rn(rmin, eps);
   qr_max[q] = rmax;
-  const float lmin = ql_min[q], lmax = ql_max[q];
-  const float s = __fdiv_rn(__fsub_rn(rmax, rmin), __fsub_rn(lmax, lmin));
-  const float z = __fsub_rn(lmin, __fdiv_rn(rmin, s));
-  float zp;
-  if (z <= lmin)
-    zp = lmin;
-  else if (z >= lmax)
-    zp = lmax;
-  else
-    zp = roundf(z);
-  m_out[q] = __fmul_rn(__fsub_rn(lmin, zp), s);
-  M_out[q] = __fmul_rn(__fsub_rn(lmax, zp), s);
-  s_out[q] = s;
+  const MinMaxNudged r = minmax_nudge(rmin, rmax, ql_min[q], ql_max[q]);
+  m_out[q] = r.m;
+  M_out[q] = r.M;
+  s_out[q] = r.s;
   if (scale_user)
-    scale_user[q] = s;
+    scale_user[q] = r.s;
 }
 
 __device__ __forceinline__ float minmax_apply_one(float x, float m, float M, float s) {
@@ -822,6 +842,81 @@ struct MinMaxOp {
   }
 };
 
+// The three steps of one range in one block: extrema, parameters, quantizer. Ranges of up to kSmallRange elements; the
+// chain of four launches (initialise, reduce, parameters, quantize) spends its time between them: [16, 24, 49] with 24
+// ranges 12.4 us.
+constexpr size_t kSmallRange = 8192;
+constexpr int kSmallThreads = 512;
+
+__global__ void __launch_bounds__(kSmallThreads)
+    minmax_small_kernel(const float *__restrict__ x, MinMaxView V, float *qr_min, float *qr_max,
+                        const float *__restrict__ ql_min, const float *__restrict__ ql_max, int x_min_max, int ema,
+                        float decay_f, float one_minus_decay_f, float eps, float *__restrict__ y, float *scale_user) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ unsigned long long s_lo[kSmallThreads / 32], s_hi[kSmallThreads / 32];
+  __shared__ MinMaxNudged s_range;
+  const uint32_t q = blockIdx.x, inner = (uint32_t)V.inner, per_q = (uint32_t)V.outer * inner;
+  const size_t step = V.Q * V.inner; // from one outer index to the next
+  const float *xq = x + (size_t)q * inner;
+  if (x_min_max) {
+    unsigned long long klo = extremum_start(true), khi = extremum_start(false);
+    float lo = 1e8f, hi = -1e8f;
+#pragma unroll 4
+    for (uint32_t t = threadIdx.x; t < per_q; t += kSmallThreads) {
+      const uint32_t o = t / inner;
+      const float v = __ldg(xq + o * step + (t - o * inner));
+      if (v < lo)
+        lo = v, klo = extremum_key(v, t, true);
+      if (v > hi)
+        hi = v, khi = extremum_key(v, t, false);
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const unsigned long long lo2 = __shfl_xor_sync(0xffffffffu, klo, d), hi2 = __shfl_xor_sync(0xffffffffu, khi, d);
+      klo = lo2 > klo ? lo2 : klo;
+      khi = hi2 > khi ? hi2 : khi;
+    }
+    if ((threadIdx.x & 31) == 0) {
+      s_lo[threadIdx.x >> 5] = klo;
+      s_hi[threadIdx.x >> 5] = khi;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    float rmin = qr_min[q], rmax = qr_max[q], mn = 0.0f, mx = 0.0f;
+    if (x_min_max) {
+      unsigned long long klo = s_lo[0], khi = s_hi[0];
+      for (int w = 1; w < kSmallThreads / 32; ++w) {
+        klo = s_lo[w] > klo ? s_lo[w] : klo;
+        khi = s_hi[w] > khi ? s_hi[w] : khi;
+      }
+      mn = extremum_value(klo, true), mx = extremum_value(khi, false);
+    }
+    minmax_update(rmin, rmax, mn, mx, x_min_max, ema, decay_f, one_minus_decay_f, eps);
+    if (x_min_max)
+      qr_min[q] = rmin;
+    qr_max[q] = rmax;
+    s_range = minmax_nudge(rmin, rmax, ql_min[q], ql_max[q]);
+    if (scale_user)
+      scale_user[q] = s_range.s;
+  }
+  __syncthreads();
+  const MinMaxNudged r = s_range;
+  float *yq = y + (size_t)q * inner;
+#pragma unroll 4
+  for (uint32_t t = threadIdx.x; t < per_q; t += kSmallThreads) {
+    const uint32_t o = t / inner;
+    const size_t e = o * step + (t - o * inner);
+    yq[e] = minmax_apply_one(__ldg(xq + e), r.m, r.M, r.s);
+  }
+}
+
+// One block per range, where a range is short and the ranges' blocks do not leave most of a large tensor to one block.
+inline bool minmax_small_applies(const MinMaxView &V) {
+  return V.size > 0 && V.outer * V.inner <= kSmallRange && V.Q < (1u << 31);
+}
+
 int minmax_view(const int64_t *xs, const int64_t *qs, int ndim, MinMaxView *V) {
   NB_CHECK(ndim >= 1 && ndim <= 8, NB200_EVALUE, "ndim must be in 1..8 (got %d)", ndim);
   size_t size = 1, Q = 1;
@@ -863,6 +958,13 @@ int minmax_view(const int64_t *xs, const int64_t *qs, int ndim, MinMaxView *V) {
 int minmax_run(const float *x, const MinMaxView &V, float *qr_min, float *qr_max, const float *ql_min,
                const float *ql_max, float decay, int x_min_max, int ema, float eps, float *y, float *scale,
                float *scratch, cudaStream_t st) {
+  // (T)decay_ and (T)(1.0 - decay_) as in min_max_quantize.cpp:105-106.
+  const float d1 = decay, d2 = (float)(1.0 - (double)decay);
+  if (minmax_small_applies(V)) {
+    NB_CUDA(launch_dependent(minmax_small_kernel, dim3((unsigned)V.Q), dim3(kSmallThreads), 0, st, x, V, qr_min, qr_max,
+                             ql_min, ql_max, x_min_max, ema, d1, d2, eps, y, scale));
+    return NB200_OK;
+  }
   unsigned long long *mn = reinterpret_cast<unsigned long long *>(scratch), *mx = mn + V.Q;
   float *m = scratch + 4 * V.Q, *M = scratch + 5 * V.Q, *s = scratch + 6 * V.Q;
   const unsigned qblocks = (unsigned)((V.Q + 255) / 256);
@@ -884,8 +986,6 @@ int minmax_run(const float *x, const MinMaxView &V, float *qr_min, float *qr_max
                              mn, mx));
     NB_LAUNCH_CHECK();
   }
-  // (T)decay_ and (T)(1.0 - decay_) as in min_max_quantize.cpp:105-106.
-  const float d1 = decay, d2 = (float)(1.0 - (double)decay);
   NB_CUDA(launch_dependent(minmax_params_kernel, dim3(qblocks), dim3(256), 0, st, V.Q, qr_min, qr_max, ql_min, ql_max,
                            mn, mx, x_min_max, ema, d1, d2, eps, m, M, s, scale));
   NB_LAUNCH_CHECK();

@@ -99,8 +99,8 @@ int launch_gradient_t(const float *x, const float *dy, float *dx, size_t size, c
                              size, op));
   } else {
     const size_t n4 = size / 4;
-    NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum>, dim3(grid_for((n4 + kUnroll - 1) / kUnroll)), dim3(kThreads),
-                             0, st, x, dy, dx, size, n4, op));
+    NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum>, dim3(grid_for_quads(n4)), dim3(kThreads), 0,
+                             st, x, dy, dx, size, n4, op));
   }
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -207,18 +207,9 @@ __global__ void minmax_nudged_kernel(size_t Q, const float *qr_min, const float 
   const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (q >= Q)
     return;
-  const float rmin = qr_min[q], rmax = qr_max[q], lmin = ql_min[q], lmax = ql_max[q];
-  const float s = __fdiv_rn(__fsub_rn(rmax, rmin), __fsub_rn(lmax, lmin));
-  const float z = __fsub_rn(lmin, __fdiv_rn(rmin, s));
-  float zp;
-  if (z <= lmin)
-    zp = lmin;
-  else if (z >= lmax)
-    zp = lmax;
-  else
-    zp = roundf(z);
-  m_out[q] = __fmul_rn(__fsub_rn(lmin, zp), s);
-  M_out[q] = __fmul_rn(__fsub_rn(lmax, zp), s);
+  const MinMaxNudged r = minmax_nudge(qr_min[q], qr_max[q], ql_min[q], ql_max[q]);
+  m_out[q] = r.m;
+  M_out[q] = r.M;
 }
 
 // Gradient w.r.t. x with ste_fine_grained (:268-287): (x >= m) * (x <= M) * dy.
@@ -368,11 +359,65 @@ __global__ void __launch_bounds__(kThreads) minmax_range_finish_kernel(const flo
   }
 }
 
+// Gradient w.r.t. x of one range per block (as minmax_small_kernel): mask and pass in one launch. zero_min / zero_max
+// (may be NULL) receive 0: range gradients that this call does not produce.
+template <bool kFine, bool kAccum>
+__global__ void __launch_bounds__(kSmallThreads)
+    minmax_small_grad_kernel(const float *__restrict__ x, const float *__restrict__ dy, MinMaxView V,
+                             const float *__restrict__ qr_min, const float *__restrict__ qr_max,
+                             const float *__restrict__ ql_min, const float *__restrict__ ql_max, float *__restrict__ dx,
+                             float *zero_min, float *zero_max) {
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t q = blockIdx.x, inner = (uint32_t)V.inner, per_q = (uint32_t)V.outer * inner;
+  const size_t step = V.Q * V.inner;
+  MinMaxNudged r{0.0f, 0.0f, 0.0f};
+  if (kFine)
+    r = minmax_nudge(__ldg(qr_min + q), __ldg(qr_max + q), __ldg(ql_min + q), __ldg(ql_max + q));
+  if (threadIdx.x == 0) {
+    if (zero_min)
+      zero_min[q] = 0.0f;
+    if (zero_max)
+      zero_max[q] = 0.0f;
+  }
+#pragma unroll 4
+  for (uint32_t t = threadIdx.x; dx && t < per_q; t += kSmallThreads) {
+    const uint32_t o = t / inner;
+    const size_t e = (size_t)q * inner + o * step + (t - o * inner);
+    float g = dy[e];
+    if (kFine) {
+      const float v = x[e];
+      g = __fmul_rn(__fmul_rn((v >= r.m) ? 1.0f : 0.0f, (v <= r.M) ? 1.0f : 0.0f), g);
+    }
+    dx[e] = kAccum ? __fadd_rn(dx[e], g) : g;
+  }
+}
+
 int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, const float *qr_max, const float *ql_min,
                     const float *ql_max, const float *dy, int x_min_max, int ema, int fine, const int32_t *prop,
                     const int32_t *accum, float *dx, float *g_min, float *g_max, cudaStream_t st) {
-  const bool ranges = !(x_min_max || ema) && (prop[1] || prop[2]);
-  const bool need_nudged = (prop[0] && fine) || ranges;
+  const int down[3] = {prop[0] & 1, prop[1] & 1, prop[2] & 1};
+  const bool ranges = !(x_min_max || ema) && (down[1] || down[2]);
+  const bool need_nudged = (down[0] && fine) || ranges;
+  // range gradients to be zeroed: asked for (flag 2) and not produced below
+  float *zero_min = (prop[1] & 2) && !(ranges && down[1]) ? g_min : nullptr;
+  float *zero_max = (prop[2] & 2) && !(ranges && down[2]) ? g_max : nullptr;
+  if (!ranges && minmax_small_applies(V) && V.Q <= 65535) {
+    if (!down[0] && !zero_min && !zero_max)
+      return NB200_OK;
+    NB_CHECK(!(down[0] && fine) || (qr_min && qr_max && ql_min && ql_max), NB200_EVALUE, "null range pointer");
+    NB_CHECK(!down[0] || (dx && dy && (x || !fine)), NB200_EVALUE, "null data pointer");
+    const bool f = down[0] && fine, a = down[0] && accum[0];
+    auto kernel = f ? (a ? minmax_small_grad_kernel<true, true> : minmax_small_grad_kernel<true, false>)
+                    : (a ? minmax_small_grad_kernel<false, true> : minmax_small_grad_kernel<false, false>);
+    NB_CUDA(launch_dependent(kernel, dim3((unsigned)V.Q), dim3(kSmallThreads), 0, st, x, dy, V, qr_min, qr_max, ql_min,
+                             ql_max, down[0] ? dx : nullptr, zero_min, zero_max));
+    return NB200_OK;
+  }
+  if (zero_min)
+    NB_CUDA(cudaMemsetAsync(zero_min, 0, V.Q * sizeof(float), st));
+  if (zero_max)
+    NB_CUDA(cudaMemsetAsync(zero_max, 0, V.Q * sizeof(float), st));
   if (V.size == 0 && !ranges)
     return NB200_OK;
   NB_CHECK(V.Q <= 65535, NB200_ENOTIMPL, "more than 65535 quantization ranges");
@@ -391,10 +436,10 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
     NB_LAUNCH_CHECK();
   }
   // Per-tensor ranges with aligned buffers: one pass produces dx and the range sums.
-  const bool fused = ranges && prop[0] && V.Q == 1 && V.size > 0 &&
+  const bool fused = ranges && down[0] && V.Q == 1 && V.size > 0 &&
                      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) |
                        reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
-  if (prop[0] && !fused) {
+  if (down[0] && !fused) {
     if (fine) {
       MinMaxGrad op{m, M, V.Q, V.inner};
       NB_TRY(launch_gradient(x, dy, dx, V.size, accum[0], op, st));
@@ -403,7 +448,7 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
     }
   }
   if (ranges) {
-    NB_CHECK((!prop[1] || g_min) && (!prop[2] || g_max), NB200_EVALUE, "null range-gradient pointer");
+    NB_CHECK((!down[1] || g_min) && (!down[2] || g_max), NB200_EVALUE, "null range-gradient pointer");
     NB_CHECK(V.size == 0 || (x && dy), NB200_EVALUE, "null data pointer");
     const dim3 grid((unsigned)splits, (unsigned)V.Q);
     if (!fused) {
@@ -426,7 +471,7 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
     }
     NB_LAUNCH_CHECK();
     NB_CUDA(launch_dependent(minmax_range_finish_kernel, dim3((unsigned)V.Q), dim3(kThreads), 0, st, partial,
-                             (unsigned)splits, g_min, g_max, prop[1], prop[2], accum[1], accum[2]));
+                             (unsigned)splits, g_min, g_max, down[1], down[2], accum[1], accum[2]));
     NB_LAUNCH_CHECK();
   }
   return NB200_OK;

@@ -111,12 +111,12 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
     if not quantize:
         return x
     x = L.f32(x)
-    qs = [L.f32(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
-                                            (ql_max, "ql_max"))]
+    qs = (L.f32(qr_min, "qr_min"), L.f32(qr_max, "qr_max"), L.f32(ql_min, "ql_min"), L.f32(ql_max, "ql_max"))
     # Shape rules of MinMaxQuantize::setup_impl (min_max_quantize.cpp:54-83).
-    if len({t.dim() for t in qs}) != 1:
+    qshape = qs[0].shape
+    if any(t.dim() != qs[0].dim() for t in qs):
         raise RuntimeError("All input dimensions must be same.")
-    if len({tuple(t.shape) for t in qs}) != 1:
+    if any(t.shape != qshape for t in qs):
         raise RuntimeError("All shapes among ql_min, ql_max, qr_min, and qr_max must be same.")
     if qs[0].dim() != x.dim():
         raise RuntimeError("x.shape and ql_min.shape must be same except for i-th dimension where "
@@ -174,20 +174,21 @@ def min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max=F
     left in place. Returns (dx, g_qr_min, g_qr_max); the range gradients are
     produced only when neither x_min_max nor ema is set."""
     x, dy, dx = _grad_buffers(x, dy, grads[0], accum[0])
-    qs = [L.f32(t, nm) for t, nm in ((qr_min, "qr_min"), (qr_max, "qr_max"), (ql_min, "ql_min"),
-                                            (ql_max, "ql_max"))]
-    if len({tuple(t.shape) for t in qs}) != 1 or qs[0].dim() != x.dim():
+    qs = (L.f32(qr_min, "qr_min"), L.f32(qr_max, "qr_max"), L.f32(ql_min, "ql_min"), L.f32(ql_max, "ql_max"))
+    if any(t.shape != qs[0].shape for t in qs) or qs[0].dim() != x.dim():
         raise RuntimeError("All shapes among ql_min, ql_max, qr_min, and qr_max must be same.")
-    gq = []
-    for g, acc in ((grads[1], accum[1]), (grads[2], accum[2])):
+    gq, flags = [], [1 if propagate_down[0] else 0]
+    for g, acc, pd in ((grads[1], accum[1], propagate_down[1]), (grads[2], accum[2], propagate_down[2])):
+        flags.append(1 if pd else 0)
         if g is None:
             if acc:
                 raise RuntimeError("accum=True needs the gradient buffer to accumulate into")
-            g = torch.zeros_like(qs[0])
+            g = L.empty(qs[0], x)
+            flags[-1] |= 2  # zero unless the call produces it
         gq.append(L.f32(g, "range gradient"))
     L.nb200_min_max_quantize_backward_f32(x, x.shape, x.dim(), qs[0], qs[1], qs[2], qs[3], qs[0].shape, dy,
                                           bool(x_min_max), bool(ema), bool(ste_fine_grained),
-                                          [bool(v) for v in propagate_down], [bool(v) for v in accum], dx, gq[0], gq[1])
+                                          flags, [bool(v) for v in accum], dx, gq[0], gq[1])
     return dx, gq[0], gq[1]
 
 

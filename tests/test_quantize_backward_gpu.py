@@ -134,3 +134,36 @@ def test_backward_argument_errors(F):
         F.fixed_point_quantize_backward(x, x, n=0)
     with pytest.raises(RuntimeError):
         F.pow2_quantize_backward(x, x, n=1)
+
+
+# one block per range up to 8192 elements, the launches of separate steps above
+@pytest.mark.parametrize("shape,axis", [((1, 1, 1), None), ((3, 5, 7), 1), ((2, 3, 4097), 1), ((8, 24, 1024), 1),
+                                        ((8, 24, 1025), 1), ((8192,), None), ((8193,), None), ((700, 2), 0)])
+@pytest.mark.parametrize("observe", [True, False])
+@pytest.mark.parametrize("fine", [True, False])
+def test_min_max_quantize_range_lengths(shape, axis, observe, fine):
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(len(shape))
+    x, dy = (torch.randn(*shape, device="cuda", generator=g) * 3 for _ in range(2))
+    qshape = [n if i == axis else 1 for i, n in enumerate(shape)]
+    dims = [i for i in range(len(shape)) if i != axis]
+    qmin, qmax = torch.full(qshape, -1.5, device="cuda"), torch.full(qshape, 2.0, device="cuda")
+    lmin, lmax = torch.zeros(qshape, device="cuda"), torch.full(qshape, 255.0, device="cuda")
+    y = F.min_max_quantize(x, qmin, qmax, lmin, lmax, x_min_max=observe)
+    lo, hi = (x.amin(dims, keepdim=True), x.amax(dims, keepdim=True)) if observe else (qmin, qmax)
+    hi = torch.where(hi - lo < 0.01, lo + 0.01, hi)
+    assert torch.equal(qmin, lo) and torch.equal(qmax, hi)
+    s = (hi - lo) / 255
+    zp = torch.clamp(torch.round(-lo / s), 0, 255)
+    m, M = -zp * s, (255 - zp) * s
+    assert ((y - (torch.round((torch.minimum(torch.maximum(x, m), M) - m) / s) * s + m)).abs() <= 1.01 * s).all()
+    old = torch.ones_like(x)
+    for accum, buffer in ((False, None), (True, old)):
+        dx, g_lo, g_hi = F.min_max_quantize_backward(x, qmin, qmax, lmin, lmax, dy, x_min_max=observe, ste_fine_grained=fine,
+                                                     accum=(accum, False, False), grads=(buffer, None, None))
+        inside = (x >= m) & (x <= M) if fine else torch.ones_like(x, dtype=torch.bool)
+        off = dx - float(accum) - dy * inside
+        assert (off.abs() <= 1e-6 * (1 + dy.abs())).float().mean() >= 1 - 3 / x.numel()  # a bound itself may round
+        for got, side in ((g_lo, x < m), (g_hi, x > M)):
+            want = torch.zeros_like(got) if observe else (dy.double() * side).sum(dims, keepdim=True)
+            assert got.shape == torch.Size(qshape) and ((got - want).abs() <= 1e-4 * dy.abs().sum() ** 0.5 + 1e-5).all()
