@@ -606,18 +606,25 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   uint8_t *xp = at, *side = xp + x_bytes;
   q.slots = reinterpret_cast<float *>(side + side_bytes);
   const bool scaled = *did_dx && alpha;
-  NB_TRY(nhwc_pieces(dy, g.N, g.Ko, g.Ho * g.Wo, g.group, g.Kog, k_pad_g, (int)k_tot, 3, scaled ? alpha : nullptr,
-                     scaled ? dys : nullptr, scaled ? (two ? dyp : nullptr) : dyp, st));
+  ConvBackwardOperands ops{};
+  ops.N = g.N, ops.groups = g.group, ops.Kog = g.Kog, ops.Cg = g.Cg;
+  ops.dy = dy, ops.alpha = scaled ? alpha : nullptr;
+  ops.dy_pixels = g.Ho * g.Wo, ops.k_pad_g = k_pad_g, ops.k_total = (int)k_tot;
+  ops.dy_scaled = scaled ? dys : nullptr;
+  ops.dy_plain = scaled ? (two ? dyp : nullptr) : dyp;
+  ops.x = x, ops.x_pixels = g.H * g.W, ops.c_pad_g = c_pad_g, ops.c_total = (int)c_tot, ops.x_planes = x_planes;
+  ops.x_pieces = *did_dw ? xp : nullptr;
+  ops.wb = wb, ops.taps = taps, ops.k_slots = p.k_slots;
+  ops.side = *did_dx ? side : nullptr;
+  NB_TRY(conv_backward_operands(ops, st));
   if (*did_dx) {
     p.c_group_stride = k_pad_g;
     p.y = dx;
     p.accumulate = accum_dx;
-    NB_TRY(transpose_binary_weights(wb, g.Ko, g.Cg, taps, g.group, p.k_slots, side, st));
     NB_TRY(launch_planes(plan, dys, g.Ho, g.Wo, k_tot, side, taps, false, st));
   }
   if (!*did_dw)
     return NB200_OK;
-  NB_TRY(nhwc_pieces(x, g.N, g.C, g.H * g.W, g.group, g.Cg, c_pad_g, (int)c_tot, x_planes, nullptr, nullptr, xp, st));
   q.k_stride = k_pad_g;
   q.c_stride = c_pad_g;
   CUtensorMap mx, md;

@@ -66,13 +66,23 @@ int fxp8_operands(const float *x, int64_t M, int K, int64_t Kp, float delta_x, i
                   float delta_w, int8_t *wt, cudaStream_t st);
 
 // ---- convolution backward (prepare_backward.cu) ------------------------------
-// src [N][C][HW] fp32 -> channel-last bf16 pieces [planes][N][HW][ctot] (planes = 3 or 1), of src * chan_scale[c] in
-// `scaled` and of src in `plain` (either may be NULL).
-int nhwc_pieces(const float *src, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, int planes,
-                const float *chan_scale, void *scaled, void *plain, cudaStream_t st);
-// wb [Ko][Cg][taps] of values exact in bf16 -> [groups * Cg][taps][k_slots] bf16, zero padded.
-int transpose_binary_weights(const float *wb, int Ko, int Cg, int taps, int groups, int k_slots, void *side,
-                             cudaStream_t st);
+// Operands of the two gradients of a convolution, channel-last: dy [N][groups * Kog][dy_pixels] as three bf16 pieces,
+// times alpha[map] (may be NULL) in dy_scaled and as it is in dy_plain (either may be NULL); x [N][groups * Cg][x_pixels] as
+// x_planes (3 or 1) bf16 pieces in x_pieces; wb [groups * Kog][Cg][taps] of values exact in bf16 as
+// [groups * Cg][taps][k_slots] bf16, zero padded, in side. What is NULL is not made.
+struct ConvBackwardOperands {
+  int N, groups, Kog, Cg;
+  const float *dy, *alpha;
+  int dy_pixels, k_pad_g, k_total;
+  void *dy_scaled, *dy_plain;
+  const float *x;
+  int x_pixels, c_pad_g, c_total, x_planes;
+  void *x_pieces;
+  const float *wb;
+  int taps, k_slots;
+  void *side;
+};
+int conv_backward_operands(const ConvBackwardOperands &o, cudaStream_t st);
 // dy [N][Ko][Ho][Wo] -> 3 bf16 planes [N][Hs][Ws][ctot] (pre-zeroed by the caller):
 // pixel (oy, ox) at (oy * sh, ox * sw), map o of group g at slot g * k_pad_g + o - g * Kog,
 // multiplied by chan_scale[o] first when given.

@@ -116,16 +116,31 @@ __global__ void __launch_bounds__(256) image_absmax_kernel(const float *__restri
 // left in image_max[n]. The images go last to first, against the order that the maxima were taken in, so that most of
 // them still come from L2: [128, 256, 28, 28] 50 us for the two passes (82 us with the maximum of the whole tensor and
 // 4-byte stores).
+struct NhwcPieces {
+  const float *src;
+  int N, C, HW, groups, Cg, c_pad_g, ctot;
+  const float *chan_scale;
+  uint16_t *scaled, *plain;
+  const uint32_t *image_parts; // kHalf
+  int parts;
+  uint32_t *image_max;
+  __host__ __device__ int tiles_x() const { return (HW + 63) / 64; }
+  __host__ __device__ int tiles_y() const { return (ctot + 63) / 64; }
+  __host__ __device__ int64_t blocks() const { return (int64_t)tiles_x() * tiles_y() * N; }
+  bool vec() const { return HW % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0; }
+};
+
 template <bool kVec, int PLANES, bool kHalf>
-__global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restrict__ src, int C, int HW, int groups, int Cg,
-                                                          int c_pad_g, int ctot, const float *__restrict__ chan_scale,
-                                                          uint16_t *__restrict__ scaled, uint16_t *__restrict__ plain,
-                                                          int64_t plane_stride, const uint32_t *__restrict__ image_parts,
-                                                          int parts, uint32_t *__restrict__ image_max) {
-  __shared__ uint4 tile[PLANES][64][8];
-  pdl_wait();
-  pdl_trigger();
-  const int n = kHalf ? gridDim.z - 1 - blockIdx.z : blockIdx.z, p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
+__device__ __forceinline__ void nhwc_pieces_tile(const NhwcPieces &P, int block, uint4 (*tile)[64][8]) {
+  const float *__restrict__ src = P.src;
+  const float *__restrict__ chan_scale = P.chan_scale;
+  const uint32_t *__restrict__ image_parts = P.image_parts;
+  uint16_t *__restrict__ scaled = P.scaled, *__restrict__ plain = P.plain;
+  const int C = P.C, HW = P.HW, groups = P.groups, Cg = P.Cg, c_pad_g = P.c_pad_g, ctot = P.ctot, parts = P.parts;
+  const int64_t plane_stride = (int64_t)P.N * HW * ctot;
+  const int tx = P.tiles_x(), ty = P.tiles_y();
+  const int bx = block % tx, by = block / tx % ty, bz = block / (tx * ty);
+  const int n = kHalf ? P.N - 1 - bz : bz, p0 = bx * 64, d0 = by * 64;
   const int px4 = threadIdx.x & 15, chq = threadIdx.x >> 4;
   const int p = p0 + 4 * px4, dq = d0 + 4 * chq;
   const int g = dq / c_pad_g, cc0 = dq - g * c_pad_g; // c_pad_g is a multiple of 16: one group for the four slots
@@ -138,8 +153,8 @@ __global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restric
       m = max(m, __ldg(image_parts + (int64_t)n * parts + i));
     m = __reduce_max_sync(0xffffffffu, m);
     down = __int_as_float((127 - half_pair_exponent(m)) << 23);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-      image_max[n] = m;
+    if (bx == 0 && by == 0 && threadIdx.x == 0)
+      P.image_max[n] = m;
   }
   float v[4][4], f[4];
 #pragma unroll
@@ -201,20 +216,52 @@ __global__ void __launch_bounds__(256) nhwc_pieces_kernel(const float *__restric
   }
 }
 
-// wb [Ko][Cg][kh][kw] of +-1 (exact in bf16) -> side [C][kh * kw][k_slots] bf16, row g * Cg + c, maps of the group
-// innermost, zero past them: the weights of the input gradient, one block per row.
-__global__ void __launch_bounds__(256) transpose_binary_weights_kernel(const float *__restrict__ wb, int Cg, int taps,
-                                                                       int Kog, int k_slots,
-                                                                       __nv_bfloat16 *__restrict__ side) {
+template <bool kVec, int PLANES, bool kHalf>
+__global__ void __launch_bounds__(256) nhwc_pieces_kernel(const __grid_constant__ NhwcPieces P) {
+  __shared__ uint4 tile[PLANES][64][8];
   pdl_wait();
   pdl_trigger();
-  const int row = blockIdx.x, g = row / Cg, c = row - g * Cg;
-  const float *src = wb + ((int64_t)g * Kog * Cg + c) * taps;
-  __nv_bfloat16 *dst = side + (int64_t)row * taps * k_slots;
-  for (int i = threadIdx.x; i < taps * k_slots; i += 256) {
-    const int t = i / k_slots, o = i - t * k_slots;
-    dst[i] = o < Kog ? __float2bfloat16_rn(__ldg(src + (int64_t)o * Cg * taps + t)) : __float2bfloat16_rn(0.0f);
+  nhwc_pieces_tile<kVec, PLANES, kHalf>(P, blockIdx.x, tile);
+}
+
+// wb [Ko][Cg][kh][kw] of +-1 (exact in bf16) -> side [C][kh * kw][k_slots] bf16, row g * Cg + c, maps of the group
+// innermost, zero past them: the weights of the input gradient, one block per row.
+struct TransposedWeights {
+  const float *wb;
+  int rows, Cg, taps, Kog, k_slots;
+  __nv_bfloat16 *side;
+};
+
+__device__ __forceinline__ void transpose_binary_weights_row(const TransposedWeights &W, int row) {
+  const int g = row / W.Cg, c = row - g * W.Cg, taps = W.taps;
+  const float *src = W.wb + ((int64_t)g * W.Kog * W.Cg + c) * taps;
+  __nv_bfloat16 *dst = W.side + (int64_t)row * taps * W.k_slots;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < taps * W.k_slots; i += 256) {
+    const int t = i / W.k_slots, o = i - t * W.k_slots;
+    dst[i] = o < W.Kog ? __float2bfloat16_rn(__ldg(src + (int64_t)o * W.Cg * taps + t)) : __float2bfloat16_rn(0.0f);
   }
+}
+
+// Everything that the two gradients of a convolution read, in one launch: the weights' rows first (short blocks of
+// scattered loads), then the pieces of dy and of x. Three launches took 17 to 19 us at 256 maps of 14 x 14 where this takes
+// 9.
+template <bool kVecDy, bool kVecX, int XP>
+__global__ void __launch_bounds__(256) conv_backward_operands_kernel(const __grid_constant__ TransposedWeights W,
+                                                                     const __grid_constant__ NhwcPieces dy,
+                                                                     const __grid_constant__ NhwcPieces x) {
+  __shared__ uint4 tile[3][64][8];
+  pdl_wait();
+  pdl_trigger();
+  int block = blockIdx.x;
+  if (block < W.rows)
+    return transpose_binary_weights_row(W, block);
+  block -= W.rows;
+  const int dy_blocks = (int)dy.blocks();
+  if (block < dy_blocks)
+    nhwc_pieces_tile<kVecDy, 3, false>(dy, block, tile);
+  else
+    nhwc_pieces_tile<kVecX, XP, false>(x, block - dy_blocks, tile);
 }
 
 // wb [Ko][Cg][kh][kw] fp32 -> side [planes][C][kh * kw][k_slots] bf16:
@@ -360,19 +407,6 @@ int dy_to_nhwc_stuffed(const float *dy, int N, int Ko, int Ho, int Wo, int group
   return NB200_OK;
 }
 
-int nhwc_pieces(const float *src, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot, int planes,
-                const float *chan_scale, void *scaled, void *plain, cudaStream_t st) {
-  NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
-  const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
-  const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  auto kernel = planes == 3 ? (vec ? nhwc_pieces_kernel<true, 3, false> : nhwc_pieces_kernel<false, 3, false>)
-                            : (vec ? nhwc_pieces_kernel<true, 1, false> : nhwc_pieces_kernel<false, 1, false>);
-  NB_CUDA(launch_dependent(kernel, grid, dim3(256), 0, st, src, C, HW, groups, Cg, c_pad_g, ctot, chan_scale,
-                           static_cast<uint16_t *>(scaled), static_cast<uint16_t *>(plain), (int64_t)N * HW * ctot,
-                           (const uint32_t *)nullptr, 0, (uint32_t *)nullptr));
-  return NB200_OK;
-}
-
 int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int groups, int Cg, int c_pad_g, int ctot,
                                   void *out, uint32_t *image_max, cudaStream_t st) {
   NB_CHECK(N <= 65535, NB200_ENOTIMPL, "batch larger than 65535");
@@ -381,21 +415,29 @@ int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int grou
   const int64_t most = std::min<int64_t>(kHalfPairParts, 16ll * sm_count() / N);
   const int parts = (int)std::max<int64_t>(1, std::min(per_image / 4096, most));
   NB_CUDA(launch_dependent(image_absmax_kernel, dim3(parts, N), dim3(256), 0, st, x, per_image, image_max + N));
-  const dim3 grid((HW + 63) / 64, (ctot + 63) / 64, N);
-  const bool vec = HW % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  NB_CUDA(launch_dependent(vec ? nhwc_pieces_kernel<true, 2, true> : nhwc_pieces_kernel<false, 2, true>, grid,
-                           dim3(256),
-                           0, st, x, C, HW, groups, Cg, c_pad_g, ctot, (const float *)nullptr, static_cast<uint16_t *>(out),
-                           (uint16_t *)nullptr, (int64_t)N * HW * ctot, image_max + N, parts, image_max));
+  const NhwcPieces P{x,       N,       C, HW, groups, Cg, c_pad_g, ctot, nullptr, static_cast<uint16_t *>(out),
+                     nullptr, image_max + N, parts, image_max};
+  NB_CHECK(P.blocks() < (1ll << 31), NB200_ENOTIMPL, "tensor too large");
+  NB_CUDA(launch_dependent(P.vec() ? nhwc_pieces_kernel<true, 2, true> : nhwc_pieces_kernel<false, 2, true>,
+                           dim3((unsigned)P.blocks()), dim3(256), 0, st, P));
   return NB200_OK;
 }
 
-int transpose_binary_weights(const float *wb, int Ko, int Cg, int taps, int groups, int k_slots, void *side,
-                             cudaStream_t st) {
-  NB_CUDA(launch_dependent(transpose_binary_weights_kernel, dim3(groups * Cg), dim3(256), 0, st, wb, Cg, taps, Ko /
-                           groups,
-                           k_slots, static_cast<__nv_bfloat16 *>(side)));
-  NB_LAUNCH_CHECK();
+int conv_backward_operands(const ConvBackwardOperands &o, cudaStream_t st) {
+  const TransposedWeights W{o.wb, o.side ? o.groups * o.Cg : 0, o.Cg, o.taps, o.Kog, o.k_slots,
+                            static_cast<__nv_bfloat16 *>(o.side)};
+  const NhwcPieces dy{o.dy, o.N, o.groups * o.Kog, o.dy_pixels, o.groups, o.Kog, o.k_pad_g, o.k_total, o.alpha,
+                      static_cast<uint16_t *>(o.dy_scaled), static_cast<uint16_t *>(o.dy_plain), nullptr, 0, nullptr};
+  const NhwcPieces x{o.x, o.x_pieces ? o.N : 0, o.groups * o.Cg, o.x_pixels, o.groups, o.Cg, o.c_pad_g, o.c_total, nullptr,
+                     nullptr, static_cast<uint16_t *>(o.x_pieces), nullptr, 0, nullptr};
+  const int64_t blocks = W.rows + dy.blocks() + x.blocks();
+  NB_CHECK(blocks < (1ll << 31), NB200_ENOTIMPL, "tensor too large");
+  const bool vd = dy.vec(), vx = x.vec();
+  auto kernel = o.x_planes == 3 ? (vd ? (vx ? conv_backward_operands_kernel<true, true, 3> : conv_backward_operands_kernel<true, false, 3>)
+                                      : (vx ? conv_backward_operands_kernel<false, true, 3> : conv_backward_operands_kernel<false, false, 3>))
+                                : (vd ? (vx ? conv_backward_operands_kernel<true, true, 1> : conv_backward_operands_kernel<true, false, 1>)
+                                      : (vx ? conv_backward_operands_kernel<false, true, 1> : conv_backward_operands_kernel<false, false, 1>));
+  NB_CUDA(launch_dependent(kernel, dim3((unsigned)blocks), dim3(256), 0, st, W, dy, x));
   return NB200_OK;
 }
 
