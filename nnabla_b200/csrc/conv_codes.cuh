@@ -216,16 +216,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const bool tabulated = k_blocks <= kCodesKTable;
   for (int kb = threadIdx.x; kb < k_blocks && kb < kCodesKTable; kb += kGemmThreads)
     kb_table[kb] = kb_entry(kb);
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_slot, kTmemCols);
+    ptx::tmem_relinquish();
+  }
   pdl_wait();
   pdl_trigger();
   for (int c = threadIdx.x; c < prob.n_tiles * BN; c += kGemmThreads)
     sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
                                       ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)
                         : make_float2(0.0f, 0.0f);
-  if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, kTmemCols);
-    ptx::tmem_relinquish();
-  }
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
