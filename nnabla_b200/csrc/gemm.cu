@@ -215,8 +215,7 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
   void *planes = base;
   void *side = base + round_up(planes_bytes, 256);
   float *partial = reinterpret_cast<float *>(base + round_up(planes_bytes, 256) + round_up(side_bytes, 256));
-  NB_TRY(binarize_columns(w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, false, partial, st));
-  NB_TRY(split_rows_bf16(x, M, (int)K, Kp, 3, planes, st));
+  NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st));
   GemmEpilogue ep{};
   ep.y = y;
   ep.scale = 1.0f;

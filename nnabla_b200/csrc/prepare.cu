@@ -73,15 +73,12 @@ __global__ void __launch_bounds__(256) binarize_columns_kernel(const float *__re
 // The same with 128-bit accesses (C a multiple of 4, 16-byte aligned W / Wb, side-band rows
 // aligned to 8 bytes): a thread handles four columns of a row, and four rows of a side-band row.
 template <bool kInt8>
-__global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *__restrict__ w, int R, int C,
-                                                                   float zero_to, float *__restrict__ wb,
-                                                                   void *__restrict__ side, int64_t side_pitch,
-                                                                   float *__restrict__ partial) {
-  pdl_wait();
-  pdl_trigger();
+__device__ __forceinline__ void binarize_columns_vec_tile(int bx, int by, const float *__restrict__ w, int R, int C,
+                                                          float zero_to, float *__restrict__ wb, void *__restrict__ side,
+                                                          int64_t side_pitch, float *__restrict__ partial) {
   __shared__ float s_sign[kBT][kBT + 1];
   __shared__ float s_sum[16][kBT];
-  const int c0 = blockIdx.x * kBT, r0 = blockIdx.y * kBT;
+  const int c0 = bx * kBT, r0 = by * kBT;
   const int tx4 = threadIdx.x & 15, ty = threadIdx.x >> 4; // 16 column quads x 16 rows
   const int c = c0 + 4 * tx4;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -109,7 +106,7 @@ __global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *
 #pragma unroll
     for (int k = 0; k < 16; ++k)
       t += s_sum[k][threadIdx.x];
-    partial[(int64_t)blockIdx.y * C + c0 + threadIdx.x] = t;
+    partial[(int64_t)by * C + c0 + threadIdx.x] = t;
   }
   // side-band: row = output column, contiguous index = input row; four input rows per thread
   const int r = r0 + 4 * tx4;
@@ -134,6 +131,16 @@ __global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *
       *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(side) + (int64_t)oc * side_pitch + r) = out;
     }
   }
+}
+
+template <bool kInt8>
+__global__ void __launch_bounds__(256) binarize_columns_vec_kernel(const float *__restrict__ w, int R, int C,
+                                                                   float zero_to, float *__restrict__ wb,
+                                                                   void *__restrict__ side, int64_t side_pitch,
+                                                                   float *__restrict__ partial) {
+  pdl_wait();
+  pdl_trigger();
+  binarize_columns_vec_tile<kInt8>(blockIdx.x, blockIdx.y, w, R, C, zero_to, wb, side, side_pitch, partial);
 }
 
 __global__ void finalize_alpha_kernel(const float *__restrict__ partial, int blocks, int C, float inv,
@@ -268,6 +275,37 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
     if (planes > 2)
       out[2 * plane_stride + i] = l;
   }
+}
+
+// Both operands of a binary-weight affine layer in one launch: the weights' 64 x 64 tiles first, then four values of x per
+// thread into three bf16 pieces [3][rows][Kp] (Kp a multiple of 64, zero padded; K a multiple of 4, 16-byte aligned).
+__global__ void __launch_bounds__(256) binary_affine_operands_kernel(const float *__restrict__ w, int R, int C, float zero_to,
+                                                                     float *__restrict__ wb, void *__restrict__ side,
+                                                                     int64_t side_pitch, float *__restrict__ partial, int gx,
+                                                                     int w_blocks, const float *__restrict__ x, int64_t rows,
+                                                                     __nv_bfloat16 *__restrict__ pieces) {
+  pdl_wait();
+  pdl_trigger();
+  if ((int)blockIdx.x < w_blocks) {
+    binarize_columns_vec_tile<false>((int)blockIdx.x % gx, (int)blockIdx.x / gx, w, R, C, zero_to, wb, side, side_pitch,
+                                     partial);
+    return;
+  }
+  const unsigned quads = (unsigned)(side_pitch / 4); // x's rows are padded like the side-band's
+  const int64_t i = (int64_t)(blockIdx.x - w_blocks) * 256 + threadIdx.x;
+  const int64_t r = i / quads;
+  const int k = 4 * (int)(i - r * quads);
+  if (r >= rows)
+    return;
+  const float4 v = k < R ? __ldcs(reinterpret_cast<const float4 *>(x + r * R + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float e[4] = {v.x, v.y, v.z, v.w};
+  __align__(8) __nv_bfloat16 p[3][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    split3(e[j], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+  for (int pl = 0; pl < 3; ++pl)
+    *reinterpret_cast<uint2 *>(pieces + (pl * rows + r) * side_pitch + k) = *reinterpret_cast<const uint2 *>(p[pl]);
 }
 
 // Column sums of a row-major [rows, C] matrix (bias gradient, affine.cpp:130-137):
@@ -618,6 +656,25 @@ int binarize_columns(const float *w, int R, int C, float zero_to, float *wb, flo
                              inv, alpha));
     NB_LAUNCH_CHECK();
   }
+  return NB200_OK;
+}
+
+int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, int C, float zero_to, float *wb, float *alpha,
+                           void *side, int64_t pitch, float *partial_scratch, void *pieces, cudaStream_t st) {
+  const int gx = (C + kBT - 1) / kBT, gy = (R + kBT - 1) / kBT;
+  const int64_t w_blocks = (int64_t)gx * gy, x_blocks = (rows * (pitch / 4) + 255) / 256;
+  const bool vec = C % 4 == 0 && R % 4 == 0 && w_blocks + x_blocks < (1ll << 31) &&
+                   ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(wb) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
+  if (!vec) {
+    NB_TRY(binarize_columns(w, R, C, zero_to, wb, alpha, side, pitch, false, partial_scratch, st));
+    return split_rows_bf16(x, rows, R, pitch, 3, pieces, st);
+  }
+  NB_CUDA(launch_dependent(binary_affine_operands_kernel, dim3((unsigned)(w_blocks + x_blocks)), dim3(256), 0, st, w, R, C,
+                           zero_to, wb, side, pitch, alpha ? partial_scratch : nullptr, gx, (int)w_blocks, x, rows,
+                           static_cast<__nv_bfloat16 *>(pieces)));
+  if (alpha)
+    NB_CUDA(launch_dependent(finalize_alpha_kernel, dim3((C + 255) / 256), dim3(256), 0, st, partial_scratch, gy, C,
+                             (float)1 / R, alpha)); // binary_weight_affine.cpp:68
   return NB200_OK;
 }
 
