@@ -110,6 +110,10 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
     """
     if not quantize:
         return x
+    if outputs is None:
+        y = L.min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay, x_min_max, ema, eps)
+        if y is not None:
+            return y
     x = L.f32(x)
     qs = (L.f32(qr_min, "qr_min"), L.f32(qr_max, "qr_max"), L.f32(ql_min, "ql_min"), L.f32(ql_max, "ql_max"))
     # Shape rules of MinMaxQuantize::setup_impl (min_max_quantize.cpp:54-83).
@@ -173,6 +177,10 @@ def min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max=F
     Call after min_max_quantize: qr_min / qr_max are the ranges the forward
     left in place. Returns (dx, g_qr_min, g_qr_max); the range gradients are
     produced only when neither x_min_max nor ema is set."""
+    fast = L.min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max, ema, ste_fine_grained,
+                                       propagate_down, accum, grads)
+    if fast is not None:
+        return fast
     x, dy, dx = _grad_buffers(x, dy, grads[0], accum[0])
     qs = (L.f32(qr_min, "qr_min"), L.f32(qr_max, "qr_max"), L.f32(ql_min, "ql_min"), L.f32(ql_max, "ql_max"))
     if any(t.shape != qs[0].shape for t in qs) or qs[0].dim() != x.dim():

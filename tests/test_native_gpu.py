@@ -53,7 +53,24 @@ CALLS = {
                                                  propagate_down=(True, False, True)),
         lambda t: F.batch_normalization_backward(t["dy"], t["dy"], t["s"], t["b"], t["s"], accum=(False, True, False)),
     ],
+    "min_max_quantize": [
+        lambda t: F.min_max_quantize(t["x"], *ranges(t, 32), x_min_max=True, ema=True),
+        lambda t: F.min_max_quantize(t["x"], *ranges(t, 1)),
+        lambda t: F.min_max_quantize(t["x"], *ranges(t, 16)),
+    ],
+    "min_max_quantize_backward": [
+        lambda t: F.min_max_quantize_backward(t["x"], *ranges(t, 32), t["x"] * 2, x_min_max=True),
+        lambda t: F.min_max_quantize_backward(t["x"], *ranges(t, 1), t["x"] * 2, accum=(True, False, False),
+                                              grads=(torch.ones_like(t["x"]), None, None)),
+        lambda t: F.min_max_quantize_backward(t["x"], *ranges(t, 1), t["x"] * 2, propagate_down=(False, True, False),
+                                              grads=(torch.ones_like(t["x"]), None, None)),
+        lambda t: F.min_max_quantize_backward(t["x"], *ranges(t, 1), t["dy"]),
+    ],
 }
+
+
+def ranges(t, n):
+    return [torch.full((1, n, 1, 1), v, device="cuda") for v in (-1.0, 1.5, 0.0, 255.0)]
 
 
 @pytest.mark.parametrize("name,k", [(n, k) for n, calls in CALLS.items() for k in range(len(calls))])
