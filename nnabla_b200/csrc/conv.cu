@@ -499,29 +499,6 @@ bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t
   p.o_blocks = (g.Kog + 63) / 64;
   p.c_blocks = (g.Cg + 63) / 64;
   p.x_planes = x_planes;
-  int n = 0, groups = 0;
-  p.tg_tap[0] = p.tg_pair[0] = 0;
-  for (int ry = 0; ry < g.sh; ++ry)
-    for (int rx = 0; rx < g.sw; ++rx) {
-      int in_group = 0;
-      for (int ky = 0; ky < g.kh; ++ky)
-        for (int kx = 0; kx < g.kw; ++kx) {
-          if (residue(ky, g.dh, g.ph, g.sh) != ry || residue(kx, g.dw, g.pw, g.sw) != rx)
-            continue;
-          if (in_group == 0 || in_group == kWgradTaps) {
-            p.tg_ry[groups] = ry;
-            p.tg_rx[groups] = rx;
-            ++groups;
-            in_group = 0;
-          }
-          p.tap_row[n] = (offset(ky, g.dh, g.ph, g.sh) - p.y0) * p.wp + offset(kx, g.dw, g.pw, g.sw) - p.x0;
-          p.tap_id[n++] = ky * g.kw + kx;
-          ++in_group;
-          p.tg_tap[groups] = n;
-          p.tg_pair[groups] = p.tg_pair[groups - 1] + (in_group + 1) / 2;
-        }
-    }
-  p.tap_groups = groups;
   // Box height: as few accumulation steps per image as possible, where a box costs about one step beside its own. Three
   // boxes must fit in shared memory when a box has one plane of x (its MMAs take about as long as its copies: with two
   // boxes the MMAs waited), two when it has three.
@@ -551,7 +528,35 @@ bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t
   smem = 1024 + p.stages * stage;
   p.flush = 96 / p.k16;
   p.tiles_h = (g.Ho + p.h_box - 1) / p.h_box;
-  const int64_t boxes = (int64_t)g.N * p.tiles_h, group_work = boxes * p.tg_pair[groups];
+  const int64_t boxes = (int64_t)g.N * p.tiles_h;
+  // Six taps per task read every box less often (the copies' L2 reads bound four: 105 us for 64 -> 64 maps on
+  // [128, 64, 56, 56], six 82); four keep the slots smaller, which shows below some 30 us (in units of 100 cycles per SM).
+  const double steps = (double)boxes * p.k16 * ((taps + 1) / 2) * p.groups * p.o_blocks * p.c_blocks / sm_count();
+  p.task_taps = steps * (x_planes == 3 ? 2.2 : 1.0) >= 500.0 ? kWgradTaps : 4;
+  int n = 0, groups = 0;
+  p.tg_tap[0] = p.tg_pair[0] = 0;
+  for (int ry = 0; ry < g.sh; ++ry)
+    for (int rx = 0; rx < g.sw; ++rx) {
+      int in_group = 0;
+      for (int ky = 0; ky < g.kh; ++ky)
+        for (int kx = 0; kx < g.kw; ++kx) {
+          if (residue(ky, g.dh, g.ph, g.sh) != ry || residue(kx, g.dw, g.pw, g.sw) != rx)
+            continue;
+          if (in_group == 0 || in_group == p.task_taps) {
+            p.tg_ry[groups] = ry;
+            p.tg_rx[groups] = rx;
+            ++groups;
+            in_group = 0;
+          }
+          p.tap_row[n] = (offset(ky, g.dh, g.ph, g.sh) - p.y0) * p.wp + offset(kx, g.dw, g.pw, g.sw) - p.x0;
+          p.tap_id[n++] = ky * g.kw + kx;
+          ++in_group;
+          p.tg_tap[groups] = n;
+          p.tg_pair[groups] = p.tg_pair[groups - 1] + (in_group + 1) / 2;
+        }
+    }
+  p.tap_groups = groups;
+  const int64_t group_work = boxes * p.tg_pair[groups];
   const int64_t work = group_work * p.groups * p.o_blocks * p.c_blocks;
   if (work >= (1ll << 30))
     return false;
@@ -597,7 +602,7 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   const size_t x_bytes = *did_dw ? round_up((size_t)x_planes * g.N * g.H * g.W * c_tot * 2, 1024) : 0;
   const size_t side_bytes = *did_dx ? round_up((size_t)g.C * taps * p.k_slots * 2, 1024) : 0;
   const int grid_w = *did_dw ? (q.work + q.per_block - 1) / q.per_block : 0;
-  const size_t slot_bytes = *did_dw ? (size_t)(grid_w + q.tasks()) * kWgradSlotFloats * 4 : 0;
+  const size_t slot_bytes = *did_dw ? (size_t)(grid_w + q.tasks()) * q.slot_floats() * 4 : 0;
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc((two ? 2 : 1) * dy_bytes + x_bytes + side_bytes + slot_bytes));
   uint8_t *at = static_cast<uint8_t *>(scratch.p);
@@ -655,7 +660,7 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   NB_TRY(device_status_word(&status));
   NB_CUDA(launch_dependent(kernel, dim3(grid_w), dim3(kGemmThreads), smem_w, st, mx, md, q, status));
   NB_LAUNCH_CHECK();
-  NB_CUDA(launch_dependent(conv_wgrad_finish_kernel, dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), dim3(256), 0, st, q,
+  NB_CUDA(launch_dependent(conv_wgrad_finish_kernel, dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), dim3(64 * q.task_taps), 0, st, q,
                            g.Kog, g.Cg, taps, dw, accum_dw));
   NB_LAUNCH_CHECK();
   return NB200_OK;

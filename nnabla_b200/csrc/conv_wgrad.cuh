@@ -15,14 +15,16 @@
 // Pixels run over the box's padded width; dy's box is as wide as x's with zeros (the copy engine's fill) where an
 // output row has ended, and its rows up to a multiple of 16 are zeroed once.
 //
-// A task is (group, 64 maps, 64 channels, up to four taps that share a box). The tasks' boxes, weighted with their MMAs,
+// A task is (group, 64 maps, 64 channels, up to six taps that share a box; the third pair of taps has 128 columns left in
+// tensor memory: column 0 to 63 as above, all other products in the rest). The tasks' boxes, weighted with their MMAs,
 // are dealt out evenly to one block per SM; a block that ends a task or its share leaves its partial sums in a slot of
 // its own and a second kernel adds the slots in order (deterministic). Every 96 accumulation steps the tensor memory
 // is emptied into fp32 registers (gemm.cuh: the tensor core's additions truncate).
 //
-// What bounds it: 100 cycles per MMA of 192 columns and 16 pixels, and the shared-memory traffic beside it (80 % for the
-// operands, the rest for the copies). The previous form made the batch the K axis of an implicit GEMM (two transposing
-// passes, K padded to 64 images per pixel): 216 us and 165 us of passes for 64 -> 64 maps on [128, 64, 56, 56], and
+// What bounds it: 100 cycles per MMA of 192 columns and 16 pixels, the shared-memory traffic beside it (80 % for the
+// operands, the rest for the copies), and beside both the L2: every task of up to six taps reads the boxes again. The
+// previous form made the batch the K axis of an implicit GEMM (two transposing passes, K padded to 64 images per pixel):
+// 216 us and 165 us of passes for 64 -> 64 maps on [128, 64, 56, 56], now 82 and a share of the preparation's 88, and
 // 3 x the work at 20 images.
 #pragma once
 #include "gemm.cuh"
@@ -30,8 +32,7 @@
 namespace nb200 {
 
 constexpr int kWgradMaxTaps = 64;
-constexpr int kWgradTaps = 4;                          // per task
-constexpr int kWgradSlotFloats = kWgradTaps * 64 * 64; // one slot of partial sums: [tap][channel][map]
+constexpr int kWgradTaps = 6;                          // per task at most: three pairs
 
 struct ConvWgradProblem {
   int tiles_h, boxes;               // boxes per image, in all
@@ -46,13 +47,16 @@ struct ConvWgradProblem {
   int stages, flush;                // ring depth; boxes per accumulation in tensor memory
   int work, per_block;              // all boxes times their tasks' MMAs (x_planes == 1 counts), and a block's share
   int group_work;                   // work of one (group, o block, c block): boxes * pairs of all tap groups
-  int tg_tap[kWgradMaxTaps + 1];    // taps of tap group k: [tg_tap[k], tg_tap[k + 1]), at most four, by ascending shift
+  int task_taps;                    // taps per task at most: 4 or kWgradTaps
+  int tg_tap[kWgradMaxTaps + 1];    // taps of tap group k: [tg_tap[k], tg_tap[k + 1]), at most six, by ascending shift
   int tg_pair[kWgradMaxTaps + 1];   // pairs of taps before tap group k
   int tg_ry[kWgradMaxTaps], tg_rx[kWgradMaxTaps]; // residues of a tap group's x rows and columns
   int tap_row[kWgradMaxTaps];       // shift of a tap, in rows of the box
   int tap_id[kWgradMaxTaps];        // its index in the filter
   float *slots;
 
+  // one slot of partial sums: [tap][channel][map]
+  __host__ __device__ __forceinline__ int slot_floats() const { return task_taps * 64 * 64; }
   __host__ __device__ __forceinline__ int tasks() const { return groups * o_blocks * c_blocks * tap_groups; }
   // first unit of work of a task, and its pairs
   __host__ __device__ __forceinline__ int task_begin(int task, int &pairs) const {
@@ -200,9 +204,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint32_t smem16 = ptx::smem_u32(smem) >> 4;
       walk([&](int task, int pairs, int b0, int b1) {
         const int tg = task % prob.tap_groups, t0 = prob.tg_tap[tg], t1 = prob.tg_tap[tg + 1];
-        uint32_t a_off[2];
+        uint32_t a_off[3];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < 3; ++q) {
           const int ta = t0 + 2 * q < t1 ? t0 + 2 * q : t0, tb = ta + 1 < t1 ? ta + 1 : ta;
           a_off[q] = (uint32_t)prob.tap_row[ta] * 8u + ((uint32_t)(prob.tap_row[tb] - prob.tap_row[ta]) * 8u << 16);
         }
@@ -226,6 +230,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             auto step = [&](int k, int q) { // 16 pixels of one pair of taps
               const uint32_t d = tmem_base + (uint32_t)q * 192u;
               const uint64_t bd = ((uint64_t)hi << 32) | (b_lo + b_lbo + (uint32_t)k * 128u);
+              if (q == 2) {
+                // the third pair has 128 columns: the product of the first pieces, and all the others together
+                const uint64_t plane = (uint32_t)prob.dy_bytes >> 4;
+                auto ad = [&](int p) {
+                  return ((uint64_t)hi << 32) | (a_lo + ((uint32_t)(p * prob.x_bytes) >> 4) + a_off[2] + (uint32_t)k * 128u);
+                };
+                ptx::mma_bf16(d, ad(0), bd, idesc1, accumulate);
+                ptx::mma_bf16(d + 64u, ad(0), bd + 2 * plane, idesc2, 1u);
+                if constexpr (kPx == 3) {
+                  ptx::mma_bf16(d + 64u, ad(1), bd, idesc2, 1u);
+                  ptx::mma_bf16(d + 64u, ad(1), bd + plane, idesc2, 1u);
+                  ptx::mma_bf16(d + 64u, ad(2), bd, idesc2, 1u);
+                }
+                return;
+              }
 #pragma unroll
               for (int p = 0; p < kPx; ++p) {
                 const uint64_t ad =
@@ -235,33 +254,29 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                               p == 0 ? accumulate : 1u);
               }
             };
-            if (pairs == 2) {
+            auto steps = [&](auto count) { // all pairs of the task, four steps of straight code at a time
               int k = 0;
               for (; k + 4 <= prob.k16; k += 4)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                  step(k + u, 0);
-                  step(k + u, 1);
-                  accumulate = 1;
-                }
-              for (; k < prob.k16; ++k) {
-                step(k, 0);
-                step(k, 1);
-                accumulate = 1;
-              }
-            } else {
-              int k = 0;
-              for (; k + 4 <= prob.k16; k += 4)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  step(k + u, 0);
+                  for (int q = 0; q < decltype(count)::value; ++q)
+                    step(k + u, q);
                   accumulate = 1;
                 }
               for (; k < prob.k16; ++k) {
-                step(k, 0);
+#pragma unroll
+                for (int q = 0; q < decltype(count)::value; ++q)
+                  step(k, q);
                 accumulate = 1;
               }
-            }
+            };
+            if (pairs == 3)
+              steps(std::integral_constant<int, 3>{});
+            else if (pairs == 2)
+              steps(std::integral_constant<int, 2>{});
+            else
+              steps(std::integral_constant<int, 1>{});
             ptx::mma_commit(empty + st);
             if (++st == prob.stages) {
               st = 0;
@@ -279,9 +294,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + 32u * set;
     int chunk = 0;
     walk([&](int task, int pairs, int b0, int b1) {
-      float acc[2][32];
+      float acc[3][32];
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < 3; ++q)
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           acc[q][j] = 0.0f;
@@ -294,17 +309,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         ptx::tc_fence_after_sync();
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < 3; ++q)
           if (q < pairs) {
-            uint32_t r0[32], r1[32], r2[32];
-            ptx::tmem_ld_32x32(lane_base + 192u * q, r0);
+            uint32_t r0[32], r1[32];
+            float low[32]; // the products of the smaller pieces
             ptx::tmem_ld_32x32(lane_base + 192u * q + 64u, r1);
-            ptx::tmem_ld_32x32(lane_base + 192u * q + 128u, r2);
+            if (q < 2)
+              ptx::tmem_ld_32x32(lane_base + 192u * q + 128u, r0);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              acc[q][j] = __fadd_rn(acc[q][j], __fadd_rn(__uint_as_float(r0[j]),
-                                                         __fadd_rn(__uint_as_float(r1[j]), __uint_as_float(r2[j]))));
+              low[j] = q < 2 ? __fadd_rn(__uint_as_float(r1[j]), __uint_as_float(r0[j])) : __uint_as_float(r1[j]);
+            ptx::tmem_ld_32x32(lane_base + 192u * q, r0);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              acc[q][j] = __fadd_rn(acc[q][j], __fadd_rn(__uint_as_float(r0[j]), low[j]));
           }
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -312,9 +332,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           ptx::mbar_arrive(&tmem_empty);
       }
       // slot of this (block, task): [tap][channel][map]
-      float *slot = prob.slots + (int64_t)((int)blockIdx.x + task) * kWgradSlotFloats;
+      float *slot = prob.slots + (int64_t)((int)blockIdx.x + task) * prob.slot_floats();
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < 3; ++q)
         if (q < pairs) {
           float4 *dst = reinterpret_cast<float4 *>(slot + (2 * q * 64 + quarter * 32 + lane) * 64 + 32 * set);
 #pragma unroll
@@ -342,7 +362,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
 // dW[o][c][tap] (+)= the slots of a task in block order; one thread block per (task, channel), the maps of a slot are
 // contiguous. Only the first and the last slot can be missing (per_block >= 2 pairs).
-__global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const __grid_constant__ ConvWgradProblem prob, int Kog,
+__global__ void __launch_bounds__(64 * kWgradTaps) conv_wgrad_finish_kernel(const __grid_constant__ ConvWgradProblem prob, int Kog,
                                                                 int Cg, int taps, float *__restrict__ dw,
                                                                 int accumulate) {
   pdl_wait();
@@ -364,19 +384,19 @@ __global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const __grid_con
   first += b0 < b1 ? 0 : 1;
   prob.share(last, begin, pairs, b0, b1);
   last -= b0 < b1 ? 0 : 1;
-  const float *src = prob.slots + (int64_t)(first + task) * kWgradSlotFloats + (t * 64 + blockIdx.y) * 64 + (threadIdx.x & 63);
+  const float *src = prob.slots + (int64_t)(first + task) * prob.slot_floats() + (t * 64 + blockIdx.y) * 64 + (threadIdx.x & 63);
   float s = 0.0f;
   int b = first;
-  for (; b + 8 <= last + 1; b += 8, src += (int64_t)8 * kWgradSlotFloats) {
+  for (; b + 8 <= last + 1; b += 8, src += (int64_t)8 * prob.slot_floats()) {
     float v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      v[u] = __ldcs(src + (int64_t)u * kWgradSlotFloats);
+      v[u] = __ldcs(src + (int64_t)u * prob.slot_floats());
 #pragma unroll
     for (int u = 0; u < 8; ++u)
       s = __fadd_rn(s, v[u]);
   }
-  for (; b <= last; ++b, src += kWgradSlotFloats)
+  for (; b <= last; ++b, src += prob.slot_floats())
     s = __fadd_rn(s, __ldcs(src));
   float *dst = dw + ((int64_t)(g * Kog + o) * Cg + c) * taps + prob.tap_id[t0 + t];
   *dst = accumulate ? __fadd_rn(*dst, s) : s;
