@@ -221,7 +221,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     ptx::tmem_relinquish();
   }
   pdl_wait();
-  pdl_trigger();
+  // (codes and channel-last results are read by convolutions)
+  if (!ep.y_nchw || early_trigger((int64_t)prob.Nimg * prob.Ko * prob.Ho * prob.Wo))
+    pdl_trigger();
   for (int c = threadIdx.x; c < prob.n_tiles * BN; c += kGemmThreads)
     sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
                                       ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)

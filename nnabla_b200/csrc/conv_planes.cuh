@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
   pdl_wait();
-  pdl_trigger();
+  if (early_trigger((int64_t)prob.Nimg * prob.total_maps * prob.H * prob.W))
+    pdl_trigger();
 
   struct TileAt {
     int n0, cls, group, row0, img;

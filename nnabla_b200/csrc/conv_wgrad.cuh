@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
   pdl_wait();
-  pdl_trigger();
+  if (prob.task_taps < kWgradTaps) // small problems (early_trigger's reason)
+    pdl_trigger();
   auto gave_up = [&](int code) {
     if (*abort_flag == 0)
       atomicCAS(status, 0, code);

@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
-  pdl_trigger();
+  if (num_tiles <= (int)gridDim.x) // one round of tiles (early_trigger's reason)
+    pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer

@@ -168,8 +168,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   ptx::cluster_sync(); // the peer's barriers are initialised before anything is signalled remotely
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
-  pdl_trigger();
+  pdl_wait(); // (large results only: no early trigger)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)

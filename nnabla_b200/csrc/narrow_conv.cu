@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
     ptx::tmem_relinquish();
   }
   pdl_wait();
-  pdl_trigger();
+  if (early_trigger((int64_t)g.N * g.Ko * g.Ho * g.Wo))
+    pdl_trigger();
   // bias of every map (0 past Ko or without bias), times 2 / delta (ReLU: over 256) when codes are written
   __shared__ __align__(16) float bias_s[kN];
   if (threadIdx.x < kN)

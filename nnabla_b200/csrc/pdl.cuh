@@ -8,17 +8,25 @@
 // global-memory access: as its first statement, or in the tensor-core kernels after the barriers and the tensor
 // memory are set up, which touches nothing outside the SM (so its completion implies the predecessor's, and
 // ordering stays transitive along the stream); (2) pdl_trigger() only says "my
-// successor may be scheduled", it orders nothing. Kernels launched the ordinary way in between serialize
+// successor may be scheduled", it orders nothing. A kernel with a large share of the SM's shared memory triggers early
+// only while its result is small (early_trigger): the successor's blocks become resident beside it, the SM then never
+// drains, and streaming kernels go on with the little L1 that such a split leaves (their loads in flight live there):
+// max-pooling behind the stem 280 us instead of 180, a batch-256 network 5.0 ms instead of 4.5. Kernels launched the ordinary way in between serialize
 // fully, as before. NNABLA_B200_PDL=0 turns the attribute off (ordinary launches; the waits are no-ops).
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstdlib>
 
 namespace nb200 {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Whether a large-shared-memory kernel with this many result values should let its successor in before it ends: up to
+// 16 MB, where the next launch's start is a tenth of the kernel.
+__device__ __forceinline__ bool early_trigger(int64_t values) { return values <= (4 << 20); }
 
 inline bool pdl_enabled() {
   static const bool on = []() {
