@@ -21,7 +21,7 @@ def _output_like(x, outputs):
     if outputs is None:
         return L.empty(x, x)
     y = outputs[0] if isinstance(outputs, (list, tuple)) else outputs
-    _sideband.pop(id(y), None)  # about to be overwritten
+    _wrote(y)
     if y.shape != x.shape or y.dtype != x.dtype or y.device != x.device or not y.is_contiguous():
         raise RuntimeError("outputs[0] must be a contiguous tensor of x's shape, dtype and device")
     return y
@@ -37,16 +37,41 @@ _sideband = {}
 SIDEBAND_MIN_VALUES = 1 << 23
 
 
+def _memory(t):
+    return t.untyped_storage().data_ptr()
+
+
 def _sideband_put(y, codes, delta):
     key = id(y)
-    _sideband[key] = (weakref.ref(y, lambda _r, key=key: _sideband.pop(key, None)), y._version, codes, float(delta))
+    _sideband[key] = (weakref.ref(y, lambda _r, key=key: _sideband.pop(key, None)), y._version, codes, float(delta),
+                      _memory(y))
 
 
 def _sideband_get(x, delta):
     e = _sideband.get(id(x))
-    if e is None or e[0]() is not x or x._version != e[1] or e[3] != float(delta):
+    if e is None or e[0]() is not x or x._version != e[1] or e[3] != float(delta) or e[4] != _memory(x):
         return None
     return e[2]
+
+
+def _wrote(*tensors):
+    """Every function that writes into a tensor of its caller says so here: the kernels do not move torch's version
+    counter, and the codes kept with that tensor, or with another one in the same memory, no longer hold."""
+    if not _sideband:
+        return
+    for t in tensors:
+        if isinstance(t, torch.Tensor):
+            m = _memory(t)
+            for key in [k for k, e in list(_sideband.items()) if e[4] == m]:
+                _sideband.pop(key, None)
+
+
+def _result(shape, like, outputs):
+    """The output of a function whose result is not shaped like an input: a new tensor, or the caller's."""
+    if outputs is None:
+        return L.empty(shape, like)
+    _wrote(outputs[0])
+    return outputs[0]
 
 
 def fixed_point_quantize(x, sign=True, n=8, delta=2 ** -4, quantize=True, ste_fine_grained=True, outputs=None,
@@ -58,8 +83,9 @@ def fixed_point_quantize(x, sign=True, n=8, delta=2 ** -4, quantize=True, ste_fi
     n - sign <= 7; otherwise the plain quantizer runs): the same pass also
     writes the result's int8 channel-last codes and keeps them with the returned tensor; a binary-weight
     convolution called on that tensor with fixed_point_delta=delta then reads the codes. The result is the
-    same, bit for bit. The codes are dropped when the tensor is modified through torch or passed as `outputs`
-    of a function of this module; do not write into it any other way.
+    same, bit for bit. The codes are dropped when the tensor is modified through torch, or when a function of this
+    module writes into its memory (outputs=, inplace=, a gradient buffer); do not write into it any other way, such as
+    through .data, which torch does not count.
     """
     if not quantize:
         return x
@@ -110,6 +136,7 @@ def min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay=0.999, x_min_max=F
     """
     if not quantize:
         return x
+    _wrote(qr_min, qr_max)
     if outputs is None:
         y = L.min_max_quantize(x, qr_min, qr_max, ql_min, ql_max, decay, x_min_max, ema, eps)
         if y is not None:
@@ -150,6 +177,8 @@ def _grad_buffers(x, dy, dx, accum):
         dx = L.empty(x, x)
     elif dx.shape != x.shape or dx.dtype != torch.float32 or dx.device != x.device or not dx.is_contiguous():
         raise RuntimeError("dx must be a contiguous float32 tensor of x's shape and device")
+    else:
+        _wrote(dx)
     return x, dy, dx
 
 
@@ -177,6 +206,7 @@ def min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max=F
     Call after min_max_quantize: qr_min / qr_max are the ranges the forward
     left in place. Returns (dx, g_qr_min, g_qr_max); the range gradients are
     produced only when neither x_min_max nor ema is set."""
+    _wrote(*grads)
     fast = L.min_max_quantize_backward(x, qr_min, qr_max, ql_min, ql_max, dy, x_min_max, ema, ste_fine_grained,
                                        propagate_down, accum, grads)
     if fast is not None:
@@ -261,7 +291,8 @@ def binary_weight_affine(x, weight, binary_weight, alpha, bias=None, base_axis=1
     _same_shape(weight, binary_weight, "float vs binary")
     if alpha.numel() != w_col:
         raise RuntimeError("Size of alpha must be equal to output size.")
-    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    _wrote(binary_weight, alpha)
+    y = _result(out_shape, x, outputs)
     L.nb200_binary_weight_affine_f32(x, weight, binary_weight, alpha, bias, y, rows, w_row, w_col, quantize_zero_to)
     return y
 
@@ -277,7 +308,8 @@ def binary_connect_affine(x, weight, binary_weight, bias=None, base_axis=1, quan
     bias = L.f32(bias, "bias") if bias is not None else None
     rows, w_row, w_col, out_shape = _affine_dims(x, weight, base_axis, bias)
     _same_shape(weight, binary_weight, "float vs binary")
-    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    _wrote(binary_weight)
+    y = _result(out_shape, x, outputs)
     L.nb200_binary_connect_affine_f32(x, weight, binary_weight, bias, y, rows, w_row, w_col, quantize_zero_to)
     return y
 
@@ -292,7 +324,7 @@ def affine(x, weight, bias=None, base_axis=1, n_outputs=-1, outputs=None, fixed_
     x, weight = L.f32(x), L.f32(weight, "weight")
     bias = L.f32(bias, "bias") if bias is not None else None
     rows, w_row, w_col, out_shape = _affine_dims(x, weight, base_axis, bias)
-    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    y = _result(out_shape, x, outputs)
     if fixed_point is not None:
         dx, dw = fixed_point
         L.nb200_affine_fxp8_f32(x, weight, dx, dw, bias, y, rows, w_row, w_col)
@@ -316,6 +348,7 @@ def affine_from_codes(x_codes, w_codes, delta_x, delta_w, bias=None):
 def _affine_backward(entry, x, w, alpha, dy, base_axis, propagate_down, accum, grads):
     """Shared driver of the affine backward entry points. Returns (dx, dw, db);
     an entry whose propagate_down flag is false is returned as passed in."""
+    _wrote(*grads)
     x, w, dy = L.f32(x), L.f32(w, "weight"), L.f32(dy, "dy")
     rows, w_row, w_col, out_shape = _affine_dims(x, w, base_axis, None)
     if tuple(dy.shape) != tuple(out_shape):
@@ -387,7 +420,8 @@ def affine_from_kmajor_codes(x_codes, w_codes_kmajor, w_row, delta_x, delta_w, b
 
 
 def _rank_pointers(y_ranks):
-    """ctypes array of the per-rank output matrices' device addresses (tensors or plain integers)."""
+    """ctypes array of the per-rank output matrices' device addresses (tensors or plain integers), to be written."""
+    _wrote(*y_ranks)
     addrs = [int(y.data_ptr()) if hasattr(y, "data_ptr") else int(y) for y in y_ranks]
     return (ctypes.c_void_p * len(addrs))(*addrs)
 
@@ -484,6 +518,7 @@ def _conv_geometry(x, w, bias, base_axis, pad, stride, dilation, group):
 
 def _binary_convolution(entry, x, weight, binary_weight, alpha, bias, base_axis, pad, stride, dilation, group,
                         quantize_zero_to, outputs, fixed_point_delta):
+    _wrote(binary_weight, alpha)
     if fixed_point_delta is not None and group == 1 and base_axis == 1 and x.dim() == 4:
         codes = _sideband_get(x, fixed_point_delta)
         if codes is not None:  # the quantizer that made x left its channel-last codes
@@ -501,7 +536,7 @@ def _binary_convolution(entry, x, weight, binary_weight, alpha, bias, base_axis,
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, weight, bias, base_axis, pad, stride, dilation, group)
     _same_shape(weight, binary_weight, "float vs binary")
-    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    y = _result(out_shape, x, outputs)
     scaled = (alpha,) if alpha is not None else ()
     getattr(L, entry)(x, weight, binary_weight, *scaled, bias, y, batch, Cin, H, W, Ko, kh, kw, *pad, *stride, *dilation,
                       group, quantize_zero_to, fixed_point_delta or 0.0)
@@ -540,6 +575,7 @@ def binary_connect_convolution(x, weight, binary_weight, bias=None, base_axis=1,
 
 def _binary_convolution_backward(entry, x, binary_weight, alpha, dy, base_axis, pad, stride, dilation, group,
                                  propagate_down, accum, grads, fixed_point_delta):
+    _wrote(*grads)
     if base_axis == 1:
         out = L.binary_convolution_backward(x, binary_weight, alpha, dy, pad, stride, dilation, group, propagate_down,
                                             accum, grads, fixed_point_delta)
@@ -599,6 +635,7 @@ def convolution_backward(x, weight_shape, dy, base_axis=1, pad=None, stride=None
     """Gradients of the full-precision convolution
     (Convolution::backward_impl, src/nbla/function/generic/convolution.cpp:199-300).
     Returns (dx, dw, db), None where propagate_down is False; dx needs `weight`."""
+    _wrote(*grads)
     x, dy = L.f32(x), L.f32(dy, "dy")
     if weight is not None:
         weight_shape = tuple(L.f32(weight, "weight").shape)
@@ -645,7 +682,7 @@ def convolution(x, weight, bias=None, base_axis=1, pad=None, stride=None, dilati
     bias = L.f32(bias, "bias") if bias is not None else None
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x, weight, bias, base_axis, pad, stride, dilation, group)
-    y = L.empty(out_shape, x) if outputs is None else outputs[0]
+    y = _result(out_shape, x, outputs)
     if fixed_point is not None:
         L.nb200_convolution_fxp8_f32(x, weight, fixed_point[0], fixed_point[1], bias, y, batch, Cin, H, W, Ko, kh, kw,
                                      pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1], group)
@@ -662,6 +699,8 @@ def batch_normalization(x, beta, gamma, mean, variance, axes=[1], decay_rate=0.9
     (src/nbla/function/generic/batch_normalization.cpp:228-260). batch_stat=True: forward_impl_batch
     (:157-226): normalises with the statistics of x and updates `mean` / `variance` (the running
     statistics) in place; output_stat=True also returns the batch mean and variance."""
+    if batch_stat:
+        _wrote(mean, variance)
     fast = L.batch_normalization(x, beta, gamma, mean, variance, axes, decay_rate, eps, batch_stat, output_stat)
     if fast is not None:
         return fast
@@ -703,6 +742,8 @@ def relu(x, inplace=False, n_outputs=-1, outputs=None):
     """ReLU (function_bases.relu; src/nbla/function/generic/relu.cpp)."""
     x = L.f32(x)
     y = x if inplace else _output_like(x, outputs)
+    if inplace:
+        _wrote(y)
     L.nb200_relu_f32(x, y, x.numel())
     return y
 
@@ -714,6 +755,8 @@ def add2(x0, x1, inplace=False, n_outputs=-1, outputs=None):
         raise C.NB200Error(4, "broadcasting add2 is not implemented: shapes %s and %s" % (tuple(x0.shape),
                                                                                          tuple(x1.shape)))
     y = x0 if inplace else _output_like(x0, outputs)
+    if inplace:
+        _wrote(y)
     L.nb200_add2_f32(x0, x1, y, x0.numel())
     return y
 
@@ -779,6 +822,7 @@ def inq_update_weights(weight, indicators, state, num_bits=4, inq_iterations=(),
     weight = L.f32(weight, "weight")
     if indicators.dtype != torch.int32 or indicators.shape != weight.shape or not indicators.is_contiguous():
         raise RuntimeError("Indicators and weights must have same size (indicators as contiguous int32).")
+    _wrote(weight)
     n = weight.numel()
     its = [int(v) for v in inq_iterations]
     L.nb200_inq_restore_f32(weight, state.old_weights, state.old_indicators, n)
@@ -830,6 +874,7 @@ def _grad_out(like, accum, dx):
         if accum:
             raise RuntimeError("accum needs the gradient buffer to add to")
         return L.empty(like, like)
+    _wrote(dx)
     return L.f32(dx, "dx")
 
 
@@ -839,6 +884,7 @@ def batch_normalization_backward(x, dy, gamma, mean, variance, axes=[1], eps=1e-
     """BatchNormalization::backward_impl (batch_normalization.cpp:262-486). mean / variance: the batch
     statistics the forward pass returned (batch_stat) or the running ones. Returns (dx, dbeta, dgamma),
     None where propagate_down is False."""
+    _wrote(*grads)
     fast = L.batch_normalization_backward(x, dy, gamma, mean, variance, axes, eps, batch_stat, dmean, dvar, propagate_down,
                                           accum, grads)
     if fast is not None:
@@ -1072,6 +1118,7 @@ def binary_weight_convolution_from_codes(x_codes, x_shape, weight, binary_weight
     """binary_weight_convolution (binary_connect_convolution when alpha is
     None) on activations given as int8 channel-last codes of a tensor of shape
     x_shape = (batch, channels, height, width) with step activation_delta."""
+    _wrote(binary_weight, alpha)
     weight = L.f32(weight, "weight")
     binary_weight = L.f32(binary_weight, "binary_weight")
     bias = L.f32(bias, "bias") if bias is not None else None
@@ -1086,7 +1133,7 @@ def binary_weight_convolution_from_codes(x_codes, x_shape, weight, binary_weight
         alpha = L.f32(alpha, "alpha")
         if alpha.numel() != Ko:
             raise RuntimeError("Size of alpha must be equal to the number of output maps.")
-    y = L.empty(out_shape, weight) if outputs is None else outputs[0]
+    y = _result(out_shape, weight, outputs)
     L.nb200_binary_convolution_codes_f32(x_codes, weight, binary_weight, alpha, bias, y, batch, Cin, H, W, Ko, kh, kw,
                                          pad[0], pad[1], stride[0], stride[1], dilation[0], dilation[1], group,
                                          quantize_zero_to, activation_delta)
@@ -1134,7 +1181,7 @@ def binary_convolution_from_codes_prepared(x_codes, x_shape, prepared, bias=None
     batch, Cin, H, W, Ko, kh, kw, pad, stride, dilation, out_shape = _conv_geometry(
         x_shape, prepared.shape, bias, 1, pad, stride, dilation, prepared.group)
     x_codes = _check_codes(x_codes, batch, H * W, Cin, prepared.group, "x_codes")
-    y = L.empty(out_shape, x_codes) if outputs is None else outputs[0]
+    y = _result(out_shape, x_codes, outputs)
     L.nb200_binary_convolution_codes_prepared_f32(x_codes, prepared.side, prepared.alpha, bias, y, batch, Cin, H, W, Ko,
                                                   kh, kw, pad[0], pad[1], stride[0], stride[1], dilation[0],
                                                   dilation[1], prepared.group, activation_delta)
@@ -1282,6 +1329,7 @@ def quantize_linear(x, scale, zero_point, round_mode="HALF_AWAY_FROM_ZERO", narr
         raise RuntimeError("round_mode must be HALF_AWAY_FROM_ZERO or HALF_TO_EVEN")
     if dtype not in _QL_DTYPES:
         raise C.NB200Error(4, "dtype must be int8 (BYTE) or uint8 (UBYTE)")
+    _wrote(zero_point)
     y = _output_like(x, outputs)
     L.nb200_quantize_linear_f32(x, x.shape, x.dim(), scale, scale.shape, zero_point, zero_point.shape, y,
                                 _ROUND_MODES[round_mode], bool(narrow_range), _QL_DTYPES[dtype])

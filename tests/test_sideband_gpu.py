@@ -86,6 +86,60 @@ def test_convolution_reads_the_codes_and_stale_codes_are_dropped(F, small_thresh
     F.check_device_status()
 
 
+WRITERS = ["relu inplace", "add2 inplace", "relu outputs", "relu outputs, a view", "relu outputs, detached",
+           "quantizer outputs", "binary connect convolution outputs", "prepared convolution outputs", "relu gradient",
+           "quantizer gradient", "min-max gradient", "convolution gradient", "batch normalization gradient",
+           "another tensor's memory"]
+
+
+def _into(F, q):
+    """Calls that write into q, or into the memory of q, which holds multiples of the step before and after."""
+    one = torch.ones_like(q)
+    eye = torch.zeros(32, 32, 1, 1, device="cuda")
+    eye.view(32, 32).fill_diagonal_(0.5)
+    rng = lambda v: torch.full((1, 1, 1, 1), v, device="cuda")
+    return {
+        "relu inplace": lambda: F.relu(q, inplace=True),
+        "add2 inplace": lambda: F.add2(q, one, inplace=True),
+        "relu outputs": lambda: F.relu(one, outputs=[q]),
+        "relu outputs, a view": lambda: F.relu(one, outputs=[q.view(q.shape)]),
+        "relu outputs, detached": lambda: F.relu(one, outputs=[q.detach()]),
+        "quantizer outputs": lambda: F.fixed_point_quantize(one, outputs=[q]),
+        "binary connect convolution outputs": lambda: F.binary_connect_convolution(
+            one, eye, torch.empty_like(eye), outputs=[q]),
+        "prepared convolution outputs": lambda: F.binary_convolution_from_codes_prepared(
+            F.fixed_point_codes_nhwc(one), one.shape, F.prepare_binary_weights(eye), outputs=[q]),
+        "relu gradient": lambda: F.relu_backward(one, one, dx=q),
+        "quantizer gradient": lambda: F.fixed_point_quantize_backward(one, one, dx=q),
+        "min-max gradient": lambda: F.min_max_quantize_backward(
+            one, rng(-2.0), rng(2.0), rng(0.0), rng(255.0), one, propagate_down=(True, False, False),
+            grads=(q, None, None)),
+        "convolution gradient": lambda: F.binary_connect_convolution_backward(
+            one, eye.fill_(1.0), one, propagate_down=(True, False, False), grads=(q, None, None)),
+        "batch normalization gradient": lambda: F.batch_normalization_backward(
+            one, one, torch.ones(32, device="cuda"), torch.ones(32, device="cuda"), torch.ones(32, device="cuda"),
+            propagate_down=(True, False, False), grads=(q, None, None)),
+        "another tensor's memory": lambda: setattr(q, "data", one),
+    }
+
+
+@pytest.mark.parametrize("name", WRITERS)
+def test_codes_do_not_outlive_a_write(F, small_threshold, name):
+    rng = np.random.RandomState(3)
+    d = 2.0 ** -4
+    q = F.fixed_point_quantize(torch.from_numpy((rng.randn(2, 32, 8, 8) * 3).astype(np.float32)).cuda(), True, 8, d,
+                               codes_sideband=True)
+    before = q.clone()
+    assert F._sideband_get(q, d) is not None
+    _into(F, q)[name]()
+    assert not torch.equal(q, before)
+    assert F._sideband_get(q, d) is None
+    w = torch.from_numpy(rng.randn(16, 32, 3, 3).astype(np.float32)).cuda()
+    conv = lambda t: F.binary_connect_convolution(t, w, torch.empty_like(w), None, 1, (1, 1), fixed_point_delta=d)
+    assert torch.equal(conv(q), conv(q.clone()))
+    F.check_device_status()
+
+
 def test_resnet18_as_written_with_the_codes_sideband(F, small_threshold):
     from nnabla_b200 import resnet18
     rng = np.random.RandomState(2)
