@@ -220,6 +220,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();
   }
+  ptx::tc_fence_before_sync();
+  __syncthreads(); // the block has its tensor memory before it lets the successor in
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
   // (codes and channel-last results are read by convolutions)
   if (!ep.y_nchw || early_trigger((int64_t)prob.Nimg * prob.Ko * prob.Ho * prob.Wo))
@@ -228,10 +232,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
                                       ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)
                         : make_float2(0.0f, 0.0f);
-  ptx::tc_fence_before_sync();
   __syncthreads();
-  ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
 
   // tile -> (column tile, pixel box); the column tiles of one box are neighbours in time (the box stays in L2)
   auto decode = [&](int tile, int &n0, int &img0, int &oy0) {

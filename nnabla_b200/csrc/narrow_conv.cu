@@ -300,6 +300,10 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
     ptx::tmem_alloc(tmem_slot, kTmemCols);
     ptx::tmem_relinquish();
   }
+  ptx::tc_fence_before_sync();
+  __syncthreads(); // the block has its tensor memory before it lets the successor in
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
   if (early_trigger((int64_t)g.N * g.Ko * g.Ho * g.Wo))
     pdl_trigger();
@@ -320,10 +324,7 @@ __global__ void __launch_bounds__(kThreadsNC, 1)
       reinterpret_cast<uint4 *>(ring + kRing * slot_bytes)[i] = make_uint4(0, 0, 0, 0);
     fence_async_smem();
   }
-  ptx::tc_fence_before_sync();
   __syncthreads();
-  ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
 
   if (warp == kLoadWarp) {
     // ------------------------------------------------------------ loader: the new rows of every tile

@@ -4,15 +4,26 @@
 // dozen images per GPU a network is a chain of kernels of a few microseconds each, and the gap between two
 // kernels (launch processing, grid start) is a large part of the step; this hides most of it.
 //
-// Rules that keep it correct: (1) every kernel launched this way executes pdl_wait() in every thread, before any
-// global-memory access: as its first statement, or in the tensor-core kernels after the barriers and the tensor
-// memory are set up, which touches nothing outside the SM (so its completion implies the predecessor's, and
-// ordering stays transitive along the stream); (2) pdl_trigger() only says "my
-// successor may be scheduled", it orders nothing. A kernel with a large share of the SM's shared memory triggers early
-// only while its result is small (early_trigger): the successor's blocks become resident beside it, the SM then never
-// drains, and streaming kernels go on with the little L1 that such a split leaves (their loads in flight live there):
-// max-pooling behind the stem 280 us instead of 180, a batch-256 network 5.0 ms instead of 4.5. Kernels launched the ordinary way in between serialize
-// fully, as before. NNABLA_B200_PDL=0 turns the attribute off (ordinary launches; the waits are no-ops).
+// Rules that keep it correct:
+// (1) Every kernel launched this way executes pdl_wait() in every thread, before any global-memory access: as its first
+//     statement, or in the tensor-core kernels after the barriers and the tensor memory are set up, which touches
+//     nothing outside the SM. Its completion then implies the predecessor's, and ordering stays transitive along the
+//     stream.
+// (2) pdl_trigger() only says "my successor may be scheduled", it orders nothing. It comes after pdl_wait(), and after
+//     the block has its tensor memory: a __syncthreads() stands between the allocation, which one warp makes, and the
+//     trigger, for which one thread counts as the block. Otherwise, with another stream's kernel on the SM, the
+//     successor's blocks could get the columns that this kernel's block is still waiting for, and keep them while they
+//     wait for this kernel.
+// Kernels launched the ordinary way in between serialize fully, as before. NNABLA_B200_PDL=0 turns the attribute off
+// (ordinary launches; the waits are no-ops).
+//
+// When to trigger is a matter of time only. A kernel with a large share of the SM's shared memory that triggers early
+// has the successor's blocks become resident beside it; the SM then never drains, and a streaming kernel goes on with
+// the little L1 that such a split leaves (its loads in flight live there): max-pooling behind the stem 280 us instead
+// of 180, a batch-256 network 5.0 ms instead of 4.5. So the stem, the pixel-major convolutions and the int8
+// convolutions with an fp32 NCHW result trigger early up to early_trigger() values; gemm.cuh while its tiles make one
+// round; the weight gradient while it is small (four taps per task), gemm2.cuh never. The int8 convolutions whose
+// result is codes or channel-last trigger early at any size: what follows them in a network is the next convolution.
 #pragma once
 #include <cuda_runtime.h>
 
