@@ -842,10 +842,9 @@ struct MinMaxOp {
   }
 };
 
-// The three steps of one range in one block: extrema, parameters, quantizer. Ranges of up to kSmallRange elements; the
-// chain of four launches (initialise, reduce, parameters, quantize) spends its time between them: [16, 24, 49] with 24
-// ranges 12.4 us.
-constexpr size_t kSmallRange = 8192;
+// The three steps of one range in one block: extrema, parameters, quantizer. The chain of four launches (initialise,
+// reduce, parameters, quantize) spends its time between them: [16, 24, 49] with 24 ranges 12.4 us. Taken where
+// minmax_one_block says so.
 constexpr int kSmallThreads = 512;
 
 __global__ void __launch_bounds__(kSmallThreads)
@@ -912,9 +911,30 @@ __global__ void __launch_bounds__(kSmallThreads)
   }
 }
 
-// One block per range, where a range is short and the ranges' blocks do not leave most of a large tensor to one block.
-inline bool minmax_small_applies(const MinMaxView &V) {
-  return V.size > 0 && V.outer * V.inner <= kSmallRange && V.Q < (1u << 31);
+// Whether one launch with a block per range is the faster form; else the chain over the whole tensor runs. Device
+// times in us as (block per range, chain), from sweeps of outer x Q x inner; a call from Python pays 2 us of host time
+// for the chain's second launch, 6 us for its four.
+//  * A block of 512 threads walks its range serially: up to 8192 elements (one range of 8192: observed 9.8, 9.9;
+//    gradient 5.2, 7.2). The forward without observation is only two launches as a chain, and with few ranges, whose
+//    blocks leave the chip idle, level at some 4096 elements (64 ranges of 4096: 5.7, 4.6; of 8192: 9.4, 5.7).
+//  * Runs of less than 16 bytes leave most of each 32-byte sector to other blocks. Weights [inmaps, outmaps] with a
+//    range per column, 4096 x 4096: forward 177, 74, observed 242, 147, gradient 242, 50; 1024 x 1024: 14, 10 and 21,
+//    17 and 17, 13; 1024 x 256: 5.3, 4.9 and 7.8, 9.4 and 6.3, 8.6. Runs of two, 1024 x 512 x 2: 8.6, 10.1 and 12, 16
+//    and 11, 13; of four, 1024 x 1024 x 4: 17, 22 and 26, 35 and 16, 21.
+//  * A wave of blocks costs 1 to 2 us whatever its ranges hold: 1024 ranges of one element 3.8, 4.5, but 4096 of 64
+//    elements 11, 5 and 16384 of one element 34, 5; 4096 ranges of 1024 elements 20, 22, gradient 13.4, 16.3, whose
+//    chain is the better one again above 2^22 elements (8192 each: 97, 90).
+enum class MinMaxCall { kForward, kObserve, kGradient };
+inline bool minmax_one_block(const MinMaxView &V, MinMaxCall call) {
+  const size_t per_q = V.outer * V.inner;
+  if (V.size == 0 || per_q > 8192 || (call == MinMaxCall::kForward && V.Q < 256 && per_q > 4096))
+    return false;
+  if (V.Q > 65535) // more than the chain's reduction takes
+    return call == MinMaxCall::kObserve && V.Q < (1u << 31);
+  if (V.inner < 4 && (per_q > 2048 || V.size > (V.inner == 1 ? 1u << 18 : 1u << 20)))
+    return false;
+  return V.Q <= 1024 ||
+         (V.Q <= 4096 && per_q >= 1024 && !(call == MinMaxCall::kGradient && V.size > (1u << 22)));
 }
 
 int minmax_view(const int64_t *xs, const int64_t *qs, int ndim, MinMaxView *V) {
@@ -960,7 +980,7 @@ int minmax_run(const float *x, const MinMaxView &V, float *qr_min, float *qr_max
                float *scratch, cudaStream_t st) {
   // (T)decay_ and (T)(1.0 - decay_) as in min_max_quantize.cpp:105-106.
   const float d1 = decay, d2 = (float)(1.0 - (double)decay);
-  if (minmax_small_applies(V)) {
+  if (minmax_one_block(V, x_min_max ? MinMaxCall::kObserve : MinMaxCall::kForward)) {
     NB_CUDA(launch_dependent(minmax_small_kernel, dim3((unsigned)V.Q), dim3(kSmallThreads), 0, st, x, V, qr_min, qr_max,
                              ql_min, ql_max, x_min_max, ema, d1, d2, eps, y, scale));
     return NB200_OK;

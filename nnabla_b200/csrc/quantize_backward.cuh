@@ -402,7 +402,7 @@ int minmax_backward(const float *x, const MinMaxView &V, const float *qr_min, co
   // range gradients to be zeroed: asked for (flag 2) and not produced below
   float *zero_min = (prop[1] & 2) && !(ranges && down[1]) ? g_min : nullptr;
   float *zero_max = (prop[2] & 2) && !(ranges && down[2]) ? g_max : nullptr;
-  if (!ranges && minmax_small_applies(V) && V.Q <= 65535) {
+  if (!ranges && minmax_one_block(V, MinMaxCall::kGradient)) {
     if (!down[0] && !zero_min && !zero_max)
       return NB200_OK;
     NB_CHECK(!(down[0] && fine) || (qr_min && qr_max && ql_min && ql_max), NB200_EVALUE, "null range pointer");

@@ -167,3 +167,62 @@ def test_min_max_quantize_range_lengths(shape, axis, observe, fine):
         for got, side in ((g_lo, x < m), (g_hi, x > M)):
             want = torch.zeros_like(got) if observe else (dy.double() * side).sum(dims, keepdim=True)
             assert got.shape == torch.Size(qshape) and ((got - want).abs() <= 1e-4 * dy.abs().sum() ** 0.5 + 1e-5).all()
+
+
+def _kernels(fn):
+    """Kernel launches of fn, from its CUDA graph."""
+    from cuda.bindings import runtime
+    fn()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    graph = runtime.cudaGraph_t(g.raw_cuda_graph())
+    _, _, count = runtime.cudaGraphGetNodes(graph)
+    err, nodes, _ = runtime.cudaGraphGetNodes(graph, count)
+    assert err == runtime.cudaError_t.cudaSuccess
+    return sum(runtime.cudaGraphNodeGetType(n)[1] == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel
+               for n in nodes[:count])
+
+
+# the lines of minmax_one_block: (forward, observed, gradient) in one launch
+@pytest.mark.parametrize("shape,one", [
+    ((16, 24, 49), (True, True, True)),          # an activation, a range per channel
+    ((1, 1, 4096), (True, True, True)),
+    ((1, 1, 8192), (False, True, True)),         # a single long range
+    ((1, 1, 8193), (False, False, False)),
+    ((1024, 256, 1), (True, True, True)),        # weights with a range per output column: a small matrix
+    ((1024, 257, 1), (False, False, False)),
+    ((2049, 16, 1), (False, False, False)),
+    ((1024, 512, 2), (True, True, True)),
+    ((1024, 513, 2), (False, False, False)),
+    ((4096, 4096, 1), (False, False, False)),
+    ((1024, 256, 4), (True, True, True)),        # runs of 16 bytes
+    ((2, 1024, 3), (True, True, True)),          # many ranges
+    ((2, 1025, 3), (False, False, False)),
+    ((4, 4096, 256), (True, True, True)),
+    ((5, 4096, 256), (True, True, False)),
+    ((4, 4097, 256), (False, False, False)),
+    ((1, 65536, 4), (False, True, None)),        # more ranges than the reduction over the whole tensor takes
+])
+def test_min_max_quantize_route(F, shape, one):
+    """Each call takes the form that was measured to be the faster one, and both give the oracle's bits."""
+    rng = np.random.RandomState(shape[1])
+    x = rng.uniform(-4.5, 4.5, shape).astype(np.float32)
+    dy = rng.randn(*shape).astype(np.float32)
+    q = [np.full((1, shape[1], 1), v, np.float32) for v in (-4.0, 4.0, 0.0, 255.0)]
+    gx, gdy, r = dev(x), dev(dy), [dev(v) for v in q]
+    for observe in (False, True):
+        want, lo, hi, _ = oracle.min_max_quantize(x, *q, 0.9, observe, observe)
+        mine = [t.clone() for t in r]
+        got = F.min_max_quantize(gx, *mine, 0.9, observe, observe)
+        for a, b in ((got, want), (mine[0], lo), (mine[1], hi)):
+            assert np.array_equal(bits(host(a)), bits(b))
+        assert (_kernels(lambda: F.min_max_quantize(gx, *mine, 0.9, observe, observe)) == 1) == one[int(observe)]
+    if one[2] is None:
+        with pytest.raises(RuntimeError, match="65535"):
+            F.min_max_quantize_backward(gx, *r, gdy, x_min_max=True)
+        return
+    want, _, _ = oracle.min_max_quantize_backward(x, *q, dy, True, True)
+    got, glo, ghi = F.min_max_quantize_backward(gx, *r, gdy, x_min_max=True, ema=True)
+    assert np.array_equal(bits(host(got)), bits(want)) and not glo.any() and not ghi.any()
+    assert (_kernels(lambda: F.min_max_quantize_backward(gx, *r, gdy, x_min_max=True, ema=True)) == 1) == one[2]
