@@ -145,6 +145,8 @@ struct PlanesAxis {
   int k, dil, pad, s;
   bool flip; // the gradient's direction: the classes are the output's
   int residue(int t) const { return ((t * dil - pad) % s + s) % s; }
+  // first input pixel of a box whose first class pixel is u, of input class r
+  int first_pixel(int u, int r) const { return flip ? u : u * s + r; }
   int offset(int t) const { return (flip ? residue(t) + pad - t * dil : t * dil - pad - residue(t)) / s; }
   int min_offset() const {
     int m = offset(0);
@@ -175,6 +177,48 @@ inline int64_t planes_slots(int group, int c_pad_g) {
 
 constexpr size_t kPlanesSmem = 226 * 1024; // of 227 KB; the barriers are static
 
+// How a tile takes its images' pixels. A halo box covers an image's rows and columns once for all taps, and the rows
+// of a second image do not fit behind it: of images of at most 64 pixels half of a tile's 128 rows are empty.
+enum class PlanesSpan {
+  kHalo, // one image, or a part of one, per tile; one box per tile and channel block
+  kRows, // several images, whose boxes have the halo along the columns only: one box per filter row
+  kTaps, // as many images as have room: one box per tap
+};
+
+// Images (class grids of rows x p.Wu pixels) per tile of a span, whose boxes have span_x columns of halo.
+inline int planes_images(const ConvPlanesProblem &p, PlanesSpan span, int rows, int span_x) {
+  if (span == PlanesSpan::kHalo)
+    return 1;
+  const int wp = p.Wu + (span == PlanesSpan::kRows ? span_x : 0);
+  const int last = (rows - 1) * wp + p.Wu; // MMA rows of the last image
+  const int n = last > kTileM ? 0 : (kTileM - last) / (rows * wp) + 1;
+  return n < p.Nimg ? n : p.Nimg;
+}
+
+// The span with the shortest time: rounds of tiles over the SMs, where a round of 512 channels and 3 x 3 taps takes 25
+// us with two planes from halo boxes, 28 with a box per filter row, 38 with a box per tap (34, 37 and 43 with three
+// planes). Measured, in us, forward and input gradient of 512 -> 512 maps on 256 images: 7 x 7 halo 197 and 255, by
+// rows 136 and 167 (by taps 174 and 193); 8 x 8 halo 198 and 257, by taps 175 and 195; 5 x 5 halo 191 and 249, by rows
+// 106 and 129, by taps 99 and 108. (The kernel with the maps on the MMA rows took 146 and 212, 157 and 231, 91 and
+// 125.) Where the halo form needs one round it stays: 16 images of 7 x 7, 43 and 52 against 46 and 53.
+inline PlanesSpan choose_planes_span(const ConvPlanesProblem &p, int rows, int span_x) {
+  if (2 * rows * p.Wu > kTileM || rows * p.in_sy > 256 || (p.Wu + span_x) * p.in_sx > 256)
+    return PlanesSpan::kHalo;
+  auto cost = [&](PlanesSpan span, int weight) {
+    const int images = planes_images(p, span, rows, span_x);
+    if (images < 2 && span != PlanesSpan::kHalo)
+      return (int64_t)1 << 40;
+    const int64_t tiles = (int64_t)p.n_tiles * p.groups * p.sy * p.sx * (span == PlanesSpan::kHalo ? p.tiles_h : 1) *
+                          ((p.Nimg + images - 1) / images);
+    return (tiles + sm_count() - 1) / sm_count() * weight;
+  };
+  const int64_t halo = cost(PlanesSpan::kHalo, 20), by_row = cost(PlanesSpan::kRows, 22),
+                by_tap = cost(PlanesSpan::kTaps, p.planes == 2 ? 30 : 26);
+  if (by_tap < by_row && by_tap < halo)
+    return PlanesSpan::kTaps;
+  return by_row < halo ? PlanesSpan::kRows : PlanesSpan::kHalo;
+}
+
 // Fills p's tiling for an output of p.H x p.W with p.maps maps per group; false: the kernel does not apply.
 bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, int channels_g) {
   ConvPlanesProblem &p = plan.p;
@@ -185,12 +229,13 @@ bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, i
   p.sx = ax.flip ? ax.s : 1;
   p.in_sy = ay.flip ? 1 : ay.s;
   p.in_sx = ax.flip ? 1 : ax.s;
+  p.n_box = 1;
+  p.img_rows = kTileM;
   p.Wu = (p.W + p.sx - 1) / p.sx;
   const int Hu = (p.H + p.sy - 1) / p.sy;
-  p.y0 = ay.min_offset();
-  p.x0 = ax.min_offset();
-  p.wp = p.Wu + ax.max_offset() - p.x0;
-  const int span_y = ay.max_offset() - p.y0;
+  const int y0 = ay.min_offset(), x0 = ax.min_offset(); // a box's origin relative to its class's first row / column
+  const int span_y = ay.max_offset() - y0, span_x = ax.max_offset() - x0;
+  p.wp = p.Wu + span_x;
   p.cblocks = (channels_g + 63) / 64;
   p.k_slots = p.cblocks * 64;
   if (p.Wu > 128 || p.wp * p.in_sx > 256)
@@ -208,46 +253,86 @@ bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, i
     return false;
   p.tiles_h = (Hu + p.h_box - 1) / p.h_box;
   p.plane_bytes = (p.hp * p.wp + 7) / 8 * 8 * kRowBytes;
+  // one box per class of taps: an output class has its own, or a tile sums those of all input classes
   int n = 0, max_row = 0;
   for (int ry = 0; ry < ay.s; ++ry)
     for (int rx = 0; rx < ax.s; ++rx) {
-      p.class_tap[ry * ax.s + rx] = n;
+      const int box = ry * ax.s + rx;
+      p.box_tap[box] = n;
+      p.box_y[box] = (int16_t)ay.first_pixel(y0, ry);
+      p.box_x[box] = (int16_t)ax.first_pixel(x0, rx);
       for (int ky = 0; ky < ay.k; ++ky)
         for (int kx = 0; kx < ax.k; ++kx)
           if (ay.residue(ky) == ry && ax.residue(kx) == rx) {
-            p.tap_row[n] = (ay.offset(ky) - p.y0) * p.wp + ax.offset(kx) - p.x0;
+            p.tap_row[n] = (ay.offset(ky) - y0) * p.wp + ax.offset(kx) - x0;
             max_row = p.tap_row[n] > max_row ? p.tap_row[n] : max_row;
             p.tap_k[n++] = ky * ax.k + kx;
           }
     }
-  p.class_tap[ay.s * ax.s] = n;
-  // the 128 rows read from the last tap's row on may reach past the last box
-  int over = (max_row + kTileM) * kRowBytes - p.plane_bytes;
-  over = over > 0 ? over : 0;
+  p.box_tap[ay.s * ax.s] = n;
+  const int classes = p.sy * p.sx, boxes_per_class = p.in_sy * p.in_sx; // one of the two is 1
+  for (int c = 0; c <= classes; ++c)
+    p.class_box[c] = c * boxes_per_class;
   plan.bn = p.maps <= 64 ? 64 : 128;
   p.n_tiles = (p.maps + plan.bn - 1) / plan.bn;
-  const size_t b_tile = (size_t)plan.bn * kRowBytes, fixed = 1024 + over;
+  const size_t b_tile = (size_t)plan.bn * kRowBytes;
+  // the 128 rows read from the last tap's row on may reach past the last box
+  auto fixed = [&]() {
+    const int over = (max_row + kTileM) * kRowBytes - p.plane_bytes;
+    return (size_t)1024 + (over > 0 ? over : 0);
+  };
   // all weights beside three single-plane boxes at least, and the accumulation short enough without chunks
   const size_t b_all = (size_t)taps * p.cblocks * b_tile;
   plan.resident = p.groups == 1 && p.n_tiles == 1 && taps * p.cblocks * 4 <= 96 &&
-                  fixed + b_all + 3 * (size_t)p.plane_bytes <= kPlanesSmem;
+                  fixed() + b_all + 3 * (size_t)p.plane_bytes <= kPlanesSmem;
   if (plan.resident) {
-    int st = (int)((kPlanesSmem - fixed - b_all) / p.plane_bytes);
+    int st = (int)((kPlanesSmem - fixed() - b_all) / p.plane_bytes);
     p.a_stages = st > 4 ? 4 : st;
     p.b_stages = 1;
     p.chunk = 0;
-    plan.smem = fixed + b_all + (size_t)p.a_stages * p.plane_bytes;
+    plan.smem = fixed() + b_all + (size_t)p.a_stages * p.plane_bytes;
     return true;
   }
-  const size_t stage = (size_t)p.planes * p.plane_bytes;
   p.a_stages = 2;
-  if (fixed + 2 * stage + 2 * b_tile > kPlanesSmem)
+  const PlanesSpan span = choose_planes_span(p, Hu, span_x);
+  if (span != PlanesSpan::kHalo) {
+    const bool by_tap = span == PlanesSpan::kTaps;
+    p.n_box = planes_images(p, span, Hu, span_x);
+    p.wp = p.Wu + (by_tap ? 0 : span_x);
+    p.hp = p.h_box = Hu;
+    p.tiles_h = 1;
+    p.img_rows = Hu * p.wp;
+    p.plane_bytes = (p.n_box * p.img_rows + 7) / 8 * 8 * kRowBytes;
+    max_row = by_tap ? 0 : span_x;
+    // a box of few taps is used up soon
+    p.a_stages = fixed() + 4 * ((size_t)p.planes * p.plane_bytes + b_tile) <= kPlanesSmem ? 4 : 3;
+    // the same taps in the same order, in more boxes; a class that no tap reaches has none
+    int box = 0, cls = -1;
+    for (int i = 0, last = -1; i < taps; ++i) {
+      const int ky = p.tap_k[i] / ax.k, kx = p.tap_k[i] - ky * ax.k, ry = ay.residue(ky), rx = ax.residue(kx);
+      while (cls < (classes > 1 ? ry * p.sx + rx : 0))
+        p.class_box[++cls] = box;
+      const int key = by_tap ? i : ky * ax.s + rx;
+      if (key != last) {
+        p.box_y[box] = (int16_t)ay.first_pixel(ay.offset(ky), ry);
+        p.box_x[box] = (int16_t)ax.first_pixel(by_tap ? ax.offset(kx) : x0, rx);
+        p.box_tap[box++] = i;
+        last = key;
+      }
+      p.tap_row[i] = by_tap ? 0 : ax.offset(kx) - x0;
+    }
+    while (cls < classes)
+      p.class_box[++cls] = box;
+    p.box_tap[box] = taps;
+  }
+  const size_t boxes = fixed() + p.a_stages * (size_t)p.planes * p.plane_bytes;
+  if (boxes + 2 * b_tile > kPlanesSmem)
     return false;
-  int st = (int)((kPlanesSmem - fixed - 2 * stage) / b_tile);
+  int st = (int)((kPlanesSmem - boxes) / b_tile);
   p.b_stages = st >= 6 ? 6 : (st >= 4 ? 4 : 2); // even: they alternate between the issuing warps
   // two accumulators share a chunk; half the usual length each: no step of a strided gradient multiplies zeros here
   p.chunk = 2 * k_chunk_blocks(p.planes * 8);
-  plan.smem = fixed + 2 * stage + (size_t)p.b_stages * b_tile;
+  plan.smem = boxes + (size_t)p.b_stages * b_tile;
   return true;
 }
 
@@ -278,7 +363,7 @@ int launch_planes(const PlanesPlan &plan, const void *act, int Hin, int Win, int
   const uint64_t dims[5] = {(uint64_t)ctot, (uint64_t)Win, (uint64_t)Hin, (uint64_t)p.Nimg, (uint64_t)p.planes};
   const uint64_t strides[4] = {(uint64_t)ctot * 2, (uint64_t)ctot * 2 * Win, (uint64_t)ctot * 2 * Win * Hin,
                                (uint64_t)ctot * 2 * Win * Hin * p.Nimg};
-  const uint32_t box[5] = {64, (uint32_t)(p.wp * p.in_sx), (uint32_t)(p.hp * p.in_sy), 1, 1};
+  const uint32_t box[5] = {64, (uint32_t)(p.wp * p.in_sx), (uint32_t)(p.hp * p.in_sy), (uint32_t)p.n_box, 1};
   const uint32_t estr[5] = {1, (uint32_t)p.in_sx, (uint32_t)p.in_sy, 1, 1};
   NB_TRY(encode_tiled(&ma, 0, 5, act, dims, strides, box, estr, kRowBytes));
   const int64_t pitch = (int64_t)taps * p.k_slots;

@@ -16,6 +16,11 @@
 // fetched a box of pixels per filter tap: 540 us for the input gradient of a 64 -> 64 3 x 3 layer on [128, 64, 56, 56],
 // now 100 to 120, 71 of them MMAs at the rates above; the forward of 256 -> 256 maps on [128, 256, 28, 28] 183 us, now 172.
 //
+// A tile is a part of an image, or several small images: the box then holds them one behind the other, n_box deep, each
+// with the halo along its columns only (a box per filter row) or with none (a box per tap), see choose_planes_span. A box
+// and its place in the weights are tables in the problem, and all three roles walk them by counters: divisions per box took
+// longer than the MMAs of one tap (512 -> 512 maps of 8 x 8, a box per tap, 256 images: 207 us, 175 without them).
+//
 // Warp 0 loads (TMA), two warps issue the MMAs, eight epilogue warps store. The issuing warps take alternate tiles
 // (kResident) or alternate weight tiles into accumulators of their own: a thread that decodes a tile, waits for
 // barriers and comes back to the head of its unrolled loop leaves the tensor core idle, 27 % of the time with one. A
@@ -38,11 +43,11 @@ struct ConvPlanesProblem {
   int Nimg, maps, total_maps, groups; // output maps per group and in all
   int H, W;                           // output image
   int sy, sx;                         // output pixel (sy * u + ry, sx * v + rx) belongs to class ry * sx + rx
-  int in_sy, in_sx;                   // a tile sums in_sy * in_sx classes of input pixels (1 with output classes)
+  int in_sy, in_sx;                   // step between the input pixels of a box
   int Wu;                             // columns of a class's grid: ceil(W / sx)
   int h_box, tiles_h, n_tiles;        // class rows per tile, tiles per class and image, column tiles
+  int n_box, img_rows;                // images per tile (1 with tiles_h > 1) and MMA rows from one to the next
   int wp, hp;                         // input box: hp rows of wp pixels
-  int y0, x0;                         // its origin relative to the tile's first class row / column (class pixels)
   int cblocks;                        // 64-channel blocks of one group
   int c_group_stride;                 // channel slots between groups in A
   int k_slots;                        // weight slots per tap
@@ -50,14 +55,18 @@ struct ConvPlanesProblem {
   int planes;                         // planes of A
   int chunk;                          // weight tiles (tap, channel block) per accumulation in tensor memory, even; 0 = all
   int a_stages, b_stages;
-  int class_tap[17];                  // taps of class k: [class_tap[k], class_tap[k + 1])
+  int class_box[17];                  // boxes that a tile of output class k sums: [class_box[k], class_box[k + 1])
+  int box_tap[kPlanesMaxTaps + 1];    // taps that read box b: [box_tap[b], box_tap[b + 1]); may be none
+  int16_t box_y[kPlanesMaxTaps], box_x[kPlanesMaxTaps]; // first input row (of a tile at row 0) and column
   int tap_row[kPlanesMaxTaps];        // first row of the box that tap reads
   int tap_k[kPlanesMaxTaps];          // its index in the weights
   const float *scale, *bias;          // per output map, may be NULL
   const uint32_t *image_max;          // per image: bits of the magnitude that its scaling was chosen from, may be NULL
   float *y;
   int accumulate;
-  __host__ __device__ __forceinline__ int num_tiles() const { return n_tiles * sy * sx * groups * tiles_h * Nimg; }
+  __host__ __device__ __forceinline__ int num_tiles() const {
+    return n_tiles * sy * sx * groups * tiles_h * ((Nimg + n_box - 1) / n_box);
+  }
 };
 
 template <int BN, int PG, bool kResident, bool kF16>
@@ -72,9 +81,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t stage_bytes = (uint32_t)PG * prob.plane_bytes;
   uint8_t *b_base = smem; // weights first: MMAs may read up to 128 rows past a box (rows of no stored pixel)
-  const int in_classes = prob.in_sy * prob.in_sx;
-  const uint32_t b_tiles =
-      kResident ? (uint32_t)(prob.class_tap[prob.sy * prob.sx * in_classes] * prob.cblocks) : (uint32_t)prob.b_stages;
+  const uint32_t b_tiles = kResident ? (uint32_t)(prob.box_tap[prob.class_box[prob.sy * prob.sx]] * prob.cblocks)
+                                     : (uint32_t)prob.b_stages;
   uint8_t *a_base = smem + b_tiles * kBBytes;
 
   __shared__ __align__(8) uint64_t a_full[kPlanesMaxStages], a_empty[kPlanesMaxStages], b_full[kPlanesMaxStages],
@@ -128,28 +136,28 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
     t.group = tile % prob.groups;
     tile /= prob.groups;
     t.row0 = (tile % prob.tiles_h) * prob.h_box;
-    t.img = tile / prob.tiles_h;
+    t.img = tile / prob.tiles_h * prob.n_box;
     return t;
   };
-  // boxes of a tile, in the order of the ring: (channel block, input class, plane group)
-  struct BoxAt {
-    int cb, cls, pg, ry, rx;
+  // the boxes of a tile, in the order of the ring: (channel block, box of its class, plane group)
+  struct BoxWalk {
+    int first, end, cb, box, pg; // box counts from first, the first of the class, to end
   };
-  const int boxes_per_tile = prob.cblocks * in_classes * plane_groups;
-  auto box_at = [&](const TileAt &t, int i) {
-    BoxAt b;
-    b.pg = i % plane_groups;
-    i /= plane_groups;
-    const int ic = i % in_classes;
-    b.cb = i / in_classes;
-    b.cls = t.cls * in_classes + ic; // one of the two counts is 1
-    b.ry = ic / prob.in_sx;
-    b.rx = ic - b.ry * prob.in_sx;
-    return b;
+  auto boxes_of = [&](const TileAt &t) {
+    const int first = prob.class_box[t.cls];
+    return BoxWalk{first, prob.class_box[t.cls + 1], 0, first, 0};
   };
-  // whether a tile has any tap (an output class may have none)
-  auto empty_tile = [&](const TileAt &t) {
-    return prob.class_tap[t.cls * in_classes] == prob.class_tap[(t.cls + 1) * in_classes];
+  auto next_box = [&](BoxWalk &b) {
+    if (++b.pg == plane_groups) {
+      b.pg = 0;
+      if (++b.box == b.end) {
+        b.box = b.first;
+        ++b.cb;
+      }
+    }
+  };
+  auto taps_of = [&](const TileAt &t) { // 0: an output class that no tap reaches
+    return prob.box_tap[prob.class_box[t.cls + 1]] - prob.box_tap[prob.class_box[t.cls]];
   };
   auto gave_up = [&](int code) {
     if (*abort_flag == 0)
@@ -172,9 +180,10 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
       }
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileAt t = decode(tile);
-        for (int i = 0; i < boxes_per_tile && ok; ++i) {
-          const BoxAt at = box_at(t, i);
-          const int cb = at.cb, pg = at.pg, tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+        if (taps_of(t) == 0)
+          continue;
+        for (BoxWalk at = boxes_of(t); at.cb < prob.cblocks && ok; next_box(at)) {
+          const int cb = at.cb, pg = at.pg, tap0 = prob.box_tap[at.box], tap1 = prob.box_tap[at.box + 1];
           if (tap0 == tap1)
             continue;
           if (!ptx::mbar_wait(a_empty + as, aphase ^ 1u, abort_flag)) {
@@ -182,12 +191,12 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
             ok = false;
             break;
           }
-          ptx::mbar_expect_tx(a_full + as, (uint32_t)(PG * prob.hp * prob.wp * kRowBytes));
+          ptx::mbar_expect_tx(a_full + as, (uint32_t)(PG * prob.n_box * prob.hp * prob.wp * kRowBytes));
 #pragma unroll
           for (int p = 0; p < PG; ++p)
             ptx::tma_load_5d(a_base + as * stage_bytes + p * prob.plane_bytes, &map_a, a_full + as,
-                             t.group * prob.c_group_stride + cb * 64, prob.x0 * prob.in_sx + at.rx,
-                             (t.row0 + prob.y0) * prob.in_sy + at.ry, t.img,
+                             t.group * prob.c_group_stride + cb * 64, prob.box_x[at.box],
+                             t.row0 * prob.in_sy + prob.box_y[at.box], t.img,
                              prob.planes - 1 - (pg * PG + p)); // smallest pieces first
           if (++as == prob.a_stages) {
             as = 0;
@@ -261,13 +270,12 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
         ok = wait(b_full, 0u);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const TileAt t = decode(tile);
-        if (empty_tile(t))
+        if (taps_of(t) == 0)
           continue;
         if constexpr (kResident) {
           if ((local & 1) != who) { // the other issuer's tile: its boxes are released as soon as they have come
-            for (int i = 0; i < boxes_per_tile; ++i) {
-              const int cls = box_at(t, i).cls;
-              if (prob.class_tap[cls] == prob.class_tap[cls + 1])
+            for (BoxWalk at = boxes_of(t); at.cb < prob.cblocks; next_box(at)) {
+              if (prob.box_tap[at.box] == prob.box_tap[at.box + 1])
                 continue;
               if (!(ok = wait(a_full + as, aphase)))
                 break;
@@ -278,9 +286,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
             continue;
           }
           ok = open_chunk();
-          for (int i = 0; i < boxes_per_tile && ok; ++i) {
-            const BoxAt at = box_at(t, i);
-            const int cb = at.cb, tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+          for (BoxWalk at = boxes_of(t); at.cb < prob.cblocks && ok; next_box(at)) {
+            const int cb = at.cb, tap0 = prob.box_tap[at.box], tap1 = prob.box_tap[at.box + 1];
             if (tap0 == tap1)
               continue;
             if (!(ok = wait(a_full + as, aphase)))
@@ -307,9 +314,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
           // Weight stages alternate between the issuers (their number is even), so that each sees every phase of its own.
           int in_chunk = 0;
           ok = open_chunk();
-          for (int i = 0; i < boxes_per_tile && ok; ++i) {
-            const BoxAt at = box_at(t, i);
-            const int tap0 = prob.class_tap[at.cls], tap1 = prob.class_tap[at.cls + 1];
+          for (BoxWalk at = boxes_of(t); at.cb < prob.cblocks && ok; next_box(at)) {
+            const int tap0 = prob.box_tap[at.box], tap1 = prob.box_tap[at.box + 1];
             if (tap0 == tap1)
               continue;
             if (!(ok = wait(a_full + as, aphase)))
@@ -348,7 +354,8 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3, set = (warp - 2) >> 2; // TMEM lanes [32 * quarter, + 32); even / odd column chunks
-    const int row = quarter * 32 + lane, box_y = row / prob.wp, box_x = row - box_y * prob.wp;
+    const int row = quarter * 32 + lane, box_img = row / prob.img_rows, in_img = row - box_img * prob.img_rows;
+    const int box_y = in_img / prob.wp, box_x = in_img - box_y * prob.wp;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int64_t plane = (int64_t)prob.H * prob.W;
     constexpr int kMine = BN / 64; // chunks of 32 columns per warp
@@ -356,10 +363,12 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const TileAt t = decode(tile);
-      const int taps = prob.class_tap[(t.cls + 1) * in_classes] - prob.class_tap[t.cls * in_classes];
+      const int taps = taps_of(t);
       const int ry = t.cls / prob.sx, rx = t.cls - ry * prob.sx;
       const int iy = (t.row0 + box_y) * prob.sy + ry, ix = box_x * prob.sx + rx;
-      const bool pix_ok = box_y < prob.h_box && box_x < prob.Wu && iy < prob.H && ix < prob.W;
+      const int img = t.img + box_img;
+      const bool pix_ok = box_img < prob.n_box && img < prob.Nimg && box_y < prob.h_box && box_x < prob.Wu &&
+                          iy < prob.H && ix < prob.W;
       const int tiles_k = kResident ? 1 : taps * prob.cblocks;
       const int chunks = taps == 0 ? 0 : (kResident || prob.chunk == 0 ? 1 : (tiles_k + prob.chunk - 1) / prob.chunk);
       float acc[kMine][32];
@@ -412,17 +421,18 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
         if (left <= 0)
           continue;
         const int map0 = t.group * prob.maps + col;
-        float *yp = prob.y + ((int64_t)t.img * prob.total_maps + map0) * plane + (int64_t)iy * prob.W + ix;
+        float *yp = prob.y + ((int64_t)img * prob.total_maps + map0) * plane + (int64_t)iy * prob.W + ix;
         if (prob.scale || prob.bias || prob.image_max) {
           // one rounding per operation, like the reference's product and bias addition (the image's factor is a power
           // of two)
-          const float up = prob.image_max ? __int_as_float((127 + half_pair_exponent(__ldg(prob.image_max + t.img))) << 23)
-                                          : 1.0f;
-          const float ls = __fmul_rn(prob.scale && lane < left ? __ldg(prob.scale + map0 + lane) : 1.0f, up);
+          const float up = prob.image_max && pix_ok
+                               ? __int_as_float((127 + half_pair_exponent(__ldg(prob.image_max + img))) << 23)
+                               : 1.0f;
+          const float ls = prob.scale && lane < left ? __ldg(prob.scale + map0 + lane) : 1.0f;
           const float lb = prob.bias && lane < left ? __ldg(prob.bias + map0 + lane) : 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            acc[ci][j] = __fmul_rn(acc[ci][j], __shfl_sync(0xffffffffu, ls, j));
+            acc[ci][j] = __fmul_rn(acc[ci][j], __fmul_rn(__shfl_sync(0xffffffffu, ls, j), up));
             if (prob.bias)
               acc[ci][j] = __fadd_rn(acc[ci][j], __shfl_sync(0xffffffffu, lb, j));
           }

@@ -58,3 +58,64 @@ def test_forward(n, c, h, w, o, k, pad, stride, dil, group):
     want = torch.nn.functional.conv2d(x.double(), wb.double() * alpha.double().view(-1, 1, 1, 1), None, stride, pad, dil, group)
     error = (y.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
     assert error.max() <= 2e-6
+
+
+# batch, channels, height, width, maps, kernel, pad, stride, group; blocks of the forward and of the input gradient: a
+# tile each, up to one per SM
+SMALL = [
+    (64, 96, 7, 7, 512, 3, 1, 1, 1, 128, 64),       # two images a tile, a box per filter row; one round as it is
+    (75, 512, 8, 8, 200, 3, 1, 1, 1, 76, 148),      # a box per tap; one image in the last tile
+    (400, 130, 5, 5, 64, 3, 1, 1, 1, 134, 148),     # three images a tile; 64 columns
+    (100, 256, 7, 7, 130, 1, 0, 1, 1, 100, 100),    # no halo
+    (100, 64, 13, 15, 130, 3, 1, 2, 1, 100, 148),   # a stride: classes of taps, and of pixels
+    (90, 128, 6, 6, 256, 3, 1, 1, 2, 90, 90),       # groups
+    (700, 512, 2, 2, 128, 3, 1, 1, 1, 44, 88),      # many images a tile
+    (30, 300, 9, 8, 300, 5, 2, 2, 1, 90, 96),       # classes of 5 x 4 pixels and fewer
+    (50, 260, 9, 9, 200, 1, 0, 2, 1, 100, 120),     # three classes that no tap reaches
+]
+
+
+def _blocks(fn):
+    """Blocks of the pixel-major kernel (the one with 352 threads) in fn, from its CUDA graph."""
+    from cuda.bindings import driver
+    fn()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    graph = driver.CUgraph(g.raw_cuda_graph())
+    _, _, count = driver.cuGraphGetNodes(graph)
+    _, nodes, _ = driver.cuGraphGetNodes(graph, count)
+    kernel = driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL
+    params = [driver.cuGraphKernelNodeGetParams(n)[1] for n in nodes[:count] if driver.cuGraphNodeGetType(n)[1] == kernel]
+    return [p.gridDimX for p in params if p.blockDimX == 352]
+
+
+@pytest.mark.parametrize("n,c,h,w,o,k,pad,stride,group,blocks,blocks_dx", SMALL)
+def test_small_images_share_tiles(n, c, h, w, o, k, pad, stride, group, blocks, blocks_dx):
+    """Images of at most 64 pixels, of very different magnitudes: several in a tile where that takes fewer rounds."""
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(n + c)
+    x = torch.randn(n, c, h, w, device="cuda", generator=g)
+    x *= torch.exp2(torch.randint(-30, 30, (n, 1, 1, 1), device="cuda", generator=g).float())
+    wt = torch.randn(o, c // group, k, k, device="cuda", generator=g)
+    wb, alpha = torch.empty_like(wt), torch.empty(o, device="cuda")
+    b = torch.randn(o, device="cuda", generator=g)
+    geometry = dict(pad=(pad, pad), stride=(stride, stride), group=group)
+    forward = lambda bias: F.binary_weight_convolution(x, wt, wb, alpha, bias, **geometry)
+    y, yb = forward(None), forward(b)
+    assert torch.equal(yb, y + b.view(1, -1, 1, 1))
+    xd, wd = x.double().requires_grad_(), wb.double() * alpha.double().view(-1, 1, 1, 1)
+    want = torch.nn.functional.conv2d(xd, wd, None, stride, pad, 1, group)
+    per_image = lambda got, ref: (got.double() - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
+    assert per_image(y, want.detach()).max() <= 2e-6
+    dy = torch.randn(*y.shape, device="cuda", generator=g)
+    dy *= torch.exp2(torch.randint(-30, 30, (n, 1, 1, 1), device="cuda", generator=g).float())
+    want.backward(dy.double())
+    gradient = lambda **kw: F.binary_weight_convolution_backward(x, wb, alpha, dy, propagate_down=(True, False, False),
+                                                                 **geometry, **kw)[0]
+    dx = gradient()
+    assert per_image(dx, xd.grad).max() <= 2e-6
+    old = torch.randn(*x.shape, device="cuda", generator=g)
+    assert torch.equal(gradient(accum=(True, False, False), grads=(old.clone(), None, None)), old + dx)
+    F.check_device_status()
+    assert _blocks(lambda: forward(b)) == [blocks] and _blocks(gradient) == [blocks_dx]
