@@ -11,6 +11,7 @@ from golden_util import bits
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
+needs_extension = pytest.mark.skipif(not H.available(), reason="extension library not built")
 
 
 def dev(a, dtype=np.float32):
@@ -68,6 +69,7 @@ def test_inq_quantize_edge_values(F):
         assert np.array_equal(gi.cpu().numpy(), ii)
 
 
+@needs_extension
 @pytest.mark.parametrize("i", range(len(inq_cases.CASES)))
 @pytest.mark.parametrize("algorithm", [0, 1])
 def test_inq_affine_extension_against_cpu_context(i, algorithm):
@@ -98,6 +100,7 @@ def test_inq_convolution_mirror_against_oracle(F, i):
         assert close_to_rms(gy.cpu().numpy(), y)
 
 
+@needs_extension
 @pytest.mark.parametrize("i", range(len(inq_cases.CONV_CASES)))
 @pytest.mark.parametrize("algorithm", [0, 1])
 def test_inq_convolution_extension_against_cpu_context(i, algorithm):
@@ -112,6 +115,7 @@ def test_inq_convolution_extension_against_cpu_context(i, algorithm):
     assert close_to_rms(g[0][0], c[0][0])
 
 
+@needs_extension
 def test_inq_backward_goes_through_the_inner_function():
     """INQAffine / INQConvolution::backward_impl hand the gradients to the inner Affine / Convolution
     (inq_affine.cpp:218-232, inq_convolution.cpp:222-237), which under this context are the device ones."""
