@@ -248,6 +248,11 @@ def cpu_images_per_second(images, threads):
 def run_reference_arm(args):
     if int(os.environ.get("RANK", "0")) != 0:
         return
+    from oracle import ref
+    if not ref.available():  # the C restatement of this repository is not the reference
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's compiled library is not here: its source was not present at build time"}))
+        return
     threads = min(os.cpu_count() or 1, 16)
     for _ in range(1 if args.warmup > 0 else 0):
         cpu_images_per_second(threads, threads)
@@ -443,13 +448,15 @@ class FunctionTimer:
         return fam
 
 
-# DRAM bytes of the 19 binary-weight convolutions of one pass at 256 images, from one ncu capture of this file's
-# own command line (dram__bytes_read.sum + dram__bytes_write.sum over their 38 kernels: 812 MB read, 794 MB
-# written; lines of a result that were still in L2 when its kernel ended are not in the write figure; 15 of the
-# 19 read their quantizer's int8 codes, not the fp32 tensor). The tensors of the pass grow in proportion to the
-# images, so other batch sizes scale it (below 2^23 values per tensor the quantizers leave no codes and the
-# convolutions read fp32: the figure is then low).
-NCU_DRAM_BYTES_BINARY_WEIGHT_CONVOLUTIONS_AT_256 = 1605.9e6
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of each function's kernels in one pass at 256 images, from
+# one ncu capture of this file's own command line; results that were still in L2 when their kernel ended are not in the
+# write figure, and 15 of the 19 binary-weight convolutions read their quantizer's int8 codes, not the fp32 tensor. The
+# tensors of the pass grow in proportion to the images, so other batch sizes scale it (below 2^23 values per tensor the
+# quantizers leave no codes and the convolutions read fp32: the figures are then off).
+NCU_DRAM_BYTES_AT_256 = {
+    "fixed_point_quantize": 4246.6e6, "binary_weight_convolution": 1607.9e6, "batch_normalization": 4175.7e6,
+    "relu": 3985.7e6, "add2": 2060.7e6,
+}
 
 
 def function_table(F, params, gz, x, peaks, int8_peak, passes=3):
@@ -495,10 +502,11 @@ def function_table(F, params, gz, x, peaks, int8_peak, passes=3):
         unit = "TOP/s" if f["kind"] == "int8_ops" else "TFLOP/s"
         ach, peak, bound, work = f["work"] / f["ms"] / 1e9, tensor_peak, "tensor", f["work"]
     traffic = None
-    if name == "binary_weight_convolution":
-        traffic = NCU_DRAM_BYTES_BINARY_WEIGHT_CONVOLUTIONS_AT_256 * int(x.shape[0]) / 256.0 / (f["calls"] / passes)
+    if name in NCU_DRAM_BYTES_AT_256:
+        traffic = NCU_DRAM_BYTES_AT_256[name] * int(x.shape[0]) / 256.0 / (f["calls"] / passes)
     roof = {"bound": bound, "kernel": name, "achieved": ach, "peak": peak, "unit": unit, "frac": ach / peak,
-            "traffic": traffic, "traffic_note": "bytes per call, ncu capture of one pass at 256 images scaled by images",
+            "traffic": traffic,
+            "traffic_note": "bytes per call of this function, ncu capture of one pass at 256 images scaled by images",
             "share_of_step": f["ms"] / total, "ms_per_call": per_call_ms,
             "algorithmic_work_per_call": work / f["calls"],
             "floors_ms_per_pass": {"hbm": t_hbm / passes, "tensor": t_tensor / passes}}

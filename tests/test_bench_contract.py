@@ -27,6 +27,16 @@ def test_reference_arm_prints_the_contract_line():
     assert "workload" in line["config"]
 
 
+@pytest.mark.skipif(os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libnnabla_ref.so")),
+                    reason="reference CPU library built")
+def test_reference_arm_without_the_reference_says_so():
+    out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
+                          "--warmup", "1"], capture_output=True, text=True, timeout=600, cwd=ROOT)
+    assert out.returncode == 0, out.stderr[-500:]
+    line = json.loads(out.stdout.strip().splitlines()[-1])
+    assert set(line) == {"impl", "unavailable"} and line["impl"] == "reference" and "\n" not in line["unavailable"]
+
+
 @pytest.mark.gpu
 def test_own_arm_prints_the_contract_line():
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--steps", "2", "--warmup", "3",
