@@ -434,15 +434,19 @@ class FunctionTimer:
             return ("flops", 2.0 * n_out * a[1].shape[0])
         return ("bytes", 0.0)
 
-    def table(self):
+    def table(self, passes):
+        """Sums per function over `passes` equal passes, each call at its median over them: the events also bracket the
+        host's side of a call, and an allocation that has to wait for the driver in one pass is not the function's."""
         import torch
         torch.cuda.synchronize()
         fam = {}
-        for name, e0, e1, rec in self.records:
+        calls = len(self.records) // passes
+        times = [e0.elapsed_time(e1) for _, e0, e1, _ in self.records]
+        for i, (name, _, _, rec) in enumerate(self.records):
             kind, work = rec[0], rec[1]
             f = fam.setdefault(name, {"calls": 0, "ms": 0.0, "kind": kind, "work": 0.0, "bytes": 0.0})
             f["calls"] += 1
-            f["ms"] += e0.elapsed_time(e1)
+            f["ms"] += statistics.median(times[i % calls::calls])
             f["work"] += work
             f["bytes"] += rec[2] if len(rec) > 2 else (work if kind == "bytes" else 0.0)
         return fam
@@ -459,18 +463,19 @@ NCU_DRAM_BYTES_AT_256 = {
 }
 
 
-def function_table(F, params, gz, x, peaks, int8_peak, passes=3):
+def function_table(F, params, gz, x, peaks, int8_peak, passes=5):
     """Per-function time table of the as-written graph (each function's calls bracketed by CUDA
-    events, averaged over `passes` forward passes) and the roofline entry of the family with the
+    events, the median over `passes` forward passes) and the roofline entry of the family with the
     largest share."""
     from nnabla_b200 import resnet18
     timer = FunctionTimer(F)
     net = resnet18.Runner(timer, params, gz, codes_sideband=True)
-    net(x)
+    for _ in range(2):
+        net(x)
     timer.records.clear()
     for _ in range(passes):
         net(x)
-    fam = timer.table()
+    fam = timer.table(passes)
     total = sum(f["ms"] for f in fam.values())
     rows = {}
     for name, f in sorted(fam.items(), key=lambda kv: -kv[1]["ms"]):
