@@ -14,12 +14,13 @@
 // What bounds it: the tensor core (an MMA of 128 rows takes 51 / 67 cycles for 64 / 128 columns, limited by the
 // shared-memory reads of A). The previous form put the maps on the 128 MMA rows, half of them empty for 64 maps, and
 // fetched a box of pixels per filter tap: 540 us for the input gradient of a 64 -> 64 3 x 3 layer on [128, 64, 56, 56],
-// now 100 to 120, 71 of them MMAs at the rates above; the forward of 256 -> 256 maps on [128, 256, 28, 28] 183 us, now 172.
+// now 95 to 120, 71 of them MMAs at the rates above; the forward of 256 -> 256 maps on [128, 256, 28, 28] 183 us, now 169.
 //
-// A tile is a part of an image, or several small images: the box then holds them one behind the other, n_box deep, each
-// with the halo along its columns only (a box per filter row) or with none (a box per tap), see choose_planes_span. A box
-// and its place in the weights are tables in the problem, and all three roles walk them by counters: divisions per box took
-// longer than the MMAs of one tap (512 -> 512 maps of 8 x 8, a box per tap, 256 images: 207 us, 175 without them).
+// A tile is a part of an image, or several small images: the box then holds them one behind the other, n_box deep,
+// each with the halo along its columns only (a box per filter row) or with none (a box per tap), see
+// choose_planes_span. A box and its place in the weights are tables in the problem, and all three roles walk them by
+// counters: divisions per box took longer than the MMAs of one tap (512 -> 512 maps of 8 x 8, a box per tap, 256
+// images: 207 us, 175 without them).
 //
 // Warp 0 loads (TMA), two warps issue the MMAs, eight epilogue warps store. The issuing warps take alternate tiles
 // (kResident) or alternate weight tiles into accumulators of their own: a thread that decodes a tile, waits for
