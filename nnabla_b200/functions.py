@@ -44,13 +44,16 @@ def _memory(t):
 def _sideband_put(y, codes, delta):
     key = id(y)
     _sideband[key] = (weakref.ref(y, lambda _r, key=key: _sideband.pop(key, None)), y._version, codes, float(delta),
-                      _memory(y))
+                      _memory(y), C.stream_ptr(y.device).value)
 
 
 def _sideband_get(x, delta):
     e = _sideband.get(id(x))
     if e is None or e[0]() is not x or x._version != e[1] or e[3] != float(delta) or e[4] != _memory(x):
         return None
+    if e[5] != C.stream_ptr(x.device).value:
+        # read on another stream than their own: their memory must outlive that read, as the caller sees to for x
+        e[2].record_stream(torch.cuda.current_stream(x.device))
     return e[2]
 
 

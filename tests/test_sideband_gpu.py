@@ -140,6 +140,28 @@ def test_codes_do_not_outlive_a_write(F, small_threshold, name):
     F.check_device_status()
 
 
+def test_codes_outlive_a_read_on_another_stream(F, small_threshold):
+    """The caller records the tensor on the stream that reads it; its codes, which the caller does not see, follow."""
+    d = 2.0 ** -4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, w = (torch.randn(*s, device="cuda", generator=g) for s in ((8, 64, 16, 16), (64, 64, 3, 3)))
+    wb = torch.empty_like(w)
+    conv = lambda t: F.binary_connect_convolution(t, w, wb, None, 1, (1, 1), fixed_point_delta=d)
+    want = conv(F.fixed_point_quantize(x, True, 8, d))
+    q = F.fixed_point_quantize(x, True, 8, d, codes_sideband=True)
+    shape = F._sideband_get(q, d).shape
+    torch.cuda.synchronize()
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(100_000_000)  # some 50 ms: the read comes after what follows
+        got = conv(q)
+    q.record_stream(other)
+    del q
+    filled = [torch.full(shape, 77, dtype=torch.int8, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and all(bool((t == 77).all()) for t in filled)
+
+
 def test_resnet18_as_written_with_the_codes_sideband(F, small_threshold):
     from nnabla_b200 import resnet18
     rng = np.random.RandomState(2)
