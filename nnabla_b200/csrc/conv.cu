@@ -745,8 +745,10 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   NB_TRY(device_status_word(&status));
   NB_CUDA(launch_dependent(kernel, dim3(grid_w), dim3(kGemmThreads), smem_w, st, mx, md, q, status));
   NB_LAUNCH_CHECK();
+  const ConvWgradOperands operands{x,    dy,   g.N,  g.C,  g.H,  g.W,  g.Ko, g.Ho,
+                                   g.Wo, g.kw, g.sh, g.sw, g.ph, g.pw, g.dh, g.dw};
   NB_CUDA(launch_dependent(conv_wgrad_finish_kernel, dim3(q.tasks(), g.Cg < 64 ? g.Cg : 64), dim3(64 * q.task_taps), 0, st, q,
-                           g.Kog, g.Cg, taps, dw, accum_dw));
+                           operands, g.Kog, g.Cg, taps, dw, accum_dw));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

@@ -361,11 +361,39 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
 }
 
+// What the sums were made of, as the caller holds it.
+struct ConvWgradOperands {
+  const float *x, *dy;
+  int N, C, H, W, Ko, Ho, Wo, kw, sh, sw, ph, pw, dh, dw;
+};
+
+// One element of dW from the fp32 operands, by the lanes of a warp. Pixels outside the image count as zeros, like in the
+// reference's unfolded patches.
+__device__ __forceinline__ float conv_wgrad_element(const ConvWgradOperands &G, int o, int c, int tap) {
+  const int ky = tap / G.kw, kx = tap - ky * G.kw, plane = G.Ho * G.Wo;
+  float s = 0.0f;
+  for (int64_t i = threadIdx.x & 31; i < (int64_t)G.N * plane; i += 32) {
+    const int n = (int)(i / plane), p = (int)(i - (int64_t)n * plane), oy = p / G.Wo;
+    const int iy = oy * G.sh - G.ph + ky * G.dh, ix = (p - oy * G.Wo) * G.sw - G.pw + kx * G.dw;
+    const bool in = iy >= 0 && iy < G.H && ix >= 0 && ix < G.W;
+    const float xv = in ? __ldg(G.x + (((int64_t)n * G.C + c) * G.H + iy) * G.W + ix) : 0.0f;
+    s = __fmaf_rn(__ldg(G.dy + ((int64_t)n * G.Ko + o) * plane + p), xv, s);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, d);
+  return s;
+}
+
 // dW[o][c][tap] (+)= the slots of a task in block order; one thread block per (task, channel), the maps of a slot are
 // contiguous. Only the first and the last slot can be missing (per_block >= 2 pairs).
-__global__ void __launch_bounds__(64 * kWgradTaps) conv_wgrad_finish_kernel(const __grid_constant__ ConvWgradProblem prob, int Kog,
-                                                                int Cg, int taps, float *__restrict__ dw,
-                                                                int accumulate) {
+//
+// Sums that are not finite are made again from the operands: the padded columns pair zeros of dy with pixels of x that the
+// tap does not reach there, and a NaN or an infinity of x would spread to taps that have no output pixel with it (and an
+// infinity of either operand to a NaN, through its pieces).
+__global__ void __launch_bounds__(64 * kWgradTaps, 5)
+    conv_wgrad_finish_kernel(const __grid_constant__ ConvWgradProblem prob, const __grid_constant__ ConvWgradOperands G,
+                             int Kog, int Cg, int taps, float *__restrict__ dw, int accumulate) {
   pdl_wait();
   pdl_trigger();
   const int task = blockIdx.x;
@@ -376,31 +404,43 @@ __global__ void __launch_bounds__(64 * kWgradTaps) conv_wgrad_finish_kernel(cons
   const int ob = r % prob.o_blocks, g = r / prob.o_blocks;
   const int t0 = prob.tg_tap[tg], n_taps = prob.tg_tap[tg + 1] - t0;
   const int o = ob * 64 + (threadIdx.x & 63), c = cb * 64 + blockIdx.y, t = threadIdx.x >> 6;
-  if (t >= n_taps || c >= Cg || o >= Kog)
+  if (t >= n_taps || c >= Cg) // (whole warps: a warp's threads have one tap, and maps in a row)
     return;
-  int pairs, b0, b1;
-  const int begin = prob.task_begin(task, pairs);
-  int first = begin / prob.per_block, last = (begin + prob.boxes * pairs - 1) / prob.per_block;
-  prob.share(first, begin, pairs, b0, b1);
-  first += b0 < b1 ? 0 : 1;
-  prob.share(last, begin, pairs, b0, b1);
-  last -= b0 < b1 ? 0 : 1;
-  const float *src = prob.slots + (int64_t)(first + task) * prob.slot_floats() + (t * 64 + blockIdx.y) * 64 + (threadIdx.x & 63);
+  const bool live = o < Kog;
   float s = 0.0f;
-  int b = first;
-  for (; b + 8 <= last + 1; b += 8, src += (int64_t)8 * prob.slot_floats()) {
-    float v[8];
+  if (live) {
+    int pairs, b0, b1;
+    const int begin = prob.task_begin(task, pairs);
+    int first = begin / prob.per_block, last = (begin + prob.boxes * pairs - 1) / prob.per_block;
+    prob.share(first, begin, pairs, b0, b1);
+    first += b0 < b1 ? 0 : 1;
+    prob.share(last, begin, pairs, b0, b1);
+    last -= b0 < b1 ? 0 : 1;
+    const float *src =
+        prob.slots + (int64_t)(first + task) * prob.slot_floats() + (t * 64 + blockIdx.y) * 64 + (threadIdx.x & 63);
+    int b = first;
+    for (; b + 8 <= last + 1; b += 8, src += (int64_t)8 * prob.slot_floats()) {
+      float v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      v[u] = __ldcs(src + (int64_t)u * prob.slot_floats());
+      for (int u = 0; u < 8; ++u)
+        v[u] = __ldcs(src + (int64_t)u * prob.slot_floats());
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      s = __fadd_rn(s, v[u]);
+      for (int u = 0; u < 8; ++u)
+        s = __fadd_rn(s, v[u]);
+    }
+    for (; b <= last; ++b, src += prob.slot_floats())
+      s = __fadd_rn(s, __ldcs(src));
   }
-  for (; b <= last; ++b, src += prob.slot_floats())
-    s = __fadd_rn(s, __ldcs(src));
-  float *dst = dw + ((int64_t)(g * Kog + o) * Cg + c) * taps + prob.tap_id[t0 + t];
-  *dst = accumulate ? __fadd_rn(*dst, s) : s;
+  const int tap = prob.tap_id[t0 + t], lane = threadIdx.x & 31;
+  for (uint32_t again = __ballot_sync(0xffffffffu, !(fabsf(s) < __int_as_float(0x7f800000))); again; again &= again - 1) {
+    const int l = __ffs(again) - 1;
+    const float v = conv_wgrad_element(G, g * Kog + o - lane + l, g * Cg + c, tap);
+    s = lane == l ? v : s;
+  }
+  if (live) {
+    float *dst = dw + ((int64_t)(g * Kog + o) * Cg + c) * taps + tap;
+    *dst = accumulate ? __fadd_rn(*dst, s) : s;
+  }
 }
 
 } // namespace nb200

@@ -119,3 +119,35 @@ def test_small_images_share_tiles(n, c, h, w, o, k, pad, stride, group, blocks, 
     assert torch.equal(gradient(accum=(True, False, False), grads=(old.clone(), None, None)), old + dx)
     F.check_device_status()
     assert _blocks(lambda: forward(b)) == [blocks] and _blocks(gradient) == [blocks_dx]
+
+
+@pytest.mark.parametrize("n,c,h,w,o,k,pad,stride,dil,group", CASES[:6] + CASES[7:8])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_weight_gradient_of_values_that_are_not_finite(n, c, h, w, o, k, pad, stride, dil, group, bad):
+    """A value of x that is not finite reaches the taps that pair it with an output pixel, and no others."""
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(n + c)
+    x = torch.randn(n, c, h, w, device="cuda", generator=g)
+    x[0, 0, 0, 0] = x[-1, c - 1, h - 1, w - 1] = x[0, c // 2, h // 2, w - 1] = bad
+    wb = torch.randn(o, c // group, k, k, device="cuda", generator=g).sign()
+    geometry = dict(pad=(pad, pad), stride=(stride, stride), dilation=(dil, dil), group=group)
+    dy = torch.randn_like(F.binary_connect_convolution(x, wb, torch.empty_like(wb), **geometry))
+    gradient = lambda **kw: F.binary_connect_convolution_backward(x, wb, dy, propagate_down=(False, True, False),
+                                                                  **geometry, **kw)[1]
+    # the taps one by one: the pixels of x that each pairs with dy, zeros outside the image
+    xp = torch.nn.functional.pad(x.double(), (pad,) * 4)
+    want = torch.empty(o, c // group, k, k, dtype=torch.float64, device="cuda")
+    for ky in range(k):
+        for kx in range(k):
+            part = xp[:, :, ky * dil:ky * dil + (dy.shape[2] - 1) * stride + 1:stride,
+                      kx * dil:kx * dil + (dy.shape[3] - 1) * stride + 1:stride]
+            for i in range(group):
+                a = dy.double().chunk(group, 1)[i].transpose(0, 1).flatten(1)
+                b = part.chunk(group, 1)[i].transpose(0, 1).flatten(1)
+                want.chunk(group, 0)[i][:, :, ky, kx] = a @ b.t()
+    got = gradient()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf())
+    finite = want.isfinite()
+    assert (got.double() - want)[finite].norm() <= 1e-5 * want[finite].norm() and not finite.all() and finite.any()
+    assert torch.equal(gradient(accum=(False, True, False), grads=(None, torch.ones_like(wb), None)).isnan(), want.isnan())
+    F.check_device_status()
