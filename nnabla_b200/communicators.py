@@ -21,6 +21,8 @@ import os
 import torch
 import torch.distributed as dist
 
+from .functions import _wrote as wrote  # collectives move no version counter: a quantizer's codes go here
+
 
 def _as_list(data):
     return list(data) if isinstance(data, (list, tuple)) else [data]
@@ -124,6 +126,7 @@ class Communicator:
         for a in arrays:
             if not a.is_contiguous():
                 raise RuntimeError("arrays must be contiguous")
+        wrote(*arrays)
         if inplace or len(arrays) == 1:
             for a in arrays:
                 fn(a)
@@ -174,6 +177,7 @@ class Communicator:
             return
         if len(ndarray_list) != len(ranks):
             raise RuntimeError("ndarray_list needs one array per rank of the group")
+        wrote(*ndarray_list)
         dist.all_gather(list(ndarray_list), ndarray, group=pg)
 
     def reduce_scatter(self, ndarray_list, ndarray, division=False, group="world"):
@@ -184,6 +188,7 @@ class Communicator:
             return
         if len(ndarray_list) != len(ranks):
             raise RuntimeError("ndarray_list needs one array per rank of the group")
+        wrote(ndarray)
         if dist.get_backend(pg) == "gloo":  # gloo has no reduce_scatter: reduce every piece to its owner
             for pos, r in enumerate(ranks):
                 piece = ndarray_list[pos].clone()

@@ -88,8 +88,8 @@ def fixed_point_quantize(x, sign=True, n=8, delta=2 ** -4, quantize=True, ste_fi
     writes the result's int8 channel-last codes and keeps them with the returned tensor; a binary-weight
     convolution called on that tensor with fixed_point_delta=delta then reads the codes. The result is the
     same, bit for bit. The codes are dropped when the tensor is modified through torch, or when a function of this
-    module writes into its memory (outputs=, inplace=, a gradient buffer); do not write into it any other way, such as
-    through .data, which torch does not count.
+    module or a collective of the communicator writes into its memory (outputs=, inplace=, a gradient buffer); do not
+    write into it any other way, such as through .data or torch.distributed, which torch's version counter does not show.
     """
     if not quantize:
         return x

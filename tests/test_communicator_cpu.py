@@ -79,6 +79,39 @@ def test_communicator_two_ranks():
         assert all(results[r].values()), (r, {k: v for k, v in results[r].items() if not v})
 
 
+def _codes_worker(rank, world, port, results):
+    """Which collectives leave a quantizer's codes with an array that they write into."""
+    import weakref
+    sys.path.insert(0, ROOT)
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), RANK=str(rank), WORLD_SIZE=str(world),
+                      LOCAL_RANK=str(rank))
+    from nnabla_b200 import communicators as C
+    from nnabla_b200 import functions as F
+    comm = C.MultiProcessDataParallelCommunicator()
+    comm.init("gloo")
+    calls = {"all_reduce": lambda t, o: comm.all_reduce(t), "reduce": lambda t, o: comm.reduce(t, 0),
+             "bcast": lambda t, o: comm.bcast(t, 0), "packed": lambda t, o: comm.all_reduce([t, o]),
+             "all_gather": lambda t, o: comm.all_gather(o, [t]),
+             "reduce_scatter": lambda t, o: comm.reduce_scatter([o], t),
+             "callback": lambda t, o: comm.all_reduce_callback([t, o], 3)()}
+    stale = []
+    for name, call in calls.items():
+        t, other = torch.ones(4), torch.zeros(4)
+        entry = (weakref.ref(t), t._version, None, 1.0, F._memory(t), None)
+        F._sideband[id(t)] = entry
+        call(t, other)
+        if F._sideband.pop(id(t), None) is not None and t._version == entry[1]:
+            stale.append(name)
+    results[rank] = stale
+    dist.destroy_process_group()
+
+
+def test_collectives_drop_the_codes_of_what_they_write():
+    results = mp.Manager().dict()
+    mp.spawn(_codes_worker, args=(1, 29950 + os.getpid() % 40, results), nprocs=1, join=True)
+    assert results[0] == []
+
+
 def test_single_process_communicator_is_not_provided():
     sys.path.insert(0, ROOT)
     from nnabla_b200 import communicators as C
