@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kThreads) bn_inference_kernel(const float *__r
       r.y = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v.y, m), g), sd), b);
       r.z = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v.z, m), g), sd), b);
       r.w = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v.w, m), g), sd), b);
-      __stcs(reinterpret_cast<float4 *>(y) + i, r);
+      st_result(reinterpret_cast<float4 *>(y) + i, r, total * sizeof(float) <= kKeepBytes);
     }
   } else {
     const size_t first = (size_t)blockIdx.x * kThreads + threadIdx.x;
@@ -71,22 +71,24 @@ __global__ void __launch_bounds__(kThreads) bn_inference_kernel(const float *__r
 
 // The same for planes of at least a few hundred float4: one block per (plane, chunk of the plane), so the
 // channel's four parameters and the square root are taken once per thread and the loop is loads, four
-// rounded operations per value and stores. blockIdx.x = plane (n * C + c), blockIdx.y = chunk.
+// rounded operations per value and stores. Blocks count the chunks of one plane (n * C + c) after the other, the tensor's
+// last first (st_result): with the chunks outermost a pass would go through the tensor once per chunk.
 __global__ void __launch_bounds__(kThreads) bn_inference_plane_kernel(const float *__restrict__ x, const float *beta,
                                                                       const float *gamma, const float *mean,
-                                                                      const float *var, int C, int S4, float eps,
-                                                                      float *__restrict__ y) {
+                                                                      const float *var, int C, int S4, unsigned chunks,
+                                                                      float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned plane = blockIdx.x;
+  const unsigned block = gridDim.x - 1 - blockIdx.x, plane = block / chunks;
+  const bool keep = (size_t)(gridDim.x / chunks) * S4 * sizeof(float4) <= kKeepBytes;
   const int c = (int)(plane % (unsigned)C);
   const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)plane * S4;
   float4 *yp = reinterpret_cast<float4 *>(y) + (size_t)plane * S4;
   // the data loads go out first: they do not depend on the channel's constants, whose own loads, square
   // root and reciprocal would otherwise stand in front of them in every (short) block
   constexpr int kPer = 4;
-  const int step = gridDim.y * kThreads;
-  int i = blockIdx.y * kThreads + threadIdx.x;
+  const int step = chunks * kThreads;
+  int i = (block - plane * chunks) * kThreads + threadIdx.x;
   float4 v[kPer];
 #pragma unroll
   for (int u = 0; u < kPer; ++u)
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(kThreads) bn_inference_plane_kernel(const floa
 #pragma unroll
   for (int u = 0; u < kPer; ++u)
     if (i + u * step < S4)
-      __stcs(yp + i + u * step, one(v[u]));
+      st_result(yp + i + u * step, one(v[u]), keep);
   for (i += kPer * step; i < S4; i += step)
-    __stcs(yp + i, one(__ldcs(xp + i)));
+    st_result(yp + i, one(__ldcs(xp + i)), keep);
 }
 
 // Planes of 32 to 1023 values (the later stages of a network: 28 x 28, 14 x 14, 7 x 7): one WARP per plane,
@@ -123,9 +125,10 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float
                                                                      float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned plane = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  const unsigned plane = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
   if (plane >= planes)
     return;
+  const bool keep = (size_t)planes * S * sizeof(float) <= kKeepBytes;
   const int lane = threadIdx.x & 31;
   const int c = (int)(plane % (unsigned)C);
   constexpr int kPer = kVec ? 7 : 4; // a 28 x 28 plane is 196 float4: seven per lane, all in flight at once
@@ -153,9 +156,9 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
       if (lane + 32 * u < S4)
-        __stcs(yp + lane + 32 * u, one(v[u]));
+        st_result(yp + lane + 32 * u, one(v[u]), keep);
     for (int i = lane + 32 * kPer; i < S4; i += 32)
-      __stcs(yp + i, one(__ldcs(xp + i)));
+      st_result(yp + i, one(__ldcs(xp + i)), keep);
   } else {
     const float *xp = x + (size_t)plane * S;
     float *yp = y + (size_t)plane * S;
@@ -171,9 +174,9 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
       if (lane + 32 * u < S)
-        __stcs(yp + lane + 32 * u, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v[u], m), g), sd), b));
+        st_result(yp + lane + 32 * u, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v[u], m), g), sd), b), keep);
     for (int i = lane + 32 * kPer; i < S; i += 32)
-      __stcs(yp + i, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(__ldcs(xp + i), m), g), sd), b));
+      st_result(yp + i, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(__ldcs(xp + i), m), g), sd), b), keep);
   }
 }
 
@@ -187,9 +190,10 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const floa
                                                                       float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned group = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  const unsigned group = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
   if (group >= groups)
     return;
+  const bool keep = (size_t)groups * S * sizeof(float4) <= kKeepBytes;
   const int lane = threadIdx.x & 31;
   const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)group * S;
   float4 *yp = reinterpret_cast<float4 *>(y) + (size_t)group * S;
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const floa
       const int j = lane + 32 * u;
       const float4 r = one(j < S ? j : 0, j < S ? v[u] : make_float4(0.f, 0.f, 0.f, 0.f));
       if (j < S)
-        __stcs(yp + j, r);
+        st_result(yp + j, r, keep);
     }
   }
   for (int u = kPer; u < rounds; ++u) {
@@ -234,43 +238,63 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const floa
     const float4 a = j < S ? __ldcs(xp + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 r = one(j < S ? j : 0, a);
     if (j < S)
-      __stcs(yp + j, r);
+      st_result(yp + j, r, keep);
   }
 }
 
 // ReLU (src/nbla/function/generic/relu.cpp): y = max(0, x); Add2 (add2.cpp): y = a + b.
-template <int kOp, bool kVec>
+// A block takes kThreads * kPer consecutive values (vectors with kVec), upwards; the last block's first threads the
+// remainder of a vector.
+template <int kOp, bool kVec, int kPer>
 __global__ void __launch_bounds__(kThreads) unary_binary_kernel(const float *__restrict__ a,
                                                                 const float *__restrict__ b, size_t total,
                                                                 float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const size_t stride = (size_t)gridDim.x * kThreads;
+  auto one = [](float v, float w) { return kOp == 0 ? (v > 0.0f ? v : 0.0f) : __fadd_rn(v, w); };
+  const size_t first = (size_t)blockIdx.x * (kThreads * kPer) + threadIdx.x;
   if (kVec) {
     const size_t total4 = total / 4;
-    for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < total4; i += stride) {
-      const float4 v = __ldcs(reinterpret_cast<const float4 *>(a) + i);
-      float4 r;
-      if (kOp == 0) {
-        r.x = v.x > 0.0f ? v.x : 0.0f;
-        r.y = v.y > 0.0f ? v.y : 0.0f;
-        r.z = v.z > 0.0f ? v.z : 0.0f;
-        r.w = v.w > 0.0f ? v.w : 0.0f;
-      } else {
-        const float4 w = __ldcs(reinterpret_cast<const float4 *>(b) + i);
-        r.x = __fadd_rn(v.x, w.x);
-        r.y = __fadd_rn(v.y, w.y);
-        r.z = __fadd_rn(v.z, w.z);
-        r.w = __fadd_rn(v.w, w.w);
+    const bool keep = total * sizeof(float) <= kKeepBytes;
+    float4 v[kPer], w[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (first + u * kThreads < total4) {
+        v[u] = ld_stream(reinterpret_cast<const float4 *>(a) + first + u * kThreads);
+        w[u] = kOp == 0 ? v[u] : ld_stream(reinterpret_cast<const float4 *>(b) + first + u * kThreads);
       }
-      __stcs(reinterpret_cast<float4 *>(y) + i, r);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (first + u * kThreads < total4)
+        st_result(reinterpret_cast<float4 *>(y) + first + u * kThreads,
+                  make_float4(one(v[u].x, w[u].x), one(v[u].y, w[u].y), one(v[u].z, w[u].z), one(v[u].w, w[u].w)), keep);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < total - total4 * 4) {
+      const size_t i = total4 * 4 + threadIdx.x;
+      y[i] = one(a[i], kOp == 0 ? 0.0f : b[i]);
     }
-    for (size_t i = total4 * 4 + (size_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += stride)
-      y[i] = (kOp == 0) ? (a[i] > 0.0f ? a[i] : 0.0f) : __fadd_rn(a[i], b[i]);
   } else {
-    for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += stride)
-      y[i] = (kOp == 0) ? (a[i] > 0.0f ? a[i] : 0.0f) : __fadd_rn(a[i], b[i]);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const size_t i = first + u * kThreads;
+      if (i < total)
+        y[i] = one(a[i], kOp == 0 ? 0.0f : b[i]);
+    }
   }
+}
+
+// Vectors (or values, unaligned) of a thread: four, or one while that leaves every SM room for all its blocks at once.
+template <int kOp> int launch_unary_binary(const float *a, const float *b, size_t size, float *y, cudaStream_t st) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(kOp == 0 ? a : b) |
+                     reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  const size_t items = vec ? size / 4 : size;
+  const bool few = items <= (size_t)sm_count() * 4 * kThreads;
+  const size_t per = (size_t)kThreads * (few ? 1 : 4);
+  const size_t blocks = items ? (items + per - 1) / per : 1;
+  auto kernel = vec ? (few ? unary_binary_kernel<kOp, true, 1> : unary_binary_kernel<kOp, true, 4>)
+                    : (few ? unary_binary_kernel<kOp, false, 1> : unary_binary_kernel<kOp, false, 4>);
+  NB_CUDA(launch_dependent(kernel, dim3((unsigned)blocks), dim3(kThreads), 0, st, a, b, size, y));
+  NB_LAUNCH_CHECK();
+  return NB200_OK;
 }
 
 // MaxPooling forward_map (src/nbla/function/generic/max_pooling.cpp:60-84):
@@ -348,7 +372,8 @@ __global__ void __launch_bounds__(kThreads) max_pooling_3x3s2_kernel(const float
       }
       first = false;
     }
-    __stcs(reinterpret_cast<float4 *>(y + (m * Ho + oy) * (size_t)Wo) + ox4, make_float4(best[0], best[1], best[2], best[3]));
+    st_result(reinterpret_cast<float4 *>(y + (m * Ho + oy) * (size_t)Wo) + ox4,
+              make_float4(best[0], best[1], best[2], best[3]), maps * Ho * Wo * sizeof(float) <= kKeepBytes);
   }
 }
 
@@ -658,13 +683,12 @@ int nb200_batch_normalization_inference_f32(const float *x, const float *beta, c
     return NB200_OK;
   NB_CHECK(x && y && mean && var, NB200_EVALUE, "null data pointer");
   const bool vec = (inner % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  if (vec && inner >= 4 * kThreads && outer * channels < (1ll << 31)) {
+  // about four float4 per thread
+  const int64_t chunks = inner >= 64ll * 16 * kThreads ? 64 : (inner / 4 + 4 * kThreads - 1) / (4 * kThreads);
+  if (vec && inner >= 4 * kThreads && outer * channels * chunks < (1ll << 31)) {
     const int S4 = (int)(inner / 4);
-    int chunks = (S4 + 4 * kThreads - 1) / (4 * kThreads); // about four float4 per thread
-    chunks = chunks > 64 ? 64 : chunks;
-    NB_CUDA(launch_dependent(bn_inference_plane_kernel, dim3((unsigned)(outer * channels), (unsigned)chunks),
-                             dim3(kThreads), 0, as_stream(stream), x, beta, gamma, mean, var, (int)channels, S4, eps,
-                             y));
+    NB_CUDA(launch_dependent(bn_inference_plane_kernel, dim3((unsigned)(outer * channels * chunks)), dim3(kThreads), 0,
+                             as_stream(stream), x, beta, gamma, mean, var, (int)channels, S4, (unsigned)chunks, eps, y));
   } else if (inner >= 32 && inner < 4 * kThreads && outer * channels < (1ll << 31)) {
     const unsigned planes = (unsigned)(outer * channels);
     const dim3 grid((planes + kThreads / 32 - 1) / (kThreads / 32));
@@ -693,15 +717,7 @@ int nb200_relu_f32(const float *x, float *y, size_t size, void *stream) {
   if (size == 0)
     return NB200_OK;
   NB_CHECK(x && y, NB200_EVALUE, "null data pointer");
-  const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  const float *none = nullptr;
-  if (vec)
-    NB_CUDA(launch_dependent(unary_binary_kernel<0, true>, dim3(grid_for(size / 4 + 1, 2)), dim3(kThreads), 0,
-                             as_stream(stream), x, none, size, y));
-  else
-    NB_CUDA(launch_dependent(unary_binary_kernel<0, false>, dim3(grid_for(size, 4)), dim3(kThreads), 0,
-                             as_stream(stream), x, none, size, y));
-  return NB200_OK;
+  return launch_unary_binary<0>(x, nullptr, size, y, as_stream(stream));
 }
 
 namespace nb200 {
@@ -727,15 +743,7 @@ int nb200_add2_f32(const float *a, const float *b, float *y, size_t size, void *
   if (size == 0)
     return NB200_OK;
   NB_CHECK(a && b && y, NB200_EVALUE, "null data pointer");
-  const bool vec =
-      ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  if (vec)
-    NB_CUDA(launch_dependent(unary_binary_kernel<1, true>, dim3(grid_for(size / 4 + 1, 2)), dim3(kThreads), 0,
-                             as_stream(stream), a, b, size, y));
-  else
-    NB_CUDA(launch_dependent(unary_binary_kernel<1, false>, dim3(grid_for(size, 4)), dim3(kThreads), 0,
-                             as_stream(stream), a, b, size, y));
-  return NB200_OK;
+  return launch_unary_binary<1>(a, b, size, y, as_stream(stream));
 }
 
 int nb200_max_pooling_f32(const float *x, float *y, int64_t maps, int height, int width, int kernel_h, int kernel_w,

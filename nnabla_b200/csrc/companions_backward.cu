@@ -29,30 +29,63 @@ inline unsigned grid_for(size_t items, int per_thread = 1) {
 // ---------------------------------------------------------------- elementwise backward passes
 
 // relu.cpp:41-49: dx (+)= y > 0 ? dy : 0; add2.cpp: dx (+)= dy.
-template <int kOp, bool kAccum>
+// A block takes kThreads * kPer consecutive vectors (values where a tensor is not 16-byte aligned), the last block's first
+// (st_result); block 0 the remainder of a vector.
+template <int kOp, bool kAccum, bool kVec, int kPer>
 __global__ void __launch_bounds__(kThreads) grad_pass_kernel(const float *__restrict__ y, const float *__restrict__ dy,
-                                                             float *__restrict__ dx, size_t total, bool vec) {
+                                                             float *__restrict__ dx, size_t total) {
   pdl_wait();
   pdl_trigger();
-  const size_t stride = (size_t)gridDim.x * kThreads;
-  const size_t first = (size_t)blockIdx.x * kThreads + threadIdx.x;
   auto one = [](float yv, float g, float old) {
     const float v = kOp == 0 ? (yv > 0.0f ? g : 0.0f) : g;
     return kAccum ? __fadd_rn(old, v) : v;
   };
-  const size_t total4 = vec ? total / 4 : 0;
-  for (size_t i = first; i < total4; i += stride) {
-    const float4 g = __ldcs(reinterpret_cast<const float4 *>(dy) + i);
-    float4 yv = make_float4(0, 0, 0, 0), o = make_float4(0, 0, 0, 0);
-    if (kOp == 0)
-      yv = __ldcs(reinterpret_cast<const float4 *>(y) + i);
-    if (kAccum)
-      o = reinterpret_cast<const float4 *>(dx)[i];
-    reinterpret_cast<float4 *>(dx)[i] = make_float4(one(yv.x, g.x, o.x), one(yv.y, g.y, o.y), one(yv.z, g.z, o.z),
-                                                    one(yv.w, g.w, o.w));
+  const size_t first = block_descending() * (kThreads * kPer) + threadIdx.x;
+  const size_t total4 = kVec ? total / 4 : 0;
+  if (kVec) {
+    const bool keep = total * sizeof(float) <= kKeepBytes;
+    float4 g[kPer], yv[kPer], o[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (first + u * kThreads < total4) {
+        g[u] = ld_stream(reinterpret_cast<const float4 *>(dy) + first + u * kThreads);
+        yv[u] = kOp == 0 ? ld_stream(reinterpret_cast<const float4 *>(y) + first + u * kThreads) : g[u];
+        o[u] = kAccum ? reinterpret_cast<const float4 *>(dx)[first + u * kThreads] : g[u];
+      }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (first + u * kThreads < total4)
+        st_result(reinterpret_cast<float4 *>(dx) + first + u * kThreads,
+                  make_float4(one(yv[u].x, g[u].x, o[u].x), one(yv[u].y, g[u].y, o[u].y), one(yv[u].z, g[u].z, o[u].z),
+                              one(yv[u].w, g[u].w, o[u].w)),
+                  keep);
+    if (blockIdx.x == 0 && threadIdx.x < total - total4 * 4) {
+      const size_t i = total4 * 4 + threadIdx.x;
+      dx[i] = one(kOp == 0 ? y[i] : 0.0f, dy[i], kAccum ? dx[i] : 0.0f);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const size_t i = first + u * kThreads;
+      if (i < total)
+        dx[i] = one(kOp == 0 ? y[i] : 0.0f, dy[i], kAccum ? dx[i] : 0.0f);
+    }
   }
-  for (size_t i = total4 * 4 + first; i < total; i += stride)
-    dx[i] = one(kOp == 0 ? y[i] : 0.0f, dy[i], kAccum ? dx[i] : 0.0f);
+}
+
+// Vectors (or values, unaligned) of a thread: four, or one while that leaves every SM room for all its blocks at once.
+template <int kOp, bool kAccum>
+int launch_grad_pass(const float *y, const float *dy, float *dx, size_t size, cudaStream_t st) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(kOp == 0 ? y : dy) | reinterpret_cast<uintptr_t>(dy) |
+                     reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
+  const size_t items = vec ? size / 4 : size;
+  const bool few = items <= (size_t)sm_count() * 4 * kThreads;
+  const size_t per = (size_t)kThreads * (few ? 1 : 4);
+  const size_t blocks = items ? (items + per - 1) / per : 1;
+  auto kernel = vec ? (few ? grad_pass_kernel<kOp, kAccum, true, 1> : grad_pass_kernel<kOp, kAccum, true, 4>)
+                    : (few ? grad_pass_kernel<kOp, kAccum, false, 1> : grad_pass_kernel<kOp, kAccum, false, 4>);
+  NB_CUDA(launch_dependent(kernel, dim3((unsigned)blocks), dim3(kThreads), 0, st, y, dy, dx, size));
+  return NB200_OK;
 }
 
 // global_average_pooling.cpp:75-117: every pixel of map m receives dy[m] / (H W).
@@ -385,9 +418,10 @@ __global__ void __launch_bounds__(kThreads)
                                 unsigned C, int S4, unsigned runs, size_t total_runs, float *__restrict__ dx) {
   pdl_wait();
   pdl_trigger();
-  const size_t run = (size_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  const size_t run = block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
   if (run >= total_runs)
     return;
+  const bool keep = total_runs / runs * S4 * sizeof(float4) <= kKeepBytes;
   const size_t plane = run / runs;
   const int c = (int)(plane % C), i0 = (int)(run - plane * runs) * (32 * kRun) + (int)(threadIdx.x & 31);
   const float4 *xp = reinterpret_cast<const float4 *>(x) + plane * S4;
@@ -424,7 +458,8 @@ __global__ void __launch_bounds__(kThreads)
     const int i = i0 + 32 * u;
     if (i < S4) {
       const float4 a = kBatch ? xv[u] : make_float4(0, 0, 0, 0), b = kAccum ? o[u] : make_float4(0, 0, 0, 0);
-      op[i] = make_float4(one(a.x, g[u].x, b.x), one(a.y, g[u].y, b.y), one(a.z, g[u].z, b.z), one(a.w, g[u].w, b.w));
+      st_result(op + i, make_float4(one(a.x, g[u].x, b.x), one(a.y, g[u].y, b.y), one(a.z, g[u].z, b.z),
+                                    one(a.w, g[u].w, b.w)), keep);
     }
   }
 }
@@ -545,25 +580,16 @@ int nb200_relu_backward_f32(const float *y, const float *dy, float *dx, size_t s
   if (size == 0)
     return NB200_OK;
   NB_CHECK(y && dy && dx, NB200_EVALUE, "null data pointer");
-  const bool vec =
-      ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
-  const unsigned grid = grid_for(size / 4 + 1, 2);
-  NB_CUDA(launch_dependent(accum ? grad_pass_kernel<0, true> : grad_pass_kernel<0, false>, dim3(grid), dim3(kThreads),
-                           0,
-                           as_stream(stream), y, dy, dx, size, vec));
-  return NB200_OK;
+  return accum ? launch_grad_pass<0, true>(y, dy, dx, size, as_stream(stream))
+               : launch_grad_pass<0, false>(y, dy, dx, size, as_stream(stream));
 }
 
 int nb200_add2_backward_f32(const float *dy, float *dx, size_t size, int accum, void *stream) {
   if (size == 0)
     return NB200_OK;
   NB_CHECK(dy && dx, NB200_EVALUE, "null data pointer");
-  const bool vec = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
-  const unsigned grid = grid_for(size / 4 + 1, 2);
-  NB_CUDA(launch_dependent(accum ? grad_pass_kernel<1, true> : grad_pass_kernel<1, false>, dim3(grid), dim3(kThreads),
-                           0,
-                           as_stream(stream), (const float *)nullptr, dy, dx, size, vec));
-  return NB200_OK;
+  return accum ? launch_grad_pass<1, true>(nullptr, dy, dx, size, as_stream(stream))
+               : launch_grad_pass<1, false>(nullptr, dy, dx, size, as_stream(stream));
 }
 
 int nb200_global_average_pooling_backward_f32(const float *dy, float *dx, int64_t maps, int64_t spatial, int accum,

@@ -31,39 +31,39 @@ constexpr int kUnroll = 4;
 // ops with an int8 side-band store their four codes as one 32-bit word.
 template <typename Op>
 __device__ __forceinline__ void apply4(const Op &op, const typename Op::State &st, const float4 v, const size_t e,
-                                       float4 *dst) {
+                                       float4 *dst, bool keep) {
   float4 r;
   float k0, k1, k2, k3;
   r.x = op(v.x, e, k0, st);
   r.y = op(v.y, e + 1, k1, st);
   r.z = op(v.z, e + 2, k2, st);
   r.w = op(v.w, e + 3, k3, st);
-  st_stream(dst, r);
+  st_result(dst, r, keep);
   if (Op::kHasCodes)
     op.store_codes4(e, k0, k1, k2, k3);
 }
 
-template <typename Op>
+// A block takes kThreads * kPer consecutive groups, the last block's first (block_descending): with a grid-stride walk of
+// capped grids every group of a thread lies a whole grid away, and the pass has no direction that the next could follow.
+template <typename Op, int kPer>
 __global__ void __launch_bounds__(kThreads) ew_vec_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                           size_t size, size_t head, size_t n4, Op op) {
   pdl_wait();
   pdl_trigger();
   const float4 *x4 = reinterpret_cast<const float4 *>(x + head);
   float4 *y4 = reinterpret_cast<float4 *>(y + head);
-  const size_t stride = (size_t)gridDim.x * kThreads;
-  size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
+  const size_t i = block_descending() * (kThreads * kPer) + threadIdx.x;
+  const bool keep = size * sizeof(float) <= kKeepBytes;
+  float4 v[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (i + u * kThreads < n4)
+      v[u] = ld_stream(x4 + i + u * kThreads);
   const typename Op::State st = op.init(); // per-thread constants, loaded once
-  for (; i + (kUnroll - 1) * stride < n4; i += kUnroll * stride) {
-    float4 v[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
-      v[u] = ld_stream(x4 + i + u * stride);
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
-      apply4(op, st, v[u], head + 4 * (i + u * stride), y4 + i + u * stride);
-  }
-  for (; i < n4; i += stride)
-    apply4(op, st, ld_stream(x4 + i), head + 4 * i, y4 + i);
+  for (int u = 0; u < kPer; ++u)
+    if (i + u * kThreads < n4)
+      apply4(op, st, v[u], head + 4 * (i + u * kThreads), y4 + i + u * kThreads, keep);
   if (blockIdx.x == 0) {
     const size_t tail_begin = head + 4 * n4;
     const size_t n_edge = head + (size - tail_begin);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kThreads) ew_scalar_kernel(const float *__rest
 
 inline unsigned grid_for(size_t work_items) {
   size_t blocks = (work_items + kThreads - 1) / kThreads;
-  // NNABLA_B200_EW_BLOCKS_PER_SM overrides the grid size per SM (tuning aid).
+  // NNABLA_B200_EW_BLOCKS_PER_SM overrides the grid size per SM of the grid-stride kernels (tuning aid).
   static const int per_sm = []() {
     const char *e = std::getenv("NNABLA_B200_EW_BLOCKS_PER_SM");
     const int v = e ? std::atoi(e) : 0;
@@ -109,10 +109,12 @@ inline unsigned grid_for(size_t work_items) {
   return (unsigned)blocks;
 }
 
-// For the kernels that take kUnroll float4 per thread and round: one per thread as long as that leaves every SM room for
-// all its blocks at once, so that small tensors spread over the chip.
-inline unsigned grid_for_quads(size_t n4) {
-  return n4 <= (size_t)sm_count() * 4 * kThreads ? grid_for(n4) : grid_for((n4 + kUnroll - 1) / kUnroll);
+// The vector kernels take kUnroll groups per thread, or one while the tensor is so small that every SM has room for all
+// its blocks at once, so that small tensors spread over the chip.
+inline bool few_quads(size_t n4) { return n4 <= (size_t)sm_count() * 4 * kThreads; }
+inline unsigned blocks_for(size_t n4, int per_thread) {
+  const size_t blocks = (n4 + (size_t)kThreads * per_thread - 1) / ((size_t)kThreads * per_thread);
+  return (unsigned)(blocks < 1 ? 1 : blocks);
 }
 
 template <typename Op> int launch_elementwise(const float *x, float *y, size_t size, Op op, cudaStream_t st) {
@@ -131,7 +133,12 @@ template <typename Op> int launch_elementwise(const float *x, float *y, size_t s
     return NB200_OK;
   }
   const size_t n4 = (size - head) / 4;
-  NB_CUDA(launch_dependent(ew_vec_kernel<Op>, dim3(grid_for_quads(n4)), dim3(kThreads), 0, st, x, y, size, head, n4, op));
+  if (few_quads(n4))
+    NB_CUDA(launch_dependent(ew_vec_kernel<Op, 1>, dim3(blocks_for(n4, 1)), dim3(kThreads), 0, st, x, y, size, head, n4,
+                             op));
+  else
+    NB_CUDA(launch_dependent(ew_vec_kernel<Op, kUnroll>, dim3(blocks_for(n4, kUnroll)), dim3(kThreads), 0, st, x, y, size,
+                             head, n4, op));
   return NB200_OK;
 }
 
@@ -233,8 +240,9 @@ __global__ void __launch_bounds__(256)
   pdl_wait();
   pdl_trigger();
   __shared__ uint32_t tile[64][17];
-  const int n = blockIdx.z;
+  const int n = (int)(gridDim.z - 1 - blockIdx.z); // down, as the other quantizers
   const int p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
+  const bool keep = (size_t)gridDim.z * C * HW * sizeof(float) <= kKeepBytes;
   const int px4 = threadIdx.x & 15, chq = threadIdx.x >> 4;
   const int p = p0 + 4 * px4;
   const int c0 = d0 + 4 * chq;
@@ -251,7 +259,7 @@ __global__ void __launch_bounds__(256)
       q.y = op(v.y, 0, k1, st);
       q.z = op(v.z, 0, k2, st);
       q.w = op(v.w, 0, k3, st);
-      st_stream(reinterpret_cast<float4 *>(y + off), q);
+      st_result(reinterpret_cast<float4 *>(y + off), q, keep);
     }
     // the codes are small integers: 1.5 * 2^23 + k has k's two's complement in its low mantissa bits
     f[r][0] = __float_as_uint(__fadd_rn(k0, 12582912.0f));
@@ -513,7 +521,7 @@ __global__ void __launch_bounds__(kThreads) pow2_kernel(const float *__restrict_
       r.y = pow2_snap(v[u].y, P, s_cut, s_pw);
       r.z = pow2_snap(v[u].z, P, s_cut, s_pw);
       r.w = pow2_snap(v[u].w, P, s_cut, s_pw);
-      st_stream(y4 + i + u * stride, r);
+      __stcs(y4 + i + u * stride, r);
     }
   }
   for (; i < n4; i += stride) {
@@ -523,7 +531,7 @@ __global__ void __launch_bounds__(kThreads) pow2_kernel(const float *__restrict_
     r.y = pow2_snap(v.y, P, s_cut, s_pw);
     r.z = pow2_snap(v.z, P, s_cut, s_pw);
     r.w = pow2_snap(v.w, P, s_cut, s_pw);
-    st_stream(y4 + i, r);
+    __stcs(y4 + i, r);
   }
   if (blockIdx.x == 0) {
     const size_t tail_begin = head + 4 * n4;

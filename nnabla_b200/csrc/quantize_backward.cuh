@@ -5,8 +5,8 @@
 // All three are HBM-bound: 4 B of x + 4 B of dy read and 4 B of dx written per
 // element (plus 4 B of dx read when accumulating; x is not read at all without
 // ste_fine_grained). Same access pattern as the forward kernels: 128-bit
-// streaming accesses, four independent groups in flight per thread, many
-// short CTAs per SM.
+// accesses, four independent groups in flight per thread, a short CTA per
+// 16 KB, but from the tensor's start up (the forward pass goes down).
 //
 // A gradient op provides
 //   bool operator()(float x, float dy, size_t i, float &g, const State &) const
@@ -28,7 +28,7 @@ __device__ __forceinline__ float grad_combine(const Op &op, const typename Op::S
   return pass ? g : 0.0f;
 }
 
-template <typename Op, bool kAccum>
+template <typename Op, bool kAccum, int kPer>
 __global__ void __launch_bounds__(kThreads) grad_vec_kernel(const float *__restrict__ x, const float *__restrict__ dy,
                                                             float *__restrict__ dx, size_t size, size_t n4, Op op) {
   pdl_wait();
@@ -36,41 +36,29 @@ __global__ void __launch_bounds__(kThreads) grad_vec_kernel(const float *__restr
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   const float4 *dy4 = reinterpret_cast<const float4 *>(dy);
   float4 *dx4 = reinterpret_cast<float4 *>(dx);
-  const size_t stride = (size_t)gridDim.x * kThreads;
-  size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x;
-  const typename Op::State st = op.init();
+  const size_t i = (size_t)blockIdx.x * (kThreads * kPer) + threadIdx.x;
+  const bool keep = size * sizeof(float) <= kKeepBytes;
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (; i + (kUnroll - 1) * stride < n4; i += kUnroll * stride) {
-    float4 vx[kUnroll], vg[kUnroll], vd[kUnroll];
+  float4 vx[kPer], vg[kPer], vd[kPer];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      vx[u] = Op::kNeedsX ? ld_stream(x4 + i + u * stride) : zero4;
-      vg[u] = ld_stream(dy4 + i + u * stride);
-      vd[u] = kAccum ? ld_stream(dx4 + i + u * stride) : zero4;
+  for (int u = 0; u < kPer; ++u)
+    if (i + u * kThreads < n4) {
+      vx[u] = Op::kNeedsX ? ld_stream(x4 + i + u * kThreads) : zero4;
+      vg[u] = ld_stream(dy4 + i + u * kThreads);
+      vd[u] = kAccum ? ld_stream(dx4 + i + u * kThreads) : zero4;
     }
+  const typename Op::State st = op.init();
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const size_t e = 4 * (i + u * stride);
+  for (int u = 0; u < kPer; ++u)
+    if (i + u * kThreads < n4) {
+      const size_t e = 4 * (i + u * kThreads);
       float4 r;
       r.x = grad_combine<Op, kAccum>(op, st, vx[u].x, vg[u].x, vd[u].x, e);
       r.y = grad_combine<Op, kAccum>(op, st, vx[u].y, vg[u].y, vd[u].y, e + 1);
       r.z = grad_combine<Op, kAccum>(op, st, vx[u].z, vg[u].z, vd[u].z, e + 2);
       r.w = grad_combine<Op, kAccum>(op, st, vx[u].w, vg[u].w, vd[u].w, e + 3);
-      st_stream(dx4 + i + u * stride, r);
+      st_result(dx4 + i + u * kThreads, r, keep);
     }
-  }
-  for (; i < n4; i += stride) {
-    const float4 vx = Op::kNeedsX ? ld_stream(x4 + i) : zero4;
-    const float4 vg = ld_stream(dy4 + i);
-    const float4 vd = kAccum ? ld_stream(dx4 + i) : zero4;
-    const size_t e = 4 * i;
-    float4 r;
-    r.x = grad_combine<Op, kAccum>(op, st, vx.x, vg.x, vd.x, e);
-    r.y = grad_combine<Op, kAccum>(op, st, vx.y, vg.y, vd.y, e + 1);
-    r.z = grad_combine<Op, kAccum>(op, st, vx.z, vg.z, vd.z, e + 2);
-    r.w = grad_combine<Op, kAccum>(op, st, vx.w, vg.w, vd.w, e + 3);
-    st_stream(dx4 + i, r);
-  }
   if (blockIdx.x == 0) {
     for (size_t e = 4 * n4 + threadIdx.x; e < size; e += kThreads)
       dx[e] = grad_combine<Op, kAccum>(op, st, Op::kNeedsX ? x[e] : 0.0f, dy[e], kAccum ? dx[e] : 0.0f, e);
@@ -99,8 +87,12 @@ int launch_gradient_t(const float *x, const float *dy, float *dx, size_t size, c
                              size, op));
   } else {
     const size_t n4 = size / 4;
-    NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum>, dim3(grid_for_quads(n4)), dim3(kThreads), 0,
-                             st, x, dy, dx, size, n4, op));
+    if (few_quads(n4))
+      NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum, 1>, dim3(blocks_for(n4, 1)), dim3(kThreads), 0, st, x, dy, dx,
+                               size, n4, op));
+    else
+      NB_CUDA(launch_dependent(grad_vec_kernel<Op, kAccum, kUnroll>, dim3(blocks_for(n4, kUnroll)), dim3(kThreads), 0, st,
+                               x, dy, dx, size, n4, op));
   }
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -268,6 +260,7 @@ __global__ void __launch_bounds__(kThreads) minmax_range_grad_kernel(const float
     const float4 *g4 = reinterpret_cast<const float4 *>(dy);
     float4 *d4 = reinterpret_cast<float4 *>(dx);
     const size_t n4 = per_q / 4;
+    const bool keep = per_q * sizeof(float) <= kKeepBytes;
     // gradient w.r.t. x of one element: (x >= m) * (x <= M) * dy, or dy itself
     auto gx = [&](float a, float g, float d) {
       const float v = __fmul_rn(a >= lo ? 1.0f : 0.0f, a <= hi ? 1.0f : 0.0f);
@@ -287,7 +280,7 @@ __global__ void __launch_bounds__(kThreads) minmax_range_grad_kernel(const float
         r.y = gx(a.y, g.y, d.y);
         r.z = gx(a.z, g.z, d.z);
         r.w = gx(a.w, g.w, d.w);
-        st_stream(d4 + t, r);
+        st_result(d4 + t, r, keep);
       }
     }
     if (blockIdx.x == 0)
