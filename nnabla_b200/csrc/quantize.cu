@@ -227,54 +227,82 @@ int fxp_launch(const float *x, float *y, int8_t *codes, size_t size, int sign, i
   return launch_elementwise(x, y, size, op, st);
 }
 
+// One value and its code as 12582912 + code (1.5 * 2^23, whose low mantissa byte is the code in two's complement), for a
+// step that is a power of two and codes of at most 7 bits: FxpOp's results bit for bit in 8 instructions instead of some
+// 20. The quotient's rounding half up is floor(q + 0.5), and both additions are made rounding down, so that neither can
+// carry a value just below a tie over it; limits by min and max that keep a NaN; x + 0 makes -0 the +0 that FxpOp returns
+// for it (values below zero that round to zero keep their sign, as there).
+struct FxpFastOp {
+  float maxv, delta, inv_delta;
+  int sign;
+  __device__ __forceinline__ float operator()(float x, float &code) const {
+    const float xs = __fadd_rn(x, 0.0f);
+    float a = fabsf(xs);
+    if (!sign)
+      asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(a) : "f"(xs));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(a), "f"(maxv));
+    const float m = __fadd_rd(__fmaf_rd(a, inv_delta, 0.5f), 8388608.0f);
+    const float r = __fmul_rn(__fsub_rn(m, 8388608.0f), delta);
+    const float y = sign ? __uint_as_float(__float_as_uint(r) | (__float_as_uint(xs) & 0x80000000u)) : r;
+    code = __fmaf_rn(y, inv_delta, 12582912.0f);
+    return y;
+  }
+};
+
+// The same for any step.
+struct FxpAnyOp {
+  FxpOp<false, false> op;
+  __device__ __forceinline__ float operator()(float x, float &code) const {
+    float k;
+    const float y = op(x, 0, k, {});
+    code = __fadd_rn(k, 12582912.0f);
+    return y;
+  }
+};
+
 // FixedPointQuantize of an [N, C, S] tensor that also leaves the result as int8 channel-last codes
 // [N][S][slots] (the layout the int8 convolutions read): the quantizer of a layer and the re-layout pass of
 // the convolution behind it in one pass over the activations (4 B read, 4 + 1 B written per value instead of
-// 4 + 4 and then 4 + 1). Blocks of 64 pixels x 64 channel slots; a thread quantizes four neighbouring
+// 4 + 4 and then 4 + 1). Blocks of 128 pixels x 64 channel slots; a thread quantizes four neighbouring
 // channels of four pixels, stores the fp32 results where they came from and hands the four codes of each
 // pixel to shared memory as one word; the codes leave as 64-byte runs per pixel. S % 4 == 0, 16-byte aligned.
-template <bool kPow2Delta>
-__global__ void __launch_bounds__(256)
+// Bound by HBM since FxpFastOp; before, by instruction issue: [256, 64, 56, 56] 92 -> 76 us (71 at the copy bandwidth),
+// [256, 128, 28, 28] 53 -> 43, [256, 256, 14, 14] 35 -> 25 from a cold L2. Blocks of 64 pixels and 256 threads 78, 43, 27.
+constexpr int kCodePixels = 128, kCodeThreads = 512;
+template <typename Op>
+__global__ void __launch_bounds__(kCodeThreads)
     fxp_nhwc_codes_kernel(const float *__restrict__ x, float *__restrict__ y, int8_t *__restrict__ codes, int C, int HW,
-                          int slots, FxpOp<kPow2Delta, false> op) {
+                          int slots, Op op) {
   pdl_wait();
   pdl_trigger();
-  __shared__ uint32_t tile[64][17];
+  __shared__ uint32_t tile[kCodePixels][17];
   const int n = (int)(gridDim.z - 1 - blockIdx.z); // down, as the other quantizers
-  const int p0 = blockIdx.x * 64, d0 = blockIdx.y * 64;
+  const int p0 = (int)(gridDim.x - 1 - blockIdx.x) * kCodePixels, d0 = blockIdx.y * 64;
   const bool keep = (size_t)gridDim.z * C * HW * sizeof(float) <= kKeepBytes;
-  const int px4 = threadIdx.x & 15, chq = threadIdx.x >> 4;
+  const int px4 = threadIdx.x % (kCodePixels / 4), chq = threadIdx.x / (kCodePixels / 4);
   const int p = p0 + 4 * px4;
   const int c0 = d0 + 4 * chq;
-  const typename FxpOp<kPow2Delta, false>::State st = op.init();
-  uint32_t f[4][4];
+  const size_t off = ((size_t)n * C + c0) * HW + p;
+  float4 v[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    v[r] = (c0 + r < C && p < HW) ? ld_stream(reinterpret_cast<const float4 *>(x + off + (size_t)r * HW))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+  float f[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
-    if (c0 + r < C && p < HW) {
-      const size_t off = ((size_t)n * C + (c0 + r)) * HW + p;
-      const float4 v = ld_stream(reinterpret_cast<const float4 *>(x + off));
-      float4 q;
-      q.x = op(v.x, 0, k0, st);
-      q.y = op(v.y, 0, k1, st);
-      q.z = op(v.z, 0, k2, st);
-      q.w = op(v.w, 0, k3, st);
-      st_result(reinterpret_cast<float4 *>(y + off), q, keep);
-    }
-    // the codes are small integers: 1.5 * 2^23 + k has k's two's complement in its low mantissa bits
-    f[r][0] = __float_as_uint(__fadd_rn(k0, 12582912.0f));
-    f[r][1] = __float_as_uint(__fadd_rn(k1, 12582912.0f));
-    f[r][2] = __float_as_uint(__fadd_rn(k2, 12582912.0f));
-    f[r][3] = __float_as_uint(__fadd_rn(k3, 12582912.0f));
+    const float4 q = make_float4(op(v[r].x, f[r][0]), op(v[r].y, f[r][1]), op(v[r].z, f[r][2]), op(v[r].w, f[r][3]));
+    if (c0 + r < C && p < HW)
+      st_result(reinterpret_cast<float4 *>(y + off + (size_t)r * HW), q, keep);
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    tile[4 * px4 + k][chq] = __byte_perm(__byte_perm(f[0][k], f[1][k], 0x0040), __byte_perm(f[2][k], f[3][k], 0x0040),
-                                         0x5410);
+    tile[4 * px4 + k][chq] = __byte_perm(__byte_perm(__float_as_uint(f[0][k]), __float_as_uint(f[1][k]), 0x0040),
+                                         __byte_perm(__float_as_uint(f[2][k]), __float_as_uint(f[3][k]), 0x0040), 0x5410);
   __syncthreads();
   const int word = threadIdx.x & 15, prow = threadIdx.x >> 4;
 #pragma unroll
-  for (int pp = prow; pp < 64; pp += 16) {
+  for (int pp = prow; pp < kCodePixels; pp += kCodeThreads / 16) {
     const int pix = p0 + pp, d = d0 + 4 * word;
     if (pix < HW && d < slots)
       *reinterpret_cast<uint32_t *>(codes + ((size_t)n * HW + pix) * slots + d) = tile[pp][word];
@@ -295,19 +323,14 @@ int fxp_nhwc_codes(const float *x, float *y, int8_t *codes, int64_t batch, int64
                (reinterpret_cast<uintptr_t>(codes) & 3) == 0,
            NB200_ENOTIMPL, "the quantizer with channel-last codes needs planes of a multiple of 4 values and aligned tensors");
   NB_CHECK(slots >= channels && slots % 16 == 0, NB200_EVALUE, "bad slot count");
-  const dim3 grid((unsigned)((inner + 63) / 64), (unsigned)((slots + 63) / 64), (unsigned)batch);
-  if (L.pow2) {
-    FxpOp<true, false> op{L.maxv, L.minv, delta, L.inv, L.code_max, L.code_min, nullptr};
-    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<true>, grid, dim3(256), 0, st, x, y, codes, (int)channels,
-                             (int)inner,
-                             slots, op));
-  } else {
-    FxpOp<false, false> op{L.maxv, L.minv, delta, L.inv, L.code_max, L.code_min, nullptr};
-    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<false>, grid, dim3(256), 0, st, x, y, codes, (int)channels,
-                             (int)inner,
-                             slots, op));
-  }
-  NB_LAUNCH_CHECK();
+  const dim3 grid((unsigned)((inner + kCodePixels - 1) / kCodePixels), (unsigned)((slots + 63) / 64), (unsigned)batch);
+  if (L.pow2)
+    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<FxpFastOp>, grid, dim3(kCodeThreads), 0, st, x, y, codes,
+                             (int)channels, (int)inner, slots, FxpFastOp{L.maxv, delta, L.inv, sign}));
+  else
+    NB_CUDA(launch_dependent(fxp_nhwc_codes_kernel<FxpAnyOp>, grid, dim3(kCodeThreads), 0, st, x, y, codes,
+                             (int)channels, (int)inner, slots,
+                             FxpAnyOp{{L.maxv, L.minv, delta, L.inv, L.code_max, L.code_min, nullptr}}));
   return NB200_OK;
 }
 
