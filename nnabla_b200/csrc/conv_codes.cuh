@@ -113,6 +113,7 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
   return d;
 }
 
+constexpr int kWeightParts = 4;    // barriers of the resident weights
 constexpr int kCodesKTable = 64; // K blocks whose coordinates are tabulated once per block
 
 // kResidentB: all tiles use the same weights (one column tile) and all their K blocks fit in
@@ -170,10 +171,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t *empty_bar = bars + STAGES;
   uint64_t *tmem_full = bars + 2 * STAGES;
   uint64_t *tmem_empty = bars + 2 * STAGES + 2;
-  uint64_t *b_full = bars + 2 * STAGES + 4;
-  uint64_t *a_full = bars + 2 * STAGES + 5;  // halo form: two pixel-tile buffers
-  uint64_t *a_empty = bars + 2 * STAGES + 7;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 9);
+  uint64_t *b_full = bars + 2 * STAGES + 4; // resident weights, kWeightParts runs of K blocks
+  uint64_t *a_full = b_full + kWeightParts; // halo form: two pixel-tile buffers
+  uint64_t *a_empty = a_full + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(a_empty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // (scale, bias) of every output map, times out_scale; read as float4 pairs, so 16-byte aligned
   float2 *sb = reinterpret_cast<float2 *>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));
@@ -197,7 +198,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       ptx::mbar_init(tmem_full + b, 1);
       ptx::mbar_init(tmem_empty + b, 4 * kSets);
     }
-    ptx::mbar_init(b_full, 1);
+    for (int q = 0; q < kWeightParts; ++q)
+      ptx::mbar_init(b_full + q, 1);
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(a_full + b, 1);
       ptx::mbar_init(a_empty + b, 1);
@@ -228,11 +230,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // (codes and channel-last results are read by convolutions)
   if (!ep.y_nchw || early_trigger((int64_t)prob.Nimg * prob.Ko * prob.Ho * prob.Wo))
     pdl_trigger();
-  for (int c = threadIdx.x; c < prob.n_tiles * BN; c += kGemmThreads)
-    sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
-                                      ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)
-                        : make_float2(0.0f, 0.0f);
-  __syncthreads();
+  // K blocks of one part of the resident weights
+  const int part_blocks = (k_blocks + kWeightParts - 1) / kWeightParts;
 
   // tile -> (column tile, pixel box); the column tiles of one box are neighbours in time (the box stays in L2)
   auto decode = [&](int tile, int &n0, int &img0, int &oy0) {
@@ -250,11 +249,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       uint32_t phase = 0;
       bool ok = true;
       const uint32_t tx_bytes = (uint32_t)(prob.pixels * RB) + (kResidentB ? 0u : kBBytes);
-      if (kResidentB && (int)blockIdx.x < num_tiles) {
-        ptx::mbar_expect_tx(b_full, resident_bytes);
-        for (int kb = 0; kb < k_blocks; ++kb)
-          ptx::tma_load_3d(b_resident + (size_t)kb * kBBytes, &map_w, b_full, kb * kElems, 0, 0);
-      }
+      // the weights behind the first pixels: the first MMAs need both, the others the rest of the weights
+      auto load_weights = [&]() {
+        for (int q = 0; q < kWeightParts; ++q) {
+          const int kb0 = q * part_blocks, kb1 = min(kb0 + part_blocks, k_blocks);
+          if (kb0 < kb1)
+            ptx::mbar_expect_tx(b_full + q, (uint32_t)(kb1 - kb0) * kBBytes);
+          for (int kb = kb0; kb < kb1; ++kb)
+            ptx::tma_load_3d(b_resident + (size_t)kb * kBBytes, &map_w, b_full + q, kb * kElems, 0, 0);
+        }
+      };
+      if (kResidentB && !kHalo && (int)blockIdx.x < num_tiles)
+        load_weights();
       int alocal = 0;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++alocal) {
         int n0, img0, oy0;
@@ -272,6 +278,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           for (int cb = 0; cb < prob.cblocks; ++cb)
             ptx::tma_load_5d(smem + (size_t)(ab * prob.cblocks + cb) * prob.a_tile_bytes, &map_x, a_full + ab,
                              cb * kElems, -prob.pw, oy0 - prob.ph, img0, 0);
+          if (alocal == 0)
+            load_weights();
         } else {
         for (int kb = 0; kb < k_blocks; ++kb) {
           bool got_slot;
@@ -307,15 +315,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       int local = 0;
       bool ok = true;
       const uint32_t idesc = ptx::make_idesc(2u, 1u, kTileM, BN); // s32 accumulator, s8 operands
-      if (kResidentB && (int)blockIdx.x < num_tiles) {
-        if (!ptx::mbar_wait(b_full, 0u, abort_flag)) {
-          if (*abort_flag == 0)
-            atomicCAS(status, 0, kStatusMmaTimeout);
-          *abort_flag = 1;
-          ok = false;
+      // resident weights: waited for part by part, as the first tile's MMAs come to them (a block with one tile spent
+      // as long on the wait for all of them as on its MMAs)
+      int weights_here = kResidentB ? 0 : 0x3fffffff; // K blocks
+      auto weights = [&](int kb_end) {
+        while (weights_here < kb_end) {
+          if (!ptx::mbar_wait(b_full + weights_here / part_blocks, 0u, abort_flag)) {
+            if (*abort_flag == 0)
+              atomicCAS(status, 0, kStatusMmaTimeout);
+            *abort_flag = 1;
+            ok = false;
+            return false;
+          }
+          ptx::tc_fence_after_sync();
+          weights_here += part_blocks;
         }
-        ptx::tc_fence_after_sync();
-      }
+        return true;
+      };
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
         const int buf = local & 1;
         const uint32_t buf_phase = (uint32_t)(local >> 1) & 1u;
@@ -360,7 +376,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           constexpr int kBatch = 4;
           int kb = 0;
           if (tabulated)
-            for (; kb + kBatch <= k_blocks; kb += kBatch) {
+            for (; kb + kBatch <= k_blocks && weights(kb + kBatch); kb += kBatch) {
               uint32_t off[kBatch];
 #pragma unroll
               for (int u = 0; u < kBatch; ++u)
@@ -369,8 +385,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
               for (int u = 0; u < kBatch; ++u)
                 issue(off[u], kb + u);
             }
-          for (; kb < k_blocks; ++kb)
+          for (; kb < k_blocks && weights(kb + 1); ++kb)
             issue((uint32_t)(tabulated ? kb_table[kb].x : kb_entry(kb).x), kb);
+          if (!ok)
+            break;
           ptx::mma_commit(a_empty + ab); // the pixel tile is free once these MMAs have read it
           ptx::mma_commit(tmem_full + buf);
         } else {
@@ -384,6 +402,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             ok = false;
             break;
           }
+          if (!weights(kb + 1))
+            break;
           ptx::tc_fence_after_sync();
           const uint32_t st = ptx::smem_u32(smem + stage * kStageBytes);
           const uint64_t adesc = ptx::smem_desc_k(st, RB);
@@ -411,6 +431,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int quarter = warp & 3;      // TMEM lanes [32 * quarter, +32) are visible to this warp
     const int first_col = 32 * ((warp - 2) >> 2); // this warp's first 32-column chunk of a tile's accumulators
     const float cap = (float)(2 * ep.kmax) + 0.5f;
+    // scale and bias are the epilogue's alone: the copies and MMAs do not wait for their loads (0.7 us of a launch that
+    // has one tile per block)
+    for (int c = threadIdx.x - 64; c < prob.n_tiles * BN; c += 32 * kEpilogueWarps)
+      sb[c] = c < prob.Ko ? make_float2(ep.scale ? __fmul_rn(ep.scale[c], ep.out_scale) : ep.out_scale,
+                                        ep.bias ? __fmul_rn(ep.bias[c], ep.bias_scale) : 0.0f)
+                          : make_float2(0.0f, 0.0f);
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
     // this thread's pixel of every tile: image of the box, row and column (the divisions stay out of the loop)
     const int row = quarter * 32 + lane;
     const int per_img = prob.h_box * prob.Wo, pitch = kHalo ? prob.wp : prob.Wo;
@@ -667,7 +694,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // (in the halo form the ring is replaced by the pixel-tile buffers, counted by the caller)
 template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false>
 constexpr size_t conv_codes_smem_bytes() {
-  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) + (2 * STAGES + 9) * 8 + 32 +
+  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) + (2 * STAGES + 8 + kWeightParts) * 8 + 32 +
          kCodesMaxMaps * sizeof(float2) + kCodesKTable * sizeof(int4) + 1024;
 }
 
