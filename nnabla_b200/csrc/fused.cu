@@ -458,6 +458,50 @@ __global__ void __launch_bounds__(128) global_average_pooling_codes_kernel(const
   }
 }
 
+// The same where the step is a power of two and the sums stay below 2^24 steps: every partial sum of the reference is then
+// exact, so the codes can be added as integers in any order. A block has up to 512 slots of a sample, 32 runs of 16 of them
+// by 8 shares of the pixels, so that one sample's loads are all in flight at once: 512 maps of 7 x 7 pixels 7.1 -> 5.1 us
+// for one image, launch and wait included (a thread that walks its pixels one after the other is a chain of 49 loads and additions).
+constexpr int kGapSlots = 512, kGapShares = 8;
+__global__ void __launch_bounds__(256) global_average_pooling_int_codes_kernel(const int8_t *__restrict__ codes,
+                                                                               CodesLayout L, float delta,
+                                                                               float *__restrict__ y) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ int part[kGapShares][kGapSlots];
+  const int run = threadIdx.x & 31, share = threadIdx.x >> 5, d0 = blockIdx.x * kGapSlots, d = d0 + 16 * run;
+  const int n = blockIdx.y;
+  int s[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    s[j] = 0;
+  if (d < L.slots) {
+    const int8_t *src = codes + (int64_t)n * L.HW * L.slots + d;
+#pragma unroll 8
+    for (int p = share; p < L.HW; p += kGapShares) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src + (int64_t)p * L.slots));
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        s[j] = __dp4a((int)w[j >> 2], 1 << (8 * (j & 3)), s[j]);
+    }
+  }
+#pragma unroll
+  for (int j4 = 0; j4 < 4; ++j4)
+    *reinterpret_cast<int4 *>(&part[share][16 * run + 4 * j4]) = make_int4(s[4 * j4], s[4 * j4 + 1], s[4 * j4 + 2], s[4 * j4 + 3]);
+  __syncthreads();
+#pragma unroll
+  for (int i = threadIdx.x; i < kGapSlots; i += 256) {
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < kGapShares; ++q)
+      sum += part[q][i];
+    const int slot = d0 + i, g = slot / L.c_pad_g, cc = slot - g * L.c_pad_g;
+    if (slot < L.slots && g < L.groups && cc < L.Cg)
+      y[(int64_t)n * L.C + g * L.Cg + cc] = __fdiv_rn(__fmul_rn((float)sum, delta), (float)L.HW);
+  }
+}
+
 int fill_fxp(FxpParams &P, int sign, int n, float delta) {
   // the reference's setup (fixed_point_quantize.cpp:31-42)
   NB_CHECK(n > 0 && delta > 0.f, NB200_EVALUE, "Both bit width and delta should be positive.");
@@ -607,6 +651,14 @@ extern "C" int nb200_global_average_pooling_codes_f32(const int8_t *codes, float
     return NB200_OK;
   NB_CHECK(codes && y, NB200_EVALUE, "null data pointer");
   NB_CHECK((reinterpret_cast<uintptr_t>(codes) & 3) == 0, NB200_EVALUE, "code tensors must be 4-byte aligned");
+  int ex = 0;
+  if (std::frexp(delta, &ex) == 0.5f && ex > -100 && ex < 100 && inner <= (1 << 24) / 128 &&
+      (reinterpret_cast<uintptr_t>(codes) & 15) == 0 && L.slots % 16 == 0) {
+    NB_CUDA(launch_dependent(global_average_pooling_int_codes_kernel,
+                             dim3((unsigned)((L.slots + kGapSlots - 1) / kGapSlots), (unsigned)batch), dim3(256), 0,
+                             as_stream(stream), codes, L, delta, y));
+    return NB200_OK;
+  }
   NB_CUDA(launch_dependent(global_average_pooling_codes_kernel, dim3((unsigned)((L.slots + 511) / 512), (unsigned)batch),
                            dim3(128), 0, as_stream(stream), codes, L, delta, y));
   return NB200_OK;
