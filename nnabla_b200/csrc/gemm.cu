@@ -328,18 +328,32 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
            (long long)N);
   NB_CHECK(M < (1ll << 31) && K < (1ll << 31) && N < (1ll << 31), NB200_EVALUE, "extent exceeds 2^31");
   NB_CHECK(dy != nullptr, NB200_EVALUE, "dy is NULL");
-  if (dx) {
-    NB_CHECK(w != nullptr, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
-    if (w_exact_bf16 ? small_gemm_scaled(M, K, N) : small_gemm_plain(M, K, N)) {
-      SmallGemm P{};
-      P.a = dy, P.b = w, P.y = dx;
-      P.M = (int)M, P.N = (int)K, P.K = (int)N;
-      P.a_scale = w_col_scale;
-      P.accumulate = accum_dx;
-      NB_TRY((launch_small_gemm<false, true, SmallB::kPlain>(P, st)));
-      dx = nullptr;
-    }
-  }
+  NB_CHECK(!dx || w, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
+  NB_CHECK(!dw || x, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
+  SmallGemm sx{}, sw{};
+  sx.a = dy, sx.b = w, sx.y = dx;
+  sx.M = (int)M, sx.N = (int)K, sx.K = (int)N;
+  sx.a_scale = w_col_scale;
+  sx.accumulate = accum_dx;
+  sw.a = x, sw.b = dy, sw.y = dw;
+  sw.M = (int)K, sw.N = (int)N, sw.K = (int)M;
+  sw.accumulate = accum_dw;
+  sw.sums = db;
+  sw.accumulate_sums = accum_db;
+  const bool small_dx = dx && (w_exact_bf16 ? small_gemm_scaled(M, K, N) : small_gemm_plain(M, K, N));
+  const bool small_dw = dw && small_gemm_transposed(K, N, M);
+  if (small_dx && small_dw)
+    NB_TRY(launch_small_gradients(sx, sw, st));
+  else if (small_dx)
+    NB_TRY((launch_small_gemm<false, true, SmallB::kPlain>(sx, st)));
+  else if (small_dw && db)
+    NB_TRY((launch_small_gemm<true, false, SmallB::kColumnSums>(sw, st)));
+  else if (small_dw)
+    NB_TRY((launch_small_gemm<true, false, SmallB::kPlain>(sw, st)));
+  if (small_dx)
+    dx = nullptr;
+  if (small_dw)
+    dw = db = nullptr;
   if (dx) {
     const int64_t Np = round_up(N, 64);
     const int planes_w = w_exact_bf16 ? 1 : 3;
@@ -354,22 +368,6 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
     ep.scale = 1.0f;
     ep.accumulate = accum_dx;
     NB_TRY(run_gemm(false, 3, planes_w, base, Np, base + a_bytes, Np, (int)M, (int)K, (int)N, ep, K, st));
-  }
-  if (dw) {
-    NB_CHECK(x != nullptr, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
-    if (small_gemm_transposed(K, N, M)) {
-      SmallGemm P{};
-      P.a = x, P.b = dy, P.y = dw;
-      P.M = (int)K, P.N = (int)N, P.K = (int)M;
-      P.accumulate = accum_dw;
-      P.sums = db;
-      P.accumulate_sums = accum_db;
-      if (db)
-        NB_TRY((launch_small_gemm<true, false, SmallB::kColumnSums>(P, st)));
-      else
-        NB_TRY((launch_small_gemm<true, false, SmallB::kPlain>(P, st)));
-      dw = db = nullptr;
-    }
   }
   if (dw) {
     const int64_t Mp = round_up(M, 64);
