@@ -378,6 +378,23 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           acc[ci][j] = 0.0f;
+      // With one chunk of maps per warp the values to add to are fetched before the accumulator is waited for: behind the
+      // wait, eight at a time, a tile's epilogue took longer than its MMAs (input gradient of a 64 -> 64 3 x 3 layer on
+      // [128, 64, 56, 56] added to dx 121 us, now 96; not added 91). With two chunks there are no registers for them.
+      constexpr int kAhead = kMine == 1 ? 32 : 1;
+      float ahead[kAhead];
+      auto chunk_left = [&](int ci) { return prob.maps - (t.n0 + 32 * set + 64 * ci); }; // maps of this chunk that exist
+      auto chunk_y = [&](int ci) {
+        return prob.y + ((int64_t)img * prob.total_maps + t.group * prob.maps + t.n0 + 32 * set + 64 * ci) * plane +
+               (int64_t)iy * prob.W + ix;
+      };
+      if (kMine == 1 && prob.accumulate && pix_ok) {
+        const float *yp = chunk_y(0);
+        const int left = chunk_left(0);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+          ahead[j] = j < left ? yp[(int64_t)j * plane] : 0.0f;
+      }
       for (int kc = 0; kc < chunks; ++kc, ++local) {
         const int buf = local & 1;
         const bool got = ptx::mbar_wait(tmem_full + buf, (uint32_t)(local >> 1) & 1u, abort_flag);
@@ -418,11 +435,11 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
         break;
 #pragma unroll
       for (int ci = 0; ci < kMine; ++ci) {
-        const int col = t.n0 + 32 * set + 64 * ci, left = prob.maps - col; // maps of this chunk that exist
+        const int left = chunk_left(ci);
         if (left <= 0)
           continue;
-        const int map0 = t.group * prob.maps + col;
-        float *yp = prob.y + ((int64_t)img * prob.total_maps + map0) * plane + (int64_t)iy * prob.W + ix;
+        const int map0 = t.group * prob.maps + t.n0 + 32 * set + 64 * ci;
+        float *yp = chunk_y(ci);
         if (prob.scale || prob.bias || prob.image_max) {
           // one rounding per operation, like the reference's product and bias addition (the image's factor is a power
           // of two)
@@ -446,7 +463,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
             float old[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              old[j] = j0 + j < left ? yp[(int64_t)(j0 + j) * plane] : 0.0f;
+              old[j] = kMine == 1 ? ahead[(j0 + j) % kAhead] : j0 + j < left ? yp[(int64_t)(j0 + j) * plane] : 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               if (j0 + j < left)
