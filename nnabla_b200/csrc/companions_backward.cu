@@ -213,10 +213,11 @@ template <int K> __device__ __forceinline__ void block_sums(float (&v)[K], float
   }
 }
 
-// Calls f(flat element, live) for this block's items of channel c, four at a time with their loads before their use:
-// the sums are HBM-bound and one load in flight per thread reached half of the copy bandwidth.
-template <int kW, typename Load, typename Use>
-__device__ __forceinline__ void channel_sum_loop(unsigned N, unsigned C, unsigned S, Load load, Use use) {
+// Calls use(loaded value, sum) for this block's items of channel c, four at a time with their loads before their use:
+// the sums are HBM-bound and one load in flight per thread reached half of the copy bandwidth. use adds to a sum of the
+// four, which is then added to v_sum: a quarter of the additions at the sum's full magnitude.
+template <int kW, int K, typename Load, typename Use>
+__device__ __forceinline__ void channel_sum_loop(unsigned N, unsigned C, unsigned S, float (&v_sum)[K], Load load, Use use) {
   const unsigned c = blockIdx.y, P = gridDim.x, Su = S / kW;
   ChannelItems it((size_t)blockIdx.x * kThreads + threadIdx.x, (size_t)P * kThreads, Su, N);
   while (it.valid()) {
@@ -229,10 +230,17 @@ __device__ __forceinline__ void channel_sum_loop(unsigned N, unsigned C, unsigne
         v[u] = load(((size_t)it.n * C + c) * S + (size_t)kW * it.s);
       it.next();
     }
+    float four[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      four[k] = 0.0f;
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (live[u])
-        use(v[u]);
+        use(v[u], four);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      v_sum[k] += four[k];
   }
 }
 
@@ -244,19 +252,38 @@ __global__ void __launch_bounds__(kThreads) bn_stats_kernel(const float *__restr
   pdl_trigger();
   float v[2] = {0.0f, 0.0f};
   if constexpr (kVec) {
-    channel_sum_loop<4>(N, C, S, [&](size_t i) { return __ldg(reinterpret_cast<const float4 *>(x + i)); },
-                        [&](float4 a) {
-                          v[0] += (a.x + a.y) + (a.z + a.w);
-                          v[1] += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
+    channel_sum_loop<4>(N, C, S, v, [&](size_t i) { return __ldg(reinterpret_cast<const float4 *>(x + i)); },
+                        [](float4 a, float (&s)[2]) {
+                          s[0] += (a.x + a.y) + (a.z + a.w);
+                          s[1] += (a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w);
                         });
   } else {
-    channel_sum_loop<1>(N, C, S, [&](size_t i) { return __ldg(x + i); },
-                        [&](float a) {
-                          v[0] += a;
-                          v[1] += a * a;
+    channel_sum_loop<1>(N, C, S, v, [&](size_t i) { return __ldg(x + i); },
+                        [](float a, float (&s)[2]) {
+                          s[0] += a;
+                          s[1] += a * a;
                         });
   }
   block_sums<2>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 2);
+}
+
+// Sums over the P blocks of a channel's K partial sums, by kLanes neighbouring lanes: each adds every kLanes-th block's,
+// then the lanes' sums are added pairwise; a fixed order, in double precision. One lane per channel is a chain of P loads
+// and additions ([128, 64, 56, 56], 13 blocks a channel: 3.4 us, now 2.6), a warp per channel is slower where P is 4.
+constexpr int kLanes = 8, kFinishThreads = 128;
+template <int K> __device__ __forceinline__ void channel_total(const float *__restrict__ partial, unsigned P, double (&t)[K]) {
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    t[k] = 0.0;
+  for (unsigned p = threadIdx.x % kLanes; p < P; p += kLanes)
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      t[k] += (double)partial[(size_t)p * K + k];
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1)
+      t[k] += __shfl_down_sync(0xffffffffu, t[k], o, kLanes);
 }
 
 // batch_normalization.cpp:191-205 given the channel's sums: mean, variance, running statistics.
@@ -265,16 +292,13 @@ __global__ void bn_stats_finish_kernel(const float *__restrict__ partial, unsign
                                        float *__restrict__ rm, float *__restrict__ rv) {
   pdl_wait();
   pdl_trigger();
-  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C)
+  const unsigned c = (blockIdx.x * kFinishThreads + threadIdx.x) / kLanes;
+  double t[2]; // (all lanes of a warp add and shuffle together)
+  channel_total<2>(partial + (size_t)c * P * 2, c < C ? P : 0u, t);
+  if (c >= C || threadIdx.x % kLanes != 0)
     return;
-  double s = 0.0, q = 0.0;
-  for (unsigned p = 0; p < P; ++p) {
-    s += (double)partial[((size_t)c * P + p) * 2];
-    q += (double)partial[((size_t)c * P + p) * 2 + 1];
-  }
-  const float mean = __fdiv_rn((float)s, count);
-  const float var = __fsub_rn(__fdiv_rn((float)q, count), __fmul_rn(mean, mean));
+  const float mean = __fdiv_rn((float)t[0], count);
+  const float var = __fsub_rn(__fdiv_rn((float)t[1], count), __fmul_rn(mean, mean));
   m[c] = mean;
   v[c] = var;
   if (update) {
@@ -295,31 +319,31 @@ __global__ void __launch_bounds__(kThreads)
   pdl_trigger();
   const float m = mean[blockIdx.y];
   float v[3] = {0.0f, 0.0f, 0.0f};
-  auto one = [&](float xv, float g) {
+  auto one = [&](float xv, float g, float (&s)[3]) {
     const float cx = __fsub_rn(xv, m);
-    v[0] += g;
-    v[1] += __fmul_rn(g, cx);
+    s[0] += g;
+    s[1] += __fmul_rn(g, cx);
     if (kBatch)
-      v[2] += cx;
+      s[2] += cx;
   };
   if constexpr (kVec) {
     struct Pair {
       float4 a, g;
     };
-    channel_sum_loop<4>(N, C, S,
+    channel_sum_loop<4>(N, C, S, v,
                         [&](size_t i) {
                           return Pair{__ldg(reinterpret_cast<const float4 *>(x + i)),
                                       __ldg(reinterpret_cast<const float4 *>(dy + i))};
                         },
-                        [&](const Pair &p) {
-                          one(p.a.x, p.g.x);
-                          one(p.a.y, p.g.y);
-                          one(p.a.z, p.g.z);
-                          one(p.a.w, p.g.w);
+                        [&](const Pair &p, float (&s)[3]) {
+                          one(p.a.x, p.g.x, s);
+                          one(p.a.y, p.g.y, s);
+                          one(p.a.z, p.g.z, s);
+                          one(p.a.w, p.g.w, s);
                         });
   } else {
-    channel_sum_loop<1>(N, C, S, [&](size_t i) { return make_float2(__ldg(x + i), __ldg(dy + i)); },
-                        [&](float2 p) { one(p.x, p.y); });
+    channel_sum_loop<1>(N, C, S, v, [&](size_t i) { return make_float2(__ldg(x + i), __ldg(dy + i)); },
+                        [&](float2 p, float (&s)[3]) { one(p.x, p.y, s); });
   }
   block_sums<3>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 3);
 }
@@ -334,14 +358,11 @@ __global__ void bn_backward_finish_kernel(const float *__restrict__ partial, uns
                                           float *__restrict__ dgamma, int accum_dgamma) {
   pdl_wait();
   pdl_trigger();
-  const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C)
+  const unsigned c = (blockIdx.x * kFinishThreads + threadIdx.x) / kLanes;
+  double t[3]; // (all lanes of a warp add and shuffle together)
+  channel_total<3>(partial + (size_t)c * P * 3, partial && c < C ? P : 0u, t);
+  if (c >= C || threadIdx.x % kLanes != 0)
     return;
-  double t[3] = {0, 0, 0};
-  if (partial)
-    for (unsigned p = 0; p < P; ++p)
-      for (int k = 0; k < 3; ++k)
-        t[k] += (double)partial[((size_t)c * P + p) * 3 + k];
   const float ve = __fadd_rn(var[c], eps);
   const double scale = gamma ? (double)gamma[c] : 1.0;
   // sum dy*scale*(x-m), sum dy*scale, sum (x-m), sum dy, sum dy*(x-m)/sqrt(v+eps)
@@ -479,12 +500,35 @@ int bn_backward_dx_planes(const float *x, const float *dy, const float *gamma, c
   return NB200_OK;
 }
 
-int channel_blocks(int64_t outer, int64_t channels, int64_t inner, bool vec) {
-  const int64_t items = outer * (vec ? inner / 4 : inner);
-  int64_t p = (8ll * sm_count() + channels - 1) / channels;
-  const int64_t most = (items + kThreads - 1) / kThreads;
-  p = p > most ? most : p;
-  return (int)(p < 1 ? 1 : p);
+// Blocks per channel of a pass that sums over channels. All blocks have the same share, so it takes as long as its rounds
+// of resident blocks: the counts that fill one to four rounds exactly are compared by how full their rounds are, more
+// rounds only where they are 5 % fuller (8 blocks per SM whatever the kernel's registers allow made 3 rounds of 592 blocks
+// of the gradients' 1216: [128, 64, 56, 56] 44 us, now 38).
+template <typename Kernel>
+int channel_blocks(Kernel kernel, int (&resident)[64], int64_t outer, int64_t channels, int64_t inner, bool vec, int *out) {
+  int dev = 0;
+  NB_CUDA(cudaGetDevice(&dev));
+  int per_sm = resident[dev & 63]; // the same value whichever thread stores it
+  if (per_sm == 0) {
+    NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+    resident[dev & 63] = per_sm;
+  }
+  const int64_t slots = (int64_t)per_sm * sm_count();
+  int64_t best = 1;
+  double best_full = 0.0;
+  for (int64_t rounds = 1; rounds <= 4; ++rounds) {
+    const int64_t p = rounds * slots / channels;
+    const double full = (double)(p * channels) / (double)(rounds * slots);
+    if (p >= 1 && full > best_full + 0.05)
+      best = p, best_full = full;
+  }
+  const int64_t items = outer * (vec ? inner / 4 : inner), most = (items + kThreads - 1) / kThreads;
+  // short channels, a thread's share at most one set of four loads: as many blocks as 8 per SM give (fewer loads in a row)
+  if (items <= best * kThreads * 4)
+    best = (8ll * sm_count() + channels - 1) / channels;
+  best = best > most ? most : best;
+  *out = (int)(best < 1 ? 1 : best);
+  return NB200_OK;
 }
 
 } // namespace
@@ -508,14 +552,17 @@ int nb200_batch_normalization_batch_f32(const float *x, const float *beta, const
   NB_CHECK(!update_running || (running_mean && running_var), NB200_EVALUE, "running statistics are needed");
   cudaStream_t st = as_stream(stream);
   const bool vec = (inner % 4 == 0) && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const int P = channel_blocks(outer, channels, inner, vec);
+  auto stats = vec ? bn_stats_kernel<true> : bn_stats_kernel<false>;
+  static int resident[2][64];
+  int P = 0;
+  NB_TRY(channel_blocks(stats, resident[vec], outer, channels, inner, vec, &P));
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc((size_t)channels * P * 2 * sizeof(float)));
   float *partial = static_cast<float *>(scratch.p);
-  const dim3 grid((unsigned)P, (unsigned)channels);
-  NB_CUDA(launch_dependent(vec ? bn_stats_kernel<true> : bn_stats_kernel<false>, grid, dim3(kThreads), 0, st, x,
+  const dim3 grid((unsigned)P, (unsigned)channels), finish_grid((unsigned)((channels * kLanes + kFinishThreads - 1) / kFinishThreads));
+  NB_CUDA(launch_dependent(stats, grid, dim3(kThreads), 0, st, x,
                            (unsigned)outer, (unsigned)channels, (unsigned)inner, partial));
-  NB_CUDA(launch_dependent(bn_stats_finish_kernel, dim3((unsigned)((channels + 127) / 128)), dim3(128), 0, st, partial,
+  NB_CUDA(launch_dependent(bn_stats_finish_kernel, finish_grid, dim3(kFinishThreads), 0, st, partial,
                            (unsigned)P, (unsigned)channels, (float)(outer * inner), decay_rate, update_running,
                            batch_mean, batch_var, running_mean, running_var));
   return nb200_batch_normalization_inference_f32(x, beta, gamma, batch_mean, batch_var, y, outer, channels, inner,
@@ -534,20 +581,23 @@ int nb200_batch_normalization_backward_f32(const float *x, const float *dy, cons
     return NB200_OK;
   cudaStream_t st = as_stream(stream);
   const bool vec = (inner % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
-  const int P = channel_blocks(outer, channels, inner, vec);
+  auto sums_kernel = vec ? (batch_stat ? bn_backward_sums_kernel<true, true> : bn_backward_sums_kernel<true, false>)
+                         : (batch_stat ? bn_backward_sums_kernel<false, true> : bn_backward_sums_kernel<false, false>);
+  static int resident[4][64];
+  int P = 0;
+  NB_TRY(channel_blocks(sums_kernel, resident[2 * vec + (batch_stat != 0)], outer, channels, inner, vec, &P));
   AsyncScratch scratch(st);
   NB_TRY(scratch.alloc((size_t)channels * (P * 3 + 4) * sizeof(float)));
   float *partial = static_cast<float *>(scratch.p);
   float *coef = partial + (size_t)channels * P * 3;
   const bool sums = (batch_stat && dx) || dbeta || dgamma;
+  const dim3 finish_grid((unsigned)((channels * kLanes + kFinishThreads - 1) / kFinishThreads));
   if (sums) {
     const dim3 grid((unsigned)P, (unsigned)channels);
-    auto kernel = vec ? (batch_stat ? bn_backward_sums_kernel<true, true> : bn_backward_sums_kernel<true, false>)
-                      : (batch_stat ? bn_backward_sums_kernel<false, true> : bn_backward_sums_kernel<false, false>);
-    NB_CUDA(launch_dependent(kernel, grid, dim3(kThreads), 0, st, x, dy, mean, (unsigned)outer, (unsigned)channels,
+    NB_CUDA(launch_dependent(sums_kernel, grid, dim3(kThreads), 0, st, x, dy, mean, (unsigned)outer, (unsigned)channels,
                              (unsigned)inner, partial));
   }
-  NB_CUDA(launch_dependent(bn_backward_finish_kernel, dim3((unsigned)((channels + 127) / 128)), dim3(128), 0, st,
+  NB_CUDA(launch_dependent(bn_backward_finish_kernel, finish_grid, dim3(kFinishThreads), 0, st,
                            sums ? partial : nullptr, (unsigned)P, (unsigned)channels, (float)(outer * inner), gamma, var,
                            eps, dmean, dvar, batch_stat, coef, sums ? dbeta : nullptr, accum_dbeta,
                            sums ? dgamma : nullptr, accum_dgamma));
