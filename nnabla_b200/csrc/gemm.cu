@@ -120,6 +120,18 @@ static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int 
                                                                            ep, st);
 }
 
+// Whether y = pieces of x (three) . weights (one plane) runs as GemmTransposedProblem: where 128 x 128 tiles would leave
+// SMs idle, and its rounds of 128 x 64 tiles at 40 KB a K block cost less than those of 64 columns by 128 rows of x at 56.
+// Whole layers, alpha made in the product's epilogue instead of a launch of its own: [256, 1024] . [1024, 4096] 19.7 -> 16.0
+// us, [512, 1024] . [1024, 1024] 16.7 -> 13.3, [128, 8000] . [8000, 2000] 101 -> 83.
+static bool gemm_transposes(int64_t M, int64_t N) {
+  const int64_t sms = sm_count();
+  auto rounds = [&](int64_t rows, int64_t cols) {
+    return (((M + rows - 1) / rows) * ((N + cols - 1) / cols) + sms - 1) / sms;
+  };
+  return ((M + 127) / 128) * ((N + 127) / 128) < sms && rounds(64, 128) * 40 <= rounds(128, 64) * 56;
+}
+
 // A: [planes_a][M][pitch_a], B: [planes_b][N][pitch_b], both K-major.
 int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch_a, const void *B, int64_t pitch_b,
              int M, int N, int K, const GemmEpilogue &ep, int64_t ldy, cudaStream_t st) {
@@ -165,6 +177,25 @@ int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch
     return launch_gemm<true, 1, 1, 64, 8, false>(ma, mb, M, N, k_blocks, ep, ldy, st);
   }
   if (planes_a == 3 && planes_b == 1) {
+    if (ep.n_peers == 0 && !ep.row_scale && !ep.row_bias && gemm_transposes(M, N)) {
+      GemmTransposedProblem prob;
+      prob.M = N;
+      prob.N = M;
+      prob.kblocks = k_blocks;
+      prob.m_tiles = (N + kTileM - 1) / kTileM;
+      prob.n_tiles = (M + 63) / 64;
+      prob.bn = 64;
+      prob.row_bytes = kRowBytes;
+      prob.chunk_blocks = k_chunk_blocks(3 * 4);
+      prob.ldy = ldy;
+      GemmEpilogue ept = ep;
+      ept.row_scale = ep.col_scale, ept.row_bias = ep.col_bias;
+      ept.col_scale = ept.col_bias = nullptr;
+      NB_TRY(make_operand_map(&ma, B, false, K, pitch_b, N, 1, kTileM));
+      NB_TRY(make_operand_map(&mb, A, false, K, pitch_a, M, 3, 64));
+      return launch_contraction<false, 1, 3, 64, 4, 0, GemmTransposedProblem>(ma, mb, prob, prob.m_tiles * prob.n_tiles,
+                                                                              ept, st);
+    }
     if (!narrow) {
       NB_TRY(make_operand_map(&mb, B, false, K, pitch_b, N, 1, 128));
       return launch_gemm<false, 3, 1, 128, 3, false>(ma, mb, M, N, k_blocks, ep, ldy, st);
@@ -215,11 +246,20 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
   void *planes = base;
   void *side = base + round_up(planes_bytes, 256);
   float *partial = reinterpret_cast<float *>(base + round_up(planes_bytes, 256) + round_up(side_bytes, 256));
-  NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st));
+  // the transposed product makes alpha from the partial sums itself
+  bool sums_left = alpha && gemm_transposes(M, N);
+  NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st, &sums_left));
   GemmEpilogue ep{};
   ep.y = y;
   ep.scale = 1.0f;
   ep.col_scale = alpha;
+  if (sums_left) {
+    ep.col_scale = nullptr;
+    ep.alpha_partial = partial;
+    ep.alpha_parts = (int)((K + 63) / 64);
+    ep.alpha_inv = (float)1 / K; // binary_weight_affine.cpp:68
+    ep.alpha = alpha;
+  }
   ep.col_bias = bias;
   return run_gemm(false, 3, 1, planes, Kp, side, Kp, (int)M, (int)N, (int)K, ep, N, st);
 }

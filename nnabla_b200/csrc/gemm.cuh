@@ -73,6 +73,12 @@ struct GemmEpilogue {
   int n_peers;
   float *peer_y[kMaxPeers];
   int accumulate; // y += value instead of y = value (gradient accumulation); single-CTA kernel only
+  // Transposed problem only: row_scale as partial sums [alpha_parts][M], added in order and multiplied by alpha_inv; the
+  // tiles of the first columns write the factors to alpha.
+  const float *alpha_partial;
+  int alpha_parts;
+  float alpha_inv;
+  float *alpha;
 };
 
 // Per-tile coordinates produced by a problem policy.
@@ -89,6 +95,7 @@ struct Tile {
 
 // ---- plain GEMM: A [planes][M][K], B [planes][N][K] --------------------------
 struct GemmProblem {
+  static constexpr bool kTransposed = false;
   int M, N, kblocks, m_tiles, n_tiles, bn;
   int row_bytes; // bytes of one K block per operand row (128 or 64)
   int chunk_blocks; // K blocks accumulated in tensor memory before the fp32 registers take over (0 = all)
@@ -126,6 +133,14 @@ struct GemmProblem {
   }
 };
 
+// The same product the other way round: D rows are the columns of y, D columns its rows (A: the weights, B: the pieces of
+// x). A thread owns a column of y, so that 32 lanes store 32 neighbouring values straight from their registers. With
+// three pieces of x a K block of a 128 x 64 tile is 40 KB (16 of weights, 24 of x) where 128 rows of x by 64 columns are
+// 56, and that is what such a tile is bound by: L2 to shared memory.
+struct GemmTransposedProblem : GemmProblem {
+  static constexpr bool kTransposed = true;
+};
+
 // ---- implicit-GEMM convolution -------------------------------------------------
 // A = weight side-band [planes][Ko][taps * cblocks * E] (K ordered tap-major,
 // channel-minor), B = activation planes [planes][N][H][W][Ctot] (NHWC), D rows
@@ -134,6 +149,7 @@ struct GemmProblem {
 // tile is one TMA box shifted by the tap (out-of-range rows/columns read as
 // zero = the padding).
 struct ConvProblem {
+  static constexpr bool kTransposed = false;
   int Nimg, Ko, Kog, groups, Ho, Wo;
   int h_box, n_box, tiles_h, tiles_n, m_tiles_g;
   int kw, taps, cblocks;
@@ -414,7 +430,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // column-wise ones by the column's owner after it: no loads in the loops.
       const int my_row = row_base + lane;
       const bool my_row_ok = my_row < t.m_end;
-      const float rs = (ep.row_scale && my_row_ok) ? __fmul_rn(ep.row_scale[my_row], ep.scale) : ep.scale;
+      float rs = (ep.row_scale && my_row_ok) ? __fmul_rn(ep.row_scale[my_row], ep.scale) : ep.scale;
+      if constexpr (Problem::kTransposed) {
+        if (ep.alpha_partial && my_row_ok) { // (while the first operands are on their way)
+          float sum = 0.0f;
+#pragma unroll 8
+          for (int b = 0; b < ep.alpha_parts; ++b)
+            sum += __ldg(ep.alpha_partial + (int64_t)b * prob.M + my_row);
+          const float a = __fmul_rn(sum, ep.alpha_inv);
+          if (t.n0 == 0 && half == 0)
+            ep.alpha[my_row] = a;
+          rs = __fmul_rn(a, ep.scale);
+        }
+      }
       const float rb = (ep.row_bias && my_row_ok) ? ep.row_bias[my_row] : 0.0f;
       int rows_here = t.m_end - row_base;
       rows_here = rows_here < 0 ? 0 : (rows_here > 32 ? 32 : rows_here);
@@ -467,6 +495,32 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               r[j] = __float_as_uint(acc[kInt8 ? 0 : ci][j]);
+          }
+          if constexpr (Problem::kTransposed) {
+            // one rounding per operation, as below
+            float *yp = ep.y + (int64_t)(t.n0 + c0) * prob.ldy + my_row;
+            const int left = prob.N - t.n0 - c0; // rows of y
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              float v = __fmul_rn(__uint_as_float(r[j]), rs);
+              if (ep.row_bias)
+                v = __fadd_rn(v, rb);
+              r[j] = __float_as_uint(v);
+            }
+            if (ep.accumulate) {
+              float old[32];
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                old[j] = my_row_ok && j < left ? yp[(int64_t)j * prob.ldy] : 0.0f;
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                r[j] = __float_as_uint(__fadd_rn(old[j], __uint_as_float(r[j])));
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (my_row_ok && j < left)
+                yp[(int64_t)j * prob.ldy] = __uint_as_float(r[j]);
+            continue;
           }
           if (ep.col_scale) {
 #pragma unroll

@@ -660,19 +660,20 @@ int binarize_columns(const float *w, int R, int C, float zero_to, float *wb, flo
 }
 
 int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, int C, float zero_to, float *wb, float *alpha,
-                           void *side, int64_t pitch, float *partial_scratch, void *pieces, cudaStream_t st) {
+                           void *side, int64_t pitch, float *partial_scratch, void *pieces, cudaStream_t st, bool *leave_sums) {
   const int gx = (C + kBT - 1) / kBT, gy = (R + kBT - 1) / kBT;
   const int64_t w_blocks = (int64_t)gx * gy, x_blocks = (rows * (pitch / 4) + 255) / 256;
   const bool vec = C % 4 == 0 && R % 4 == 0 && w_blocks + x_blocks < (1ll << 31) &&
                    ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(wb) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
   if (!vec) {
+    *leave_sums = false;
     NB_TRY(binarize_columns(w, R, C, zero_to, wb, alpha, side, pitch, false, partial_scratch, st));
     return split_rows_bf16(x, rows, R, pitch, 3, pieces, st);
   }
   NB_CUDA(launch_dependent(binary_affine_operands_kernel, dim3((unsigned)(w_blocks + x_blocks)), dim3(256), 0, st, w, R, C,
                            zero_to, wb, side, pitch, alpha ? partial_scratch : nullptr, gx, (int)w_blocks, x, rows,
                            static_cast<__nv_bfloat16 *>(pieces)));
-  if (alpha)
+  if (alpha && !*leave_sums)
     NB_CUDA(launch_dependent(finalize_alpha_kernel, dim3((C + 255) / 256), dim3(256), 0, st, partial_scratch, gy, C,
                              (float)1 / R, alpha)); // binary_weight_affine.cpp:68
   return NB200_OK;

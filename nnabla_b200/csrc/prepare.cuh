@@ -30,9 +30,9 @@ inline int64_t codes_slots(int64_t channels, int group) {
 int split_rows_bf16(const float *x, int64_t rows, int K, int64_t Kp, int planes, void *out, cudaStream_t st,
                     const float *col_scale = nullptr);
 // binarize_columns (bf16 side-band) and the three pieces of x [rows, R] with the side-band's row pitch, in one launch where
-// 128-bit accesses fit.
+// 128-bit accesses fit. *leave_sums: alpha may stay in partial sums, [(R + 63) / 64][C]; on return, whether it did.
 int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, int C, float zero_to, float *wb, float *alpha,
-                           void *side, int64_t pitch, float *partial_scratch, void *pieces, cudaStream_t st);
+                           void *side, int64_t pitch, float *partial_scratch, void *pieces, cudaStream_t st, bool *leave_sums);
 // out[c] (+)= sum over rows of a[rows, C]; partial: splits * C floats of scratch.
 int column_sums(const float *a, int64_t rows, int C, float *out, int accumulate, float *partial, int splits,
                 cudaStream_t st);

@@ -1,0 +1,38 @@
+"""Binary-weight affine layers and input gradients whose product runs with the weights on the MMA rows: shapes at the
+edges of its 128 x 64 tiles, with rows that 128-bit accesses do not fit, alpha made from partial sums, accumulation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (rows, inmaps, outmaps): past the sizes of the one-launch products
+SHAPES = [(256, 1024, 4096), (63, 4100, 129), (65, 2048, 700), (129, 3000, 1027), (1, 8192, 513), (300, 1111, 2050)]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+def test_forward_and_input_gradient(M, K, N):
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b, dy = r(M, K), r(K, N), r(N), r(M, N)
+    wb, alpha = torch.zeros_like(w), torch.zeros(N, device="cuda")
+    y = F.binary_weight_affine(x, w, wb, alpha, b)
+    sign = torch.where(w > 0, 1.0, torch.where(w < 0, -1.0, 1.0))
+    a = w.double().abs().mean(0)
+    assert torch.equal(wb, sign)
+    # sums of K positive values, fp32
+    assert ((alpha.double() - a).abs() <= 4 * 2.0 ** -24 * K ** 0.5 * a).all()
+    # the tensor core's sums: 1.4e-6 of the result's root mean square however long they are, three times that
+    rms = lambda t: t.square().mean().sqrt()
+    want = (x.double() @ sign.double()) * a + b.double()
+    assert rms(y.double() - want) <= 4.2e-6 * rms(want)
+    connect = F.binary_connect_affine(x, w, torch.zeros_like(w), b)
+    want = x.double() @ sign.double() + b.double()
+    assert rms(connect.double() - want) <= 4.2e-6 * rms(want)
+    old = torch.ones_like(x)
+    dx = F.binary_weight_affine_backward(x, wb, alpha, dy, propagate_down=(True, False, False))[0]
+    want = (dy.double() * alpha.double()) @ sign.double().t()
+    assert rms(dx.double() - want) <= 4.2e-6 * rms(want)
+    acc = F.binary_weight_affine_backward(x, wb, alpha, dy, propagate_down=(True, False, False),
+                                          accum=(True, False, False), grads=(old, None, None))[0]
+    assert torch.equal(acc, dx + 1.0)
