@@ -102,24 +102,130 @@ int device_status_word(int **status) {
   return NB200_OK;
 }
 
+// ---- split K ----------------------------------------------------------------
+// y (+)= (sum over the splits of parts[split][M][N], in order) * (scale * col_scale) + col_bias, each operation rounded as
+// in the contraction's own epilogue. Four columns of a row per thread (kVec: N % 4 == 0, 16-byte aligned y rows).
+template <bool kVec>
+__global__ void __launch_bounds__(256) split_sums_kernel(const float *__restrict__ parts, int splits, int M, int N,
+                                                         GemmEpilogue ep, int64_t ldy) {
+  pdl_wait();
+  pdl_trigger();
+  const int quads = (N + 3) / 4;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (int64_t)M * quads)
+    return;
+  const int m = (int)(i / quads), n = 4 * (int)(i - (int64_t)m * quads);
+  const float *p = parts + (int64_t)m * N + n;
+  float *y = ep.y + m * ldy + n;
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+  for (int k = 0; k < splits; ++k, p += (int64_t)M * N) {
+    if (kVec) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+      s[0] += v.x, s[1] += v.y, s[2] += v.z, s[3] += v.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        s[j] += n + j < N ? __ldg(p + j) : 0.0f;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (n + j < N) {
+      s[j] = __fmul_rn(s[j], ep.col_scale ? __fmul_rn(ep.scale, __ldg(ep.col_scale + n + j)) : ep.scale);
+      if (ep.col_bias)
+        s[j] = __fadd_rn(s[j], __ldg(ep.col_bias + n + j));
+      if (ep.accumulate)
+        s[j] = __fadd_rn(y[j], s[j]);
+    }
+  if (kVec) {
+    *reinterpret_cast<float4 *>(y) = make_float4(s[0], s[1], s[2], s[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < N)
+        y[j] = s[j];
+  }
+}
+
+static int launch_split_sums(const float *parts, int splits, int M, int N, const GemmEpilogue &ep, int64_t ldy,
+                             cudaStream_t st) {
+  const bool vec = N % 4 == 0 && ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(ep.y) & 15) == 0;
+  const int64_t threads = (int64_t)M * ((N + 3) / 4);
+  NB_CUDA(launch_dependent(vec ? split_sums_kernel<true> : split_sums_kernel<false>,
+                           dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, st, parts, splits, M, N, ep, ldy));
+  return NB200_OK;
+}
+
+// Into how many parts the K blocks of a floating-point product go whose tiles do not fill the chip. A tile's time is about
+// 3 us and then its blocks', bound by L2 to shared memory (10 ns a KB); parts cost 5 us, a second launch that adds up what
+// they stored. Whole layers, in one part and in parts: [60, 8192] . [8192, 1000] 64 and 29 us, [128, 8000] . [8000, 2000] 83
+// and 60, input gradient of [16, 1024] . [1024, 4096] 48 and 30; [512, 1024] . [1024, 1024] 13.3 and, in two, 15.7.
+static int k_splits_for(int64_t tiles, int k_blocks, int block_kb) {
+  const double block_us = 0.01 * block_kb;
+  int best = 1;
+  double best_us = 0.0;
+  for (int s = 1; s <= 16 && (s == 1 || k_blocks >= 4 * s); ++s) {
+    const int64_t rounds = (tiles * s + sm_count() - 1) / sm_count();
+    const double us = rounds * (3.0 + (k_blocks + s - 1) / s * block_us) + (s > 1 ? 5.0 : 0.0);
+    if (s == 1 || us < best_us)
+      best = s, best_us = us;
+  }
+  const int per = (k_blocks + best - 1) / best;
+  return (k_blocks + per - 1) / per; // no empty part
+}
+
 // ---- launch -----------------------------------------------------------------
-template <bool kInt8, int PA, int PB, int BN, int STAGES, bool kSkip>
-static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int k_blocks,
-                       const GemmEpilogue &ep, int64_t ldy, cudaStream_t st) {
-  GemmProblem prob;
+static void fill_problem(GemmProblem &prob, int M, int N, int k_blocks, int bn, int chunk_blocks, int64_t ldy) {
   prob.M = M;
   prob.N = N;
   prob.kblocks = k_blocks;
   prob.m_tiles = (M + kTileM - 1) / kTileM;
-  prob.n_tiles = (N + BN - 1) / BN;
-  prob.bn = BN;
+  prob.n_tiles = (N + bn - 1) / bn;
+  prob.bn = bn;
   prob.row_bytes = kRowBytes;
-  prob.chunk_blocks = kInt8 ? 0 : k_chunk_blocks((kSkip ? 6 : PA * PB) * 4);
+  prob.chunk_blocks = chunk_blocks;
+  prob.k_splits = 1;
+  prob.split_blocks = k_blocks;
+  prob.split_stride = 0;
   prob.ldy = ldy;
-  return launch_contraction<kInt8, PA, PB, BN, STAGES, kSkip, GemmProblem>(ma, mb, prob, prob.m_tiles * prob.n_tiles,
-                                                                           ep, st);
 }
 
+// Runs `launch(problem, epilogue)` whole or, for few tiles, in parts of K that split_sums_kernel adds up. y is M x N.
+template <typename Problem, typename Launch>
+static int run_in_parts(Problem &prob, int block_kb, int M, int N, const GemmEpilogue &ep, int64_t ldy, cudaStream_t st,
+                        Launch launch) {
+  const int splits = ep.n_peers == 0 && !ep.row_scale && !ep.row_bias && !ep.alpha_partial
+                         ? k_splits_for((int64_t)prob.m_tiles * prob.n_tiles, prob.kblocks, block_kb)
+                         : 1;
+  if (splits == 1)
+    return launch(prob, ep);
+  AsyncScratch scratch(st);
+  NB_TRY(scratch.alloc((size_t)splits * M * N * sizeof(float)));
+  prob.k_splits = splits;
+  prob.split_blocks = (prob.kblocks + splits - 1) / splits;
+  prob.split_stride = (int64_t)M * N;
+  prob.ldy = N;
+  GemmEpilogue part{};
+  part.y = static_cast<float *>(scratch.p);
+  part.scale = 1.0f;
+  NB_TRY(launch(prob, part));
+  return launch_split_sums(part.y, splits, M, N, ep, ldy, st);
+}
+
+template <bool kInt8, int PA, int PB, int BN, int STAGES, bool kSkip>
+static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int N, int k_blocks,
+                       const GemmEpilogue &ep, int64_t ldy, cudaStream_t st) {
+  GemmProblem prob;
+  fill_problem(prob, M, N, k_blocks, BN, kInt8 ? 0 : k_chunk_blocks((kSkip ? 6 : PA * PB) * 4), ldy);
+  auto launch = [&](const GemmProblem &p, const GemmEpilogue &e) {
+    return launch_contraction<kInt8, PA, PB, BN, STAGES, kSkip, GemmProblem>(ma, mb, p, p.k_splits * p.m_tiles * p.n_tiles,
+                                                                             e, st);
+  };
+  // (int32 sums are exact in one piece only)
+  return kInt8 ? launch(prob, ep)
+               : run_in_parts(prob, (PA * kTileM + PB * BN) * kRowBytes / 1024, M, N, ep, ldy, st, launch);
+}
 // Whether y = pieces of x (three) . weights (one plane) runs as GemmTransposedProblem: where 128 x 128 tiles would leave
 // SMs idle, and its rounds of 128 x 64 tiles at 40 KB a K block cost less than those of 64 columns by 128 rows of x at 56.
 // Whole layers, alpha made in the product's epilogue instead of a launch of its own: [256, 1024] . [1024, 4096] 19.7 -> 16.0
@@ -179,22 +285,16 @@ int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch
   if (planes_a == 3 && planes_b == 1) {
     if (ep.n_peers == 0 && !ep.row_scale && !ep.row_bias && gemm_transposes(M, N)) {
       GemmTransposedProblem prob;
-      prob.M = N;
-      prob.N = M;
-      prob.kblocks = k_blocks;
-      prob.m_tiles = (N + kTileM - 1) / kTileM;
-      prob.n_tiles = (M + 63) / 64;
-      prob.bn = 64;
-      prob.row_bytes = kRowBytes;
-      prob.chunk_blocks = k_chunk_blocks(3 * 4);
-      prob.ldy = ldy;
-      GemmEpilogue ept = ep;
-      ept.row_scale = ep.col_scale, ept.row_bias = ep.col_bias;
-      ept.col_scale = ept.col_bias = nullptr;
+      fill_problem(prob, N, M, k_blocks, 64, k_chunk_blocks(3 * 4), ldy);
       NB_TRY(make_operand_map(&ma, B, false, K, pitch_b, N, 1, kTileM));
       NB_TRY(make_operand_map(&mb, A, false, K, pitch_a, M, 3, 64));
-      return launch_contraction<false, 1, 3, 64, 4, 0, GemmTransposedProblem>(ma, mb, prob, prob.m_tiles * prob.n_tiles,
-                                                                              ept, st);
+      return run_in_parts(prob, 40, M, N, ep, ldy, st, [&](const GemmTransposedProblem &p, const GemmEpilogue &e) {
+        GemmEpilogue t = e;
+        t.row_scale = e.col_scale, t.row_bias = e.col_bias;
+        t.col_scale = t.col_bias = nullptr;
+        return launch_contraction<false, 1, 3, 64, 4, 0, GemmTransposedProblem>(
+            ma, mb, p, p.k_splits * p.m_tiles * p.n_tiles, t, st);
+      });
     }
     if (!narrow) {
       NB_TRY(make_operand_map(&mb, B, false, K, pitch_b, N, 1, 128));
@@ -246,8 +346,9 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
   void *planes = base;
   void *side = base + round_up(planes_bytes, 256);
   float *partial = reinterpret_cast<float *>(base + round_up(planes_bytes, 256) + round_up(side_bytes, 256));
-  // the transposed product makes alpha from the partial sums itself
-  bool sums_left = alpha && gemm_transposes(M, N);
+  // the transposed product makes alpha from the partial sums itself, unless its K is split
+  bool sums_left = alpha && gemm_transposes(M, N) &&
+                   k_splits_for(((N + kTileM - 1) / kTileM) * ((M + 63) / 64), (int)(Kp / 64), 40) == 1;
   NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st, &sums_left));
   GemmEpilogue ep{};
   ep.y = y;

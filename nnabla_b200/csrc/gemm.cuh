@@ -99,20 +99,25 @@ struct GemmProblem {
   int M, N, kblocks, m_tiles, n_tiles, bn;
   int row_bytes; // bytes of one K block per operand row (128 or 64)
   int chunk_blocks; // K blocks accumulated in tensor memory before the fp32 registers take over (0 = all)
+  int k_splits;     // the K loop is cut into this many tiles (of split_blocks K blocks, the last of the rest), each with a result of its own
+  int split_blocks;
+  int64_t split_stride; // elements between the results of consecutive splits in y
   int64_t ldy;
   __device__ __forceinline__ int k_chunk() const { return chunk_blocks; }
-  __device__ __forceinline__ int num_tiles() const { return m_tiles * n_tiles; }
+  __device__ __forceinline__ int num_tiles() const { return k_splits * m_tiles * n_tiles; }
   __device__ __forceinline__ int k_blocks() const { return kblocks; }
   __device__ __forceinline__ uint32_t umma_n() const { return (uint32_t)bn; }
   __device__ __forceinline__ uint32_t b_tx_bytes() const { return (uint32_t)(bn * row_bytes); }
   __device__ __forceinline__ void decode(int tile, Tile &t) const {
+    const int split = tile / (m_tiles * n_tiles);
+    tile -= split * (m_tiles * n_tiles);
     t.m0 = (tile % m_tiles) * kTileM;
     t.m_end = M;
     t.n0 = (tile / m_tiles) * bn;
     t.img0 = t.oy0 = t.group = 0;
-    t.kb0 = 0;
-    t.kb1 = kblocks;
-    t.y_off = 0;
+    t.kb0 = split * split_blocks;
+    t.kb1 = t.kb0 + split_blocks < kblocks ? t.kb0 + split_blocks : kblocks;
+    t.y_off = split * split_stride;
   }
   __device__ __forceinline__ void load_a(const CUtensorMap *map, void *dst, uint64_t *bar, int kb, const Tile &t,
                                          int plane, int epb) const {
@@ -498,7 +503,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           if constexpr (Problem::kTransposed) {
             // one rounding per operation, as below
-            float *yp = ep.y + (int64_t)(t.n0 + c0) * prob.ldy + my_row;
+            float *yp = ep.y + t.y_off + (int64_t)(t.n0 + c0) * prob.ldy + my_row;
             const int left = prob.N - t.n0 - c0; // rows of y
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
