@@ -502,8 +502,8 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
     AsyncScratch scratch(st);
     NB_TRY(scratch.alloc(a_bytes + b_bytes));
     uint8_t *base = static_cast<uint8_t *>(scratch.p);
-    NB_TRY(split_rows_bf16(dy, M, (int)N, Np, 3, base, st, w_col_scale));
-    NB_TRY(split_rows_bf16(w, K, (int)N, Np, planes_w, base + a_bytes, st));
+    NB_TRY(split_rows_bf16(SplitRows{dy, w_col_scale, base, M, (int)N, 3},
+                           SplitRows{w, nullptr, base + a_bytes, K, (int)N, planes_w}, Np, st));
     GemmEpilogue ep{};
     ep.y = dx;
     ep.scale = 1.0f;
@@ -521,8 +521,7 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
     uint8_t *pa = base + xt_bytes + dyt_bytes, *pb = pa + a_bytes;
     NB_TRY(transpose_f32(x, (int)M, (int)K, xt, st));
     NB_TRY(transpose_f32(dy, (int)M, (int)N, dyt, st));
-    NB_TRY(split_rows_bf16(xt, K, (int)M, Mp, 3, pa, st));
-    NB_TRY(split_rows_bf16(dyt, N, (int)M, Mp, 3, pb, st));
+    NB_TRY(split_rows_bf16(SplitRows{xt, nullptr, pa, K, (int)M, 3}, SplitRows{dyt, nullptr, pb, N, (int)M, 3}, Mp, st));
     GemmEpilogue ep{};
     ep.y = dw;
     ep.scale = 1.0f;
@@ -622,8 +621,7 @@ int nb200_affine_f32(const float *x, const float *w, const float *bias, float *y
   uint8_t *base = static_cast<uint8_t *>(scratch.p);
   float *wt32 = reinterpret_cast<float *>(base + xa + wa);
   NB_TRY(transpose_f32(w, (int)K, (int)N, wt32, st));
-  NB_TRY(split_rows_bf16(x, M, (int)K, Kp, 3, base, st));
-  NB_TRY(split_rows_bf16(wt32, N, (int)K, Kp, 3, base + xa, st));
+  NB_TRY(split_rows_bf16(SplitRows{x, nullptr, base, M, (int)K, 3}, SplitRows{wt32, nullptr, base + xa, N, (int)K, 3}, Kp, st));
   GemmEpilogue ep{};
   ep.y = y;
   ep.scale = 1.0f;

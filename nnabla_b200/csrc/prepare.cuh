@@ -25,10 +25,15 @@ inline int64_t codes_slots(int64_t channels, int group) {
   const int64_t ctot = (int64_t)group * c_pad_g;
   return ctot < E ? E : ctot;
 }
-// fp32 [rows, K] -> bf16 [planes][rows][Kp] (planes = 1 or 3; hi, mid, lo).
-// col_scale (K floats or NULL): x[r, k] is multiplied by col_scale[k] first.
-int split_rows_bf16(const float *x, int64_t rows, int K, int64_t Kp, int planes, void *out, cudaStream_t st,
-                    const float *col_scale = nullptr);
+// fp32 [rows, K] -> bf16 [planes][rows][Kp] (planes = 1 or 3; hi, mid, lo), up to two operands in one launch (rows = 0: none).
+// col_scale (K floats or NULL): x[r, k] is multiplied by col_scale[k] first. out is 16-byte aligned.
+struct SplitRows {
+  const float *x, *col_scale;
+  void *out;
+  int64_t rows;
+  int K, planes;
+};
+int split_rows_bf16(const SplitRows &a, const SplitRows &b, int64_t Kp, cudaStream_t st);
 // binarize_columns (bf16 side-band) and the three pieces of x [rows, R] with the side-band's row pitch, in one launch where
 // 128-bit accesses fit. *leave_sums: alpha may stay in partial sums, [(R + 63) / 64][C]; on return, whether it did.
 int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, int C, float zero_to, float *wb, float *alpha,
