@@ -455,7 +455,7 @@ static int affine_fxp8(const float *xq, const float *wq, float delta_x, float de
 // Backward of y = x . W (+ b) for row-major x [M, K], W [K, N], dy [M, N]
 // (Affine::backward_impl, src/nbla/function/generic/affine.cpp:98-138):
 //   dx (+)= dy . W^T     A = dy [M][N], B = W [K][N]: both already contraction-major
-//   dW (+)= x^T . dy     A = x^T [K][M], B = dy^T [N][M]: two fp32 transposes first
+//   dW (+)= x^T . dy     A = x^T [K][M], B = dy^T [N][M]: transposed while they are split
 //   db (+)= column sums of dy
 // `w_exact_bf16`: W holds values that are exact in bf16 (the +-1 / zero_to
 // weights of the binary layers); it is then used as one bf16 plane and
@@ -512,16 +512,17 @@ static int affine_backward(const float *x, const float *w, const float *w_col_sc
   }
   if (dw) {
     const int64_t Mp = round_up(M, 64);
-    const size_t xt_bytes = round_up((size_t)K * M * 4, 256), dyt_bytes = round_up((size_t)N * M * 4, 256);
     const size_t a_bytes = round_up((size_t)3 * K * Mp * 2, 256), b_bytes = round_up((size_t)3 * N * Mp * 2, 256);
+    const bool with_sums = db && Mp / 64 <= 256; // (one thread adds up a column's)
     AsyncScratch scratch(st);
-    NB_TRY(scratch.alloc(xt_bytes + dyt_bytes + a_bytes + b_bytes));
-    uint8_t *base = static_cast<uint8_t *>(scratch.p);
-    float *xt = reinterpret_cast<float *>(base), *dyt = reinterpret_cast<float *>(base + xt_bytes);
-    uint8_t *pa = base + xt_bytes + dyt_bytes, *pb = pa + a_bytes;
-    NB_TRY(transpose_f32(x, (int)M, (int)K, xt, st));
-    NB_TRY(transpose_f32(dy, (int)M, (int)N, dyt, st));
-    NB_TRY(split_rows_bf16(SplitRows{xt, nullptr, pa, K, (int)M, 3}, SplitRows{dyt, nullptr, pb, N, (int)M, 3}, Mp, st));
+    NB_TRY(scratch.alloc(a_bytes + b_bytes + (with_sums ? (size_t)(Mp / 64) * N * sizeof(float) : 0)));
+    uint8_t *pa = static_cast<uint8_t *>(scratch.p), *pb = pa + a_bytes;
+    float *sums = with_sums ? reinterpret_cast<float *>(pb + b_bytes) : nullptr;
+    NB_TRY(split_columns_bf16(SplitColumns{x, pa, nullptr, M, (int)K, 3}, SplitColumns{dy, pb, sums, M, (int)N, 3}, Mp, st));
+    if (with_sums) {
+      NB_TRY(column_sums_finish(sums, (int)N, (int)(Mp / 64), db, accum_db, st));
+      db = nullptr;
+    }
     GemmEpilogue ep{};
     ep.y = dw;
     ep.scale = 1.0f;
@@ -614,14 +615,12 @@ int nb200_affine_f32(const float *x, const float *w, const float *bias, float *y
     return launch_small_gemm<false, false, SmallB::kPlain>(P, st);
   }
   const int64_t Kp = round_up(K, 64);
-  // w [K, N] is transposed through a fp32 staging pass into [N][K] planes.
   AsyncScratch scratch(st);
   const size_t xa = round_up((size_t)3 * M * Kp * 2, 256), wa = round_up((size_t)3 * N * Kp * 2, 256);
-  NB_TRY(scratch.alloc(xa + wa + (size_t)N * K * 4));
+  NB_TRY(scratch.alloc(xa + wa));
   uint8_t *base = static_cast<uint8_t *>(scratch.p);
-  float *wt32 = reinterpret_cast<float *>(base + xa + wa);
-  NB_TRY(transpose_f32(w, (int)K, (int)N, wt32, st));
-  NB_TRY(split_rows_bf16(SplitRows{x, nullptr, base, M, (int)K, 3}, SplitRows{wt32, nullptr, base + xa, N, (int)K, 3}, Kp, st));
+  NB_TRY(split_rows_bf16(SplitRows{x, nullptr, base, M, (int)K, 3}, SplitRows{}, Kp, st));
+  NB_TRY(split_columns_bf16(SplitColumns{w, base + xa, nullptr, K, (int)N, 3}, SplitColumns{}, Kp, st));
   GemmEpilogue ep{};
   ep.y = y;
   ep.scale = 1.0f;

@@ -252,6 +252,15 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 
   l = __float2bfloat16_rn(r2);
 }
 
+// Four neighbouring values of a row of `extent` floats from column k on, zero past its end; kVec: one 128-bit load
+// (the row starts on 16 bytes and extent is a multiple of 4).
+template <bool kVec> __device__ __forceinline__ float4 load_quad(const float *__restrict__ row, int k, int extent) {
+  if (kVec)
+    return k < extent ? __ldcs(reinterpret_cast<const float4 *>(row + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(k < extent ? row[k] : 0.f, k + 1 < extent ? row[k + 1] : 0.f, k + 2 < extent ? row[k + 2] : 0.f,
+                     k + 3 < extent ? row[k + 3] : 0.f);
+}
+
 // Up to two operands with rows of Kp values in one launch. A thread takes eight values of a row (Kp is a multiple of 64): two
 // 128-bit loads (kVec: K % 4 == 0, 16-byte aligned x) and a 128-bit store per plane. Bound by HBM; with a value per
 // thread and a launch per operand the input gradient of a [16, 4096] . [4096, 4096] layer took 104 us, now 27, of
@@ -293,6 +302,59 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const SplitRows A, cons
   for (int pl = 0; pl < 3; ++pl)
     if (pl < P.planes)
       *reinterpret_cast<uint4 *>(dst + pl * P.rows * Kp) = *reinterpret_cast<const uint4 *>(piece[pl]);
+}
+
+// The same for operands along whose rows the product does not contract (x and dy of a weight gradient, plain weights):
+// source [rows][cols] -> [planes][cols][Rp], rows padded with zeros to Rp, a multiple of 64. 64 x 64 tiles through shared
+// memory, eight rows of a column per thread, 128 bytes of a plane per eight lanes. sums (may be NULL): receives the column
+// sums of each tile, [tile row][cols]. With an fp32 transpose first and the split behind it, and dy read again for its
+// sums, the weight gradient of [256, 1024] . [1024, 4096] took 43 us, now 24.5; of [1024, 2048] . [2048, 700] 56, now 36.
+template <bool kVec>
+__global__ void __launch_bounds__(256) split_columns_kernel(const SplitColumns A, const SplitColumns B, unsigned a_blocks,
+                                                            int64_t Rp) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ float tile[64][65];
+  const bool first = blockIdx.x < a_blocks;
+  const SplitColumns &P = first ? A : B;
+  const unsigned b = blockIdx.x - (first ? 0u : a_blocks), row_tiles = (unsigned)(Rp / 64);
+  const unsigned rt = b % row_tiles;
+  const int r0 = 64 * (int)rt, c0 = 64 * (int)(b / row_tiles);
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int r = (threadIdx.x >> 4) + 16 * it, c = 4 * (threadIdx.x & 15);
+    const float *row = P.x + (int64_t)(r0 + r) * P.cols;
+    const float4 v = r0 + r < P.rows ? load_quad<kVec>(row, c0 + c, P.cols) : make_float4(0.f, 0.f, 0.f, 0.f);
+    tile[r][c] = v.x, tile[r][c + 1] = v.y, tile[r][c + 2] = v.z, tile[r][c + 3] = v.w;
+  }
+  __syncthreads();
+  const int g = threadIdx.x & 7;
+  __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(P.out);
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int c = (threadIdx.x >> 3) + 32 * it;
+    __align__(16) __nv_bfloat16 piece[3][8];
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float v = tile[8 * g + j][c];
+      sum += v;
+      split3(v, piece[0][j], piece[1][j], piece[2][j]);
+    }
+    if (P.sums) {
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (g == 0 && c0 + c < P.cols)
+        P.sums[(int64_t)rt * P.cols + c0 + c] = sum;
+    }
+    if (c0 + c < P.cols)
+#pragma unroll
+      for (int pl = 0; pl < 3; ++pl)
+        if (pl < P.planes)
+          *reinterpret_cast<uint4 *>(out + ((int64_t)pl * P.cols + c0 + c) * Rp + r0 + 8 * g) =
+              *reinterpret_cast<const uint4 *>(piece[pl]);
+  }
 }
 
 // Both operands of a binary-weight affine layer in one launch: the weights' 64 x 64 tiles first, then four values of x per
@@ -554,35 +616,6 @@ __global__ void __launch_bounds__(256) transpose_i8_kernel(const int8_t *__restr
   }
 }
 
-// fp32 [R, C] -> [C][R] (transpose), tile 32 x 32 through shared memory.
-__global__ void __launch_bounds__(256) transpose_f32_kernel(const float *__restrict__ src, int R, int C,
-                                                            float *__restrict__ dst) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ float tile[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int rr = ty; rr < 32; rr += 8) {
-    const int r = r0 + rr, c = c0 + tx;
-    tile[rr][tx] = (r < R && c < C) ? src[(int64_t)r * C + c] : 0.0f;
-  }
-  __syncthreads();
-  for (int cc = ty; cc < 32; cc += 8) {
-    const int c = c0 + cc, r = r0 + tx;
-    if (c < C && r < R)
-      dst[(int64_t)c * R + r] = tile[tx][cc];
-  }
-}
-
-// Four neighbouring values of a row of `extent` floats from column k on, zero past its end; kVec: one 128-bit load
-// (the row starts on 16 bytes and extent is a multiple of 4).
-template <bool kVec> __device__ __forceinline__ float4 load_quad(const float *__restrict__ row, int k, int extent) {
-  if (kVec)
-    return k < extent ? __ldcs(reinterpret_cast<const float4 *>(row + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-  return make_float4(k < extent ? row[k] : 0.f, k + 1 < extent ? row[k + 1] : 0.f, k + 2 < extent ? row[k + 2] : 0.f,
-                     k + 3 < extent ? row[k + 3] : 0.f);
-}
-
 // Both operands of the 8-bit fixed-point affine in one launch: x [M, K] -> codes [M][Kp] and w [K, N] -> transposed
 // codes [N][Kp] (Kp = K rounded up to 128, zero padded). HBM-bound: 5 bytes per value. Blocks [0, x_blocks): a warp
 // converts four runs of 128 values, each one 512-byte load and one 128-byte store. The other blocks: a tile of 128 k
@@ -759,6 +792,18 @@ int split_rows_bf16(const SplitRows &a, const SplitRows &b, int64_t Kp, cudaStre
   return NB200_OK;
 }
 
+int split_columns_bf16(const SplitColumns &a, const SplitColumns &b, int64_t Rp, cudaStream_t st) {
+  NB_CHECK(Rp % 64 == 0, NB200_EVALUE, "the padded row count must be a multiple of 64");
+  auto blocks = [&](const SplitColumns &p) { return (Rp / 64) * ((p.cols + 63) / 64); };
+  auto vec = [](const SplitColumns &p) {
+    return p.cols == 0 || (p.cols % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
+  };
+  NB_CHECK(blocks(a) + blocks(b) < (1ll << 31), NB200_ENOTIMPL, "operand too large");
+  NB_CUDA(launch_dependent(vec(a) && vec(b) ? split_columns_kernel<true> : split_columns_kernel<false>,
+                           dim3((unsigned)(blocks(a) + blocks(b))), dim3(256), 0, st, a, b, (unsigned)blocks(a), Rp));
+  return NB200_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Two fp16 pieces of an fp32 tensor: with s = 2^-e chosen from the tensor's largest magnitude so that
 // max |x| * s lies in [2^14, 2^15), x * s = p0 + p1 with p0 = fp16(x * s), p1 = fp16(x * s - p0): 22
@@ -884,23 +929,18 @@ int column_sums(const float *a, int64_t rows, int C, float *out, int accumulate,
                 cudaStream_t st) {
   const dim3 grid((C + 255) / 256, splits);
   NB_CUDA(launch_dependent(column_partial_sums_kernel, grid, dim3(256), 0, st, a, rows, C, partial));
-  NB_LAUNCH_CHECK();
+  return column_sums_finish(partial, C, splits, out, accumulate, st);
+}
+
+int column_sums_finish(const float *partial, int C, int splits, float *out, int accumulate, cudaStream_t st) {
   NB_CUDA(launch_dependent(column_finish_kernel, dim3((C + 255) / 256), dim3(256), 0, st, partial, C, splits, out,
                            accumulate));
-  NB_LAUNCH_CHECK();
   return NB200_OK;
 }
 
 int transpose_i8(const int8_t *src, int R, int C, int8_t *dst, int64_t pitch, cudaStream_t st) {
   const dim3 grid((C + 63) / 64, (R + 63) / 64);
   NB_CUDA(launch_dependent(transpose_i8_kernel, grid, dim3(256), 0, st, src, R, C, dst, pitch));
-  NB_LAUNCH_CHECK();
-  return NB200_OK;
-}
-
-int transpose_f32(const float *src, int R, int C, float *dst, cudaStream_t st) {
-  const dim3 grid((C + 31) / 32, (R + 31) / 32);
-  NB_CUDA(launch_dependent(transpose_f32_kernel, grid, dim3(256), 0, st, src, R, C, dst));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }

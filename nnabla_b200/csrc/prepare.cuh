@@ -34,6 +34,16 @@ struct SplitRows {
   int K, planes;
 };
 int split_rows_bf16(const SplitRows &a, const SplitRows &b, int64_t Kp, cudaStream_t st);
+// fp32 [rows, cols] -> bf16 [planes][cols][Rp], rows padded with zeros to Rp (a multiple of 64); sums (or NULL): column sums of
+// every 64 rows, [Rp / 64][cols]. Up to two operands of Rp rows in one launch (cols = 0: none). out is 16-byte aligned.
+struct SplitColumns {
+  const float *x;
+  void *out;
+  float *sums;
+  int64_t rows;
+  int cols, planes;
+};
+int split_columns_bf16(const SplitColumns &a, const SplitColumns &b, int64_t Rp, cudaStream_t st);
 // binarize_columns (bf16 side-band) and the three pieces of x [rows, R] with the side-band's row pitch, in one launch where
 // 128-bit accesses fit. *leave_sums: alpha may stay in partial sums, [(R + 63) / 64][C]; on return, whether it did.
 int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, int C, float zero_to, float *wb, float *alpha,
@@ -41,6 +51,8 @@ int binary_affine_operands(const float *x, int64_t rows, const float *w, int R, 
 // out[c] (+)= sum over rows of a[rows, C]; partial: splits * C floats of scratch.
 int column_sums(const float *a, int64_t rows, int C, float *out, int accumulate, float *partial, int splits,
                 cudaStream_t st);
+// out (+)= the sums of `splits` rows of partial [splits][C], in order
+int column_sums_finish(const float *partial, int C, int splits, float *out, int accumulate, cudaStream_t st);
 // fp32 NCHW -> NHWC planes [planes][N][HW][ctot] (planes = 3 or 1: bf16 pieces;
 // planes = 0: int8 codes of multiples of delta). Channel c of group g is stored
 // at slot g * c_pad_g + (c - g * Cg); all other slots are zero.
@@ -67,8 +79,6 @@ __host__ __device__ __forceinline__ int half_pair_exponent(uint32_t maxbits) {
 }
 // int8 [R, C] -> [C][pitch].
 int transpose_i8(const int8_t *src, int R, int C, int8_t *dst, int64_t pitch, cudaStream_t st);
-// fp32 [R, C] -> [C][R].
-int transpose_f32(const float *src, int R, int C, float *dst, cudaStream_t st);
 // x [M, K] multiples of delta_x -> int8 [M][Kp] and w [K, N] multiples of delta_w -> int8 [N][Kp] (transposed);
 // Kp a multiple of 128, zero padded, xc and wt 16-byte aligned.
 int fxp8_operands(const float *x, int64_t M, int K, int64_t Kp, float delta_x, int8_t *xc, const float *w, int N,
