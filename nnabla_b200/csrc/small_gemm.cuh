@@ -15,6 +15,8 @@
 // last to end: [100, 784] . [784, 500] 10.6 us, now 9.5); the partial tiles go to shared memory in rows of 36 floats as
 // 16-byte writes (one value at a time, eight rows to a bank, x^T . dy of the same layer took 9.6 us, now 7.8).
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 #include "pdl.cuh"
 #include "prepare.cuh"
@@ -333,15 +335,22 @@ inline int64_t small_gemm_cost(int64_t M, int64_t N, int64_t K) {
   const int64_t waves = (small_gemm_tiles(M, N, 32) + sm_count() - 1) / sm_count();
   return M > 65535 * 16 ? INT64_MAX : waves * (128 + (K + kSmallK - 1) / kSmallK * kSmallK);
 }
-// The tensor-core route's time on sizes where both were measured grows with K from what its launches cost:
-// binarize + split + product 12 to 18 us, dy and weights split + product 12 to 20 (for K up to kSmallMaxK, the factors'
-// place), two three-piece operands 13 + 18 per 1024 of K, the same behind two transposes and with the column sums 21 to 37.
-inline bool small_gemm_binarized(int64_t M, int64_t N, int64_t K) { return small_gemm_cost(M, N, K) <= 1024 + K / 4; }
-inline bool small_gemm_scaled(int64_t M, int64_t N, int64_t K) {
-  return K <= kSmallMaxK && small_gemm_cost(M, N, K) <= 1024 + K * 5 / 8;
+// Lines to the tensor-core route, from both routes' times on 200 shapes of 1 to 4096 rows and 16 to 8192 columns: that
+// route's launches are a constant and a part that grows with K, and its passes over B with N * K ([1, 4096] . [4096, 4096]
+// 27 us here, 69 there, binarized 41 and 49). Where the first line of each allows more, the tensor-core route is up to a
+// third the faster one by now, but seven times as far from 64-bit sums (1.4e-6 of the result against 2e-7).
+inline bool small_gemm_binarized(int64_t M, int64_t N, int64_t K) {
+  return small_gemm_cost(M, N, K) <= std::max(1024 + K / 4, 768 + K * 3 / 8 + N * K / 8192);
 }
-inline bool small_gemm_plain(int64_t M, int64_t N, int64_t K) { return small_gemm_cost(M, N, K) <= 1024 + K * 3 / 2; }
-inline bool small_gemm_transposed(int64_t M, int64_t N, int64_t K) { return small_gemm_cost(M, N, K) <= 2048 + K * 3; }
+inline bool small_gemm_scaled(int64_t M, int64_t N, int64_t K) { // (the factors' place)
+  return K <= kSmallMaxK && small_gemm_cost(M, N, K) <= std::max(1024 + K * 5 / 8, 768 + K * 3 / 8 + N * K / 8192);
+}
+inline bool small_gemm_plain(int64_t M, int64_t N, int64_t K) {
+  return small_gemm_cost(M, N, K) <= std::max(1024 + K * 3 / 2, 1536 + K * 3 / 8 + N * K / 4096);
+}
+inline bool small_gemm_transposed(int64_t M, int64_t N, int64_t K) {
+  return small_gemm_cost(M, N, K) <= std::max(2048 + K * 3, 1024 + K / 4 + N * K / 4096);
+}
 
 template <int TM, bool kAT, bool kBT> constexpr size_t small_gemm_smem() {
   constexpr size_t smem =
