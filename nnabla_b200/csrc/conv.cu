@@ -985,6 +985,11 @@ void int8_side_layout(int Cg, int taps, int &c_slots, int64_t &wpitch) {
 long long *g_cc_trace = nullptr;
 #endif
 
+// Columns that the tiles cover: the maps, and the slots behind them of a channel-last result, which are written as zeros.
+int code_columns(const ConvGeometry &g, int slots_out, const ConvCodesEpilogue &ep) {
+  return ep.y_nchw || g.Ko > slots_out ? g.Ko : slots_out;
+}
+
 // halves = 2: two row blocks of h_box / 2 output rows each per tile (halo form).
 template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false, int kHalves = 1>
 int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot, const int8_t *side, int64_t wpitch,
@@ -1015,7 +1020,7 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
   p.n_box = n_box;
   p.tiles_h = (g.Ho + h_box - 1) / h_box;
   p.tiles_n = (g.N + n_box - 1) / n_box;
-  p.n_tiles = (g.Ko + BN - 1) / BN;
+  p.n_tiles = (code_columns(g, slots_out, ep) + BN - 1) / BN;
   p.bn = BN;
   p.kw = g.kw;
   p.taps = g.kh * g.kw;
@@ -1036,11 +1041,19 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
   const int rows_alloc =
       (((kHalves - 1) * p.h_half * wp + (g.kh - 1) * g.dh * wp + (g.kw - 1) * g.dw + kTileM) + 7) / 8 * 8;
   p.a_tile_bytes = (rows_alloc > hp * wp ? rows_alloc : (hp * wp + 7) / 8 * 8) * RB;
+  p.a_bufs = 2;
+  const int tiles = p.n_tiles * p.tiles_h * p.tiles_n;
+  if (kHalo && p.n_tiles > 1) {
+    // one tile per block, one buffer; rows behind a channel block's pixels are the next block's, or the weights'
+    NB_CHECK(tiles <= sm_count() && rows_alloc <= p.taps * p.cblocks * BN, NB200_EVALUE, "column tiles need a block each");
+    p.a_bufs = 1;
+    p.a_tile_bytes = (hp * wp + 7) / 8 * 8 * RB;
+  }
   auto kernel = conv_codes_tcgen05_kernel<BN, STAGES, RB, kResidentB, kHalo, kHalves>;
   constexpr size_t smem_fixed = conv_codes_smem_bytes<BN, STAGES, RB, kResidentB, kHalo>();
   static_assert(smem_fixed <= 227 * 1024, "shared memory budget");
   const size_t smem = smem_fixed + (kResidentB ? (size_t)p.taps * p.cblocks * BN * RB : 0) +
-                      (kHalo ? (size_t)2 * p.cblocks * p.a_tile_bytes : 0);
+                      (kHalo ? (size_t)p.a_bufs * p.cblocks * p.a_tile_bytes : 0);
   NB_CHECK(smem <= 227 * 1024, NB200_EVALUE, "resident weights do not fit in shared memory");
   static bool configured[64];
   int dev = 0;
@@ -1052,7 +1065,6 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
   }
   int *status = nullptr;
   NB_TRY(device_status_word(&status));
-  const int tiles = p.n_tiles * p.tiles_h * p.tiles_n;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   NB_CUDA(launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), smem, st, mx, mw, p, ep, status));
   NB_LAUNCH_CHECK();
@@ -1149,7 +1161,7 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
                                                     ep, st)
   // weights resident in shared memory when one column tile covers the maps and they fit beside the ring
   const size_t w_bytes = (size_t)g.kh * g.kw * cblocks * (narrow_rows ? 64 : 128);
-  if (g.sh == 1 && g.sw == 1 && g.kh * g.kw > 1 && g.Ko <= 128) {
+  if (g.sh == 1 && g.sw == 1 && g.kh * g.kw > 1) {
     // halo form: the tile's rows are h rows of the padded width wp; one input box per tile
     const int RBh = narrow_rows ? 64 : 128, BNh = g.Ko <= 64 ? 64 : 128;
     const int wp = g.Wo + (g.kw - 1) * g.dw;
@@ -1165,28 +1177,42 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
         }
       const int hp = hh + (g.kh - 1) * g.dh;
       const int rows_alloc = (((g.kh - 1) * g.dh * wp + (g.kw - 1) * g.dw + kTileM) + 7) / 8 * 8;
-      const size_t a_bytes = (size_t)(rows_alloc > hp * wp ? rows_alloc : (hp * wp + 7) / 8 * 8) * RBh;
-      const size_t need = 2 * cblocks * a_bytes + w_bytes * BNh + 8 * 1024;
-      if (need <= 220 * 1024 && wp <= 256 && hp <= 256) {
-        if (narrow_rows) {
-          if (g.Ko <= 64) {
-            // two row blocks per tile, once every SM has more than one such tile to do (below that the larger tile
-            // only makes the single round of tiles longer)
-            const int h2 = 2 * hh < g.Ho ? 2 * hh : (g.Ho + 1) / 2 * 2;
-            const int64_t pairs = (int64_t)g.N * ((g.Ho + h2 - 1) / h2);
-            const int hp2 = h2 + (g.kh - 1) * g.dh;
-            const size_t a2_bytes = (size_t)(rows_alloc + (h2 / 2) * wp > hp2 * wp ? rows_alloc + (h2 / 2) * wp
-                                                                                   : (hp2 * wp + 7) / 8 * 8) * RBh;
-            if (pairs > sm_count() && h2 / 2 >= 1 && hp2 <= 256 && 2 * a2_bytes + w_bytes * BNh + 8 * 1024 <= 220 * 1024)
-              return launch_conv_codes<64, 1, 64, true, true, 2>(g, x_codes, ctot, side, wpitch, cblocks, h2, 1,
-                                                                 (int)slots_out, ep, st);
-            NB_CC_HALO(64, 64);
-          }
-          NB_CC_HALO(128, 64);
-        }
-        if (g.Ko <= 64)
+      if (!narrow_rows && g.Ko > 64 && wp <= 256 && hp <= 256) {
+        // column tiles of 32 or 64 maps while every block has one
+        const int64_t boxes = (int64_t)g.N * ((g.Ho + hh - 1) / hh);
+        auto fits = [&](int bn) {
+          return boxes * ((code_columns(g, (int)slots_out, ep) + bn - 1) / bn) <= sm_count() && rows_alloc <= g.kh * g.kw * cblocks * bn &&
+                 (size_t)cblocks * ((hp * wp + 7) / 8 * 8) * 128 + w_bytes * bn + 8 * 1024 <= 220 * 1024;
+        };
+        if (fits(32))
+          NB_CC_HALO(32, 128);
+        if (g.Ko > 128 && fits(64))
           NB_CC_HALO(64, 128);
-        NB_CC_HALO(128, 128);
+      }
+      if (g.Ko <= 128) {
+        const size_t a_bytes = (size_t)(rows_alloc > hp * wp ? rows_alloc : (hp * wp + 7) / 8 * 8) * RBh;
+        const size_t need = 2 * cblocks * a_bytes + w_bytes * BNh + 8 * 1024;
+        if (need <= 220 * 1024 && wp <= 256 && hp <= 256) {
+          if (narrow_rows) {
+            if (g.Ko <= 64) {
+              // two row blocks per tile, once every SM has more than one such tile to do (below that the larger tile
+              // only makes the single round of tiles longer)
+              const int h2 = 2 * hh < g.Ho ? 2 * hh : (g.Ho + 1) / 2 * 2;
+              const int64_t pairs = (int64_t)g.N * ((g.Ho + h2 - 1) / h2);
+              const int hp2 = h2 + (g.kh - 1) * g.dh;
+              const size_t a2_bytes = (size_t)(rows_alloc + (h2 / 2) * wp > hp2 * wp ? rows_alloc + (h2 / 2) * wp
+                                                                                     : (hp2 * wp + 7) / 8 * 8) * RBh;
+              if (pairs > sm_count() && h2 / 2 >= 1 && hp2 <= 256 && 2 * a2_bytes + w_bytes * BNh + 8 * 1024 <= 220 * 1024)
+                return launch_conv_codes<64, 1, 64, true, true, 2>(g, x_codes, ctot, side, wpitch, cblocks, h2, 1,
+                                                                   (int)slots_out, ep, st);
+              NB_CC_HALO(64, 64);
+            }
+            NB_CC_HALO(128, 64);
+          }
+          if (g.Ko <= 64)
+            NB_CC_HALO(64, 128);
+          NB_CC_HALO(128, 128);
+        }
       }
     }
   }
@@ -1220,6 +1246,8 @@ int convolution_codes_folded(const int8_t *x_codes, const int8_t *side, const fl
         const int64_t blocks = ptiles * ((g.Ko + bn - 1) / bn);
         return (double)((blocks + sms - 1) / sms) * (55.0 + 0.6 * bn);
       };
+      if (cost(32) < cost(64) && cost(32) < cost(128) && cost(32) < cost(256))
+        NB_CC(32, 10, 128);
       if (cost(64) < cost(128) && cost(64) < cost(256))
         NB_CC(64, 8, 128);
       if (cost(128) < cost(256))

@@ -45,6 +45,7 @@ struct ConvCodesProblem {
   int wp, hp;          // wp = Wo + (kw - 1) * dw, hp = h_box + (kh - 1) * dh
   int h_half;          // output rows of one MMA row block (h_box, or half of it with two row blocks per tile)
   int a_tile_bytes;    // bytes of one channel block's pixel tile in shared memory (readable rows included)
+  int a_bufs;          // pixel-tile buffers: 2, or 1 where every block has one tile
   __device__ __forceinline__ int num_tiles() const { return n_tiles * tiles_h * tiles_n; }
   __device__ __forceinline__ int k_blocks() const { return taps * cblocks; }
 };
@@ -132,6 +133,11 @@ constexpr int kCodesKTable = 64; // K blocks whose coordinates are tabulated onc
 // field is needed; setting one breaks it). This cuts the copy engine's rows per tile by the number
 // of taps.
 //
+// Several column tiles (more maps than BN) in the halo form: every block then has one tile, with the weights of its own
+// columns (launch_conv_codes checks it). For the few pixels of late stages and small batches this takes an image's pixels
+// once instead of once per tap, and narrow tiles spread the weights, which one SM's port brings in at 64 bytes a cycle:
+// 512 -> 512 maps of 7 x 7 pixels, one image, 10.4 us with a box per tap and 64 columns, now 8.4 (launch and wait included).
+//
 // kHalves = 2 (halo form, at most 64 maps): a tile is two MMA row blocks, rows [0, 128) and the 128 rows from
 // h_half * wp on, of ONE input box of 2 * h_half output rows; their accumulators lie side by side in tensor memory.
 // With one block of 18 small MMAs per tile the hand-over between the roles (four barriers, the commits, the
@@ -163,8 +169,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // resident weights (kResidentB): [k block][BN rows] behind the ring
   const uint32_t resident_bytes = kResidentB ? (uint32_t)(prob.taps * prob.cblocks) * kBBytes : 0u;
-  // halo form: the ring's place is taken by two buffers of cblocks pixel tiles each
-  const uint32_t ring_bytes = kHalo ? 2u * (uint32_t)(prob.cblocks * prob.a_tile_bytes) : (uint32_t)STAGES * kStageBytes;
+  // halo form: the ring's place is taken by two buffers (one) of cblocks pixel tiles each
+  const uint32_t ring_bytes =
+      kHalo ? (uint32_t)(prob.a_bufs * prob.cblocks * prob.a_tile_bytes) : (uint32_t)STAGES * kStageBytes;
   uint8_t *b_resident = smem + ring_bytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + ring_bytes + resident_bytes);
   uint64_t *full_bar = bars;
@@ -250,17 +257,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       bool ok = true;
       const uint32_t tx_bytes = (uint32_t)(prob.pixels * RB) + (kResidentB ? 0u : kBBytes);
       // the weights behind the first pixels: the first MMAs need both, the others the rest of the weights
-      auto load_weights = [&]() {
+      auto load_weights = [&](int n0) {
         for (int q = 0; q < kWeightParts; ++q) {
           const int kb0 = q * part_blocks, kb1 = min(kb0 + part_blocks, k_blocks);
           if (kb0 < kb1)
             ptx::mbar_expect_tx(b_full + q, (uint32_t)(kb1 - kb0) * kBBytes);
           for (int kb = kb0; kb < kb1; ++kb)
-            ptx::tma_load_3d(b_resident + (size_t)kb * kBBytes, &map_w, b_full + q, kb * kElems, 0, 0);
+            ptx::tma_load_3d(b_resident + (size_t)kb * kBBytes, &map_w, b_full + q, kb * kElems, n0, 0);
         }
       };
       if (kResidentB && !kHalo && (int)blockIdx.x < num_tiles)
-        load_weights();
+        load_weights(0);
       int alocal = 0;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++alocal) {
         int n0, img0, oy0;
@@ -279,7 +286,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             ptx::tma_load_5d(smem + (size_t)(ab * prob.cblocks + cb) * prob.a_tile_bytes, &map_x, a_full + ab,
                              cb * kElems, -prob.pw, oy0 - prob.ph, img0, 0);
           if (alocal == 0)
-            load_weights();
+            load_weights(n0);
         } else {
         for (int kb = 0; kb < k_blocks; ++kb) {
           bool got_slot;
@@ -446,16 +453,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const bool box_ok = box_img < prob.n_box && box_x < prob.Wo && box_y < prob.h_half;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     if constexpr (kHalo) {
-      // one column tile: this warp's maps are the same for every tile
+      // one column tile, or one tile for this block: this warp's maps are the same for every tile
+      const int own = (int)(blockIdx.x % (unsigned)prob.n_tiles) * BN;
       for (int c = first_col; c < BN; c += 32 * kSets) {
         uint32_t t[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-          t[j] = __float_as_uint(sb[c + j].x);
+          t[j] = __float_as_uint(sb[own + c + j].x);
         ptx::tmem_st_32x32(lane_base + kScaleCol + c, t);
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-          t[j] = __float_as_uint(sb[c + j].y);
+          t[j] = __float_as_uint(sb[own + c + j].y);
         ptx::tmem_st_32x32(lane_base + kScaleCol + BN + c, t);
       }
       ptx::tmem_st_wait();
