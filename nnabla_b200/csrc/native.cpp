@@ -11,6 +11,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
 #include <array>
@@ -20,6 +21,7 @@
 #include <tuple>
 #include <type_traits>
 #include <utility>
+#include <vector>
 
 #include "nnabla_b200.h"
 
@@ -438,6 +440,121 @@ PyObject *folded_convolution(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+PyObject *attribute(PyObject *o, const char *name) { // new reference; NULL without an exception
+  PyObject *v = PyObject_GetAttrString(o, name);
+  if (!v)
+    PyErr_Clear();
+  return v;
+}
+
+// folded_convolutions(x_codes, x_shape, steps, n, delta): functions.folded_convolutions. All steps are read and checked
+// before the first is launched.
+PyObject *folded_convolutions(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 5)
+    return PyErr_Format(PyExc_TypeError, "expected 5 arguments, got %zd", nargs);
+  struct Step {
+    Geometry g;
+    at::Tensor side; // (held: the prepared weights' attribute could be set anew while other threads run)
+    const at::Tensor *scale, *bias;
+    int64_t source, residual;
+    bool relu, codes;
+    int64_t last_use; // of its result
+  };
+  Plain p;
+  const at::Tensor *x = p.i8(a[0]);
+  c10::SmallVector<int64_t, 8> xs;
+  const long n = p.integer(a[3]);
+  const float delta = p.number(a[4]);
+  if (!p.ok || !read_shape(a[1], xs) || xs.size() != 4 || !PyTuple_Check(a[2]))
+    return not_plain();
+  const int64_t count = PyTuple_GET_SIZE(a[2]), want_x[3] = {xs[0], xs[2] * xs[3], nb200_codes_nhwc_slots(xs[1], 1)};
+  p.require(count > 0 && x->sizes() == at::IntArrayRef(want_x, 3));
+  std::vector<Step> steps((size_t)count);
+  for (int64_t i = 0; p.ok && i < count; ++i) {
+    PyObject *t = PyTuple_GET_ITEM(a[2], i);
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 9)
+      return not_plain();
+    auto item = [&](int k) { return PyTuple_GET_ITEM(t, k); };
+    Step &s = steps[(size_t)i];
+    s.last_use = i;
+    s.source = p.integer(item(0));
+    PyObject *prepared = item(1), *side = attribute(prepared, "side"), *shape = attribute(prepared, "shape"),
+             *group = attribute(prepared, "group");
+    if (const at::Tensor *t8 = side ? p.i8(side) : p.fail())
+      s.side = *t8;
+    c10::SmallVector<int64_t, 8> in, ws;
+    p.require(group && p.integer(group) == 1 && shape && read_shape(shape, ws) && s.source >= 0 && s.source <= i);
+    Py_XDECREF(side);
+    Py_XDECREF(shape);
+    Py_XDECREF(group);
+    s.scale = p.f32(item(2)), s.bias = p.f32_or_none(item(3));
+    s.residual = item(6) == Py_None ? -1 : p.integer(item(6));
+    s.relu = p.truth(item(7)), s.codes = p.truth(item(8));
+    p.require(s.residual >= -1 && s.residual <= i);
+    if (!p.ok)
+      return not_plain();
+    if (s.source == 0) {
+      in = xs;
+    } else {
+      const Step &from = steps[(size_t)s.source - 1];
+      p.require(from.codes);
+      in = {from.g.x[0], from.g.w[0], from.g.out[0], from.g.out[1]};
+    }
+    p.require(s.g.read(in, ws, item(4), item(5), Py_None, 1) && s.scale->numel() == s.g.w[0] &&
+              (!s.bias || (s.bias->dim() == 1 && s.bias->numel() == s.g.w[0])));
+    if (p.ok && s.residual >= 0) { // of the result's own shape
+      const int64_t *o = s.residual == 0 ? xs.data() : nullptr;
+      const Step *from = o ? nullptr : &steps[(size_t)s.residual - 1];
+      const int64_t r[4] = {o ? o[0] : from->g.x[0], o ? o[1] : from->g.w[0], o ? o[2] : from->g.out[0], o ? o[3] : from->g.out[1]};
+      p.require(r[0] == s.g.x[0] && r[1] == s.g.w[0] && r[2] == s.g.out[0] && r[3] == s.g.out[1]);
+      if (s.residual > 0)
+        steps[(size_t)s.residual - 1].last_use = i;
+    }
+    if (s.source > 0)
+      steps[(size_t)s.source - 1].last_use = i;
+  }
+  if (!p.ok)
+    return not_plain();
+  std::vector<at::Tensor> results((size_t)count);
+  int rc = 0;
+  {
+    const int device = x->get_device(), current = c10::cuda::current_device();
+    if (device != current)
+      c10::cuda::set_device((c10::DeviceIndex)device);
+    void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    pybind11::gil_scoped_release no_gil;
+    for (int64_t i = 0; i < count && rc == 0; ++i) {
+      const Step &s = steps[(size_t)i];
+      const Geometry &g = s.g;
+      const int64_t want[3] = {g.x[0], g.out[0] * g.out[1], nb200_codes_nhwc_slots(g.w[0], 1)};
+      at::Tensor &y = results[(size_t)i];
+      y = empty_like_of(*x, at::IntArrayRef(want, 3), s.codes ? at::kChar : at::kFloat);
+      const at::Tensor *from = s.source == 0 ? x : &results[(size_t)s.source - 1];
+      const at::Tensor *res = s.residual < 0 ? nullptr : s.residual == 0 ? x : &results[(size_t)s.residual - 1];
+      const bool res_codes = res && res->scalar_type() == at::kChar;
+      g_calls.fetch_add(1, std::memory_order_relaxed);
+      rc = nb200_convolution_codes_folded_nhwc(
+          data<int8_t>(from), data<int8_t>(&s.side), data<float>(s.scale), data<float>(s.bias),
+          res_codes ? data<int8_t>(res) : nullptr, res_codes ? delta : 0.0f, res_codes ? nullptr : data<float>(res),
+          s.codes ? data<int8_t>(&y) : nullptr, s.codes ? nullptr : data<float>(&y), (int)g.x[0], (int)g.x[1], (int)g.x[2],
+          (int)g.x[3], (int)g.w[0], (int)g.w[2], (int)g.w[3], (int)g.pad[0], (int)g.pad[1], (int)g.stride[0],
+          (int)g.stride[1], (int)g.dil[0], (int)g.dil[1], s.relu, 1, (int)n, delta, stream);
+      for (int64_t j = 0; j < i; ++j)
+        if (steps[(size_t)j].last_use == i)
+          results[(size_t)j].reset();
+    }
+    if (device != current)
+      c10::cuda::set_device((c10::DeviceIndex)current);
+  }
+  if (rc != 0)
+    return raise_status(rc);
+  const Geometry &g = steps.back().g;
+  return Py_BuildValue("N(LLLL)", THPVariable_Wrap(results.back()), (long long)g.x[0], (long long)g.w[0], (long long)g.out[0],
+                       (long long)g.out[1]);
+  END_HANDLE_TH_ERRORS
+}
+
 // binary_convolution(x, weight, binary_weight, alpha, bias, pad, stride, dilation, group, quantize_zero_to, delta):
 // y of binary_weight_convolution (alpha a tensor) or binary_connect_convolution (alpha None); delta None or a number
 PyObject *binary_convolution(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
@@ -821,6 +938,7 @@ PyMethodDef methods[] = {
     HELPER("empty_i8", empty<at::kChar>),
     HELPER("conv2d", conv2d),
     HELPER("folded_convolution", folded_convolution),
+    HELPER("folded_convolutions", folded_convolutions),
     HELPER("binary_convolution", binary_convolution),
     HELPER("binary_convolution_backward", binary_convolution_backward),
     HELPER("batch_normalization", batch_normalization),

@@ -292,11 +292,20 @@ class FoldedRunner:
             k0, k1 = fold[bn]
             scale = (host(prep.alpha) * k0).astype(np.float32) * np.float32(DELTA)
             self.layers[conv] = (prep, up(scale), up(k1))
+        steps, block_in = [], 0  # the convolutions in one call (functions.folded_convolutions)
         for name, cin, c, st, has_sc in folded_layers():
             add(name + "/conv1", name + "/bn1")
             add(name + "/conv2", name + "/bn2")
             if has_sc:
                 add(name + "/shortcut", name + "/bn_s")
+            steps.append((block_in,) + self.layers[name + "/conv1"] + ((1, 1), (st, st), None, True, True))
+            hidden, residual = len(steps), block_in
+            if has_sc:
+                steps.append((block_in,) + self.layers[name + "/shortcut"] + ((0, 0), (st, st), None, False, False))
+                residual = len(steps)
+            steps.append((hidden,) + self.layers[name + "/conv2"] + ((1, 1), (1, 1), residual, True, True))
+            block_in = len(steps)
+        self.steps = tuple(steps)
         self.head = (params["head/W"], params["head/b"])
 
     def _rec(self, name, x, y, shape, **kw):
@@ -311,7 +320,10 @@ class FoldedRunner:
         pc, pshape = o.max_pooling_codes(hc, shape, (3, 3), (2, 2), True, (1, 1))
         self._rec("stem/pool", hc, pc, pshape, in_shape=shape)
         hc, shape = pc, pshape
-        for name, cin, c, st, has_sc in folded_layers():
+        whole = getattr(o, "folded_convolutions", None) if self.trace is None else None
+        if whole is not None:
+            hc, shape = whole(hc, shape, self.steps, DELTA)
+        for name, cin, c, st, has_sc in folded_layers() if whole is None else ():
             p1, s1, b1 = self.layers[name + "/conv1"]
             r, rshape = o.convolution_codes_folded(hc, shape, p1, s1, b1, (1, 1), (st, st), (1, 1))
             self._rec(name + "/conv1", hc, r, rshape, in_shape=shape, stride=st, k=3)
