@@ -275,6 +275,7 @@ bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, i
     p.class_box[c] = c * boxes_per_class;
   plan.bn = p.maps <= 64 ? 64 : 128;
   p.n_tiles = (p.maps + plan.bn - 1) / plan.bn;
+  p.bn = (int)round_up((p.maps + p.n_tiles - 1) / p.n_tiles, 16);
   const size_t b_tile = (size_t)plan.bn * kRowBytes;
   // the 128 rows read from the last tap's row on may reach past the last box
   auto fixed = [&]() {
@@ -367,7 +368,7 @@ int launch_planes(const PlanesPlan &plan, const void *act, int Hin, int Win, int
   const uint32_t estr[5] = {1, (uint32_t)p.in_sx, (uint32_t)p.in_sy, 1, 1};
   NB_TRY(encode_tiled(&ma, 0, 5, act, dims, strides, box, estr, kRowBytes));
   const int64_t pitch = (int64_t)taps * p.k_slots;
-  NB_TRY(make_operand_map(&mb, side, false, pitch, pitch, p.total_maps, 1, plan.bn));
+  NB_TRY(make_operand_map(&mb, side, false, pitch, pitch, p.total_maps, 1, p.bn));
   if (f16) {
     NB_CHECK(p.planes == 2, NB200_EVALUE, "fp16 planes come in pairs");
     if (plan.resident)

@@ -11,6 +11,10 @@
 //  * the forward convolution of fp32 activations: A = two fp16 pieces of the scaled activations, B = +-1 weights. A
 //    stride s makes s * s classes of taps, each reading one of the s * s interleaved images of x.
 //
+// A column tile has as many maps as spread them evenly (160 as 80 + 80, not as 128 + 32 and 96 empty columns): an MMA's
+// time follows its columns (a [24, 96, 35, 29] layer of 160 maps 29.6 us forward, 26.6 with even tiles; its input gradient,
+// 96 columns, 31.9 and 29.3).
+//
 // What bounds it: the tensor core (an MMA of 128 rows takes 51 / 67 cycles for 64 / 128 columns, limited by the
 // shared-memory reads of A). The previous form put the maps on the 128 MMA rows, half of them empty for 64 maps, and
 // fetched a box of pixels per filter tap: 540 us for the input gradient of a 64 -> 64 3 x 3 layer on [128, 64, 56, 56],
@@ -47,6 +51,7 @@ struct ConvPlanesProblem {
   int in_sy, in_sx;                   // step between the input pixels of a box
   int Wu;                             // columns of a class's grid: ceil(W / sx)
   int h_box, tiles_h, n_tiles;        // class rows per tile, tiles per class and image, column tiles
+  int bn;                             // columns of a tile, a multiple of 16 up to BN: the maps spread evenly over the tiles
   int n_box, img_rows;                // images per tile (1 with tiles_h > 1) and MMA rows from one to the next
   int wp, hp;                         // input box: hp rows of wp pixels
   int cblocks;                        // 64-channel blocks of one group
@@ -95,6 +100,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = prob.num_tiles();
   const int plane_groups = prob.planes / PG;
+  const uint32_t b_bytes = (uint32_t)prob.bn * kRowBytes; // of a weight tile, in kBBytes of shared memory
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kPlanesMaxStages; ++i) {
@@ -130,7 +136,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
   // the column tiles of a box are neighbours in time, then the classes: the box stays in L2
   auto decode = [&](int tile) {
     TileAt t;
-    t.n0 = (tile % prob.n_tiles) * BN;
+    t.n0 = (tile % prob.n_tiles) * prob.bn;
     tile /= prob.n_tiles;
     t.cls = tile % (prob.sy * prob.sx);
     tile /= prob.sy * prob.sx;
@@ -173,7 +179,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
       uint32_t aphase = 0, bphase = 0;
       bool ok = true;
       if (kResident && (int)blockIdx.x < num_tiles) { // one group, one column tile
-        ptx::mbar_expect_tx(b_full, b_tiles * kBBytes);
+        ptx::mbar_expect_tx(b_full, b_tiles * b_bytes);
         for (uint32_t i = 0; i < b_tiles; ++i) {
           const int tap = (int)i / prob.cblocks, cb = (int)i - tap * prob.cblocks;
           ptx::tma_load_3d(b_base + i * kBBytes, &map_b, b_full, prob.tap_k[tap] * prob.k_slots + cb * 64, 0, 0);
@@ -210,7 +216,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
                 ok = false;
                 break;
               }
-              ptx::mbar_expect_tx(b_full + bs, kBBytes);
+              ptx::mbar_expect_tx(b_full + bs, b_bytes);
               ptx::tma_load_3d(b_base + bs * kBBytes, &map_b, b_full + bs, prob.tap_k[tap] * prob.k_slots + cb * 64,
                                t.group * prob.maps + t.n0, 0);
               if (++bs == prob.b_stages) {
@@ -228,7 +234,7 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
       int as = 0, bs = 0, local = 0; // stages and chunk (or tile) counted over both issuers' work
       uint32_t aphase = 0, bphase = 0;
       bool ok = true;
-      const uint32_t idesc = ptx::make_idesc(1u, kF16 ? 0u : 1u, kTileM, BN);
+      const uint32_t idesc = ptx::make_idesc(1u, kF16 ? 0u : 1u, kTileM, (uint32_t)prob.bn);
       const uint32_t hi = (uint32_t)(ptx::smem_desc_k(0, kRowBytes) >> 32);
       const uint32_t a_lo = ptx::smem_u32(a_base) >> 4, b_lo = ptx::smem_u32(b_base) >> 4; // below 2^14
       auto next_a = [&]() {
@@ -383,7 +389,10 @@ __global__ void __launch_bounds__(kPlanesThreads, 1)
       // [128, 64, 56, 56] added to dx 121 us, now 96; not added 91). With two chunks there are no registers for them.
       constexpr int kAhead = kMine == 1 ? 32 : 1;
       float ahead[kAhead];
-      auto chunk_left = [&](int ci) { return prob.maps - (t.n0 + 32 * set + 64 * ci); }; // maps of this chunk that exist
+      auto chunk_left = [&](int ci) { // maps of this chunk that the tile has
+        const int c = 32 * set + 64 * ci;
+        return min(prob.maps - t.n0, prob.bn) - c;
+      };
       auto chunk_y = [&](int ci) {
         return prob.y + ((int64_t)img * prob.total_maps + t.group * prob.maps + t.n0 + 32 * set + 64 * ci) * plane +
                (int64_t)iy * prob.W + ix;
