@@ -459,8 +459,6 @@ int binary_convolution(const float *x, const float *w, float *wb, float *alpha, 
            "activation codes and prepared weights must be 16-byte aligned");
   bool operands_done = false;
   if (!prepared_side) {
-    if (c_slots != g.Cg)
-      NB_CUDA(cudaMemsetAsync(side, 0, side_bytes, st));
     if (fxp_weights)
       NB_TRY(codes_conv_weights(w, g.Ko, g.Cg, g.kh, g.kw, weight_delta, side, wpitch, c_slots, st));
     else if (int8 && !x_codes && binary_conv_operands_i8_applies(x, g.N, g.H * g.W, (int)ctot, g.Ko)) {
@@ -657,8 +655,8 @@ bool plan_wgrad(ConvWgradProblem &p, const ConvGeometry &g, int x_planes, size_t
 // Input gradient (dx) and weight gradient (dw) from the channel-last pieces of dy and x, for weights exact in one bf16
 // piece. *did_dx / *did_dw: which of the two it computed (the geometries its kernels do not take are left to the caller).
 int planes_backward(const float *x, const float *wb, const float *alpha, const float *dy, float *dx, float *dw,
-                    const ConvGeometry &g, int accum_dx, int accum_dw, float act_delta, cudaStream_t st, bool *did_dx,
-                    bool *did_dw) {
+                    float *db, const ConvGeometry &g, int accum_dx, int accum_dw, int accum_db, float act_delta,
+                    cudaStream_t st, bool *did_dx, bool *did_dw, bool *did_db) {
   const int taps = g.kh * g.kw, k_pad_g = (int)round_up(g.Kog, 16), c_pad_g = (int)round_up(g.Cg, 16);
   // activations that are multiples of act_delta with |code| <= 127 are exact in one bf16 piece
   const int x_planes = act_delta > 0.0f ? 1 : 3;
@@ -689,13 +687,19 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   const size_t side_bytes = *did_dx ? round_up((size_t)g.C * taps * p.k_slots * 2, 1024) : 0;
   const int grid_w = *did_dw ? (q.work + q.per_block - 1) / q.per_block : 0;
   const size_t slot_bytes = *did_dw ? (size_t)(grid_w + q.tasks()) * q.slot_floats() * 4 : 0;
+  // the bias gradient's sums on the way, while there are few: a pass over dy and its finish cost 8 us (a [24, 160, 35, 29]
+  // dy), the finish of 384 rows of sums 3; with thousands of rows a pass of its own is faster
+  const int64_t sum_rows = conv_dy_sum_rows(g.N, g.Ho * g.Wo);
+  *did_db = db != nullptr && sum_rows <= 1024;
+  const size_t sum_bytes = *did_db ? round_up((size_t)sum_rows * g.Ko * 4, 1024) : 0;
   AsyncScratch scratch(st);
-  NB_TRY(scratch.alloc((two ? 2 : 1) * dy_bytes + x_bytes + side_bytes + slot_bytes));
+  NB_TRY(scratch.alloc((two ? 2 : 1) * dy_bytes + x_bytes + side_bytes + sum_bytes + slot_bytes));
   uint8_t *at = static_cast<uint8_t *>(scratch.p);
   uint8_t *dys = at, *dyp = two ? at + dy_bytes : at; // pieces of dy * alpha (or dy) and of dy
   at += (two ? 2 : 1) * dy_bytes;
   uint8_t *xp = at, *side = xp + x_bytes;
-  q.slots = reinterpret_cast<float *>(side + side_bytes);
+  float *sums = reinterpret_cast<float *>(side + side_bytes);
+  q.slots = reinterpret_cast<float *>(side + side_bytes + sum_bytes);
   const bool scaled = *did_dx && alpha;
   ConvBackwardOperands ops{};
   ops.N = g.N, ops.groups = g.group, ops.Kog = g.Kog, ops.Cg = g.Cg;
@@ -703,11 +707,14 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
   ops.dy_pixels = g.Ho * g.Wo, ops.k_pad_g = k_pad_g, ops.k_total = (int)k_tot;
   ops.dy_scaled = scaled ? dys : nullptr;
   ops.dy_plain = scaled ? (two ? dyp : nullptr) : dyp;
+  ops.dy_sums = *did_db ? sums : nullptr;
   ops.x = x, ops.x_pixels = g.H * g.W, ops.c_pad_g = c_pad_g, ops.c_total = (int)c_tot, ops.x_planes = x_planes;
   ops.x_pieces = *did_dw ? xp : nullptr;
   ops.wb = wb, ops.taps = taps, ops.k_slots = p.k_slots;
   ops.side = *did_dx ? side : nullptr;
   NB_TRY(conv_backward_operands(ops, st));
+  if (*did_db)
+    NB_TRY(channel_rows_finish(sums, g.Ko, (int)sum_rows, db, accum_db, st));
   if (*did_dx) {
     p.c_group_stride = k_pad_g;
     p.y = dx;
@@ -888,17 +895,17 @@ int convolution_backward(const float *x, const float *w_exact, const float *alph
   NB_CHECK(dy != nullptr, NB200_EVALUE, "dy is NULL");
   NB_CHECK(!dx || w_exact != nullptr, NB200_EVALUE, "the gradient w.r.t. x needs the weights");
   NB_CHECK(!dw || x != nullptr, NB200_EVALUE, "the gradient w.r.t. the weights needs x");
-  bool did_dx = false, did_dw = false;
+  bool did_dx = false, did_dw = false, did_db = false;
   if ((dx && !full_precision_weights) || dw)
-    NB_TRY(planes_backward(x, w_exact, alpha, dy, full_precision_weights ? nullptr : dx, dw, g, accum_dx, accum_dw,
-                           act_delta, st, &did_dx, &did_dw));
+    NB_TRY(planes_backward(x, w_exact, alpha, dy, full_precision_weights ? nullptr : dx, dw, db, g, accum_dx, accum_dw,
+                           accum_db, act_delta, st, &did_dx, &did_dw, &did_db));
   if (dx && !did_dx) {
     NB_TRY(conv_input_grad(w_exact, alpha, dy, dx, g, accum_dx, st, full_precision_weights));
   }
   if (dw && !did_dw) {
     NB_TRY(conv_weight_grad(x, dy, dw, g, accum_dw, act_delta, st));
   }
-  if (db) {
+  if (db && !did_db) {
     int splits = g.N < 32 ? g.N : 32;
     AsyncScratch scratch(st);
     NB_TRY(scratch.alloc((size_t)splits * g.Ko * 4));
@@ -1287,8 +1294,6 @@ int nb200_binary_weights_prepare_i8(const float *w, float *wb, float *alpha, int
   int64_t wpitch;
   int8_side_layout(Cg, kernel_h * kernel_w, c_slots, wpitch);
   cudaStream_t st = as_stream(stream);
-  if (c_slots != Cg)
-    NB_CUDA(cudaMemsetAsync(side, 0, (size_t)outmaps * wpitch, st));
   return binarize_rows(w, outmaps, Cg, kernel_h, kernel_w, quantize_zero_to, wb, alpha, side, wpitch, c_slots, true, st);
 }
 

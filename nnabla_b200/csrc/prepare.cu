@@ -164,6 +164,16 @@ __global__ void finalize_alpha_kernel(const float *__restrict__ partial, int blo
 // block is one filter tap over consecutive channels, matching the NHWC
 // activation planes.
 // ---------------------------------------------------------------------------
+// Zeros in the channel slots [Cg, c_pad) of every tap of one row of weights (a memset of all weights in front cost 4 us: a
+// launch that the ones around it do not overlap).
+__device__ __forceinline__ void zero_slots(uint8_t *row, int taps, int Cg, int c_pad, int bytes) {
+  const int pad = (c_pad - Cg) * bytes;
+  for (int i = threadIdx.x; i < taps * pad; i += 256) {
+    const int t = i / pad;
+    row[(t * c_pad + Cg) * bytes + (i - t * pad)] = 0;
+  }
+}
+
 // kMode: 0 = bf16 signs, 1 = int8 signs, 2 = fp16 signs.
 template <int kMode>
 __device__ __forceinline__ void binarize_row(int o, const float *__restrict__ w, int Cg, int kh, int kw,
@@ -172,6 +182,8 @@ __device__ __forceinline__ void binarize_row(int o, const float *__restrict__ w,
                                              int c_pad) {
   const int taps = kh * kw, Kd = Cg * taps;
   const float *wr = w + (int64_t)o * Kd;
+  zero_slots(reinterpret_cast<uint8_t *>(side) + (int64_t)o * side_pitch * (kMode == 1 ? 1 : 2), taps, Cg, c_pad,
+             kMode == 1 ? 1 : 2);
   float acc = 0.0f;
   for (int k0 = threadIdx.x; k0 < Kd; k0 += 8 * 256) { // eight loads in flight
     float v[8];
@@ -234,6 +246,7 @@ __global__ void __launch_bounds__(256) codes_conv_weights_kernel(const float *__
   const int o = blockIdx.x;
   const int taps = kh * kw, Kd = Cg * taps;
   const float *wr = wq + (int64_t)o * Kd;
+  zero_slots(reinterpret_cast<uint8_t *>(side) + (int64_t)o * side_pitch, taps, Cg, c_pad, 1);
   for (int k = threadIdx.x; k < Kd; k += 256) {
     const int c = k / taps, t = k - c * taps;
     side[(int64_t)o * side_pitch + (int64_t)t * c_pad + c] = (int8_t)__float2int_rn(__fmul_rn(wr[k], inv_delta));

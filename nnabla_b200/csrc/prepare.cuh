@@ -94,6 +94,7 @@ struct ConvBackwardOperands {
   const float *dy, *alpha;
   int dy_pixels, k_pad_g, k_total;
   void *dy_scaled, *dy_plain;
+  float *dy_sums; // NULL, or [conv_dy_sum_rows(N, dy_pixels)][maps]: the maps' sums over 64 pixels each
   const float *x;
   int x_pixels, c_pad_g, c_total, x_planes;
   void *x_pieces;
@@ -102,6 +103,9 @@ struct ConvBackwardOperands {
   void *side;
 };
 int conv_backward_operands(const ConvBackwardOperands &o, cudaStream_t st);
+inline int64_t conv_dy_sum_rows(int N, int pixels) { return (int64_t)N * ((pixels + 63) / 64); }
+// out[o] (+)= the sum of `rows` rows of partial [rows][Ko]
+int channel_rows_finish(const float *partial, int Ko, int rows, float *out, int accumulate, cudaStream_t st);
 // dy [N][Ko][Ho][Wo] -> 3 bf16 planes [N][Hs][Ws][ctot] (pre-zeroed by the caller):
 // pixel (oy, ox) at (oy * sh, ox * sw), map o of group g at slot g * k_pad_g + o - g * Kog,
 // multiplied by chan_scale[o] first when given.

@@ -124,6 +124,7 @@ struct NhwcPieces {
   const uint32_t *image_parts; // kHalf
   int parts;
   uint32_t *image_max;
+  float *sums; // not kHalf: the channels' sums over each tile's pixels, [N * tiles_x][C], or NULL
   __host__ __device__ int tiles_x() const { return (HW + 63) / 64; }
   __host__ __device__ int tiles_y() const { return (ctot + 63) / 64; }
   __host__ __device__ int64_t blocks() const { return (int64_t)tiles_x() * tiles_y() * N; }
@@ -169,6 +170,17 @@ __device__ __forceinline__ void nhwc_pieces_tile(const NhwcPieces &P, int block,
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         v[r][k] = live && p + k < HW ? __ldcs(base + (int64_t)r * HW + k) : 0.0f;
+    }
+  }
+  if (!kHalf && P.sums) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float s = (v[r][0] + v[r][1]) + (v[r][2] + v[r][3]);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (px4 == 0 && ok && cc0 + r < Cg)
+        P.sums[((int64_t)n * tx + bx) * C + g * Cg + cc0 + r] = s;
     }
   }
 #pragma unroll
@@ -368,6 +380,32 @@ __global__ void channel_finish_kernel(const float *__restrict__ partial, int Ko,
   out[o] = accumulate ? __fadd_rn(out[o], s) : s;
 }
 
+// The same where the pass that converts dy has left its sums, `rows` of them per map: 32 rows by 8 maps per block.
+__global__ void __launch_bounds__(256) channel_rows_finish_kernel(const float *__restrict__ partial, int Ko, int rows,
+                                                                  float *__restrict__ out, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ float warps[8][8];
+  const int o = blockIdx.x * 8 + (threadIdx.x & 7);
+  float s = 0.0f;
+  if (o < Ko) {
+#pragma unroll 8
+    for (int r = threadIdx.x >> 3; r < rows; r += 32)
+      s += __ldg(partial + (int64_t)r * Ko + o);
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  if ((threadIdx.x & 31) < 8)
+    warps[threadIdx.x >> 5][threadIdx.x & 7] = s;
+  __syncthreads();
+  if (threadIdx.x < 8 && o < Ko) {
+    s = 0.0f;
+    for (int w = 0; w < 8; ++w)
+      s += warps[w][threadIdx.x];
+    out[o] = accumulate ? __fadd_rn(out[o], s) : s;
+  }
+}
+
 // staged [splits][Cg][Kog][taps] (the contraction's NCHW-shaped output with the
 // input channel as the image axis, one partial result per K split) ->
 // dW[o][c][taps]: the splits are added in order, then dW is overwritten or added to.
@@ -416,7 +454,7 @@ int nchw_to_nhwc_half_pair_images(const float *x, int N, int C, int HW, int grou
   const int parts = (int)std::max<int64_t>(1, std::min(per_image / 4096, most));
   NB_CUDA(launch_dependent(image_absmax_kernel, dim3(parts, N), dim3(256), 0, st, x, per_image, image_max + N));
   const NhwcPieces P{x,       N,       C, HW, groups, Cg, c_pad_g, ctot, nullptr, static_cast<uint16_t *>(out),
-                     nullptr, image_max + N, parts, image_max};
+                     nullptr, image_max + N, parts, image_max, nullptr};
   NB_CHECK(P.blocks() < (1ll << 31), NB200_ENOTIMPL, "tensor too large");
   NB_CUDA(launch_dependent(P.vec() ? nhwc_pieces_kernel<true, 2, true> : nhwc_pieces_kernel<false, 2, true>,
                            dim3((unsigned)P.blocks()), dim3(256), 0, st, P));
@@ -427,9 +465,9 @@ int conv_backward_operands(const ConvBackwardOperands &o, cudaStream_t st) {
   const TransposedWeights W{o.wb, o.side ? o.groups * o.Cg : 0, o.Cg, o.taps, o.Kog, o.k_slots,
                             static_cast<__nv_bfloat16 *>(o.side)};
   const NhwcPieces dy{o.dy, o.N, o.groups * o.Kog, o.dy_pixels, o.groups, o.Kog, o.k_pad_g, o.k_total, o.alpha,
-                      static_cast<uint16_t *>(o.dy_scaled), static_cast<uint16_t *>(o.dy_plain), nullptr, 0, nullptr};
+                      static_cast<uint16_t *>(o.dy_scaled), static_cast<uint16_t *>(o.dy_plain), nullptr, 0, nullptr, o.dy_sums};
   const NhwcPieces x{o.x, o.x_pieces ? o.N : 0, o.groups * o.Cg, o.x_pixels, o.groups, o.Cg, o.c_pad_g, o.c_total, nullptr,
-                     nullptr, static_cast<uint16_t *>(o.x_pieces), nullptr, 0, nullptr};
+                     nullptr, static_cast<uint16_t *>(o.x_pieces), nullptr, 0, nullptr, nullptr};
   const int64_t blocks = W.rows + dy.blocks() + x.blocks();
   NB_CHECK(blocks < (1ll << 31), NB200_ENOTIMPL, "tensor too large");
   const bool vd = dy.vec(), vx = x.vec();
@@ -479,6 +517,12 @@ int channel_sums(const float *dy, int N, int Ko, int HW, float *out, int accumul
   NB_CUDA(launch_dependent(channel_finish_kernel, dim3((Ko + 255) / 256), dim3(256), 0, st, partial, Ko, splits, out,
                            accumulate));
   NB_LAUNCH_CHECK();
+  return NB200_OK;
+}
+
+int channel_rows_finish(const float *partial, int Ko, int rows, float *out, int accumulate, cudaStream_t st) {
+  NB_CUDA(launch_dependent(channel_rows_finish_kernel, dim3((Ko + 7) / 8), dim3(256), 0, st, partial, Ko, rows, out,
+                           accumulate));
   return NB200_OK;
 }
 
