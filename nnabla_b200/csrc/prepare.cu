@@ -630,8 +630,9 @@ __global__ void __launch_bounds__(256) transpose_i8_kernel(const int8_t *__restr
 }
 
 // Both operands of the 8-bit fixed-point affine in one launch: x [M, K] -> codes [M][Kp] and w [K, N] -> transposed
-// codes [N][Kp] (Kp = K rounded up to 128, zero padded). HBM-bound: 5 bytes per value. Blocks [0, x_blocks): a warp
-// converts four runs of 128 values, each one 512-byte load and one 128-byte store. The other blocks: a tile of 128 k
+// codes [N][Kp] (Kp = K rounded up to 128, zero padded). HBM-bound: 5 bytes per value. The last x_blocks blocks: a warp
+// converts four runs of 128 values, each one 512-byte load and one 128-byte store. The blocks before them, since w is what
+// was quantized last and begins in L2: a tile of 128 k
 // x 64 n; a thread converts 4 x 4 values, the word of four k of one n goes through shared memory (16-byte chunks
 // XORed with the n quad, so that the transposed stores meet at most two to a bank) and leaves in 128-byte rows.
 // 8192 x 4096 and 4096 x 8192: 54 us, 6.2 TB/s; one pass to codes per operand (one value per thread and store) and
@@ -640,14 +641,14 @@ template <bool kVecX, bool kVecW>
 __global__ void __launch_bounds__(256) fxp8_operands_kernel(const float *__restrict__ x, int64_t M, int K, int64_t Kp,
                                                             float inv_dx, int8_t *__restrict__ xc,
                                                             const float *__restrict__ w, int N, float inv_dw,
-                                                            int8_t *__restrict__ wt, unsigned x_blocks, int k_tiles) {
+                                                            int8_t *__restrict__ wt, unsigned w_blocks, int k_tiles) {
   __shared__ uint4 tile[64][8];
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (blockIdx.x < x_blocks) {
+  if (blockIdx.x >= w_blocks) {
     const int64_t runs_row = Kp / 128, runs = M * runs_row;
-    const int64_t s0 = ((int64_t)blockIdx.x * 8 + warp) * 4;
+    const int64_t s0 = ((int64_t)(blockIdx.x - w_blocks) * 8 + warp) * 4;
     float4 v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(256) fxp8_operands_kernel(const float *__restr
         reinterpret_cast<uint32_t *>(xc)[(s0 + j) * 32 + lane] = pack_codes(v[j].x, v[j].y, v[j].z, v[j].w, inv_dx);
     return;
   }
-  const unsigned t = blockIdx.x - x_blocks;
+  const unsigned t = blockIdx.x;
   const int k0 = (int)(t % k_tiles) * 128, n0 = (int)(t / k_tiles) * 64;
   const int nq = threadIdx.x & 15, kr = threadIdx.x >> 4; // n quad, first k quad
   float4 v[2][4];
@@ -967,7 +968,7 @@ int fxp8_operands(const float *x, int64_t M, int K, int64_t Kp, float delta_x, i
   auto kernel = vx ? (vw ? fxp8_operands_kernel<true, true> : fxp8_operands_kernel<true, false>)
                    : (vw ? fxp8_operands_kernel<false, true> : fxp8_operands_kernel<false, false>);
   NB_CUDA(launch_dependent(kernel, dim3((unsigned)(x_blocks + w_blocks)), dim3(256), 0, st, x, M, K, Kp, 1.0f / delta_x,
-                           xc, w, N, 1.0f / delta_w, wt, (unsigned)x_blocks, (int)k_tiles));
+                           xc, w, N, 1.0f / delta_w, wt, (unsigned)w_blocks, (int)k_tiles));
   NB_LAUNCH_CHECK();
   return NB200_OK;
 }
