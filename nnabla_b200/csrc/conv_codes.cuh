@@ -45,7 +45,7 @@ struct ConvCodesProblem {
   int wp, hp;          // wp = Wo + (kw - 1) * dw, hp = h_box + (kh - 1) * dh
   int h_half;          // output rows of one MMA row block (h_box, or half of it with two row blocks per tile)
   int a_tile_bytes;    // bytes of one channel block's pixel tile in shared memory (readable rows included)
-  int a_bufs;          // pixel-tile buffers: 2, or 1 where every block has one tile
+  int a_bufs;          // pixel-tile buffers: 2 to kTileBufs, or 1 where every block has one tile
   __device__ __forceinline__ int num_tiles() const { return n_tiles * tiles_h * tiles_n; }
   __device__ __forceinline__ int k_blocks() const { return taps * cblocks; }
 };
@@ -114,6 +114,7 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
   return d;
 }
 
+constexpr int kTileBufs = 4;       // barriers of the halo form's pixel tiles
 constexpr int kWeightParts = 4;    // barriers of the resident weights
 constexpr int kCodesKTable = 64; // K blocks whose coordinates are tabulated once per block
 
@@ -179,9 +180,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint64_t *tmem_full = bars + 2 * STAGES;
   uint64_t *tmem_empty = bars + 2 * STAGES + 2;
   uint64_t *b_full = bars + 2 * STAGES + 4; // resident weights, kWeightParts runs of K blocks
-  uint64_t *a_full = b_full + kWeightParts; // halo form: two pixel-tile buffers
-  uint64_t *a_empty = a_full + 2;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(a_empty + 2);
+  uint64_t *a_full = b_full + kWeightParts; // halo form: pixel-tile buffers
+  uint64_t *a_empty = a_full + kTileBufs;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(a_empty + kTileBufs);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // (scale, bias) of every output map, times out_scale; read as float4 pairs, so 16-byte aligned
   float2 *sb = reinterpret_cast<float2 *>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     for (int q = 0; q < kWeightParts; ++q)
       ptx::mbar_init(b_full + q, 1);
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kTileBufs; ++b) {
       ptx::mbar_init(a_full + b, 1);
       ptx::mbar_init(a_empty + b, 1);
     }
@@ -268,14 +269,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       };
       if (kResidentB && !kHalo && (int)blockIdx.x < num_tiles)
         load_weights(0);
-      int alocal = 0;
+      int alocal = 0, ab = 0;
+      uint32_t ab_phase = 0;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++alocal) {
         int n0, img0, oy0;
         decode(tile, n0, img0, oy0);
         NB_CC_STAMP(0, (tile - (int)blockIdx.x) / (int)gridDim.x);
         if constexpr (kHalo) {
-          const int ab = alocal & 1;
-          if (!ptx::mbar_wait(a_empty + ab, ((uint32_t)(alocal >> 1) & 1u) ^ 1u, abort_flag)) {
+          if (!ptx::mbar_wait(a_empty + ab, ab_phase ^ 1u, abort_flag)) {
             if (*abort_flag == 0)
               atomicCAS(status, 0, kStatusProducerTimeout);
             *abort_flag = 1;
@@ -287,6 +288,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                              cb * kElems, -prob.pw, oy0 - prob.ph, img0, 0);
           if (alocal == 0)
             load_weights(n0);
+          if (++ab == prob.a_bufs) {
+            ab = 0;
+            ab_phase ^= 1u;
+          }
         } else {
         for (int kb = 0; kb < k_blocks; ++kb) {
           bool got_slot;
@@ -319,7 +324,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      int local = 0;
+      int local = 0, ab = 0;
+      uint32_t ab_phase = 0;
       bool ok = true;
       const uint32_t idesc = ptx::make_idesc(2u, 1u, kTileM, BN); // s32 accumulator, s8 operands
       // resident weights: waited for part by part, as the first tile's MMAs come to them (a block with one tile spent
@@ -354,8 +360,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kCols);
         uint32_t accumulate = 0;
         if constexpr (kHalo) {
-          const int ab = local & 1;
-          if (!ptx::mbar_wait(a_full + ab, (uint32_t)(local >> 1) & 1u, abort_flag)) {
+          if (!ptx::mbar_wait(a_full + ab, ab_phase, abort_flag)) {
             if (*abort_flag == 0)
               atomicCAS(status, 0, kStatusMmaTimeout);
             *abort_flag = 1;
@@ -397,6 +402,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           if (!ok)
             break;
           ptx::mma_commit(a_empty + ab); // the pixel tile is free once these MMAs have read it
+          if (++ab == prob.a_bufs) {
+            ab = 0;
+            ab_phase ^= 1u;
+          }
           ptx::mma_commit(tmem_full + buf);
         } else {
         for (int kb = 0; kb < k_blocks; ++kb) {
@@ -702,7 +711,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // (in the halo form the ring is replaced by the pixel-tile buffers, counted by the caller)
 template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false>
 constexpr size_t conv_codes_smem_bytes() {
-  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) + (2 * STAGES + 8 + kWeightParts) * 8 + 32 +
+  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) + (2 * STAGES + 4 + 2 * kTileBufs + kWeightParts) * 8 + 32 +
          kCodesMaxMaps * sizeof(float2) + kCodesKTable * sizeof(int4) + 1024;
 }
 
