@@ -484,11 +484,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int buf = local & 1;
       const uint32_t buf_phase = (uint32_t)(local >> 1) & 1u;
       const int img = img0 + box_img;
-      // the residual of this warp's first chunk is requested before the accumulator is waited for
-      uint4 ra = make_uint4(0, 0, 0, 0), rb = make_uint4(0, 0, 0, 0);
-      auto load_residual = [&](int64_t off, bool upper) {
-        ra = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off));
-        rb = upper ? __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off) + 1) : make_uint4(0, 0, 0, 0);
+      // the residual of this warp's first chunk, and of its second where it has two, is requested before the accumulator is
+      // waited for: the second's load inside its chunk was a latency per tile. [256, 64, 56, 56] 68.3 us, now 58.5, [256,
+      // 128, 28, 28] 34.5 and 33.1; batch 64 17.1 and 16.5, 13.3 and 12.5. (Requested a tile ahead: 53.5 and 30.6, but
+      // batch 64 17.9 and 13.0, since a launch of few tiles waits for its instructions.)
+      constexpr bool kTwo = kCols == 64 * kSets;
+      uint4 ra = make_uint4(0, 0, 0, 0), rb = ra, ra2 = ra, rb2 = ra;
+      auto load_residual = [&](int64_t off, bool upper, uint4 &a, uint4 &b) {
+        a = __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off));
+        b = upper ? __ldg(reinterpret_cast<const uint4 *>(ep.res_codes + off) + 1) : make_uint4(0, 0, 0, 0);
       };
       auto pixel_ok = [&](int half) {
         const int y = box_y + half * prob.h_half;
@@ -497,7 +501,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       auto in_plane_of = [&](int half) { return (oy0 + box_y + half * prob.h_half) * prob.Wo + box_x; };
       const int64_t plane0 = (int64_t)img * prob.Ho * prob.Wo; // pixels before this image
       if (ep.res_codes && pixel_ok(0) && n0 + first_col < prob.slots_out)
-        load_residual((plane0 + in_plane_of(0)) * prob.slots_out + n0 + first_col, n0 + first_col + 16 < prob.slots_out);
+        load_residual((plane0 + in_plane_of(0)) * prob.slots_out + n0 + first_col, n0 + first_col + 16 < prob.slots_out, ra, rb);
+      if (kTwo && ep.res_codes) {
+        constexpr int kNext = 32 * kSets;
+        const int half = kNext / BN, col = n0 + first_col + kNext % BN;
+        if (pixel_ok(half) && col < prob.slots_out)
+          load_residual((plane0 + in_plane_of(half)) * prob.slots_out + col, col + 16 < prob.slots_out, ra2, rb2);
+      }
       if (threadIdx.x == 64)
         NB_CC_STAMP(5, local);
       const bool got = ptx::mbar_wait(tmem_full + buf, buf_phase, abort_flag);
@@ -520,8 +530,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const int in_plane = in_plane_of(half); // inside the image's plane
         const int64_t off = (plane0 + in_plane) * prob.slots_out + col;
         const bool upper = col + 16 < prob.slots_out; // the pixel's row ends in the middle of this chunk otherwise
-        if (c0 != first_col && ep.res_codes && live) // later chunks: fetched here
-          load_residual(off, upper);
+        if (kTwo && c0 != first_col)
+          ra = ra2, rb = rb2;
+        else if (!kTwo && c0 != first_col && ep.res_codes && live) // later chunks: fetched here
+          load_residual(off, upper, ra, rb);
         uint32_t r[32];
         ptx::tmem_ld_32x32(lane_base + (uint32_t)(buf * kCols + c0), r);
         float scale[32], bias[32]; // (maps past Ko have scale = bias = 0)
