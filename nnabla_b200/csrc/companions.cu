@@ -7,6 +7,7 @@
 // CPU code; the convolution accumulates with fused multiply-adds (tolerance
 // parity, like the other contractions).
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "narrow_conv.cuh"
@@ -114,102 +115,99 @@ __global__ void __launch_bounds__(kThreads) bn_inference_plane_kernel(const floa
     st_result(yp + i, one(__ldcs(xp + i)), keep);
 }
 
-// Planes of 32 to 1023 values (the later stages of a network: 28 x 28, 14 x 14, 7 x 7): one WARP per plane,
-// eight planes per block. The channel's constants are taken once per lane instead of once per value, the
-// data loads go out before them, and nothing divides by the plane size. kVec: S % 4 == 0 and 16-byte
-// aligned tensors (float4 lanes), otherwise scalar lanes (a 7 x 7 plane is 49 values).
-template <bool kVec>
+constexpr int kBnSamples = 2; // samples of a warp in the two kernels below
+
+// Planes of 32 to 1023 values (the later stages of a network: 28 x 28, 14 x 14, 7 x 7): one WARP per channel and kSamples
+// samples, eight channels per block. The channel's constants are taken once per lane and kSamples planes, the data loads go
+// out before them, and nothing divides by the plane size. kVec: S % 4 == 0 and 16-byte aligned tensors (float4 lanes),
+// otherwise scalar lanes. A lane's first kPer values of every plane are in flight at once. What bounds it: a plane per warp
+// lived for the latency of its loads, its constants and its stores, with 784 bytes of a 14 x 14 plane on the way: [256, 256,
+// 14, 14] 18.9 us, with two samples 12.1, four 13.6, eight 16.7 (fewer warps); the divisions are next.
+template <bool kVec, int kPer, int kSamples>
 __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float *__restrict__ x, const float *beta,
                                                                      const float *gamma, const float *mean,
-                                                                     const float *var, unsigned planes, int C, int S,
+                                                                     const float *var, unsigned outer, unsigned C, int S,
                                                                      float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned plane = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
-  if (plane >= planes)
+  typedef typename std::conditional<kVec, float4, float>::type V;
+  const unsigned w = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
+  const unsigned n0 = w / C * kSamples, c = w % C;
+  if (n0 >= outer)
     return;
-  const bool keep = (size_t)planes * S * sizeof(float) <= kKeepBytes;
-  const int lane = threadIdx.x & 31;
-  const int c = (int)(plane % (unsigned)C);
-  constexpr int kPer = kVec ? 7 : 4; // a 28 x 28 plane is 196 float4: seven per lane, all in flight at once
-  if (kVec) {
-    const int S4 = S / 4;
-    const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)plane * S4;
-    float4 *yp = reinterpret_cast<float4 *>(y) + (size_t)plane * S4;
-    float4 v[kPer];
+  const bool keep = (size_t)outer * C * S * sizeof(float) <= kKeepBytes;
+  const int lane = threadIdx.x & 31, Sv = kVec ? S / 4 : S;
+  const size_t step = (size_t)C * Sv; // from a sample's plane to the next's
+  const V *xp = reinterpret_cast<const V *>(x) + n0 * step + (size_t)c * Sv;
+  V *yp = reinterpret_cast<V *>(y) + n0 * step + (size_t)c * Sv;
+  V v[kSamples][kPer];
+#pragma unroll
+  for (int r = 0; r < kSamples; ++r)
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
-      if (lane + 32 * u < S4)
-        v[u] = __ldcs(xp + lane + 32 * u);
-    const float m = __ldg(mean + c);
-    const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
-    const float g = gamma ? __ldg(gamma + c) : 1.0f;
-    const float b = beta ? __ldg(beta + c) : 0.0f;
-    auto one = [&](float4 a) {
-      float4 r;
-      r.x = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(a.x, m), g), sd), b);
-      r.y = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(a.y, m), g), sd), b);
-      r.z = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(a.z, m), g), sd), b);
-      r.w = __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(a.w, m), g), sd), b);
-      return r;
-    };
+      if (n0 + r < outer && lane + 32 * u < Sv)
+        v[r][u] = __ldcs(xp + r * step + lane + 32 * u);
+  const float m = __ldg(mean + c);
+  const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
+  const float g = gamma ? __ldg(gamma + c) : 1.0f;
+  const float b = beta ? __ldg(beta + c) : 0.0f;
+  auto value = [&](float t) { return __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(t, m), g), sd), b); };
+  auto one = [&](V a) {
+    if constexpr (kVec)
+      return make_float4(value(a.x), value(a.y), value(a.z), value(a.w));
+    else
+      return value(a);
+  };
 #pragma unroll
-    for (int u = 0; u < kPer; ++u)
-      if (lane + 32 * u < S4)
-        st_result(yp + lane + 32 * u, one(v[u]), keep);
-    for (int i = lane + 32 * kPer; i < S4; i += 32)
-      st_result(yp + i, one(__ldcs(xp + i)), keep);
-  } else {
-    const float *xp = x + (size_t)plane * S;
-    float *yp = y + (size_t)plane * S;
-    float v[kPer];
+  for (int r = 0; r < kSamples; ++r)
+    if (n0 + r < outer) {
 #pragma unroll
-    for (int u = 0; u < kPer; ++u)
-      if (lane + 32 * u < S)
-        v[u] = __ldcs(xp + lane + 32 * u);
-    const float m = __ldg(mean + c);
-    const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
-    const float g = gamma ? __ldg(gamma + c) : 1.0f;
-    const float b = beta ? __ldg(beta + c) : 0.0f;
-#pragma unroll
-    for (int u = 0; u < kPer; ++u)
-      if (lane + 32 * u < S)
-        st_result(yp + lane + 32 * u, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(v[u], m), g), sd), b), keep);
-    for (int i = lane + 32 * kPer; i < S; i += 32)
-      st_result(yp + i, __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(__ldcs(xp + i), m), g), sd), b), keep);
-  }
+      for (int u = 0; u < kPer; ++u)
+        if (lane + 32 * u < Sv)
+          st_result(yp + r * step + lane + 32 * u, one(v[r][u]), keep);
+      for (int i = lane + 32 * kPer; i < Sv; i += 32)
+        st_result(yp + r * step + i, one(__ldcs(xp + r * step + i)), keep);
+    }
 }
 
 // Planes whose size is not a multiple of 4 (7 x 7 = 49 values): four consecutive planes are S float4, 16-byte
-// aligned when the plane count is a multiple of 4, and a warp takes such a group. Lanes 0..3 hold the constants of
+// aligned when the plane count is a multiple of 4, and a warp takes such a group of kSamples samples (C % 4 == 0, unit =
+// C / 4 groups a sample), or one group of all (kSamples = 1, unit = groups, outer = 1). Lanes 0..3 hold the constants of
 // the group's four channels; a float4 lies in one channel or across two neighbours (S >= 32), whose constants come
-// by shuffle. A quarter of the load / store instructions of the scalar form, the same rounded operations.
+// by shuffle, once for the samples. A quarter of the load / store instructions of the scalar form, the same rounded
+// operations. [256, 512, 7, 7] 13.7 us, with two samples 12.1 (the selections and divisions bound it).
+template <int kSamples>
 __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const float *__restrict__ x, const float *beta,
                                                                       const float *gamma, const float *mean,
-                                                                      const float *var, unsigned groups, int C, int S,
-                                                                      float eps, float *__restrict__ y) {
+                                                                      const float *var, unsigned outer, unsigned unit, int C,
+                                                                      int S, float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned group = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
-  if (group >= groups)
+  const unsigned w = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
+  const unsigned n0 = w / unit * kSamples, group = w % unit;
+  if (n0 >= outer)
     return;
-  const bool keep = (size_t)groups * S * sizeof(float4) <= kKeepBytes;
+  const bool keep = (size_t)outer * unit * S * sizeof(float4) <= kKeepBytes;
   const int lane = threadIdx.x & 31;
-  const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)group * S;
-  float4 *yp = reinterpret_cast<float4 *>(y) + (size_t)group * S;
+  const size_t step = (size_t)unit * S;
+  const float4 *xp = reinterpret_cast<const float4 *>(x) + n0 * step + (size_t)group * S;
+  float4 *yp = reinterpret_cast<float4 *>(y) + n0 * step + (size_t)group * S;
   constexpr int kPer = 2;
-  float4 v[kPer];
+  float4 v[kSamples][kPer];
 #pragma unroll
-  for (int u = 0; u < kPer; ++u)
-    if (lane + 32 * u < S)
-      v[u] = __ldcs(xp + lane + 32 * u);
+  for (int r = 0; r < kSamples; ++r)
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (n0 + r < outer && lane + 32 * u < S)
+        v[r][u] = __ldcs(xp + r * step + lane + 32 * u);
   const int c = (int)((group * 4u + (unsigned)(lane & 3)) % (unsigned)C);
   const float m = __ldg(mean + c);
   const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
   const float g = gamma ? __ldg(gamma + c) : 1.0f;
   const float b = beta ? __ldg(beta + c) : 0.0f;
-  auto one = [&](int j, float4 a) { // all lanes of the warp call this together (shuffles)
-    const int e = 4 * j;
+  const int rounds = (S + 31) / 32;
+  auto round = [&](int u, auto load) { // all lanes of the warp call this together (shuffles)
+    const int j = lane + 32 * u, e = 4 * (j < S ? j : 0);
     const int k0 = (e >= S) + (e >= 2 * S) + (e >= 3 * S);
     const int k1 = k0 < 3 ? k0 + 1 : 3;
     const float m0 = __shfl_sync(0xffffffffu, m, k0), m1 = __shfl_sync(0xffffffffu, m, k1);
@@ -221,25 +219,19 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const floa
       const bool nx = idx >= edge;
       return __fadd_rn(__fdiv_rn(__fmul_rn(__fsub_rn(t, nx ? m1 : m0), nx ? g1 : g0), nx ? s1 : s0), nx ? b1 : b0);
     };
-    return make_float4(el(a.x, e), el(a.y, e + 1), el(a.z, e + 2), el(a.w, e + 3));
-  };
-  const int rounds = (S + 31) / 32;
 #pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    if (u < rounds) { // warp-uniform
-      const int j = lane + 32 * u;
-      const float4 r = one(j < S ? j : 0, j < S ? v[u] : make_float4(0.f, 0.f, 0.f, 0.f));
-      if (j < S)
-        st_result(yp + j, r, keep);
-    }
-  }
-  for (int u = kPer; u < rounds; ++u) {
-    const int j = lane + 32 * u;
-    const float4 a = j < S ? __ldcs(xp + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 r = one(j < S ? j : 0, a);
-    if (j < S)
-      st_result(yp + j, r, keep);
-  }
+    for (int r = 0; r < kSamples; ++r)
+      if (n0 + r < outer && j < S) {
+        const float4 a = load(r, j);
+        st_result(yp + r * step + j, make_float4(el(a.x, e), el(a.y, e + 1), el(a.z, e + 2), el(a.w, e + 3)), keep);
+      }
+  };
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (u < rounds) // warp-uniform
+      round(u, [&](int r, int) { return v[r][u]; });
+  for (int u = kPer; u < rounds; ++u)
+    round(u, [&](int r, int j) { return __ldcs(xp + r * step + j); });
 }
 
 // ReLU (src/nbla/function/generic/relu.cpp): y = max(0, x); Add2 (add2.cpp): y = a + b.
@@ -692,20 +684,30 @@ int nb200_batch_normalization_inference_f32(const float *x, const float *beta, c
     NB_CUDA(launch_dependent(bn_inference_plane_kernel, dim3((unsigned)(outer * channels * chunks)), dim3(kThreads), 0,
                              as_stream(stream), x, beta, gamma, mean, var, (int)channels, S4, (unsigned)chunks, eps, y));
   } else if (inner >= 32 && inner < 4 * kThreads && outer * channels < (1ll << 31)) {
-    const unsigned planes = (unsigned)(outer * channels);
-    const dim3 grid((planes + kThreads / 32 - 1) / (kThreads / 32));
+    const int64_t planes = outer * channels;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-    if (vec)
-      NB_CUDA(launch_dependent(bn_inference_warp_kernel<true>, grid, dim3(kThreads), 0, as_stream(stream), x, beta,
-                               gamma,
-                               mean, var, planes, (int)channels, (int)inner, eps, y));
-    else if (aligned && planes % 4 == 0)
-      NB_CUDA(launch_dependent(bn_inference_warp4_kernel, dim3((planes / 4 + kThreads / 32 - 1) / (kThreads / 32)),
-                               dim3(kThreads), 0, as_stream(stream), x, beta, gamma, mean, var, planes / 4,
+    // two samples per warp where every SM still has a block ([16, 256, 14, 14] 4.0 us, now 2.4) and a plane is two vectors
+    // of a lane or less (a 28 x 28 plane fills a lane's registers by itself)
+    auto blocks = [&](int64_t warps) { return dim3((unsigned)((warps + kThreads / 32 - 1) / (kThreads / 32))); };
+    const int64_t full = (int64_t)sm_count() * (kThreads / 32); // warps
+    auto launch = [&](auto kernel, int samples) {
+      return launch_dependent(kernel, blocks((outer + samples - 1) / samples * channels), dim3(kThreads), 0, as_stream(stream), x,
+                              beta, gamma, mean, var, (unsigned)outer, (unsigned)channels, (int)inner, eps, y);
+    };
+    if (vec && inner <= 256 && planes >= kBnSamples * full)
+      NB_CUDA(launch(bn_inference_warp_kernel<true, 2, kBnSamples>, kBnSamples));
+    else if (vec)
+      NB_CUDA(launch(bn_inference_warp_kernel<true, 7, 1>, 1)); // a 28 x 28 plane is 196 float4: seven per lane
+    else if (aligned && channels % 4 == 0 && planes / 4 >= kBnSamples * full)
+      NB_CUDA(launch_dependent(bn_inference_warp4_kernel<kBnSamples>,
+                               blocks((outer + kBnSamples - 1) / kBnSamples * (channels / 4)), dim3(kThreads), 0,
+                               as_stream(stream), x, beta, gamma, mean, var, (unsigned)outer, (unsigned)(channels / 4),
                                (int)channels, (int)inner, eps, y));
+    else if (aligned && planes % 4 == 0)
+      NB_CUDA(launch_dependent(bn_inference_warp4_kernel<1>, blocks(planes / 4), dim3(kThreads), 0, as_stream(stream), x, beta,
+                               gamma, mean, var, 1u, (unsigned)(planes / 4), (int)channels, (int)inner, eps, y));
     else
-      NB_CUDA(launch_dependent(bn_inference_warp_kernel<false>, grid, dim3(kThreads), 0, as_stream(stream), x, beta,
-                               gamma, mean, var, planes, (int)channels, (int)inner, eps, y));
+      NB_CUDA(launch(bn_inference_warp_kernel<false, 4, 1>, 1));
   } else if (vec)
     NB_CUDA(launch_dependent(bn_inference_kernel<true>, dim3(grid_for(total / 4, 2)), dim3(kThreads), 0,
                              as_stream(stream), x, beta, gamma, mean, var, total, (int)channels, (int)inner, eps, y));

@@ -62,6 +62,14 @@ def test_batch_normalization_chunks(F, shape):
     assert same(y, want)
 
 
+# small planes, two samples per warp and one: odd numbers of samples, the largest planes of each form, groups of four planes
+# that are one sample's and that are not
+@pytest.mark.parametrize("shape", [(19, 256, 14, 14), (9, 512, 4, 9), (5, 1000, 16, 16), (5, 1000, 10, 26), (41, 516, 7, 7),
+                                   (41, 515, 7, 7), (40, 515, 5, 7), (11, 1024, 31, 33), (3, 8, 14, 14), (1, 4, 7, 7)])
+def test_batch_normalization_small_planes(F, shape):
+    test_batch_normalization_chunks(F, shape)
+
+
 def test_streaming_results(F):
     """Past 240 MB results leave with the streaming policy: the same values."""
     n = (240 << 20) // 4 + 4099
