@@ -1,8 +1,7 @@
 // Elementwise quantizers for sm_100a: FixedPointQuantize, Pow2Quantize and
 // MinMaxQuantize forward. All three are HBM-bound (4 B read + 4 B written per
-// element): 128-bit coalesced streaming accesses, grid-stride loops with four
-// independent loads in flight per thread, grid sized in multiples of the SM
-// count. Arithmetic is arranged to be bit-identical to the reference's scalar
+// element): 128-bit coalesced accesses, up to four independent loads in flight
+// per thread, blocks of consecutive elements. Arithmetic is arranged to be bit-identical to the reference's scalar
 // CPU loops; each kernel names the loop it replaces.
 #include <cmath>
 #include <cstdio>
@@ -109,7 +108,7 @@ inline unsigned grid_for(size_t work_items) {
   return (unsigned)blocks;
 }
 
-// The vector kernels take kUnroll groups per thread, or one while the tensor is so small that every SM has room for all
+// The vector kernels take kUnroll groups per thread (the quantizers two for some sizes), or one while the tensor is so small that every SM has room for all
 // its blocks at once, so that small tensors spread over the chip.
 inline bool few_quads(size_t n4) { return n4 <= (size_t)sm_count() * 4 * kThreads; }
 inline unsigned blocks_for(size_t n4, int per_thread) {
@@ -135,6 +134,11 @@ template <typename Op> int launch_elementwise(const float *x, float *y, size_t s
   const size_t n4 = (size - head) / 4;
   if (few_quads(n4))
     NB_CUDA(launch_dependent(ew_vec_kernel<Op, 1>, dim3(blocks_for(n4, 1)), dim3(kThreads), 0, st, x, y, size, head, n4,
+                             op));
+  else if (n4 <= (size_t)sm_count() * 8 * kThreads * 2 * kUnroll)
+    // four a thread would be less than two rounds of resident blocks, the last one nearly empty. FixedPointQuantize of 2^20
+    // values 2.7 us with four, 2.3 with two, 2^22 5.2 and 4.9; Pow2Quantize 3.6 and 3.0, 7.1 and 6.4; 2^24 23.4 and 24.9
+    NB_CUDA(launch_dependent(ew_vec_kernel<Op, 2>, dim3(blocks_for(n4, 2)), dim3(kThreads), 0, st, x, y, size, head, n4,
                              op));
   else
     NB_CUDA(launch_dependent(ew_vec_kernel<Op, kUnroll>, dim3(blocks_for(n4, kUnroll)), dim3(kThreads), 0, st, x, y, size,
@@ -582,45 +586,38 @@ struct Pow2FastOp {
   __device__ __forceinline__ void store_codes4(size_t, float, float, float, float) const {}
   struct State {};
   __device__ __forceinline__ State init() const { return State(); }
+  // the snapped power of a magnitude that the addition below does not decide
+  __device__ __forceinline__ float special(float a, uint32_t bits) const {
+    const uint32_t E = bits >> 23;
+    if (E == 255u)
+      return a;
+    if (E != 0u) { // a few ulp from the cut; 2^k for k in [-126, 128], where 128 assembles +inf like powf(2, 128)
+      const int k = (int)E - 127;
+      return __uint_as_float((E + ((bits & 0x7fffffu) > __ldg(&tables->cut[k - kMinExp]) ? 1u : 0u)) << 23);
+    }
+    const int p = 31 - __clz(bits); // denormal
+    const int e = p - 149;
+    const uint32_t frac = (bits << (23 - p)) & 0x7fffffu;
+    const int k = e + ((frac > __ldg(&tables->cut[e - kMinExp])) ? 1 : 0);
+    return __ldg(&tables->pw[k - kMinExp]);
+  }
+  // The mantissa's comparison with the cut is one addition whose carry goes into the exponent, and zero needs no test of
+  // its own: with a branch per kind of value 2^30 values took 1.47 ms and 2^26 96 us, now 1.22 ms and 81 us (HBM).
   __device__ __forceinline__ float operator()(float x, size_t, float &, const State &) const {
     const float a = fabsf(x);
-    const uint32_t bits = __float_as_uint(a);
-    const uint32_t E = bits >> 23;
-    float q;
-    if (E - 1u < 254u) { // normal number
-      const uint32_t frac = bits & 0x7fffffu;
-      int k = (int)E - 127;
-      if (frac >= kCutCentre + margin) {
-        k += 1;
-      } else if (frac + margin > kCutCentre) {
-        k += (frac > __ldg(&tables->cut[k - kMinExp])) ? 1 : 0;
-      }
-      // 2^k for k in [-126, 128]; k = 128 assembles +inf like powf(2, 128); k = -126 - 1 cannot occur here
-      q = __uint_as_float((uint32_t)(k + 127) << 23);
-    } else if (bits == 0u) {
-      q = 0.0f;
-    } else if (E == 255u) {
-      q = a;
-    } else { // denormal input
-      const int p = 31 - __clz(bits);
-      const int e = p - 149;
-      const uint32_t frac = (bits << (23 - p)) & 0x7fffffu;
-      const int k = e + ((frac > __ldg(&tables->cut[e - kMinExp])) ? 1 : 0);
-      q = __ldg(&tables->pw[k - kMinExp]);
-    }
-    if (q > P.p_max) {
+    const uint32_t bits = __float_as_uint(a), frac = bits & 0x7fffffu;
+    float q = __uint_as_float((bits + (0x800000u - (kCutCentre + margin))) & 0x7f800000u);
+    const bool normal = bits - 0x800000u < 0x7f000000u, near = frac - (kCutCentre - margin + 1u) < 2u * margin - 1u;
+    if ((!normal && bits != 0u) || near)
+      q = special(a, bits);
+    if (q > P.p_max)
       q = P.p_max;
-    } else if (q < P.p_min) {
-      q = P.with_zero ? (a < P.prune ? 0.0f : P.p_min) : P.p_min;
-    }
+    else if (q < P.p_min)
+      q = P.with_zero && a < P.prune ? 0.0f : P.p_min;
     const bool neg = x < 0.0f;
     if (P.sign)
-      q = neg ? -q : q;
-    else if (P.with_zero)
-      q = neg ? 0.0f : q;
-    else
-      q = neg ? P.p_min : q;
-    return q;
+      return neg ? -q : q;
+    return neg ? (P.with_zero ? 0.0f : P.p_min) : q;
   }
 };
 

@@ -62,6 +62,27 @@ def test_batch_normalization_chunks(F, shape):
     assert same(y, want)
 
 
+# two vectors a thread up to 148 * 8 * 256 * 8 of them, four above; and every kind of magnitude of Pow2Quantize: all exponents,
+# mantissas around the cut at sqrt(2), zeros of both signs, denormals, infinities, NaN
+@pytest.mark.parametrize("form", [(True, True, 8, 1), (True, False, 4, 0), (False, True, 5, 2), (False, False, 3, -3)])
+@pytest.mark.parametrize("size", [FEW + 4, 4 * 148 * 8 * 256 * 8 - 1, 4 * 148 * 8 * 256 * 8 + 4 * 1024 + 3])
+def test_quantizers_two_and_four_vectors(F, size, form):
+    rng = np.random.RandomState(size % 1000)
+    a = rng.uniform(-9, 9, size).astype(np.float32)
+    cut = np.float32(np.sqrt(2.0)).view(np.int32) & 0x7fffff
+    exponents = np.arange(256, dtype=np.int64)[:, None] << 23
+    mantissas = np.concatenate([cut + np.arange(-40, 41), [0, 1, 2, 0x400000, 0x7ffffe, 0x7fffff]])[None, :]
+    special = (exponents | mantissas).astype(np.uint32).reshape(-1).view(np.float32)
+    special = np.concatenate([special, -special])
+    a[:special.size] = special
+    a[-special.size:] = special[::-1]
+    got, want = F.pow2_quantize(tensor(a), *form).cpu().numpy(), oracle.pow2_quantize(a, *form)
+    nan = np.isnan(want)
+    assert np.array_equal(np.isnan(got), nan) and np.array_equal(bits(got)[~nan], bits(want)[~nan])
+    b = rng.uniform(-9, 9, size).astype(np.float32)
+    assert same(F.fixed_point_quantize(tensor(b), True, 8, 2.0 ** -4), oracle.fixed_point_quantize(b, True, 8, 2.0 ** -4))
+
+
 # small planes, two samples per warp and one: odd numbers of samples, the largest planes of each form, groups of four planes
 # that are one sample's and that are not
 @pytest.mark.parametrize("shape", [(19, 256, 14, 14), (9, 512, 4, 9), (5, 1000, 16, 16), (5, 1000, 10, 26), (41, 516, 7, 7),
