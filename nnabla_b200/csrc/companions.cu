@@ -77,11 +77,10 @@ __global__ void __launch_bounds__(kThreads) bn_inference_kernel(const float *__r
 __global__ void __launch_bounds__(kThreads) bn_inference_plane_kernel(const float *__restrict__ x, const float *beta,
                                                                       const float *gamma, const float *mean,
                                                                       const float *var, int C, int S4, unsigned chunks,
-                                                                      float eps, float *__restrict__ y) {
+                                                                      bool keep, float eps, float *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const unsigned block = gridDim.x - 1 - blockIdx.x, plane = block / chunks;
-  const bool keep = (size_t)(gridDim.x / chunks) * S4 * sizeof(float4) <= kKeepBytes;
+  const unsigned block = gridDim.x - 1 - blockIdx.x, plane = chunks == 1 ? block : block / chunks;
   const int c = (int)(plane % (unsigned)C);
   const float4 *xp = reinterpret_cast<const float4 *>(x) + (size_t)plane * S4;
   float4 *yp = reinterpret_cast<float4 *>(y) + (size_t)plane * S4;
@@ -274,16 +273,21 @@ __global__ void __launch_bounds__(kThreads) unary_binary_kernel(const float *__r
   }
 }
 
-// Vectors (or values, unaligned) of a thread: four, or one while that leaves every SM room for all its blocks at once.
+// Vectors (or values, unaligned) of a thread: four; two while four would be less than two rounds of resident blocks, the last
+// one nearly empty (ReLU of 2^21 values 3.4 us with four, 2.6 with two; Add2 3.4 and 2.9); or one while that leaves every SM room for all its blocks at once.
 template <int kOp> int launch_unary_binary(const float *a, const float *b, size_t size, float *y, cudaStream_t st) {
   const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(kOp == 0 ? a : b) |
                      reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   const size_t items = vec ? size / 4 : size;
-  const bool few = items <= (size_t)sm_count() * 4 * kThreads;
-  const size_t per = (size_t)kThreads * (few ? 1 : 4);
+  const int each = items <= (size_t)sm_count() * 4 * kThreads ? 1 : items <= (size_t)sm_count() * 8 * kThreads * 8 ? 2 : 4;
+  const size_t per = (size_t)kThreads * each;
   const size_t blocks = items ? (items + per - 1) / per : 1;
-  auto kernel = vec ? (few ? unary_binary_kernel<kOp, true, 1> : unary_binary_kernel<kOp, true, 4>)
-                    : (few ? unary_binary_kernel<kOp, false, 1> : unary_binary_kernel<kOp, false, 4>);
+  auto kernel = vec ? (each == 1   ? unary_binary_kernel<kOp, true, 1>
+                       : each == 2 ? unary_binary_kernel<kOp, true, 2>
+                                   : unary_binary_kernel<kOp, true, 4>)
+                    : (each == 1   ? unary_binary_kernel<kOp, false, 1>
+                       : each == 2 ? unary_binary_kernel<kOp, false, 2>
+                                   : unary_binary_kernel<kOp, false, 4>);
   NB_CUDA(launch_dependent(kernel, dim3((unsigned)blocks), dim3(kThreads), 0, st, a, b, size, y));
   NB_LAUNCH_CHECK();
   return NB200_OK;
@@ -682,7 +686,8 @@ int nb200_batch_normalization_inference_f32(const float *x, const float *beta, c
   if (vec && inner >= 4 * kThreads && outer * channels * chunks < (1ll << 31)) {
     const int S4 = (int)(inner / 4);
     NB_CUDA(launch_dependent(bn_inference_plane_kernel, dim3((unsigned)(outer * channels * chunks)), dim3(kThreads), 0,
-                             as_stream(stream), x, beta, gamma, mean, var, (int)channels, S4, (unsigned)chunks, eps, y));
+                             as_stream(stream), x, beta, gamma, mean, var, (int)channels, S4, (unsigned)chunks,
+                             total * sizeof(float) <= kKeepBytes, eps, y));
   } else if (inner >= 32 && inner < 4 * kThreads && outer * channels < (1ll << 31)) {
     const int64_t planes = outer * channels;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
