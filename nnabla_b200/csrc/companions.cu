@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(kThreads) unary_binary_kernel(const float *__r
 }
 
 // Vectors (or values, unaligned) of a thread: four; two while four would be less than two rounds of resident blocks, the last
-// one nearly empty (ReLU of 2^21 values 3.4 us with four, 2.6 with two; Add2 3.4 and 2.9); or one while that leaves every SM room for all its blocks at once.
+// one nearly empty (ReLU of 2^21 values 3.4 us with four, 2.6 with two; Add2 3.4 and 2.9); or one while that leaves every SM
+// room for all its blocks at once.
 template <int kOp> int launch_unary_binary(const float *a, const float *b, size_t size, float *y, cudaStream_t st) {
   const bool vec = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(kOp == 0 ? a : b) |
                      reinterpret_cast<uintptr_t>(y)) & 15) == 0;

@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // (in the halo form the ring is replaced by the pixel-tile buffers, counted by the caller)
 template <int BN, int STAGES, int RB, bool kResidentB = false, bool kHalo = false>
 constexpr size_t conv_codes_smem_bytes() {
-  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) + (2 * STAGES + 4 + 2 * kTileBufs + kWeightParts) * 8 + 32 +
-         kCodesMaxMaps * sizeof(float2) + kCodesKTable * sizeof(int4) + 1024;
+  return (kHalo ? 0 : (size_t)STAGES * (kTileM * RB + (kResidentB ? 0 : BN * RB))) +
+         (2 * STAGES + 4 + 2 * kTileBufs + kWeightParts) * 8 + 32 + kCodesMaxMaps * sizeof(float2) + kCodesKTable * sizeof(int4) + 1024;
 }
 
 } // namespace nb200
