@@ -91,6 +91,13 @@ def test_batch_normalization_small_planes(F, shape):
     test_batch_normalization_chunks(F, shape)
 
 
+# a thread per map (fewer than 24 values, but not 16); values of a map in one run of 64, in several and in parts of one; maps that fill a block of 64 and that do not
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (9, 31, 1, 23), (4, 17, 4, 4), (4, 16, 6, 4), (3, 21, 7, 7), (2, 32, 8, 8), (5, 13, 5, 13), (1, 129, 11, 19), (2, 3, 56, 56)])
+def test_global_average_pooling(F, shape):
+    x = np.random.RandomState(shape[1]).randn(*shape).astype(np.float32)
+    assert same(F.global_average_pooling(tensor(x.reshape(-1)).reshape(shape)), oracle.global_average_pooling(x))
+
+
 def test_streaming_results(F):
     """Past 240 MB results leave with the streaming policy: the same values."""
     n = (240 << 20) // 4 + 4099
