@@ -131,14 +131,16 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float
   pdl_trigger();
   typedef typename std::conditional<kVec, float4, float>::type V;
   const unsigned w = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
-  const unsigned n0 = w / C * kSamples, c = w % C;
-  if (n0 >= outer)
+  // (one sample: the plane is the warp's number, and the division for its channel waits behind the loads)
+  const unsigned n0 = kSamples == 1 ? 0 : w / C * kSamples;
+  if (kSamples == 1 ? w >= outer * C : n0 >= outer)
     return;
   const bool keep = (size_t)outer * C * S * sizeof(float) <= kKeepBytes;
   const int lane = threadIdx.x & 31, Sv = kVec ? S / 4 : S;
   const size_t step = (size_t)C * Sv; // from a sample's plane to the next's
-  const V *xp = reinterpret_cast<const V *>(x) + n0 * step + (size_t)c * Sv;
-  V *yp = reinterpret_cast<V *>(y) + n0 * step + (size_t)c * Sv;
+  const size_t first = kSamples == 1 ? (size_t)w * Sv : n0 * step + (size_t)(w % C) * Sv;
+  const V *xp = reinterpret_cast<const V *>(x) + first;
+  V *yp = reinterpret_cast<V *>(y) + first;
   V v[kSamples][kPer];
 #pragma unroll
   for (int r = 0; r < kSamples; ++r)
@@ -146,6 +148,7 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp_kernel(const float
     for (int u = 0; u < kPer; ++u)
       if (n0 + r < outer && lane + 32 * u < Sv)
         v[r][u] = __ldcs(xp + r * step + lane + 32 * u);
+  const unsigned c = w % C;
   const float m = __ldg(mean + c);
   const float sd = __fsqrt_rn(__fadd_rn(__ldg(var + c), eps));
   const float g = gamma ? __ldg(gamma + c) : 1.0f;
@@ -183,8 +186,8 @@ __global__ void __launch_bounds__(kThreads) bn_inference_warp4_kernel(const floa
   pdl_wait();
   pdl_trigger();
   const unsigned w = (unsigned)block_descending() * (kThreads / 32) + (threadIdx.x >> 5);
-  const unsigned n0 = w / unit * kSamples, group = w % unit;
-  if (n0 >= outer)
+  const unsigned n0 = kSamples == 1 ? 0 : w / unit * kSamples, group = kSamples == 1 ? w : w % unit;
+  if (kSamples == 1 ? w >= unit : n0 >= outer)
     return;
   const bool keep = (size_t)outer * unit * S * sizeof(float4) <= kKeepBytes;
   const int lane = threadIdx.x & 31;
