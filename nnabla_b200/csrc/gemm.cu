@@ -238,6 +238,36 @@ static bool gemm_transposes(int64_t M, int64_t N) {
   return ((M + 127) / 128) * ((N + 127) / 128) < sms && rounds(64, 128) * 40 <= rounds(128, 64) * 56;
 }
 
+// Which kernel a product takes: the one answer that run_gemm launches by and binary_affine prepares alpha by. `ep` as
+// run_gemm gets it, but for col_scale and alpha's fields.
+enum class GemmRoute { kPair, kTransposed, kSingle };
+static GemmRoute gemm_route(bool int8, int planes_a, int planes_b, int M, int N, int k_blocks, const GemmEpilogue &ep,
+                            int64_t ldy) {
+  // Large problems: two-SM tiles (256 x 256 per CTA pair) halve the B traffic per SM.
+  // NNABLA_B200_GEMM_PAIR=0 forces the single-CTA kernel (debugging aid).
+  static const bool pair_enabled = []() {
+    const char *e = std::getenv("NNABLA_B200_GEMM_PAIR");
+    return !(e && e[0] == '0');
+  }();
+  const int64_t pair_tiles = (int64_t)((M + kPairTileM - 1) / kPairTileM) * ((N + kPairTileN - 1) / kPairTileN);
+  // (the bulk stores of its epilogue need a 16-byte aligned y with a row pitch that is a multiple of 16 bytes)
+  const bool y_tma_ok = (reinterpret_cast<uintptr_t>(ep.y) & 15) == 0 && (ldy % 4) == 0;
+  // (peer copies of y and accumulation into y need the plain stores of the single-CTA kernel's epilogue)
+  // (the two-SM kernel accumulates a whole tile in tensor memory; long floating-point K loops go to the
+  // single-CTA kernel, whose chunked accumulation bounds the truncation error)
+  if (pair_enabled && y_tma_ok && ep.n_peers == 0 && !ep.accumulate && planes_b == 1 && pair_tiles >= sm_count() / 2 &&
+      (int8 || (planes_a == 3 && k_blocks * 12 <= 384)))
+    return GemmRoute::kPair;
+  return !int8 && planes_a == 3 && planes_b == 1 && ep.n_peers == 0 && !ep.row_scale && !ep.row_bias && gemm_transposes(M, N)
+             ? GemmRoute::kTransposed
+             : GemmRoute::kSingle;
+}
+// The transposed product's tiles (128 of y's columns by 64 rows) and the KB that a K block of one takes.
+constexpr int kTransposedRows = 64, kTransposedBlockKb = 40;
+static int64_t transposed_tiles(int M, int N) {
+  return (int64_t)((N + kTileM - 1) / kTileM) * ((M + kTransposedRows - 1) / kTransposedRows);
+}
+
 // A: [planes_a][M][pitch_a], B: [planes_b][N][pitch_b], both K-major.
 int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch_a, const void *B, int64_t pitch_b,
              int M, int N, int K, const GemmEpilogue &ep, int64_t ldy, cudaStream_t st) {
@@ -249,24 +279,12 @@ int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch
   const bool narrow = (int64_t)m_tiles * ((N + 127) / 128) < sm_count();
   CUtensorMap ma, mb;
   NB_TRY(make_operand_map(&ma, A, int8, K, pitch_a, M, planes_a, kTileM));
-  // Large problems: two-SM tiles (256 x 256 per CTA pair) halve the B traffic per SM.
-  // NNABLA_B200_GEMM_PAIR=0 forces the single-CTA kernel (debugging aid).
-  static const bool pair_enabled = []() {
-    const char *e = std::getenv("NNABLA_B200_GEMM_PAIR");
-    return !(e && e[0] == '0');
-  }();
-  const int64_t pair_tiles = (int64_t)((M + kPairTileM - 1) / kPairTileM) * ((N + kPairTileN - 1) / kPairTileN);
-  // (the bulk stores of its epilogue need a 16-byte aligned y with a row pitch that is a multiple of 16 bytes)
-  const bool y_tma_ok = (reinterpret_cast<uintptr_t>(ep.y) & 15) == 0 && (ldy % 4) == 0;
-  // (peer copies of y and accumulation into y need the plain stores of the single-CTA kernel's epilogue)
-  if (pair_enabled && y_tma_ok && ep.n_peers == 0 && !ep.accumulate && planes_b == 1 && pair_tiles >= sm_count() / 2) {
+  const GemmRoute route = gemm_route(int8, planes_a, planes_b, M, N, k_blocks, ep, ldy);
+  NB_CHECK(!ep.alpha_partial || route == GemmRoute::kTransposed, NB200_EVALUE, "this route does not make alpha");
+  if (route == GemmRoute::kPair) {
     NB_TRY(make_operand_map(&mb, B, int8, K, pitch_b, N, 1, kPairTileN / 2));
-    if (int8)
-      return launch_pair_gemm<true, 1, 6>(ma, mb, M, N, k_blocks, ep, ldy, st);
-    // (the two-SM kernel accumulates a whole tile in tensor memory; long floating-point K loops go to the
-    // single-CTA kernel, whose chunked accumulation bounds the truncation error)
-    if (planes_a == 3 && k_blocks * 12 <= 384)
-      return launch_pair_gemm<false, 3, 3>(ma, mb, M, N, k_blocks, ep, ldy, st);
+    return int8 ? launch_pair_gemm<true, 1, 6>(ma, mb, M, N, k_blocks, ep, ldy, st)
+                : launch_pair_gemm<false, 3, 3>(ma, mb, M, N, k_blocks, ep, ldy, st);
   }
   if (int8) {
     NB_CHECK(planes_a == 1 && planes_b == 1, NB200_EVALUE, "int8 operands have one plane");
@@ -283,18 +301,19 @@ int run_gemm(bool int8, int planes_a, int planes_b, const void *A, int64_t pitch
     return launch_gemm<true, 1, 1, 64, 8, false>(ma, mb, M, N, k_blocks, ep, ldy, st);
   }
   if (planes_a == 3 && planes_b == 1) {
-    if (ep.n_peers == 0 && !ep.row_scale && !ep.row_bias && gemm_transposes(M, N)) {
+    if (route == GemmRoute::kTransposed) {
       GemmTransposedProblem prob;
-      fill_problem(prob, N, M, k_blocks, 64, k_chunk_blocks(3 * 4), ldy);
+      fill_problem(prob, N, M, k_blocks, kTransposedRows, k_chunk_blocks(3 * 4), ldy);
       NB_TRY(make_operand_map(&ma, B, false, K, pitch_b, N, 1, kTileM));
-      NB_TRY(make_operand_map(&mb, A, false, K, pitch_a, M, 3, 64));
-      return run_in_parts(prob, 40, M, N, ep, ldy, st, [&](const GemmTransposedProblem &p, const GemmEpilogue &e) {
+      NB_TRY(make_operand_map(&mb, A, false, K, pitch_a, M, 3, kTransposedRows));
+      auto launch = [&](const GemmTransposedProblem &p, const GemmEpilogue &e) {
         GemmEpilogue t = e;
         t.row_scale = e.col_scale, t.row_bias = e.col_bias;
         t.col_scale = t.col_bias = nullptr;
-        return launch_contraction<false, 1, 3, 64, 4, 0, GemmTransposedProblem>(
+        return launch_contraction<false, 1, 3, kTransposedRows, 4, 0, GemmTransposedProblem>(
             ma, mb, p, p.k_splits * p.m_tiles * p.n_tiles, t, st);
-      });
+      };
+      return run_in_parts(prob, kTransposedBlockKb, M, N, ep, ldy, st, launch);
     }
     if (!narrow) {
       NB_TRY(make_operand_map(&mb, B, false, K, pitch_b, N, 1, 128));
@@ -346,14 +365,16 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
   void *planes = base;
   void *side = base + round_up(planes_bytes, 256);
   float *partial = reinterpret_cast<float *>(base + round_up(planes_bytes, 256) + round_up(side_bytes, 256));
-  // the transposed product makes alpha from the partial sums itself, unless its K is split
-  bool sums_left = alpha && gemm_transposes(M, N) &&
-                   k_splits_for(((N + kTileM - 1) / kTileM) * ((M + 63) / 64), (int)(Kp / 64), 40) == 1;
-  NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st, &sums_left));
   GemmEpilogue ep{};
   ep.y = y;
   ep.scale = 1.0f;
   ep.col_scale = alpha;
+  ep.col_bias = bias;
+  // the transposed product makes alpha from the partial sums itself, unless its K is split
+  const int k_blocks = (int)(Kp / 64);
+  bool sums_left = alpha && gemm_route(false, 3, 1, (int)M, (int)N, k_blocks, ep, N) == GemmRoute::kTransposed &&
+                   k_splits_for(transposed_tiles((int)M, (int)N), k_blocks, kTransposedBlockKb) == 1;
+  NB_TRY(binary_affine_operands(x, M, w, (int)K, (int)N, zero_to, wb, alpha, side, Kp, partial, planes, st, &sums_left));
   if (sums_left) {
     ep.col_scale = nullptr;
     ep.alpha_partial = partial;
@@ -361,7 +382,6 @@ static int binary_affine(const float *x, const float *w, float *wb, float *alpha
     ep.alpha_inv = (float)1 / K; // binary_weight_affine.cpp:68
     ep.alpha = alpha;
   }
-  ep.col_bias = bias;
   return run_gemm(false, 3, 1, planes, Kp, side, Kp, (int)M, (int)N, (int)K, ep, N, st);
 }
 

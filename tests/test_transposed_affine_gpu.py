@@ -36,3 +36,25 @@ def test_forward_and_input_gradient(M, K, N):
     acc = F.binary_weight_affine_backward(x, wb, alpha, dy, propagate_down=(True, False, False),
                                           accum=(True, False, False), grads=(old, None, None))[0]
     assert torch.equal(acc, dx + 1.0)
+
+
+# Around the line to the two-SM kernel, which makes no alpha: 148 SMs take 74 of its 256 x 256 tiles, while 147 of 128 x 128
+# leave one of them idle. On either side of it in outputs, in rows and in the length of K; bias and no bias.
+@pytest.mark.parametrize("M,K,N", [(64, 1024, 18704), (128, 512, 18816), (128, 512, 18688), (128, 512, 18820),
+                                   (64, 2048, 18692), (64, 2052, 18692), (64, 1024, 18702), (64, 1022, 18704),
+                                   (18816, 256, 100), (18688, 256, 100), (18689, 512, 128)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_alpha_at_the_line_to_the_two_sm_kernel(M, K, N, bias):
+    from nnabla_b200 import functions as F
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b = r(M, K), r(K, N), r(N) if bias else None
+    wb, alpha = torch.zeros_like(w), torch.full((N,), -1.0, device="cuda")
+    y = F.binary_weight_affine(x, w, wb, alpha, b)
+    a = w.double().abs().mean(0)
+    assert ((alpha.double() - a).abs() <= 4 * 2.0 ** -24 * K ** 0.5 * a).all()
+    sign = torch.where(w < 0, -1.0, 1.0)  # (a few of the many normal values are zero)
+    want = (x.double() @ sign.double()) * a + (b.double() if bias else 0.0)
+    # a whole tile's sums in tensor memory: 2.6e-6 of the root mean square at K = 1024, growing with K up to 2048
+    rms = lambda t: t.square().mean().sqrt()
+    assert rms(y.double() - want) <= 1e-5 * rms(want)
