@@ -132,6 +132,23 @@ bool read_args(Tuple &a, PyObject *const *args, int &device, std::index_sequence
   return (std::get<I>(a).read(args[I], device) && ...);
 }
 
+// Makes `device` the current one, and the caller's again on every way out of the block, exceptions among them.
+class OnDevice {
+  const int device_, before_;
+
+public:
+  explicit OnDevice(int device) : device_(device), before_(c10::cuda::current_device()) {
+    if (device_ != before_)
+      c10::cuda::set_device((c10::DeviceIndex)device_);
+  }
+  ~OnDevice() {
+    if (device_ != before_)
+      (void)c10::cuda::SetDevice((c10::DeviceIndex)before_); // (the one of the two that does not throw)
+  }
+  OnDevice(const OnDevice &) = delete;
+  OnDevice &operator=(const OnDevice &) = delete;
+};
+
 // The entry point as a Python function of its parameters without the last one, `stream`: that is torch's current
 // stream of the tensors' device, which is made the current device for the call.
 template <auto Fn> struct Entry;
@@ -145,17 +162,15 @@ template <typename... A, int (*Fn)(A...)> struct Entry<Fn> {
     int device = -1;
     if (!read_args(a, args, device, std::make_index_sequence<n>{}))
       return nullptr;
-    const int current = c10::cuda::current_device();
-    if (device >= 0 && device != current)
-      c10::cuda::set_device((c10::DeviceIndex)device);
-    std::get<n>(a).v = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)(device >= 0 ? device : current)).stream();
+    if (device < 0) // (no tensor among the arguments)
+      device = c10::cuda::current_device();
+    const OnDevice on(device);
+    std::get<n>(a).v = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
     g_calls.fetch_add(1, std::memory_order_relaxed);
     int rc;
     Py_BEGIN_ALLOW_THREADS;
     rc = std::apply([](auto &...x) { return Fn(x.v...); }, a);
     Py_END_ALLOW_THREADS;
-    if (device >= 0 && device != current)
-      c10::cuda::set_device((c10::DeviceIndex)current);
     if (rc != 0)
       return raise_status(rc);
     Py_RETURN_NONE;
@@ -377,17 +392,14 @@ at::Tensor empty_like_of(const at::Tensor &like, at::IntArrayRef shape, at::Scal
 
 // Runs an entry point on the tensors' device and torch's current stream of it; NULL after raising its error.
 template <typename F> bool run_on(const at::Tensor &t, F &&f) {
-  const int device = t.get_device(), current = c10::cuda::current_device();
-  if (device != current)
-    c10::cuda::set_device((c10::DeviceIndex)device);
+  const int device = t.get_device();
+  const OnDevice on(device);
   void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
   g_calls.fetch_add(1, std::memory_order_relaxed);
   int rc;
   Py_BEGIN_ALLOW_THREADS;
   rc = f(stream);
   Py_END_ALLOW_THREADS;
-  if (device != current)
-    c10::cuda::set_device((c10::DeviceIndex)current);
   if (rc != 0)
     raise_status(rc);
   return rc == 0;
@@ -519,9 +531,8 @@ PyObject *folded_convolutions(PyObject *, PyObject *const *a, Py_ssize_t nargs) 
   std::vector<at::Tensor> results((size_t)count);
   int rc = 0;
   {
-    const int device = x->get_device(), current = c10::cuda::current_device();
-    if (device != current)
-      c10::cuda::set_device((c10::DeviceIndex)device);
+    const int device = x->get_device();
+    const OnDevice on(device); // (an allocation below may throw)
     void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
     pybind11::gil_scoped_release no_gil;
     for (int64_t i = 0; i < count && rc == 0; ++i) {
@@ -544,8 +555,6 @@ PyObject *folded_convolutions(PyObject *, PyObject *const *a, Py_ssize_t nargs) 
         if (steps[(size_t)j].last_use == i)
           results[(size_t)j].reset();
     }
-    if (device != current)
-      c10::cuda::set_device((c10::DeviceIndex)current);
   }
   if (rc != 0)
     return raise_status(rc);

@@ -1,4 +1,8 @@
 """The binding's shape arithmetic against the mirror's full checks, without a GPU."""
+import os
+import re
+import subprocess
+
 import pytest
 
 from nnabla_b200 import functions as F
@@ -23,3 +27,36 @@ def test_operands_that_do_not_fit_are_left_to_the_full_checks(x, w, pad, group):
     assert F.L.conv2d(x, w, None, 1, pad, None, None, group) is None
     with pytest.raises(RuntimeError):
         F._conv_geometry(x, w, None, 1, pad, None, None, group)
+
+
+def test_the_callers_device_comes_back_on_every_way_out(tmp_path):
+    """The binding changes the current device in one class only; that class, compiled against a stand-in for torch's two
+    calls, puts the caller's device back after a block that ends and after one that throws."""
+    text = open(os.path.join(os.path.dirname(F.__file__), "csrc", "native.cpp")).read()
+    guard = re.search(r"^class OnDevice \{.*?^\};\n", text, re.S | re.M).group(0)
+    assert re.search(r"set_?device\(", text.replace(guard, ""), re.I) is None
+    source, program = tmp_path / "guard.cpp", tmp_path / "guard"
+    source.write_text("""
+#include <stdexcept>
+namespace c10 {
+using DeviceIndex = signed char;
+namespace cuda {
+int now = 2, changes = 0;
+DeviceIndex current_device() { return (DeviceIndex)now; }
+void set_device(DeviceIndex d) { now = d, ++changes; }
+int SetDevice(DeviceIndex d) { return now = d, ++changes, 0; }
+} // namespace cuda
+} // namespace c10
+%s
+using namespace c10::cuda;
+int main() {
+  { const OnDevice on(2); if (now != 2 || changes != 0) return 1; }
+  if (now != 2 || changes != 0) return 2;
+  { const OnDevice on(5); if (now != 5) return 3; }
+  if (now != 2 || changes != 2) return 4;
+  try { const OnDevice on(7); throw std::runtime_error("out of memory"); } catch (const std::runtime_error &) {}
+  return now == 2 ? 0 : 5;
+}
+""" % guard)
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-std=c++17", "-o", str(program), str(source)])
+    assert subprocess.run([str(program)]).returncode == 0
