@@ -929,7 +929,7 @@ int nb200_convolution_f32(const float *x, const float *w, const float *bias, flo
         // taps pair up into 64-bit shared loads when the first tap of every pixel sits at an odd column
         const bool pairs = ((4 - pad_w) & 1) == 1;
         auto kernel = pairs ? direct_conv_tile_kernel<OT, PX7, 7, 2, true> : direct_conv_tile_kernel<OT, PX7, 7, 2, false>;
-        static bool configured[64][2];
+        static std::atomic<bool> configured[64][2]{};
         int dev = 0;
         NB_CUDA(cudaGetDevice(&dev));
         if (!configured[dev & 63][pairs]) {

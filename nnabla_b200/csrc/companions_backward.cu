@@ -505,7 +505,8 @@ int bn_backward_dx_planes(const float *x, const float *dy, const float *gamma, c
 // rounds only where they are 5 % fuller (8 blocks per SM whatever the kernel's registers allow made 3 rounds of 592 blocks
 // of the gradients' 1216: [128, 64, 56, 56] 44 us, now 38).
 template <typename Kernel>
-int channel_blocks(Kernel kernel, int (&resident)[64], int64_t outer, int64_t channels, int64_t inner, bool vec, int *out) {
+int channel_blocks(Kernel kernel, std::atomic<int> (&resident)[64], int64_t outer, int64_t channels, int64_t inner, bool vec,
+                   int *out) {
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   int per_sm = resident[dev & 63]; // the same value whichever thread stores it
@@ -553,7 +554,7 @@ int nb200_batch_normalization_batch_f32(const float *x, const float *beta, const
   cudaStream_t st = as_stream(stream);
   const bool vec = (inner % 4 == 0) && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   auto stats = vec ? bn_stats_kernel<true> : bn_stats_kernel<false>;
-  static int resident[2][64];
+  static std::atomic<int> resident[2][64]{};
   int P = 0;
   NB_TRY(channel_blocks(stats, resident[vec], outer, channels, inner, vec, &P));
   AsyncScratch scratch(st);
@@ -583,7 +584,7 @@ int nb200_batch_normalization_backward_f32(const float *x, const float *dy, cons
   const bool vec = (inner % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
   auto sums_kernel = vec ? (batch_stat ? bn_backward_sums_kernel<true, true> : bn_backward_sums_kernel<true, false>)
                          : (batch_stat ? bn_backward_sums_kernel<false, true> : bn_backward_sums_kernel<false, false>);
-  static int resident[4][64];
+  static std::atomic<int> resident[4][64]{};
   int P = 0;
   NB_TRY(channel_blocks(sums_kernel, resident[2 * vec + (batch_stat != 0)], outer, channels, inner, vec, &P));
   AsyncScratch scratch(st);

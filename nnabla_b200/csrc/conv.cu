@@ -340,7 +340,7 @@ bool plan_planes(PlanesPlan &plan, const PlanesAxis &ay, const PlanesAxis &ax, i
 template <int BN, int PG, bool kResident, bool kF16>
 int launch_planes_kernel(const CUtensorMap &ma, const CUtensorMap &mb, const PlanesPlan &plan, cudaStream_t st) {
   auto kernel = conv_planes_tcgen05_kernel<BN, PG, kResident, kF16>;
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
@@ -742,7 +742,7 @@ int planes_backward(const float *x, const float *wb, const float *alpha, const f
     NB_TRY(encode_tiled(&md, 0, 5, dyp, dims, strides, box, nullptr, kRowBytes));
   }
   auto kernel = x_planes == 1 ? conv_wgrad_tcgen05_kernel<1> : conv_wgrad_tcgen05_kernel<3>;
-  static bool configured[64][2];
+  static std::atomic<bool> configured[64][2]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63][x_planes == 3]) {
@@ -1071,7 +1071,7 @@ int launch_conv_codes(const ConvGeometry &g, const int8_t *x_codes, int64_t ctot
     smem += tile_bytes;
   }
   NB_CHECK(smem <= 227 * 1024, NB200_EVALUE, "resident weights do not fit in shared memory");
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {

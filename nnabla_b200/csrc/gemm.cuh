@@ -704,7 +704,7 @@ inline int launch_contraction(const CUtensorMap &ma, const CUtensorMap &mb, cons
   // a resident A operand adds its K blocks; the attribute is set to the device maximum once
   const size_t smem = smem_fixed + (kResidentA ? (size_t)resident_k_blocks * PA * kTileM * RB : 0);
   NB_CHECK(smem <= 227 * 1024, NB200_EVALUE, "resident operand does not fit in shared memory");
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {

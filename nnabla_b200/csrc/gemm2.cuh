@@ -385,7 +385,7 @@ inline int launch_pair_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M,
   auto kernel = gemm_pair_tcgen05_kernel<kInt8, PA, STAGES>;
   constexpr size_t smem = gemm_pair_smem_bytes<kInt8, PA, STAGES>();
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {

@@ -660,7 +660,7 @@ int narrow_conv_tc(const float *x, const float *w, const float *bias, float *y, 
   auto split = stride_w == 2 ? (split_rows == 8 ? narrow_conv_split_kernel<2, 4> : narrow_conv_split_kernel<2, 1>)
                              : (split_rows == 8 ? narrow_conv_split_kernel<1, 4> : narrow_conv_split_kernel<1, 1>);
   NB_CUDA(launch_dependent(split, split_grid, dim3(256), 0, st, x, g, split_rows, maxbits, parts, xs, xscale));
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {

@@ -27,7 +27,7 @@ int fail(int code, const char *fmt, ...) {
 void clear_error() { g_error.clear(); }
 
 int sm_count() {
-  static int cached[64];
+  static std::atomic<int> cached[64]{}; // (threads that come here first all find the same)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
     return 148;

@@ -359,7 +359,7 @@ template <int TM, bool kAT, bool kBT> constexpr size_t small_gemm_smem() {
   return smem;
 }
 
-template <typename Kernel> int allow_small_gemm_smem(Kernel kernel, size_t smem, bool (&configured)[64]) {
+template <typename Kernel> int allow_small_gemm_smem(Kernel kernel, size_t smem, std::atomic<bool> (&configured)[64]) {
   int dev = 0;
   NB_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
@@ -373,7 +373,7 @@ template <int TM, bool kAT, bool kBT, SmallB kMode>
 int launch_small_gemm_tile(const SmallGemm &P, cudaStream_t st) {
   constexpr size_t smem = small_gemm_smem<TM, kAT, kBT>();
   auto kernel = small_gemm_kernel<TM, kAT, kBT, kMode>;
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   NB_TRY(allow_small_gemm_smem(kernel, smem, configured));
   const dim3 grid((unsigned)((P.N + 31) / 32), (unsigned)((P.M + TM - 1) / TM));
   NB_CUDA(launch_dependent(kernel, grid, dim3(256), smem, st, P));
@@ -385,7 +385,7 @@ int launch_small_gradients_tile(const SmallGemm &X, const SmallGemm &W, cudaStre
   constexpr size_t sx = small_gemm_smem<TMX, false, true>(), sw = small_gemm_smem<TMW, true, false>();
   constexpr size_t smem = sx > sw ? sx : sw;
   auto kernel = small_gemm_gradients_kernel<TMX, TMW, kSums>;
-  static bool configured[64];
+  static std::atomic<bool> configured[64]{};
   NB_TRY(allow_small_gemm_smem(kernel, smem, configured));
   const unsigned n_dx = (unsigned)small_gemm_tiles(X.M, X.N, TMX);
   NB_CUDA(launch_dependent(kernel, dim3(n_dx + (unsigned)small_gemm_tiles(W.M, W.N, TMW)), dim3(256), smem, st, X, W,
