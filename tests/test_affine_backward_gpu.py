@@ -7,6 +7,7 @@ import pytest
 import torch
 
 import cases
+from launches import kernels
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -97,3 +98,46 @@ def test_backward_shape_errors(F):
         F.affine_backward(x, w, torch.zeros(4, 5, device="cuda"))
     with pytest.raises(RuntimeError):
         F.affine_backward(x, w, torch.zeros(4, 6, device="cuda"), accum=(True, False, False))
+
+
+# Past the sizes of the one-launch products: operands of every product in pieces. Rows that 128-bit accesses fit and rows that
+# they do not, column sums of more than 256 row tiles, contractions in parts. Kernels of the weight gradient with db, then
+# of the input gradient.
+V, S = ["split_columns<1>", "column_finish"], ["split_columns<0>", "column_finish"]
+LARGE = [
+    (256, 1024, 4096, V + ["gemm_tcgen05"], ["split_rows<1>", "gemm_tcgen05", "split_sums<1>"]),
+    (300, 1111, 2050, S + ["gemm_tcgen05"], ["split_rows<0>", "gemm_tcgen05", "split_sums<0>"]),
+    (16500, 1024, 1024, ["split_columns<1>", "gemm_tcgen05", "column_partial_sums", "column_finish"],
+     ["split_rows<1>", "gemm_tcgen05"]),
+    (8000, 1024, 600, V + ["gemm_tcgen05", "split_sums<1>"], ["split_rows<1>", "gemm_tcgen05"]),
+    (8001, 1021, 602, S + ["gemm_tcgen05", "split_sums<0>"], ["split_rows<0>", "gemm_tcgen05"]),
+]
+
+
+@pytest.mark.parametrize("M,K,N,route_dw,route_dx", LARGE)
+@pytest.mark.parametrize("offset", [0, 1])
+def test_large_affine_backward(F, M, K, N, route_dw, route_dx, offset):
+    """offset: x and W begin so many values behind a 16-byte boundary."""
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    r = lambda *s: torch.randn(offset + int(np.prod(s)), device="cuda", generator=g)[offset:].view(*s)
+    x, w, dy = r(M, K), r(K, N), torch.randn(M, N, device="cuda", generator=g)
+    run = lambda down, **kw: F.affine_backward(x, w, dy, propagate_down=down, **kw)
+    dx, dw, db = run((True, True, True))
+    dw_alone, db_alone = run((False, True, True))[1:]
+    assert torch.equal(dw, dw_alone) and torch.equal(db, db_alone)
+    assert torch.equal(dw, run((False, True, False))[1])
+    acc = run((True, True, True), accum=(True, True, True),
+              grads=(torch.ones_like(x), torch.ones_like(w), torch.ones(N, device="cuda")))
+    F.check_device_status()
+    for a, b in zip(acc, (dx, dw, db)):
+        assert torch.equal(a, b + 1.0)
+    rms = lambda t: t.square().mean().sqrt()
+    # products: the tensor core's sums and the pieces' products that are left out, 2.0e-6 of the result's root mean square
+    # at every one of these sizes, three times that; column sums: fp32 sums of M values, 2^-24 * sqrt(M), four times that
+    for got, want, bound in ((dx, dy.double() @ w.double().t(), 6e-6), (dw, x.double().t() @ dy.double(), 6e-6),
+                             (db, dy.double().sum(0), 4 * 2.0 ** -24 * M ** 0.5)):
+        assert rms(got.double() - want) <= bound * rms(want)
+    if offset == 0:
+        routes = [kernels(lambda: run(down)) for down in ((False, True, True), (True, False, False))]
+        print("dW, db:", *routes[0], "dx:", *routes[1])
+        assert routes == [route_dw, route_dx]

@@ -7,6 +7,7 @@ import torch
 
 import cases
 from golden_util import bits, golden, sha
+from launches import kernels
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -132,6 +133,30 @@ def test_full_precision_affine(F, M, K, N):
     y = F.affine(dev(x), dev(w), dev(b))
     F.check_device_status()
     assert cases.rel_rms(y.cpu().numpy(), oracle.affine(x, w, b, f64=True)) < TOL
+
+
+# Past the sizes of the one-launch products: operands in pieces, with rows that 128-bit accesses fit and rows that they do not;
+# contractions in one part and in several.
+@pytest.mark.parametrize("M,K,N,route", [
+    (256, 1024, 4096, ["split_rows<1>", "split_columns<1>", "gemm_tcgen05"]),
+    (300, 1111, 2050, ["split_rows<0>", "split_columns<0>", "gemm_tcgen05"]),
+    (600, 8000, 1024, ["split_rows<1>", "split_columns<1>", "gemm_tcgen05", "split_sums<1>"]),
+    (603, 8001, 1022, ["split_rows<0>", "split_columns<0>", "gemm_tcgen05", "split_sums<0>"])])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_large_full_precision_affine(F, M, K, N, route, offset):
+    """offset: x and W begin so many values behind a 16-byte boundary."""
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    r = lambda *s: torch.randn(offset + int(np.prod(s)), device="cuda", generator=g)[offset:].view(*s)
+    x, w, b = r(M, K), r(K, N), torch.randn(N, device="cuda", generator=g)
+    y = F.affine(x, w, b)
+    F.check_device_status()
+    want = x.double() @ w.double() + b.double()
+    # 2.0e-6 at every one of these sizes, three times that
+    assert (y.double() - want).norm() <= 6e-6 * want.norm()
+    if offset == 0:
+        taken = kernels(lambda: F.affine(x, w, b))
+        print(*taken)
+        assert taken == route
 
 
 def test_shape_errors(F):

@@ -3,6 +3,8 @@ edges of its 128 x 64 tiles, with rows that 128-bit accesses do not fit, alpha m
 import pytest
 import torch
 
+from launches import kernels
+
 pytestmark = pytest.mark.gpu
 
 # (rows, inmaps, outmaps): past the sizes of the one-launch products
@@ -40,11 +42,14 @@ def test_forward_and_input_gradient(M, K, N):
 
 # Around the line to the two-SM kernel, which makes no alpha: 148 SMs take 74 of its 256 x 256 tiles, while 147 of 128 x 128
 # leave one of them idle. On either side of it in outputs, in rows and in the length of K; bias and no bias.
-@pytest.mark.parametrize("M,K,N", [(64, 1024, 18704), (128, 512, 18816), (128, 512, 18688), (128, 512, 18820),
-                                   (64, 2048, 18692), (64, 2052, 18692), (64, 1024, 18702), (64, 1022, 18704),
-                                   (18816, 256, 100), (18688, 256, 100), (18689, 512, 128)])
+@pytest.mark.parametrize("M,K,N,last", [
+    (64, 1024, 18704, "gemm_pair_tcgen05"), (128, 512, 18816, "gemm_pair_tcgen05"), (128, 512, 18820, "gemm_pair_tcgen05"),
+    (64, 2048, 18692, "gemm_pair_tcgen05"), (64, 1022, 18704, "gemm_pair_tcgen05"), (18816, 256, 100, "gemm_pair_tcgen05"),
+    (18689, 512, 128, "gemm_pair_tcgen05"), (64, 2052, 18692, "gemm_tcgen05_transposed"),
+    (128, 512, 18688, "gemm_tcgen05_transposed"), (64, 1024, 18702, "gemm_tcgen05_transposed"),
+    (18688, 256, 100, "gemm_tcgen05_transposed")])
 @pytest.mark.parametrize("bias", [True, False])
-def test_alpha_at_the_line_to_the_two_sm_kernel(M, K, N, bias):
+def test_alpha_at_the_line_to_the_two_sm_kernel(M, K, N, last, bias):
     from nnabla_b200 import functions as F
     g = torch.Generator(device="cuda").manual_seed(M + K + N)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)
@@ -58,3 +63,6 @@ def test_alpha_at_the_line_to_the_two_sm_kernel(M, K, N, bias):
     # a whole tile's sums in tensor memory: 2.6e-6 of the root mean square at K = 1024, growing with K up to 2048
     rms = lambda t: t.square().mean().sqrt()
     assert rms(y.double() - want) <= 1e-5 * rms(want)
+    taken = kernels(lambda: F.binary_weight_affine(x, w, wb, alpha, b))
+    print(*taken)
+    assert taken[-1] == last
