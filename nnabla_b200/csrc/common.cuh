@@ -52,9 +52,14 @@ __device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p);
 // 31.0, 205 MB 57 against 62). The direction is each kernel's own, chosen so that the functions of a layer alternate:
 // convolutions and their operand passes go up, batch normalization (inference) down, ReLU and Add2 up, the quantizers
 // down; backward, ReLU's gradient down, batch normalization's sums up, its dx down, the quantizers' gradients up.
-// Results of up to kKeepBytes are stored with the ordinary policy (51 MB, 13.5 us a pass with streaming stores, 12.3
-// without; ResNet-18 on 256 images, results of up to 205 MB: 3989 us where only those up to 128 MB are kept, 3951 with all),
-// larger ones streaming, since little of them would be left (a quantizer of 268 MB and its gradient 192 us; kept 200).
+// Results of up to kKeepBytes are stored with the ordinary policy, larger ones streaming. Kept results are faster where the
+// next call reads them, streamed ones where it reads something else that lay in L2, at every size: time of all kept by time of
+// all streamed, for results of 48 / 96 / 144 / 192 / 240 / 288 MB: quantizers and ReLU in turn, each reading the other's result
+// .85 .89 .93 .95 .96 .97; a layer's batch normalization, Add2 and ReLU and the next quantizer .89 .95 .99 .99 1.00 1.00; the
+// gradients of ReLU, batch normalization and a quantizer .98 1.00 1.00 1.01 1.01 1.01; a quantizer and its gradient, whose
+// results nobody reads, 1.13 1.07 1.05 1.04 1.04 1.04 (ResNet-18 on 256 images, results of up to 205 MB: 3951 us, 3989 where
+// only those up to 128 MB are kept). A call does not know who reads its result, and either policy loses 2 to 4 us a call where
+// it is the wrong one; the line lies where the layer no longer gains (288 MB: 390 us both ways).
 constexpr size_t kKeepBytes = (size_t)240 << 20;
 template <typename T> __device__ __forceinline__ void st_result(T *p, T v, bool keep) {
   if (keep)

@@ -228,8 +228,10 @@ static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, int M, int 
 }
 // Whether y = pieces of x (three) . weights (one plane) runs as GemmTransposedProblem: where 128 x 128 tiles would leave
 // SMs idle, and its rounds of 128 x 64 tiles at 40 KB a K block cost less than those of 64 columns by 128 rows of x at 56.
-// Whole layers, alpha made in the product's epilogue instead of a launch of its own: [256, 1024] . [1024, 4096] 19.7 -> 16.0
-// us, [512, 1024] . [1024, 1024] 16.7 -> 13.3, [128, 8000] . [8000, 2000] 101 -> 83.
+// Whole layers, alpha made in the product's epilogue instead of a launch of its own, operands in L2 and, in brackets, read
+// from HBM: [256, 1024] . [1024, 4096] 19.3 -> 16.1 us (23.5 -> 19.3), [512, 1024] . [1024, 1024] 16.3 -> 13.3 (19.0 ->
+// 15.5), [64, 2048] . [2048, 8192] 53.6 -> 48.7 (55.7 -> 50.5), [128, 8000] . [8000, 2000], in parts, 63.8 -> 59.5 (65.4 ->
+// 61.5).
 static bool gemm_transposes(int64_t M, int64_t N) {
   const int64_t sms = sm_count();
   auto rounds = [&](int64_t rows, int64_t cols) {
