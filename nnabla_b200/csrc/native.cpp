@@ -501,9 +501,10 @@ PyObject *folded_convolutions(PyObject *, PyObject *const *a, Py_ssize_t nargs) 
     Py_XDECREF(shape);
     Py_XDECREF(group);
     s.scale = p.f32(item(2)), s.bias = p.f32_or_none(item(3));
-    s.residual = item(6) == Py_None ? -1 : p.integer(item(6));
+    const bool adds = item(6) != Py_None;
+    s.residual = adds ? p.integer(item(6)) : -1;
     s.relu = p.truth(item(7)), s.codes = p.truth(item(8));
-    p.require(s.residual >= -1 && s.residual <= i);
+    p.require(!adds || (s.residual >= 0 && s.residual <= i));
     if (!p.ok)
       return not_plain();
     if (s.source == 0) {

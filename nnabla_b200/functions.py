@@ -1265,6 +1265,9 @@ def folded_convolutions(x_codes, x_shape, steps, delta=2 ** -4, n=8):
         return fast
     results = [(x_codes, tuple(int(v) for v in x_shape), True)]
     for source, prepared, scale, bias, pad, stride, residual, relu, codes in steps:
+        for i in (source,) if residual is None else (source, residual):
+            if not 0 <= i < len(results):
+                raise IndexError("step %d reads result %d, which no step before it has" % (len(results), i))
         added = None if residual is None else results[residual]
         is_codes = added is not None and added[2]
         y, shape = convolution_codes_folded(

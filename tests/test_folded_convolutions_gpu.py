@@ -62,6 +62,12 @@ def test_wrong_steps_raise(F):
                 (4,) + good[1:], (0,) + layer(F, 64, 32, 3, 1) + good[4:]):
         with pytest.raises(Exception):
             F.folded_convolutions(codes, (1, 64, 8, 8), (good, bad), 2.0 ** -4)
+    # results that no step before has, counted from the end too: on the fast path and in the mirror's own loop
+    for odd in (good, good[:2] + (torch.stack([scale, scale], 1)[:, 0],) + good[3:]):
+        for source, residual in ((-1, None), (2, None), (0, -1), (0, 2), (-1, -1)):
+            bad = (source,) + good[1:6] + (residual, True, True)
+            with pytest.raises(IndexError):
+                F.folded_convolutions(codes, (1, 64, 8, 8), (odd, bad), 2.0 ** -4)
 
 
 def test_network(F):

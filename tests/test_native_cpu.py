@@ -4,6 +4,7 @@ import re
 import subprocess
 
 import pytest
+import torch
 
 from nnabla_b200 import functions as F
 
@@ -60,3 +61,13 @@ int main() {
 """ % guard)
     subprocess.check_call([os.environ.get("CXX", "g++"), "-std=c++17", "-o", str(program), str(source)])
     assert subprocess.run([str(program)]).returncode == 0
+
+
+@pytest.mark.parametrize("source,residual", [(-1, None), (1, None), (0, -1), (0, 1)])
+def test_folded_convolutions_of_results_that_do_not_exist(source, residual):
+    """No step reads a result that no step before it has: -1 is neither the last result nor no residual."""
+    import types
+    prepared = types.SimpleNamespace(side=torch.zeros(64, 576, dtype=torch.int8), group=1, shape=(64, 64, 3, 3))
+    step = (source, prepared, torch.ones(64), None, (1, 1), (1, 1), residual, True, True)
+    with pytest.raises(IndexError):
+        F.folded_convolutions(torch.zeros(1, 64, 64, dtype=torch.int8), (1, 64, 8, 8), (step,), 2.0 ** -4)
