@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // resident weights (kResidentB): [k block][BN rows] behind the ring
   const uint32_t resident_bytes = kResidentB ? (uint32_t)(prob.taps * prob.cblocks) * kBBytes : 0u;
-  // halo form: the ring's place is taken by two buffers (one) of cblocks pixel tiles each
+  // halo form: the ring's place is taken by prob.a_bufs buffers (1, or 2 to kTileBufs) of cblocks pixel tiles each
   const uint32_t ring_bytes =
       kHalo ? (uint32_t)(prob.a_bufs * prob.cblocks * prob.a_tile_bytes) : (uint32_t)STAGES * kStageBytes;
   uint8_t *b_resident = smem + ring_bytes;
