@@ -833,9 +833,12 @@ int nb200_global_average_pooling_f32(const float *x, float *y, int64_t maps, int
   if (maps == 0)
     return NB200_OK;
   NB_CHECK(x && y, NB200_EVALUE, "null data pointer");
-  // 131072 maps of 1, 9, 12, 16 and 20 values: 1.6, 2.4, 3.3, 5.9 (64 bytes apart) and 4.2 us by a thread per map, 5.0 to 5.7
-  // through shared memory
-  if (spatial < 24 && spatial != 16)
+  // A thread per map loads S times, its warp's 32 values S apart, and is paid for by the lines that a load touches and by the
+  // banks that it meets: values 16 apart lie in two of the 32 banks, values 8 apart in four. 131072 maps of 1, 9, 15, 16, 17, 20,
+  // 23, 24, 25, 32 values by a thread per map 1.4, 2.2, 2.9, 5.5, 3.1, 3.9, 4.1, 5.7, 4.8, 18.1 us, through shared memory 4.7 to
+  // 5.4; 524288 maps of 15, 16, 17, 23, 24, 28 values 6.1, 16.5, 7.2, 10.8, 16.2, 16.0 and 15.7 to 16.7. Of 8192 maps and fewer
+  // either way takes 1.2 to 2.5 us.
+  if (spatial < 24 && spatial % 16 != 0)
     NB_CUDA(launch_dependent(global_average_pooling_short_kernel, dim3((unsigned)((maps + kThreads - 1) / kThreads)),
                              dim3(kThreads), 0, as_stream(stream), x, (size_t)maps, (int)spatial, y));
   else
